@@ -163,6 +163,7 @@ class BatchExecutor {
     }
     uint32_t num_checks = 0; /* checks captured so far (levels, then VARCHAR totals) */
     std::vector<DevPtr> keep_checks;
+    DevPtr col_states; /* ColumnState of every decoded column */
     int levels(PlanState &p, uint64_t node, int depth);
     void decode_all();
     Decoded &dec(size_t plan, uint64_t t, uint64_t c) { return decoded.at({plan, t, c}); }
@@ -189,9 +190,7 @@ int BatchExecutor::levels(PlanState &p, uint64_t node, int depth) {
 }
 
 void BatchExecutor::decode_all() {
-    std::vector<DecodeTask> tasks;
     std::vector<std::tuple<size_t, uint64_t, uint64_t>> keys;
-    uint64_t total_pages = 0;
     for (size_t i = 0; i < ps.size(); ++i) {
         PlanState &p = ps[i];
         if (p.status) continue;
@@ -213,35 +212,22 @@ void BatchExecutor::decode_all() {
                 else
                     upload_pages(ctx, plan.inputs[sn.base_table_id].columns[sn.output_attrs[a].index], d.src,
                                  &stats.h2d_bytes);
-                const uint64_t words = std::max<uint64_t>((d.rows + 31) / 32, 1);
-                d.valid = ctx.alloc(words * 4);
-                ck(cudaMemsetAsync(d.valid->ptr, 0, words * 4, ctx.stream), "memset");
-                if (d.type == CJ_VARCHAR) d.desc = ctx.alloc(d.rows * 8);
-                else d.values = ctx.alloc(d.rows * (d.type == CJ_INT32 ? 4 : 8));
-                DecodeTask t{};
-                t.pages = d.src.dev;
-                t.num_pages = d.src.num_pages;
-                t.page_base = total_pages;
-                t.rows = d.rows;
-                t.type = d.type;
-                t.values = d.values ? d.values->ptr : nullptr;
-                t.desc = d.desc ? d.desc->as<uint64_t>() : nullptr;
-                t.valid = d.valid->as<uint32_t>();
-                total_pages += t.num_pages;
-                tasks.push_back(t);
                 keys.push_back(key);
                 decoded.emplace(key, std::move(d));
             }
         }
     }
-    if (tasks.empty()) return;
+    if (keys.empty()) return;
+    col_states = ctx.alloc(keys.size() * sizeof(ColumnState));
+    ck(cudaMemsetAsync(col_states->ptr, 0, keys.size() * sizeof(ColumnState), ctx.stream), "memset");
+    std::vector<ColumnTask> tasks;
+    for (size_t k = 0; k < keys.size(); ++k) {
+        tasks.push_back(column_task(ctx, decoded.at(keys[k]), col_states->as<ColumnState>() + k));
+        tasks.back().err = &ctx.d_status->errors;
+    }
+    const ColumnGrid grid = place_columns(L, tasks.data(), tasks.size());
     DevPtr td = upload_tasks(tasks);
-    DevPtr rows_pp = ctx.alloc(std::max<uint64_t>(total_pages, 1) * 4);
-    DevPtr row_start = ctx.alloc((total_pages + 1) * 8);
-    DevPtr tmp = ctx.alloc(scan_temp_bytes(total_pages));
-    ck(launch_decode_grouped(L, td->as<DecodeTask>(), (uint32_t)tasks.size(), total_pages, rows_pp->as<uint32_t>(),
-                             row_start->as<uint64_t>(), tmp->ptr),
-       "decode_grouped");
+    ck(launch_columns_grouped(L, td->as<ColumnTask>(), (uint32_t)tasks.size(), grid), "decode_grouped");
 }
 
 void BatchExecutor::run_level(int lvl) {
@@ -548,7 +534,6 @@ void BatchExecutor::run_level(int lvl) {
 void BatchExecutor::materialize_roots() {
     const uint32_t TR = (uint32_t)std::max<int64_t>(64, std::min<int64_t>(ctx.opt.varchar_tile_rows, 8192));
     std::vector<PageTask> ptasks;
-    uint64_t pages = 0;
     struct VarJob {
         size_t plan, col;
         DevPtr temp;
@@ -575,12 +560,16 @@ void BatchExecutor::materialize_roots() {
             const uint32_t R = rows_per_page_fixed(p.root_types[c]);
             res->num_pages[c] = (p.root_rows + R - 1) / R;
             res->dev_pages[c] = ctx.alloc(res->num_pages[c] * kPageSize);
-            ptasks.push_back({p.root_cols[c], p.root_rows, res->dev_pages[c]->as<uint8_t>(), pages});
-            pages += res->num_pages[c];
+            PageTask t{};
+            t.col = p.root_cols[c];
+            t.rows = p.root_rows;
+            t.out = res->dev_pages[c]->as<uint8_t>();
+            ptasks.push_back(t);
         }
     }
+    const uint32_t page_grid = place_pages(L, ptasks.data(), ptasks.size());
     DevPtr pt = upload_tasks(ptasks);
-    ck(launch_write_fixed_grouped(L, pt->as<PageTask>(), (uint32_t)ptasks.size(), pages), "write_fixed_grouped");
+    ck(launch_write_pages_grouped(L, pt->as<PageTask>(), (uint32_t)ptasks.size(), page_grid), "write_pages_grouped");
     if (!var.empty()) {
         DevPtr totals = ctx.alloc(var.size() * 8);
         for (size_t k = 0; k < var.size(); ++k) {

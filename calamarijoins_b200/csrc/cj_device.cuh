@@ -93,6 +93,11 @@ template <typename T> CJ_DEV T block_exclusive_scan(T v, T *warp_buf, T *total) 
     return res;
 }
 
+/* First row of page p by its column's page index (k_page_index). */
+CJ_DEV uint64_t page_first_row(const uint64_t *base, const uint32_t *loc, uint64_t p) {
+    return __ldg(base + p / kIndexChunk) + __ldg(loc + p);
+}
+
 /* Relation row -> base row through the view's indirections. */
 CJ_DEV uint32_t base_row(const ColView &c, uint32_t i) {
     if (c.rid_a) i = __ldg(c.rid_a + i);

@@ -3,9 +3,10 @@
  *
  * Device data layout (all in HBM, one allocation per array):
  *   pages        a column's 8 KiB pages, consecutive, exactly as on the host
- *   row_start    u64[num_pages + 1], first row of each page (prefix sum of
- *                the rows each page holds: n_rows, 1 for a long-string start
- *                page 0xffff, 0 for a continuation page 0xfffe)
+ *   page index   u64 base per 256 pages and u32 loc per page, whose sum is
+ *                the page's first row (a page holds n_rows rows, a
+ *                long-string start page 0xffff one, a continuation page
+ *                0xfffe none)
  *   values       dense fixed-width values, one per row (0 where NULL)
  *   valid        validity bitmap, u32 words, bit r = row r present
  *   str_desc     VARCHAR: one u64 per row, see CJ_DESC_* below
@@ -62,6 +63,17 @@ enum DevError : uint32_t {
     DEV_ERR_INTERNAL = 1u << 31
 };
 
+/* What a column's page index leaves on the device. Zero before the launch. */
+struct ColumnState {
+    unsigned int flags; /* COL_* flags, from the page headers      */
+    unsigned int done;  /* blocks of the index that have finished  */
+    unsigned int err;   /* DevError bits of this column            */
+    unsigned int pad;
+};
+/* Columns whose state lives in the status block: their errors count only
+ * once the plan reads them (Context::sync_status). */
+constexpr uint32_t kStatusColumns = 64;
+
 /* Small pinned block the host reads at each synchronisation point. */
 struct StatusBlock {
     unsigned int errors;          /* DevError bits                          */
@@ -72,6 +84,7 @@ struct StatusBlock {
                                      in the open-addressing table          */
     unsigned long long stale[3];  /* DEV_ERR_STALE: check index, count found,
                                      count recorded (one of the mismatches) */
+    ColumnState cols[kStatusColumns];
 };
 
 /* How a kernel reads one column of a relation: row i of the relation is
@@ -136,7 +149,7 @@ struct MatchOut {
     uint8_t *key_pages = nullptr;   /* null, or the join key written straight
                                        into 8 KiB result pages: value pos % R
                                        of page pos / R (R = 1984 or 1007 by
-                                       key_bytes); launch_finish_dense_pages
+                                       key_bytes); a PageTask with `finish`
                                        adds headers and bitmaps */
     int32_t key_bytes = 4;
     unsigned long long capacity = 0;
@@ -187,45 +200,36 @@ cudaError_t scan_u32_to_u64(const Launch &L, const uint32_t *in, uint64_t *out,
                             size_t n, void *temp);
 
 /* Decode */
-/* Page index of one column: rows_pp[p] = rows of page p, row_start[p] =
- * rows before page p (row_start[num_pages] = total; only the total when
- * the column is read in place), state[0] |= the column's COL_* flags;
- * a total other than `rows` raises DEV_ERR_ROW_COUNT and sets
- * COL_NOT_DIRECT. state (2 words) must be zero; partials holds
- * page_index_blocks(num_pages) entries. Two launches. */
-uint64_t page_index_blocks(const Launch &L, uint64_t num_pages);
-cudaError_t launch_page_index(const Launch &L, const uint8_t *pages, uint64_t num_pages, int32_t type,
-                              uint64_t rows, uint32_t *rows_pp, uint64_t *partials, uint64_t *row_start,
-                              uint32_t *state);
-/* Rows past max_rows are never written; a page that would write them
- * raises DEV_ERR_ROW_COUNT instead. Does nothing when *col_flags is 0
- * (readers then take the values from the pages). */
-cudaError_t launch_decode_fixed(const Launch &L, const uint8_t *pages,
-                                uint64_t num_pages, int32_t type,
-                                const uint64_t *row_start, uint64_t max_rows,
-                                void *values, uint32_t *valid, const uint32_t *col_flags);
-cudaError_t launch_decode_varchar(const Launch &L, const uint8_t *pages,
-                                  uint64_t num_pages,
-                                  const uint64_t *row_start, uint64_t max_rows,
-                                  uint64_t *desc, uint32_t *valid);
-/* Grouped decode of many columns: task k's pages are global pages
- * [page_base, page_base + num_pages). rows_pp / row_start are scratch of
- * total_pages / total_pages + 1 entries; scan_temp of
- * scan_temp_bytes(total_pages). */
-struct DecodeTask {
+/* One column to index and decode. The index gives row base[p >> 8] + loc[p]
+ * as page p's first (page_first_row), the column's COL_* flags, its errors,
+ * and a cleared validity bitmap; the decode writes the dense arrays of a
+ * column that is not read in place. Rows past `rows` are never written; a
+ * page that would write them raises DEV_ERR_ROW_COUNT instead. */
+constexpr int kIndexChunk = 256; /* pages per block of the index */
+struct ColumnTask {
     const uint8_t *pages;
     uint64_t num_pages;
-    uint64_t page_base;
     uint64_t rows;
+    uint32_t *loc;       /* num_pages entries               */
+    uint64_t *base;      /* index_blocks(num_pages) entries */
+    ColumnState *state;
+    unsigned int *err;
+    void *values;        /* fixed width                     */
+    uint64_t *desc;      /* VARCHAR                         */
+    uint32_t *valid;     /* max(1, ceil(rows / 32)) words   */
     int32_t type;
-    int32_t pad;
-    void *values;
-    uint64_t *desc;
-    uint32_t *valid; /* zeroed */
+    uint32_t index_base, index_blocks, decode_base, decode_blocks; /* place_columns */
 };
-cudaError_t launch_decode_grouped(const Launch &L, const DecodeTask *tasks_dev, uint32_t ntasks,
-                                  uint64_t total_pages, uint32_t *rows_pp, uint64_t *row_start,
-                                  void *scan_temp);
+constexpr int kColumnArgs = 32; /* tasks passed by value */
+struct ColumnGrid {
+    uint32_t index = 0, decode = 0; /* blocks of the two launches */
+};
+uint32_t index_blocks(uint64_t num_pages);
+ColumnGrid place_columns(const Launch &L, ColumnTask *tasks, size_t n);
+/* Index (or decode) of n columns, a launch per kColumnArgs of them. */
+cudaError_t launch_columns(const Launch &L, ColumnTask *tasks, size_t n, bool index);
+/* Index and decode of the columns of a batch, placed by place_columns. */
+cudaError_t launch_columns_grouped(const Launch &L, const ColumnTask *tasks_dev, uint32_t n, const ColumnGrid &g);
 
 /* Build */
 struct BuildPlan {
@@ -379,16 +383,6 @@ cudaError_t launch_check_counts(const Launch &L, const unsigned long long *count
                                 const unsigned long long *expected, uint32_t n,
                                 unsigned long long *detail, uint32_t check_id);
 
-/* Headers (n_rows = n_values), zero gaps and all-ones bitmaps of the
- * ceil(rows / R) pages of a NULL-free fixed-width column whose values are
- * already in place (R by type, as rows_per_page_fixed). */
-/* The page writers below take `rows` as the rows to write, or, with
- * `rows_dev` set, as the capacity the pages were sized for while the count
- * itself is read on the device from *rows_dev (a match counter the host has
- * not read yet). */
-cudaError_t launch_finish_dense_pages(const Launch &L, uint8_t *pages, uint64_t rows, int32_t type,
-                                      const unsigned long long *rows_dev = nullptr);
-
 /* Intermediates: out[i] = src[idx[i]] */
 cudaError_t launch_gather_u32(const Launch &L, const uint32_t *src,
                               const uint32_t *idx, uint64_t n, uint32_t *out);
@@ -405,20 +399,26 @@ struct GatherTask {
 };
 cudaError_t launch_gather_grouped(const Launch &L, const GatherTask *tasks_dev, uint32_t ntasks,
                                   uint64_t total_chunks);
+/* One fixed-width result column. `rows` are the rows to write or, with
+ * `rows_dev` set, the capacity the pages were sized for while the count
+ * itself is read on the device (a match counter the host has not read yet).
+ * finish: the values are in place already (a NULL-free column written by the
+ * probe); headers (n_rows = n_values), zero gaps and all-ones bitmaps only. */
 struct PageTask {
     ColView col;
     uint64_t rows;
+    const unsigned long long *rows_dev;
     uint8_t *out;
-    uint64_t page_base;
+    int32_t finish;
+    uint32_t block_base, blocks; /* place_pages */
 };
-cudaError_t launch_write_fixed_grouped(const Launch &L, const PageTask *tasks_dev, uint32_t ntasks,
-                                      uint64_t total_pages);
+constexpr int kPageArgs = 24; /* tasks passed by value */
+uint32_t place_pages(const Launch &L, PageTask *tasks, size_t n); /* returns the grid */
+cudaError_t launch_write_pages(const Launch &L, PageTask *tasks, size_t n);
+cudaError_t launch_write_pages_grouped(const Launch &L, const PageTask *tasks_dev, uint32_t n, uint32_t grid);
 
 /* Output pages */
 uint32_t rows_per_page_fixed(int32_t type);
-cudaError_t launch_write_fixed_pages(const Launch &L, const ColView &col,
-                                     uint64_t rows, uint8_t *out_pages,
-                                     const unsigned long long *rows_dev = nullptr);
 size_t varchar_temp_bytes(uint64_t rows, uint32_t tile_rows);
 /* Pass 1: page count per tile; total pages into *total_pages_dev. */
 cudaError_t launch_varchar_plan(const Launch &L, const ColView &col, uint64_t rows,

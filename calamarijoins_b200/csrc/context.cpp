@@ -226,11 +226,13 @@ cudaEvent_t Context::get_event() {
 
 void Context::put_event(cudaEvent_t e) { event_pool.push_back(e); }
 
-void Context::sync_status() {
+void Context::sync_status(uint64_t used_cols) {
     check_cuda(cudaMemcpyAsync(h_status, d_status, sizeof(StatusBlock), cudaMemcpyDeviceToHost, stream),
                "status copy");
     check_cuda(cudaStreamSynchronize(stream), "stream synchronize");
     unsigned int err = h_status->errors;
+    for (uint32_t c = 0; c < kStatusColumns; ++c)
+        if ((used_cols >> c) & 1u) err |= h_status->cols[c].err;
     if (err) {
         /* clear for the next call */
         cudaMemsetAsync(&d_status->errors, 0, sizeof(unsigned int), stream);

@@ -120,10 +120,11 @@ class Executor {
     std::map<std::pair<uint64_t, uint64_t>, Prefetched> prefetched;
     std::vector<PhaseEv> phase_events;
     cj_exec_stats stats{};
+    uint64_t used_cols = 0;   /* columns of the status block the plan has read */
     bool synced_last = false; /* the last thing enqueued was a synchronisation */
     /* Brings the status block to the host, counting the synchronisation. */
     void sync() {
-        ctx.sync_status();
+        ctx.sync_status(used_cols);
         stats.host_syncs++;
     }
     /* A result written with a device-side row count (materialize with
@@ -147,6 +148,7 @@ class Executor {
 
     void validate();
     void prefetch();
+    void decode_columns(std::vector<ColumnTask> &tasks);
     Decoded &decode(uint64_t t, uint64_t c);
     Relation resolve(uint64_t node, int depth);
     Relation exec_join(uint64_t node, int depth, bool is_root, cj_result **out);
@@ -171,7 +173,13 @@ void Executor::validate() { validate_plan(ctx, plan); }
  * context's upload stream, in the order the kernels need them: join keys
  * bottom-up, then the root's outputs. The kernel stream waits for a
  * column's copy only when it decodes that column, so later columns (the
- * payloads) cross PCIe while the joins below the root run. */
+ * payloads) cross PCIe while the joins below the root run.
+ *
+ * The resident columns among them are indexed and decoded here, all in one
+ * launch each (per column those were two to three launches and two memsets:
+ * 212 us of a six-table plan's 1.9 ms). Each keeps its errors to itself
+ * until the plan reads it: a plan that never gets to a malformed column
+ * (an empty join below) still runs. */
 void Executor::prefetch() {
     using TC = std::pair<uint64_t, uint64_t>;
     std::vector<TC> order;
@@ -197,6 +205,20 @@ void Executor::prefetch() {
         return out;
     };
     for (const TC &tc : cols(plan.root, 0)) add(tc);
+    std::vector<ColumnTask> tasks;
+    for (const TC &tc : order) {
+        const cj_table *r = resident(tc.first);
+        if (!r || r->num_rows > 0xFFFFFFFFull || tasks.size() == kStatusColumns) continue;
+        Decoded d;
+        d.type = column_type(tc.first, tc.second);
+        d.rows = r->num_rows;
+        d.src = r->cols[tc.second];
+        d.status_col = (int)tasks.size();
+        tasks.push_back(column_task(ctx, d, &ctx.d_status->cols[tasks.size()]));
+        decoded.emplace(tc, std::move(d));
+    }
+    ck(cudaMemsetAsync(ctx.d_status, 0, sizeof(StatusBlock), ctx.stream), "memset");
+    if (!tasks.empty()) decode_columns(tasks);
     cudaEvent_t first = nullptr;
     for (const TC &tc : order) {
         if (resident(tc.first)) continue;
@@ -217,10 +239,23 @@ void Executor::prefetch() {
     }
 }
 
+void Executor::decode_columns(std::vector<ColumnTask> &tasks) {
+    PhaseScope ph(*this, PH_DECODE);
+    {
+        KScope k(*this, "page_index");
+        ck(launch_columns(L, tasks.data(), tasks.size(), true), "page_index");
+    }
+    KScope k(*this, "decode");
+    ck(launch_columns(L, tasks.data(), tasks.size(), false), "decode");
+}
+
 Decoded &Executor::decode(uint64_t t, uint64_t c) {
     auto key = std::make_pair(t, c);
     auto it = decoded.find(key);
-    if (it != decoded.end()) return it->second;
+    if (it != decoded.end()) {
+        if (it->second.status_col >= 0) used_cols |= 1ull << it->second.status_col;
+        return it->second;
+    }
     Decoded d;
     d.type = column_type(t, c);
     d.rows = table_rows(t);
@@ -237,36 +272,8 @@ Decoded &Executor::decode(uint64_t t, uint64_t c) {
         PhaseScope ph(*this, PH_UPLOAD);
         upload_pages(ctx, plan.inputs[t].columns[c], d.src, &stats.h2d_bytes);
     }
-    PhaseScope ph(*this, PH_DECODE);
-    const uint64_t np = d.src.num_pages;
-    DevPtr rows_pp = ctx.alloc(std::max<uint64_t>(np, 1) * 4);
-    DevPtr row_start = ctx.alloc((np + 1) * 8);
-    DevPtr partials = ctx.alloc(page_index_blocks(L, np) * 8);
-    d.col_flags = ctx.alloc(8); /* COL_* flags, then the index's finished-block count */
-    ck(cudaMemsetAsync(d.col_flags->ptr, 0, 8, ctx.stream), "memset");
-    {
-        KScope k(*this, "page_index");
-        ck(launch_page_index(L, d.src.dev, np, d.type, d.rows, rows_pp->as<uint32_t>(), partials->as<uint64_t>(),
-                             row_start->as<uint64_t>(), d.col_flags->as<uint32_t>()),
-           "page_index");
-    }
-    const uint64_t words = (d.rows + 31) / 32;
-    d.valid = ctx.alloc(std::max<uint64_t>(words, 1) * 4);
-    ck(cudaMemsetAsync(d.valid->ptr, 0, std::max<uint64_t>(words, 1) * 4, ctx.stream), "memset");
-    if (d.type == CJ_VARCHAR) {
-        d.desc = ctx.alloc(d.rows * 8);
-        KScope k(*this, "decode_varchar");
-        ck(launch_decode_varchar(L, d.src.dev, np, row_start->as<uint64_t>(), d.rows, d.desc->as<uint64_t>(),
-                                 d.valid->as<uint32_t>()),
-           "decode_varchar");
-    } else {
-        const uint64_t w = d.type == CJ_INT32 ? 4 : 8;
-        d.values = ctx.alloc(d.rows * w);
-        KScope k(*this, d.type == CJ_INT32 ? "decode_int32" : "decode_8byte");
-        ck(launch_decode_fixed(L, d.src.dev, np, d.type, row_start->as<uint64_t>(), d.rows, d.values->ptr,
-                               d.valid->as<uint32_t>(), d.col_flags->as<uint32_t>()),
-           "decode_fixed");
-    }
+    std::vector<ColumnTask> tasks{column_task(ctx, d, nullptr)};
+    decode_columns(tasks);
     return decoded.emplace(key, std::move(d)).first->second;
 }
 
@@ -710,31 +717,39 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
                 h += res->num_pages[c] * kPageSize;
             }
         }
+        /* A host result's columns are written one by one, each downloaded
+         * while the next is written (and still uploaded); a result left in
+         * HBM has its fixed-width columns written by one launch. */
+        std::vector<PageTask> ptasks;
+        auto write_pages = [&]() {
+            KScope ks(*this, "write_pages");
+            ck(launch_write_pages(L, ptasks.data(), ptasks.size()), "write_pages");
+            ptasks.clear();
+        };
         for (size_t c = 0; c < nc; ++c) {
             if (!rows) continue;
+            PageTask t{};
+            t.rows = rows;
+            t.rows_dev = rows_dev;
             if (cols[c].pages) {
                 /* values already in place: headers and bitmaps, once per
                  * shared page array */
                 res->dev_pages[c] = cols[c].pages;
-                if (alias[c] < 0) {
-                    KScope ks(*this, "finish_pages");
-                    ck(launch_finish_dense_pages(L, cols[c].pages->as<uint8_t>(), rows, types[c], rows_dev),
-                       "finish_pages");
-                }
+                t.col.type = types[c];
+                t.finish = 1;
             } else {
                 /* decoded here, not before the loop: the kernel stream waits
                  * for a column's upload only when its pages are written */
-                const ColView cv = out_view(cols[c]);
+                t.col = out_view(cols[c]);
                 res->dev_pages[c] = ctx.alloc(res->num_pages[c] * kPageSize);
-                if (types[c] != CJ_VARCHAR) {
-                    KScope ks(*this, types[c] == CJ_INT32 ? "write_pages_int32" : "write_pages_8byte");
-                    ck(launch_write_fixed_pages(L, cv, rows, res->dev_pages[c]->as<uint8_t>(), rows_dev),
-                       "write_fixed");
-                } else {
-                    KScope ks(*this, "varchar_write");
-                    ck(launch_varchar_write(L, cv, rows, TR, vtemp[c]->ptr, res->dev_pages[c]->as<uint8_t>()),
-                       "varchar_write");
-                }
+            }
+            t.out = res->dev_pages[c]->as<uint8_t>();
+            if (types[c] == CJ_VARCHAR) {
+                KScope ks(*this, "varchar_write");
+                ck(launch_varchar_write(L, t.col, rows, TR, vtemp[c]->ptr, t.out), "varchar_write");
+            } else if (alias[c] < 0) {
+                ptasks.push_back(t);
+                if (to_host) write_pages();
             }
             const size_t bytes = res->num_pages[c] * kPageSize;
             if (to_host && bytes && alias[c] < 0) {
@@ -752,6 +767,7 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
                 stats.d2h_bytes += bytes;
             }
         }
+        if (!ptasks.empty()) write_pages();
     }
     if (dl.first) {
         dl.last = ctx.get_event();

@@ -172,8 +172,9 @@ struct Context {
     cudaEvent_t get_event();
     void put_event(cudaEvent_t e);
     /* Copies the status block to the host, waits for the stream and throws
-     * on any device-side error bit. */
-    void sync_status();
+     * on any device-side error bit, those of the status block's columns in
+     * `used_cols` among them. */
+    void sync_status(uint64_t used_cols = 0);
     void resolve_profile();
 };
 

@@ -4,6 +4,7 @@
  */
 #pragma once
 
+#include <algorithm>
 #include <map>
 #include <string>
 #include <vector>
@@ -45,8 +46,42 @@ struct Decoded {
     uint64_t rows = 0;
     ColumnPages src;
     DevPtr values, valid, desc;
-    DevPtr col_flags; /* u32 COL_* flags from the page headers; null: not computed */
+    DevPtr loc, base;                   /* page index (page_first_row)        */
+    DevPtr own_state;                   /* the state, unless the status block's */
+    ColumnState *state = nullptr;       /* COL_* flags and errors (device)    */
+    int status_col = -1;                /* its place in the status block      */
 };
+
+/* Allocates a column's arrays and describes its index and decode. `state`
+ * (device, zero before the launches) null: one of its own, errors then go
+ * straight to the status word. */
+inline ColumnTask column_task(Context &ctx, Decoded &d, ColumnState *state) {
+    const uint64_t np = d.src.num_pages;
+    d.loc = ctx.alloc(std::max<uint64_t>(np, 1) * 4);
+    d.base = ctx.alloc(index_blocks(np) * 8);
+    d.valid = ctx.alloc(std::max<uint64_t>((d.rows + 31) / 32, 1) * 4);
+    if (d.type == CJ_VARCHAR) d.desc = ctx.alloc(std::max<uint64_t>(d.rows, 1) * 8);
+    else d.values = ctx.alloc(std::max<uint64_t>(d.rows, 1) * (d.type == CJ_INT32 ? 4 : 8));
+    ColumnTask t{};
+    t.err = state ? &state->err : &ctx.d_status->errors;
+    if (!state) {
+        d.own_state = ctx.alloc(sizeof(ColumnState));
+        check_cuda(cudaMemsetAsync(d.own_state->ptr, 0, sizeof(ColumnState), ctx.stream), "memset");
+        state = d.own_state->as<ColumnState>();
+    }
+    d.state = state;
+    t.pages = d.src.dev;
+    t.num_pages = np;
+    t.rows = d.rows;
+    t.loc = d.loc->as<uint32_t>();
+    t.base = d.base->as<uint64_t>();
+    t.state = state;
+    t.values = d.values ? d.values->ptr : nullptr;
+    t.desc = d.desc ? d.desc->as<uint64_t>() : nullptr;
+    t.valid = d.valid->as<uint32_t>();
+    t.type = d.type;
+    return t;
+}
 
 /* A column of a relation: base column (input, col) reached through row-id
  * vector `vec` of the relation (-1: the relation row is the base row). */
@@ -114,7 +149,7 @@ inline ColView make_view(const Decoded &d, const Relation &R, const RelCol &c, c
     v.rid_a = rid_a;
     v.rid_b = c.vec >= 0 ? R.vecs[c.vec]->as<uint32_t>() : nullptr;
     v.null_sentinel = (c.sentinel && c.type == CJ_INT32) ? 1 : 0;
-    v.col_flags = d.col_flags ? d.col_flags->as<uint32_t>() : nullptr;
+    v.col_flags = &d.state->flags;
     return v;
 }
 

@@ -304,7 +304,11 @@ class Filter {
                     const uint32_t R = rows_per_page_fixed(cp.type);
                     cp.num_pages = (count + R - 1) / R;
                     cp.owner = ctx.alloc(cp.num_pages * kPageSize);
-                    check_cuda(launch_write_fixed_pages(L, v, count, cp.owner->as<uint8_t>()), "write_fixed");
+                    PageTask pt{};
+                    pt.col = v;
+                    pt.rows = count;
+                    pt.out = cp.owner->as<uint8_t>();
+                    check_cuda(launch_write_pages(L, &pt, 1), "write_pages");
                 } else {
                     DevPtr temp = ctx.alloc(varchar_temp_bytes(count, TR));
                     check_cuda(launch_varchar_plan(L, v, count, TR, temp->ptr,
@@ -372,32 +376,9 @@ class Filter {
         d.type = in.cols[c].type;
         d.rows = in.num_rows;
         d.src = in.cols[c];
-        const uint64_t np = d.src.num_pages;
-        DevPtr rows_pp = ctx.alloc(std::max<uint64_t>(np, 1) * 4);
-        DevPtr row_start = ctx.alloc((np + 1) * 8);
-        DevPtr partials = ctx.alloc(page_index_blocks(L, np) * 8);
-        keep.push_back(rows_pp);
-        keep.push_back(row_start);
-        keep.push_back(partials);
-        d.col_flags = ctx.alloc(8);
-        check_cuda(cudaMemsetAsync(d.col_flags->ptr, 0, 8, ctx.stream), "memset");
-        check_cuda(launch_page_index(L, d.src.dev, np, d.type, d.rows, rows_pp->as<uint32_t>(),
-                                     partials->as<uint64_t>(), row_start->as<uint64_t>(), d.col_flags->as<uint32_t>()),
-                   "page_index");
-        const uint64_t words = std::max<uint64_t>((d.rows + 31) / 32, 1);
-        d.valid = ctx.alloc(words * 4);
-        check_cuda(cudaMemsetAsync(d.valid->ptr, 0, words * 4, ctx.stream), "memset");
-        if (d.type == CJ_VARCHAR) {
-            d.desc = ctx.alloc(std::max<uint64_t>(d.rows, 1) * 8);
-            check_cuda(launch_decode_varchar(L, d.src.dev, np, row_start->as<uint64_t>(), d.rows,
-                                             d.desc->as<uint64_t>(), d.valid->as<uint32_t>()),
-                       "decode_varchar");
-        } else {
-            d.values = ctx.alloc(std::max<uint64_t>(d.rows, 1) * (d.type == CJ_INT32 ? 4 : 8));
-            check_cuda(launch_decode_fixed(L, d.src.dev, np, d.type, row_start->as<uint64_t>(), d.rows,
-                                           d.values->ptr, d.valid->as<uint32_t>(), d.col_flags->as<uint32_t>()),
-                       "decode_fixed");
-        }
+        ColumnTask task = column_task(ctx, d, nullptr);
+        check_cuda(launch_columns(L, &task, 1, true), "page_index");
+        check_cuda(launch_columns(L, &task, 1, false), "decode");
         return decoded.emplace(c, std::move(d)).first->second;
     }
 

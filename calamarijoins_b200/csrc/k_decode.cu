@@ -66,94 +66,89 @@ CJ_DEV uint32_t page_flags(const uint8_t *pg, uint64_t p, uint64_t np, int32_t t
     return f;
 }
 
-/* Page index of one column in two launches. Block b of both kernels owns
- * pages [b * chunk, (b + 1) * chunk).
- * k_page_index: rows per page, the column's COL_* flags (ORed into
- * state[0]) and each block's row total (partials[b]); the last block to
- * finish (state[1] counts finished blocks) adds the totals, stores
- * row_start[np] and checks the row count against the table's (a mismatch
- * raises DEV_ERR_ROW_COUNT and makes the column NOT_DIRECT, so readers stay
- * inside its decoded arrays).
- * k_page_index_scan: row_start[p] = rows before page p; skipped for a
- * column read in place (state[0] == 0), which needs no row offsets. */
-constexpr int kIndexThreads = 256;
+/* ---- page index: every column of a plan (or batch) in one launch ----
+ * A block owns kIndexChunk consecutive pages of one column, one page per
+ * thread: it stores each page's first row relative to the chunk (loc) and
+ * the chunk's rows (base), ORs the column's COL_* flags and clears its share
+ * of the column's validity bitmap. The last block of a column to finish
+ * turns base into the rows before each chunk and checks the column's row
+ * count (a mismatch raises DEV_ERR_ROW_COUNT and makes the column
+ * NOT_DIRECT, so readers stay inside its decoded arrays).
+ *
+ * Bound by launch and header latency, not by bytes (one 32-byte sector per
+ * 8 KB page). Per column it used to take two launches and two memsets
+ * (10-13 us of a plan's time each on the device); now the columns share one
+ * launch, and the second pass is folded into readers, which add the two
+ * numbers (page_first_row). */
+constexpr int kIndexThreads = kIndexChunk;
 
-__global__ void __launch_bounds__(kIndexThreads)
-    k_page_index(const uint8_t *__restrict__ pages, uint64_t np, int32_t type, uint64_t chunk, uint64_t expected,
-                 uint32_t *__restrict__ rows, uint64_t *__restrict__ partials, uint64_t *__restrict__ row_start,
-                 uint32_t *state, unsigned int *err) {
-    __shared__ uint64_t wsum[kIndexThreads / 32];
+CJ_DEV void index_chunk(const ColumnTask &T, uint32_t b) {
+    __shared__ uint64_t wbuf[kIndexThreads / 32 + 1];
     __shared__ bool s_last;
-    const uint64_t p0 = (uint64_t)blockIdx.x * chunk, p1 = min(np, p0 + chunk);
-    uint64_t s = 0;
+    const uint64_t np = T.num_pages, p = (uint64_t)b * kIndexThreads + threadIdx.x;
     uint32_t f = 0;
-    for (uint64_t p = p0 + threadIdx.x; p < p1; p += blockDim.x) {
-        const uint8_t *pg = pages + p * kPageSize;
-        const uint32_t r = page_rows_of(pg, type, err);
-        rows[p] = r;
-        s += r;
-        f |= page_flags(pg, p, np, type);
+    uint64_t r = 0;
+    if (p < np) {
+        const uint8_t *pg = T.pages + p * kPageSize;
+        r = page_rows_of(pg, T.type, T.err);
+        f = page_flags(pg, p, np, T.type);
     }
     f = __reduce_or_sync(0xffffffffu, f);
-    if (f && lane_id() == 0) atomicOr(state, f);
-    s = warp_sum(s);
-    if (lane_id() == 0) wsum[threadIdx.x >> 5] = s;
-    __syncthreads();
+    if (f && lane_id() == 0) atomicOr(&T.state->flags, f);
+    uint64_t tot;
+    const uint64_t pre = block_exclusive_scan<uint64_t>(r, wbuf, &tot);
+    if (p < np) T.loc[p] = (uint32_t)pre; /* at most 256 * 65535 rows */
+    const uint64_t words = T.rows ? (T.rows + 31) / 32 : 1;
+    const uint64_t w0 = words * b / T.index_blocks, w1 = words * (b + 1) / T.index_blocks;
+    for (uint64_t w = w0 + threadIdx.x; w < w1; w += kIndexThreads) T.valid[w] = 0u;
     if (threadIdx.x == 0) {
-        uint64_t t = 0;
-        for (int w = 0; w < kIndexThreads / 32; ++w) t += wsum[w];
-        partials[blockIdx.x] = t;
+        T.base[b] = tot;
         __threadfence();
-        s_last = atomicAdd(state + 1, 1u) == gridDim.x - 1;
+        s_last = atomicAdd(&T.state->done, 1u) == T.index_blocks - 1;
     }
     __syncthreads();
     if (!s_last) return;
     __threadfence();
-    uint64_t t = 0;
-    for (uint32_t b = threadIdx.x; b < gridDim.x; b += blockDim.x) t += __ldcg(partials + b);
-    t = warp_sum(t);
-    __syncthreads();
-    if (lane_id() == 0) wsum[threadIdx.x >> 5] = t;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint64_t total = 0;
-        for (int w = 0; w < kIndexThreads / 32; ++w) total += wsum[w];
-        row_start[np] = total;
-        if (total != expected) {
-            atomicOr(err, DEV_ERR_ROW_COUNT);
-            atomicOr(state, COL_NOT_DIRECT);
-        }
-    }
-}
-
-/* A column without pages: zero rows (any other count is an error). */
-__global__ void k_page_index_empty(uint64_t expected, uint64_t *row_start, uint32_t *state, unsigned int *err) {
-    row_start[0] = 0;
-    if (expected != 0) {
-        atomicOr(err, DEV_ERR_ROW_COUNT);
-        atomicOr(state, COL_NOT_DIRECT);
-    }
-}
-
-__global__ void __launch_bounds__(kIndexThreads)
-    k_page_index_scan(const uint32_t *__restrict__ rows, uint64_t np, uint64_t chunk,
-                      const uint64_t *__restrict__ partials, uint64_t *__restrict__ row_start,
-                      const uint32_t *state) {
-    __shared__ uint64_t wbuf[kIndexThreads / 32 + 1];
-    if (*state == 0u) return; /* uniform: read in place */
-    uint64_t o = 0;
-    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += blockDim.x) o += partials[b];
-    uint64_t off;
-    block_exclusive_scan<uint64_t>(o, wbuf, &off);
-    const uint64_t p0 = (uint64_t)blockIdx.x * chunk, p1 = min(np, p0 + chunk);
-    for (uint64_t base = p0; base < p1; base += blockDim.x) {
-        const uint64_t p = base + threadIdx.x;
-        const uint64_t v = p < p1 ? rows[p] : 0;
-        uint64_t tot;
-        const uint64_t pre = block_exclusive_scan<uint64_t>(v, wbuf, &tot);
-        if (p < p1) row_start[p] = off + pre;
+    uint64_t off = 0;
+    for (uint32_t c0 = 0; c0 < T.index_blocks; c0 += kIndexThreads) {
+        const uint32_t c = c0 + threadIdx.x;
+        const uint64_t v = c < T.index_blocks ? __ldcg(T.base + c) : 0;
+        const uint64_t e = block_exclusive_scan<uint64_t>(v, wbuf, &tot);
+        if (c < T.index_blocks) T.base[c] = off + e;
         off += tot;
     }
+    if (threadIdx.x == 0 && off != T.rows) {
+        atomicOr(T.err, DEV_ERR_ROW_COUNT);
+        atomicOr(&T.state->flags, COL_NOT_DIRECT);
+    }
+}
+
+/* Task of a block: the last task whose first block is at most `block`. */
+template <bool kIndex> CJ_DEV uint32_t find_column(const ColumnTask *tasks, uint32_t ntasks, uint32_t block) {
+    uint32_t lo = 0, hi = ntasks;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if ((kIndex ? tasks[mid].index_base : tasks[mid].decode_base) <= block) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+/* Tasks travel as a kernel argument (a plan's few columns: no copy to wait
+ * for) or in device memory (a batch's hundreds). */
+struct ColumnArgs {
+    ColumnTask t[kColumnArgs];
+    uint32_t n;
+};
+
+__global__ void __launch_bounds__(kIndexThreads) k_page_index(const __grid_constant__ ColumnArgs a) {
+    const ColumnTask &T = a.t[find_column<true>(a.t, a.n, blockIdx.x)];
+    index_chunk(T, blockIdx.x - T.index_base);
+}
+
+__global__ void __launch_bounds__(kIndexThreads) k_page_index_grouped(const ColumnTask *tasks, uint32_t n) {
+    const ColumnTask &T = tasks[find_column<true>(tasks, n, blockIdx.x)];
+    index_chunk(T, blockIdx.x - T.index_base);
 }
 
 /* Loads a sparse page's bitmap into s_bm (bits past n_rows cleared) and the
@@ -374,153 +369,77 @@ CJ_DEV void decode_varchar_page(const uint8_t *__restrict__ pages, uint64_t p, u
     __syncthreads();
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kDecodeThreads, 8)
-    k_decode_fixed(const uint8_t *__restrict__ pages, uint64_t np, const uint64_t *__restrict__ row_start,
-                   uint64_t max_rows, T *__restrict__ values, uint32_t *__restrict__ valid, unsigned int *err,
-                   const uint32_t *__restrict__ col_flags) {
-    __shared__ DecodeSmem sm;
-    if (col_flags && *col_flags == 0u) return; /* read in place from the pages */
-    for (uint64_t p = blockIdx.x; p < np; p += gridDim.x)
-        decode_fixed_page<T>(pages, p, row_start[p], max_rows, values, valid, err, sm);
-}
-
-__global__ void __launch_bounds__(kDecodeThreads)
-    k_decode_varchar(const uint8_t *__restrict__ pages, uint64_t np, const uint64_t *__restrict__ row_start,
-                     uint64_t max_rows, uint64_t *__restrict__ desc, uint32_t *__restrict__ valid, unsigned int *err) {
-    __shared__ DecodeSmem sm;
-    for (uint64_t p = blockIdx.x; p < np; p += gridDim.x)
-        decode_varchar_page(pages, p, np, row_start[p], max_rows, desc, valid, err, sm);
-}
-
-/* ---- grouped: every column a batch needs, one launch per pass ---- */
-CJ_DEV uint32_t find_column(const DecodeTask *tasks, uint32_t ntasks, uint64_t gpage) {
-    uint32_t lo = 0, hi = ntasks;
-    while (hi - lo > 1) {
-        uint32_t mid = (lo + hi) >> 1;
-        if (tasks[mid].page_base <= gpage) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
-__global__ void k_page_rows_grouped(const DecodeTask *__restrict__ tasks, uint32_t ntasks, uint64_t total_pages,
-                                    uint32_t *__restrict__ rows, unsigned int *err) {
-    for (uint64_t gp = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; gp < total_pages;
-         gp += (uint64_t)gridDim.x * blockDim.x) {
-        const DecodeTask &T = tasks[find_column(tasks, ntasks, gp)];
-        const uint8_t *pg = T.pages + (gp - T.page_base) * kPageSize;
-        rows[gp] = page_rows_of(pg, T.type, err);
-    }
-}
-
-__global__ void k_check_rows_grouped(const DecodeTask *__restrict__ tasks, uint32_t ntasks,
-                                     const uint64_t *__restrict__ row_start, unsigned int *err) {
-    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < ntasks; k += gridDim.x * blockDim.x) {
-        const DecodeTask &T = tasks[k];
-        if (row_start[T.page_base + T.num_pages] - row_start[T.page_base] != T.rows) atomicOr(err, DEV_ERR_ROW_COUNT);
-    }
-}
-
-__global__ void __launch_bounds__(kDecodeThreads)
-    k_decode_grouped(const DecodeTask *__restrict__ tasks, uint32_t ntasks, uint64_t total_pages,
-                     const uint64_t *__restrict__ row_start, unsigned int *err) {
-    __shared__ DecodeSmem sm;
-    __shared__ uint32_t s_task;
-    for (uint64_t gp = blockIdx.x; gp < total_pages; gp += gridDim.x) {
-        if (threadIdx.x == 0) s_task = find_column(tasks, ntasks, gp);
-        __syncthreads();
-        const DecodeTask &T = tasks[s_task];
-        const uint64_t p = gp - T.page_base;
-        const uint64_t rs = row_start[gp] - row_start[T.page_base];
+/* Decode of every column that is not read in place: task k's blocks stride
+ * over its pages; the blocks of a column read in place (flags 0) leave at
+ * once. 32 registers and 16 KB of shared memory: 8 CTAs per SM. */
+CJ_DEV void decode_blocks(const ColumnTask &T, uint32_t b, DecodeSmem &sm) {
+    if (T.type != CJ_VARCHAR && T.state->flags == 0u) return;
+    for (uint64_t p = b; p < T.num_pages; p += T.decode_blocks) {
+        const uint64_t rs = page_first_row(T.base, T.loc, p);
         if (T.type == CJ_VARCHAR)
-            decode_varchar_page(T.pages, p, T.num_pages, rs, T.rows, T.desc, T.valid, err, sm);
+            decode_varchar_page(T.pages, p, T.num_pages, rs, T.rows, T.desc, T.valid, T.err, sm);
         else if (T.type == CJ_INT32)
-            decode_fixed_page<int32_t>(T.pages, p, rs, T.rows, reinterpret_cast<int32_t *>(T.values), T.valid, err, sm);
+            decode_fixed_page<int32_t>(T.pages, p, rs, T.rows, reinterpret_cast<int32_t *>(T.values), T.valid, T.err,
+                                       sm);
         else
             decode_fixed_page<long long>(T.pages, p, rs, T.rows, reinterpret_cast<long long *>(T.values), T.valid,
-                                         err, sm);
+                                         T.err, sm);
         __syncthreads();
     }
 }
 
-unsigned grid_for(const Launch &L, uint64_t units, int per_sm) {
-    uint64_t g = (uint64_t)L.num_sms * per_sm;
-    if (units < g) g = units;
-    return (unsigned)(g ? g : 1);
+__global__ void __launch_bounds__(kDecodeThreads, 8) k_decode(const __grid_constant__ ColumnArgs a) {
+    __shared__ DecodeSmem sm;
+    const ColumnTask &T = a.t[find_column<false>(a.t, a.n, blockIdx.x)];
+    decode_blocks(T, blockIdx.x - T.decode_base, sm);
+}
+
+__global__ void __launch_bounds__(kDecodeThreads, 8) k_decode_grouped(const ColumnTask *tasks, uint32_t n) {
+    __shared__ DecodeSmem sm;
+    const ColumnTask &T = tasks[find_column<false>(tasks, n, blockIdx.x)];
+    decode_blocks(T, blockIdx.x - T.decode_base, sm);
 }
 
 } // namespace
 
-uint64_t page_index_blocks(const Launch &L, uint64_t np) {
-    const uint64_t chunk = std::max<uint64_t>(kIndexThreads, (np + L.num_sms * 8 - 1) / (L.num_sms * 8));
-    return std::max<uint64_t>((np + chunk - 1) / chunk, 1);
+uint32_t index_blocks(uint64_t np) { return (uint32_t)std::max<uint64_t>((np + kIndexChunk - 1) / kIndexChunk, 1); }
+
+ColumnGrid place_columns(const Launch &L, ColumnTask *tasks, size_t n) {
+    ColumnGrid g;
+    const uint64_t wave = (uint64_t)L.num_sms * 8;
+    for (size_t k = 0; k < n; ++k) {
+        ColumnTask &t = tasks[k];
+        t.index_blocks = index_blocks(t.num_pages);
+        t.index_base = g.index;
+        t.decode_blocks = (uint32_t)std::min<uint64_t>(t.num_pages, wave);
+        t.decode_base = g.decode;
+        g.index += t.index_blocks;
+        g.decode += t.decode_blocks;
+    }
+    return g;
 }
 
-cudaError_t launch_page_index(const Launch &L, const uint8_t *pages, uint64_t np, int32_t type, uint64_t rows,
-                              uint32_t *rows_pp, uint64_t *partials, uint64_t *row_start, uint32_t *state) {
-    if (np == 0) {
-        k_page_index_empty<<<1, 1, 0, L.stream>>>(rows, row_start, state, L.dev_errors);
-        count_launches(1);
-        return cudaGetLastError();
+cudaError_t launch_columns(const Launch &L, ColumnTask *tasks, size_t n, bool index) {
+    for (size_t k = 0; k < n; k += kColumnArgs) {
+        ColumnArgs a;
+        a.n = (uint32_t)std::min<size_t>(n - k, kColumnArgs);
+        const ColumnGrid g = place_columns(L, tasks + k, a.n);
+        std::copy(tasks + k, tasks + k + a.n, a.t);
+        if (index) k_page_index<<<g.index, kIndexThreads, 0, L.stream>>>(a);
+        else if (g.decode) k_decode<<<g.decode, kDecodeThreads, 0, L.stream>>>(a);
+        count_launches(index || g.decode ? 1 : 0);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
     }
-    const unsigned g = (unsigned)page_index_blocks(L, np);
-    const uint64_t chunk = (np + g - 1) / g;
-    k_page_index<<<g, kIndexThreads, 0, L.stream>>>(pages, np, type, chunk, rows, rows_pp, partials, row_start,
-                                                     state, L.dev_errors);
-    k_page_index_scan<<<g, kIndexThreads, 0, L.stream>>>(rows_pp, np, chunk, partials, row_start, state);
-    count_launches(2);
+    return cudaSuccess;
+}
+
+cudaError_t launch_columns_grouped(const Launch &L, const ColumnTask *tasks_dev, uint32_t n, const ColumnGrid &g) {
+    if (!n) return cudaSuccess;
+    k_page_index_grouped<<<g.index, kIndexThreads, 0, L.stream>>>(tasks_dev, n);
+    if (g.decode) k_decode_grouped<<<g.decode, kDecodeThreads, 0, L.stream>>>(tasks_dev, n);
+    count_launches(g.decode ? 2 : 1);
     return cudaGetLastError();
 }
-
-cudaError_t launch_decode_fixed(const Launch &L, const uint8_t *pages, uint64_t np, int32_t type,
-                                const uint64_t *row_start, uint64_t max_rows, void *values,
-                                uint32_t *valid, const uint32_t *col_flags) {
-    if (np == 0) return cudaSuccess;
-    unsigned g = grid_for(L, np, 8); /* 32 registers, 16 KB shared: 8 CTAs per SM */
-    if (type == CJ_INT32) {
-        k_decode_fixed<int32_t><<<g, kDecodeThreads, 0, L.stream>>>(
-            pages, np, row_start, max_rows, reinterpret_cast<int32_t *>(values), valid, L.dev_errors, col_flags);
-        count_launches(1);
-    } else {
-        k_decode_fixed<long long><<<g, kDecodeThreads, 0, L.stream>>>(
-            pages, np, row_start, max_rows, reinterpret_cast<long long *>(values), valid, L.dev_errors,
-            col_flags);
-        count_launches(1);
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_decode_varchar(const Launch &L, const uint8_t *pages, uint64_t np,
-                                  const uint64_t *row_start, uint64_t max_rows, uint64_t *desc,
-                                  uint32_t *valid) {
-    if (np == 0) return cudaSuccess;
-    unsigned g = grid_for(L, np, 6);
-    k_decode_varchar<<<g, kDecodeThreads, 0, L.stream>>>(pages, np, row_start, max_rows, desc, valid,
-                                                          L.dev_errors);
-    count_launches(1);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_decode_grouped(const Launch &L, const DecodeTask *tasks_dev, uint32_t ntasks, uint64_t total_pages,
-                                  uint32_t *rows_pp, uint64_t *row_start, void *scan_temp) {
-    if (!ntasks) return cudaSuccess;
-    if (total_pages) {
-        unsigned g = (unsigned)std::min<uint64_t>((total_pages + 255) / 256, (uint64_t)L.num_sms * 8);
-        k_page_rows_grouped<<<g, 256, 0, L.stream>>>(tasks_dev, ntasks, total_pages, rows_pp, L.dev_errors);
-        count_launches(1);
-    }
-    cudaError_t e = scan_u32_to_u64(L, rows_pp, row_start, total_pages, scan_temp);
-    if (e != cudaSuccess) return e;
-    k_check_rows_grouped<<<(ntasks + 127) / 128, 128, 0, L.stream>>>(tasks_dev, ntasks, row_start, L.dev_errors);
-    count_launches(1);
-    if (total_pages) {
-        unsigned g = grid_for(L, total_pages, 6);
-        k_decode_grouped<<<g, kDecodeThreads, 0, L.stream>>>(tasks_dev, ntasks, total_pages, row_start, L.dev_errors);
-        count_launches(1);
-    }
-    return cudaGetLastError();
-}
-
 
 } // namespace cj

@@ -9,7 +9,7 @@
  * row-id vectors (k_gather_u32); values are read once, by the root's page
  * writers, through up to two row-id indirections.
  *
- * Fixed-width pages (k_write_fixed): output page p holds rows
+ * Fixed-width pages (k_write_pages): output page p holds rows
  * [p*R, p*R+R) with R = 1984 (INT32) or 1007 (INT64 / FP64), the fill of
  * ColumnInserter<T> (plan.h:241-250), so every page fits whatever the NULL
  * pattern. One CTA writes one page: all of the page's loads issued at
@@ -193,69 +193,77 @@ CJ_DEV uint64_t live_rows(uint64_t rows, const unsigned long long *rows_dev) {
     return n < rows ? n : rows;
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kMatThreads, kMatMinBlocks)
-    k_write_fixed(ColView col, uint64_t rows, const unsigned long long *rows_dev, uint32_t R,
-                  uint8_t *__restrict__ out) {
-    __shared__ PageSmem sm;
-    rows = live_rows(rows, rows_dev);
-    const uint64_t num_pages = (rows + R - 1) / R;
-    if (blockIdx.x >= num_pages) return;
-    zero_page(sm);
-    for (uint64_t pg = blockIdx.x; pg < num_pages; pg += gridDim.x) write_fixed_page<T>(col, rows, R, pg, out, sm);
-}
-
-/* Finishes pages whose values are in place (a NULL-free column written by
+/* Finishes a page whose values are in place (a NULL-free column written by
  * the probe): header, zero gap after the values, bitmap of nr ones. */
-template <typename T>
-__global__ void k_finish_dense_pages(uint8_t *__restrict__ pages, uint64_t rows, const unsigned long long *rows_dev) {
+template <typename T> CJ_DEV void finish_dense_page(uint8_t *__restrict__ pages, uint64_t rows, uint64_t pg) {
     constexpr uint32_t R = sizeof(T) == 4 ? kRowsPerPageInt32 : kRowsPerPage8B;
     constexpr uint32_t DB = sizeof(T) == 4 ? 4u : 8u;
-    rows = live_rows(rows, rows_dev);
-    const uint64_t num_pages = (rows + R - 1) / R;
-    for (uint64_t pg = blockIdx.x; pg < num_pages; pg += gridDim.x) {
-        uint8_t *dst = pages + pg * kPageSize;
-        const uint32_t nr = (uint32_t)min((uint64_t)R, rows - pg * R);
-        if (threadIdx.x == 0) {
-            if (DB == 8) __stcs(reinterpret_cast<unsigned long long *>(dst), (unsigned long long)nr * 0x10001ull);
-            else __stcs(reinterpret_cast<unsigned int *>(dst), nr * 0x10001u);
+    uint8_t *dst = pages + pg * kPageSize;
+    const uint32_t nr = (uint32_t)min((uint64_t)R, rows - pg * R);
+    if (threadIdx.x == 0) {
+        if (DB == 8) __stcs(reinterpret_cast<unsigned long long *>(dst), (unsigned long long)nr * 0x10001ull);
+        else __stcs(reinterpret_cast<unsigned int *>(dst), nr * 0x10001u);
+    }
+    const uint32_t bm_bytes = (nr + 7) / 8, bm0 = kPageSize - bm_bytes;
+    for (uint32_t b = DB + nr * (uint32_t)sizeof(T) + threadIdx.x; b < kPageSize; b += blockDim.x) {
+        uint8_t v = 0;
+        if (b >= bm0) {
+            const uint32_t i = b - bm0;
+            v = (i + 1) * 8 <= nr ? 0xFFu : (uint8_t)((1u << (nr - i * 8)) - 1u);
         }
-        const uint32_t bm_bytes = (nr + 7) / 8, bm0 = kPageSize - bm_bytes;
-        for (uint32_t b = DB + nr * (uint32_t)sizeof(T) + threadIdx.x; b < kPageSize; b += blockDim.x) {
-            uint8_t v = 0;
-            if (b >= bm0) {
-                const uint32_t i = b - bm0;
-                v = (i + 1) * 8 <= nr ? 0xFFu : (uint8_t)((1u << (nr - i * 8)) - 1u);
-            }
-            dst[b] = v;
-        }
+        dst[b] = v;
     }
 }
 
-/* Grouped page writer: every fixed-width output column of a batch. */
-__global__ void __launch_bounds__(kMatThreads, kMatMinBlocks)
-    k_write_fixed_grouped(const PageTask *__restrict__ tasks, uint32_t ntasks, uint64_t total_pages) {
-    __shared__ PageSmem sm;
-    __shared__ uint32_t s_task;
-    zero_page(sm);
-    for (uint64_t gp = blockIdx.x; gp < total_pages; gp += gridDim.x) {
-        if (threadIdx.x == 0) {
-            uint32_t lo = 0, hi = ntasks;
-            while (hi - lo > 1) {
-                uint32_t mid = (lo + hi) >> 1;
-                if (tasks[mid].page_base <= gp) lo = mid;
-                else hi = mid;
-            }
-            s_task = lo;
+/* Page writer: the fixed-width result columns of a plan (tasks by value) or
+ * of a batch (tasks in device memory) in one launch; task k's blocks stride
+ * over its pages. One launch for a plan's columns instead of one each: at
+ * C1's size each of those ran 6-10 us for 1-4 us of work. */
+CJ_DEV void write_page_blocks(const PageTask &T, uint32_t b, PageSmem &sm) {
+    const uint64_t rows = live_rows(T.rows, T.rows_dev);
+    const uint32_t R = rows_per_page_dev(T.col.type);
+    const uint64_t num_pages = (rows + R - 1) / R;
+    if (b >= num_pages) return;
+    if (T.finish) {
+        for (uint64_t pg = b; pg < num_pages; pg += T.blocks) {
+            if (T.col.type == CJ_INT32) finish_dense_page<int32_t>(T.out, rows, pg);
+            else finish_dense_page<long long>(T.out, rows, pg);
         }
-        __syncthreads();
-        const PageTask &T = tasks[s_task];
-        const uint64_t pg = gp - T.page_base;
-        if (T.col.type == CJ_INT32)
-            write_fixed_page<int32_t>(T.col, T.rows, rows_per_page_dev(CJ_INT32), pg, T.out, sm);
-        else
-            write_fixed_page<long long>(T.col, T.rows, rows_per_page_dev(CJ_INT64), pg, T.out, sm);
+        return;
     }
+    zero_page(sm);
+    for (uint64_t pg = b; pg < num_pages; pg += T.blocks) {
+        if (T.col.type == CJ_INT32) write_fixed_page<int32_t>(T.col, rows, kRowsPerPageInt32, pg, T.out, sm);
+        else write_fixed_page<long long>(T.col, rows, kRowsPerPage8B, pg, T.out, sm);
+    }
+}
+
+CJ_DEV uint32_t find_pages(const PageTask *tasks, uint32_t ntasks, uint32_t block) {
+    uint32_t lo = 0, hi = ntasks;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (tasks[mid].block_base <= block) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+
+struct PageArgs {
+    PageTask t[kPageArgs];
+    uint32_t n;
+};
+
+__global__ void __launch_bounds__(kMatThreads, kMatMinBlocks) k_write_pages(const __grid_constant__ PageArgs a) {
+    __shared__ PageSmem sm;
+    const PageTask &T = a.t[find_pages(a.t, a.n, blockIdx.x)];
+    write_page_blocks(T, blockIdx.x - T.block_base, sm);
+}
+
+__global__ void __launch_bounds__(kMatThreads, kMatMinBlocks)
+    k_write_pages_grouped(const PageTask *__restrict__ tasks, uint32_t ntasks) {
+    __shared__ PageSmem sm;
+    const PageTask &T = tasks[find_pages(tasks, ntasks, blockIdx.x)];
+    write_page_blocks(T, blockIdx.x - T.block_base, sm);
 }
 
 /* Grouped row-id gather: task k covers global chunks [chunk_base, ...). */
@@ -508,11 +516,35 @@ cudaError_t launch_gather_u32(const Launch &L, const uint32_t *src, const uint32
     return cudaGetLastError();
 }
 
-cudaError_t launch_write_fixed_grouped(const Launch &L, const PageTask *tasks_dev, uint32_t ntasks,
-                                      uint64_t total_pages) {
-    if (!total_pages) return cudaSuccess;
-    uint64_t g = std::min<uint64_t>(total_pages, (uint64_t)L.num_sms * kMatMinBlocks);
-    k_write_fixed_grouped<<<(unsigned)g, kMatThreads, 0, L.stream>>>(tasks_dev, ntasks, total_pages);
+uint32_t place_pages(const Launch &L, PageTask *tasks, size_t n) {
+    uint32_t grid = 0;
+    for (size_t k = 0; k < n; ++k) {
+        const uint32_t R = rows_per_page_fixed(tasks[k].col.type);
+        tasks[k].blocks = (uint32_t)std::min<uint64_t>((tasks[k].rows + R - 1) / R, (uint64_t)L.num_sms * kMatMinBlocks);
+        tasks[k].block_base = grid;
+        grid += tasks[k].blocks;
+    }
+    return grid;
+}
+
+cudaError_t launch_write_pages(const Launch &L, PageTask *tasks, size_t n) {
+    for (size_t k = 0; k < n; k += kPageArgs) {
+        PageArgs a;
+        a.n = (uint32_t)std::min<size_t>(n - k, kPageArgs);
+        const uint32_t grid = place_pages(L, tasks + k, a.n);
+        std::copy(tasks + k, tasks + k + a.n, a.t);
+        if (!grid) continue;
+        k_write_pages<<<grid, kMatThreads, 0, L.stream>>>(a);
+        count_launches(1);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+cudaError_t launch_write_pages_grouped(const Launch &L, const PageTask *tasks_dev, uint32_t n, uint32_t grid) {
+    if (!grid) return cudaSuccess;
+    k_write_pages_grouped<<<grid, kMatThreads, 0, L.stream>>>(tasks_dev, n);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -528,35 +560,6 @@ cudaError_t launch_gather_grouped(const Launch &L, const GatherTask *tasks_dev, 
 
 uint32_t rows_per_page_fixed(int32_t type) {
     return type == CJ_INT32 ? kRowsPerPageInt32 : kRowsPerPage8B;
-}
-
-cudaError_t launch_write_fixed_pages(const Launch &L, const ColView &col, uint64_t rows,
-                                     uint8_t *out, const unsigned long long *rows_dev) {
-    if (rows == 0) return cudaSuccess;
-    const uint32_t R = rows_per_page_fixed(col.type);
-    const uint64_t np = (rows + R - 1) / R;
-    uint64_t g = np, cap = (uint64_t)L.num_sms * kMatMinBlocks;
-    if (g > cap) g = cap;
-    if (col.type == CJ_INT32) {
-        k_write_fixed<int32_t><<<(unsigned)g, kMatThreads, 0, L.stream>>>(col, rows, rows_dev, R, out);
-        count_launches(1);
-    } else {
-        k_write_fixed<long long><<<(unsigned)g, kMatThreads, 0, L.stream>>>(col, rows, rows_dev, R, out);
-        count_launches(1);
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t launch_finish_dense_pages(const Launch &L, uint8_t *pages, uint64_t rows, int32_t type,
-                                      const unsigned long long *rows_dev) {
-    if (rows == 0) return cudaSuccess;
-    const uint32_t R = rows_per_page_fixed(type);
-    const uint64_t np = (rows + R - 1) / R;
-    const unsigned g = (unsigned)std::min<uint64_t>(np, (uint64_t)L.num_sms * 8);
-    if (type == CJ_INT32) k_finish_dense_pages<int32_t><<<g, 128, 0, L.stream>>>(pages, rows, rows_dev);
-    else k_finish_dense_pages<long long><<<g, 128, 0, L.stream>>>(pages, rows, rows_dev);
-    count_launches(1);
-    return cudaGetLastError();
 }
 
 size_t varchar_temp_bytes(uint64_t rows, uint32_t TR) {
