@@ -115,6 +115,10 @@ CJ_DEV bool col_direct(const ColView &c) { return c.col_flags && __ldg(c.col_fla
 /* A column without NULLs: validity need not be read. */
 CJ_DEV bool col_all_valid(const ColView &c) { return c.col_flags && (__ldg(c.col_flags) & COL_HAS_NULLS) == 0u; }
 
+/* A fixed-width column whose rows read through a view are never NULL: its
+ * result pages hold value q at a place that depends on q alone. */
+CJ_DEV bool col_null_free(const ColView &c) { return col_all_valid(c) && !(c.type == CJ_INT32 && c.null_sentinel); }
+
 /* Base row r of a direct column: value r % R of page r / R (R constant per
  * width, so the division is a multiply). */
 template <typename T> CJ_DEV T page_value(const uint8_t *pages, uint32_t r) {

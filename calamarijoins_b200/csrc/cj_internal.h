@@ -79,9 +79,8 @@ struct StatusBlock {
     unsigned int errors;          /* DevError bits                          */
     unsigned int pad;
     unsigned long long counter;   /* match counter of the last probe        */
-    unsigned long long aux[8];    /* [0, kDirectParams): direct-mapped table
-                                     parameters; [kOpenDup]: a repeated key
-                                     in the open-addressing table          */
+    unsigned long long table[8];  /* kTableWords of the last unique table   */
+    unsigned long long aux;       /* a count on its way to the host (filter) */
     unsigned long long stale[3];  /* DEV_ERR_STALE: check index, count found,
                                      count recorded (one of the mismatches) */
     ColumnState cols[kStatusColumns];
@@ -282,33 +281,76 @@ cudaError_t launch_build_grouped(const Launch &L, const BuildTask *tasks_dev, ui
                                  uint32_t total_parts, uint64_t total_cells, uint32_t max_parts, uint32_t max_slots,
                                  const uint16_t *bloom, void *temp);
 
-/* Direct-mapped build for unique keys spread densely over [lo, lo + span):
- * slots[key - lo] = build row, decided on the device. `params` (6 u64, set
- * by the caller to {~0, 0, 0, 0, 0, 0}) receives [0] min and [1] max of the
- * non-NULL keys (XOR 2^63: unsigned order is signed order), [2] their count,
- * [3] non-zero when the table cannot be used (1: span above max_span, 2: a
- * repeated key), [4] lo, [5] span. `slots` holds max_span entries. Four launches, no
- * host round trip. */
+/* Table of unique build keys (k_unique.cu): direct-mapped when their range is
+ * at most max_span, else, for INT32 keys (open_slots > 0), open-addressing.
+ * `slots` holds max(4 max_span, 8 open_slots) bytes rounded up to 16,
+ * 16-byte aligned; open_slots is at least twice the build rows. `params` (kTableWords words, zero before the build) receives what the
+ * device found. */
 constexpr uint32_t kArrayEmpty = 0xFFFFFFFFu;
-constexpr int kDirectParams = 6;
-cudaError_t launch_direct_build(const Launch &L, const ColView &key, uint32_t n, uint64_t max_span, uint32_t *slots,
-                                unsigned long long *params);
-/* Probe of a direct-mapped table; does nothing when params[3] is set. */
-cudaError_t launch_probe_tiles_array(const Launch &L, const ColView &pkey, uint32_t n_probe, const uint32_t *slots,
-                                     const unsigned long long *params, const MatchOut &out, void *sched);
-
-/* Open-addressing table for unique INT32 build keys too spread out for a
- * direct-mapped table: `nslots` 8-byte slots (key << 32 | build row, all
- * ones when empty; at most half of them full), linear probing from the
- * key's hash scaled to [0, nslots). The build sets *dup when a key repeats
- * (the table cannot be used); the probe then does nothing. Two launches. */
-constexpr int kOpenDup = kDirectParams;
 constexpr uint64_t kOpenMaxRows = 1ull << 28;
-cudaError_t launch_open_build(const Launch &L, const ColView &key, uint32_t n, unsigned long long *slots,
-                              uint64_t nslots, unsigned long long *dup);
-cudaError_t launch_probe_tiles_open(const Launch &L, const ColView &pkey, uint32_t n_probe,
-                                    const unsigned long long *slots, uint64_t nslots,
-                                    const unsigned long long *dup, const MatchOut &out, void *sched);
+enum TableWord { /* of params */
+    kTableMinC = 0,    /* ~min, max of the non-NULL keys (XOR 2^63: unsigned
+                          order is signed order) and their count           */
+    kTableMax = 1,
+    kTableCount = 2,
+    kTableRefused = 3, /* not direct-mapped: a TableRefusal                */
+    kTableLo = 4,      /* smallest key, values in the range                */
+    kTableSpan = 5,
+    kTableDup = 6,     /* the build met a repeated key: the table is unusable */
+    kTableDone = 7,    /* blocks of the range pass that have finished      */
+    kTableWords = 8
+};
+enum TableRefusal : unsigned long long {
+    kTableSpread = 1,  /* the keys' range is above max_span           */
+    kTableRepeats = 2  /* more keys than values in their range        */
+};
+struct UniqueTable {
+    void *slots;
+    unsigned long long *params;
+    uint64_t max_span;
+    uint32_t open_slots; /* 0: no open-addressing table */
+};
+/* What the params say (host copy or device): 0 unusable, 1 direct-mapped,
+ * 2 open-addressing. */
+inline int table_kind(const unsigned long long *p, uint32_t open_slots) {
+    if (p[kTableDup]) return 0;
+    if (!p[kTableRefused]) return 1;
+    return p[kTableRefused] == kTableSpread && open_slots ? 2 : 0;
+}
+cudaError_t launch_unique_build(const Launch &L, const ColView &key, uint32_t n, const UniqueTable &t);
+
+/* The probe's key column: a scan read page by page (base and loc of its page
+ * index set; the decoded arrays are not needed), or relation rows through
+ * the view (base null). */
+struct ProbeKey {
+    ColView col;
+    const uint64_t *base;
+    const uint32_t *loc;
+    uint64_t num_pages;
+    unsigned int *err; /* errors of the column's pages */
+};
+/* A fixed-width result column that the probe writes when the device finds
+ * that it holds no NULL (else its match row ids are collected). */
+struct EmitColumn {
+    ColView col; /* rid_a unused: the match row ids */
+    uint8_t *pages;
+    int32_t from_build;
+    int32_t direct_only; /* not beside an open-addressing table: the two would
+                            not stay in L2 together                       */
+};
+constexpr int kEmitColumns = 8;
+struct UniqueOut {
+    MatchOut match;      /* capacity: at least the probe rows         */
+    bool need_b, need_p; /* match row ids wanted whatever the columns */
+    int n;
+    EmitColumn cols[kEmitColumns];
+};
+/* Probe of a unique table; does nothing when the table is unusable. The
+ * match counter must be zero before. */
+cudaError_t launch_probe_unique(const Launch &L, const ProbeKey &k, uint32_t n, const UniqueTable &t,
+                                const UniqueOut &out);
+
+constexpr int kDirectParams = 6; /* words of a grouped direct-mapped table */
 
 /* Probe and nested loop share one tiled kernel; `sched` is scratch of
  * probe_sched_bytes(n_probe) bytes (the tile ticket). */
@@ -347,9 +389,13 @@ struct ProbeTask {
     uint32_t num_tiles;
     uint32_t tile_base;         /* first global tile of this task           */
 };
-/* Grouped direct-mapped builds (launch_direct_build for every task): task k
- * owns blocks [block_base, block_base + blocks) of each pass; params hold
- * kDirectParams words per task, set to {~0, 0, 0, 0, 0, 0} before. */
+/* Grouped direct-mapped builds: slots[key - lo] = build row for every task
+ * whose keys are unique and span at most max_span values; task k owns blocks
+ * [block_base, block_base + blocks) of each pass. params hold kDirectParams
+ * words per task, set to {~0, 0, 0, 0, 0, 0} before, and receive [0] min and
+ * [1] max of the non-NULL keys (XOR 2^63), [2] their count, [3] non-zero when
+ * the table cannot be used (1: span above max_span, 2: a repeated key), [4]
+ * lo, [5] span. */
 struct DirectTask {
     ColView key;
     uint32_t n;
@@ -402,14 +448,19 @@ cudaError_t launch_gather_grouped(const Launch &L, const GatherTask *tasks_dev, 
 /* One fixed-width result column. `rows` are the rows to write or, with
  * `rows_dev` set, the capacity the pages were sized for while the count
  * itself is read on the device (a match counter the host has not read yet).
- * finish: the values are in place already (a NULL-free column written by the
- * probe); headers (n_rows = n_values), zero gaps and all-ones bitmaps only. */
+ * finish 1: the values are in place already (a NULL-free column written by
+ * the probe); headers (n_rows = n_values), zero gaps and all-ones bitmaps
+ * only. finish 2: so if the device finds that `col` holds no NULL, else the
+ * pages are written through its row ids. */
 struct PageTask {
     ColView col;
     uint64_t rows;
     const unsigned long long *rows_dev;
     uint8_t *out;
     int32_t finish;
+    const unsigned long long *table; /* finish 2: also written through the row
+                                        ids when set and these table words say
+                                        open-addressing (EmitColumn::direct_only) */
     uint32_t block_base, blocks; /* place_pages */
 };
 constexpr int kPageArgs = 24; /* tasks passed by value */

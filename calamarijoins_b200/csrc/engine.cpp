@@ -28,6 +28,13 @@
 namespace cj {
 namespace {
 
+/* A probe of an open-addressing table reads a build column's values beside
+ * it while both stay in L2 (126 MB on two dies, each keeping its own copy of
+ * what it reads); a larger pair is read one after the other, through the
+ * match row ids: 64 MB of table and 33 MB of values 1513 us together, 1447
+ * apart (64M probe rows). A direct-mapped table is 16 MB there. */
+constexpr uint64_t kEmitBesideOpen = 48ull << 20;
+
 enum Phase { PH_UPLOAD, PH_DECODE, PH_BUILD, PH_PROBE, PH_NL, PH_INTER, PH_MAT, PH_DOWNLOAD, PH_COUNT };
 /* NVTX range names of the phases (host-side ranges around the enqueueing of
  * each phase; visible in Nsight Systems timelines). */
@@ -120,6 +127,14 @@ class Executor {
     std::map<std::pair<uint64_t, uint64_t>, Prefetched> prefetched;
     std::vector<PhaseEv> phase_events;
     cj_exec_stats stats{};
+    /* The match counter and table words of the status block are zero (they
+     * are when a plan starts): nothing to clear before the first join. */
+    bool join_words_clear = true;
+    void clear_join_words() {
+        ck(cudaMemsetAsync(&ctx.d_status->counter, 0, sizeof(ctx.d_status->counter) + sizeof(ctx.d_status->table),
+                           ctx.stream),
+           "memset");
+    }
     uint64_t used_cols = 0;   /* columns of the status block the plan has read */
     bool synced_last = false; /* the last thing enqueued was a synchronisation */
     /* Brings the status block to the host, counting the synchronisation. */
@@ -148,8 +163,10 @@ class Executor {
 
     void validate();
     void prefetch();
-    void decode_columns(std::vector<ColumnTask> &tasks);
+    void launch_tasks(std::vector<ColumnTask> &tasks, bool index);
+    Decoded &indexed(uint64_t t, uint64_t c);
     Decoded &decode(uint64_t t, uint64_t c);
+    int streamed_key(std::pair<uint64_t, uint64_t> *col) const;
     Relation resolve(uint64_t node, int depth);
     Relation exec_join(uint64_t node, int depth, bool is_root, cj_result **out);
     ColView view(const Relation &R, const RelCol &c, const uint32_t *rid_a);
@@ -159,7 +176,9 @@ class Executor {
         const Relation *rel; /* null: the values are already in `pages` */
         RelCol col;
         const uint32_t *rid_a;
-        DevPtr pages; /* result pages written by the probe (no NULL) */
+        DevPtr pages; /* result pages written by the probe (with `rel`: if
+                         the column holds no NULL)                       */
+        bool direct_only = false; /* ... and the table is direct-mapped */
     };
     ColView out_view(const OutCol &oc) { return view(*oc.rel, oc.col, oc.rid_a); }
     cj_result *materialize(const std::vector<OutCol> &cols, const std::vector<int32_t> &types, uint64_t rows,
@@ -205,7 +224,9 @@ void Executor::prefetch() {
         return out;
     };
     for (const TC &tc : cols(plan.root, 0)) add(tc);
-    std::vector<ColumnTask> tasks;
+    std::vector<ColumnTask> tasks, decodes;
+    TC streamed;
+    const bool stream = streamed_key(&streamed);
     for (const TC &tc : order) {
         const cj_table *r = resident(tc.first);
         if (!r || r->num_rows > 0xFFFFFFFFull || tasks.size() == kStatusColumns) continue;
@@ -215,10 +236,16 @@ void Executor::prefetch() {
         d.src = r->cols[tc.second];
         d.status_col = (int)tasks.size();
         tasks.push_back(column_task(ctx, d, &ctx.d_status->cols[tasks.size()]));
+        d.ready = !(stream && tc == streamed);
+        if (d.ready) decodes.push_back(tasks.back());
         decoded.emplace(tc, std::move(d));
     }
     ck(cudaMemsetAsync(ctx.d_status, 0, sizeof(StatusBlock), ctx.stream), "memset");
-    if (!tasks.empty()) decode_columns(tasks);
+    if (!tasks.empty()) {
+        PhaseScope ph(*this, PH_DECODE);
+        launch_tasks(tasks, true);
+        if (!decodes.empty()) launch_tasks(decodes, false);
+    }
     cudaEvent_t first = nullptr;
     for (const TC &tc : order) {
         if (resident(tc.first)) continue;
@@ -239,17 +266,42 @@ void Executor::prefetch() {
     }
 }
 
-void Executor::decode_columns(std::vector<ColumnTask> &tasks) {
-    PhaseScope ph(*this, PH_DECODE);
-    {
-        KScope k(*this, "page_index");
-        ck(launch_columns(L, tasks.data(), tasks.size(), true), "page_index");
+/* Whether the root joins two scans whose probe key column is read by the
+ * probe alone, page by page (*col): no other key and no output but the key's
+ * own reads it, so it need not be decoded. A rule on what is known before
+ * anything runs; a join that goes on to another table decodes it then. */
+int Executor::streamed_key(std::pair<uint64_t, uint64_t> *col) const {
+    const cj_plan_node &n = plan.nodes[plan.root];
+    if (n.node_type != CJ_NODE_HASH_JOIN || ctx.opt.dense_keys <= 0) return 0;
+    const cj_plan_node &l = plan.nodes[n.left], &r = plan.nodes[n.right];
+    if (l.node_type != CJ_NODE_SCAN || r.node_type != CJ_NODE_SCAN) return 0;
+    const uint64_t lrows = table_rows(l.base_table_id), rrows = table_rows(r.base_table_id);
+    const bool build_left = lrows <= rrows;
+    if ((int64_t)std::min(lrows, rrows) <= ctx.opt.nested_loop_max_build) return 0;
+    const cj_plan_node &b = build_left ? l : r, &p = build_left ? r : l;
+    const uint64_t battr = build_left ? n.left_attr : n.right_attr, pattr = build_left ? n.right_attr : n.left_attr;
+    if (battr >= b.num_output_attrs || pattr >= p.num_output_attrs) return 0;
+    *col = {p.base_table_id, p.output_attrs[pattr].index};
+    if (*col == std::make_pair(b.base_table_id, b.output_attrs[battr].index)) return 0;
+    for (uint64_t a = 0; a < n.num_output_attrs; ++a) {
+        const uint64_t i = n.output_attrs[a].index;
+        const bool left = i < l.num_output_attrs;
+        const cj_plan_node &side = left ? l : r;
+        const uint64_t k = left ? i : i - l.num_output_attrs;
+        if (k < side.num_output_attrs && &side == &b &&
+            *col == std::make_pair(b.base_table_id, b.output_attrs[k].index))
+            return 0;
     }
-    KScope k(*this, "decode");
-    ck(launch_columns(L, tasks.data(), tasks.size(), false), "decode");
+    return 1;
 }
 
-Decoded &Executor::decode(uint64_t t, uint64_t c) {
+void Executor::launch_tasks(std::vector<ColumnTask> &tasks, bool index) {
+    KScope k(*this, index ? "page_index" : "decode");
+    ck(launch_columns(L, tasks.data(), tasks.size(), index), index ? "page_index" : "decode");
+}
+
+/* A column with its page index; its dense arrays may not be written yet. */
+Decoded &Executor::indexed(uint64_t t, uint64_t c) {
     auto key = std::make_pair(t, c);
     auto it = decoded.find(key);
     if (it != decoded.end()) {
@@ -272,9 +324,21 @@ Decoded &Executor::decode(uint64_t t, uint64_t c) {
         PhaseScope ph(*this, PH_UPLOAD);
         upload_pages(ctx, plan.inputs[t].columns[c], d.src, &stats.h2d_bytes);
     }
+    PhaseScope ph(*this, PH_DECODE);
     std::vector<ColumnTask> tasks{column_task(ctx, d, nullptr)};
-    decode_columns(tasks);
+    launch_tasks(tasks, true);
     return decoded.emplace(key, std::move(d)).first->second;
+}
+
+Decoded &Executor::decode(uint64_t t, uint64_t c) {
+    Decoded &d = indexed(t, c);
+    if (!d.ready) {
+        PhaseScope ph(*this, PH_DECODE);
+        std::vector<ColumnTask> tasks{d.task};
+        launch_tasks(tasks, false);
+        d.ready = true;
+    }
+    return d;
 }
 
 ColView Executor::view(const Relation &R, const RelCol &c, const uint32_t *rid_a) {
@@ -313,6 +377,8 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         const Relation *rel;
         RelCol col;
         bool from_keys = false; /* root: read from the keys the probe writes */
+        DevPtr pages;           /* root: pages the probe writes, if the column has no NULL */
+        bool direct_only = false; /* ... and the table is direct-mapped */
     };
     std::vector<OutRef> outs;
     bool need_b = false, need_p = false;
@@ -366,6 +432,8 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 oc.pages = mk; /* o.col.type == the probe key's type */
             } else {
                 oc.rid_a = o.from_build ? (mb ? mb->as<uint32_t>() : nullptr) : (mp ? mp->as<uint32_t>() : nullptr);
+                oc.pages = o.pages;
+                oc.direct_only = o.direct_only;
             }
             cols.push_back(oc);
             types.push_back(o.col.type);
@@ -373,7 +441,6 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
     };
     if (B.rows && P.rows) {
         const ColView bv = view(B, bk, nullptr);
-        const ColView pv = view(P, pk, nullptr);
         if (is_root) {
             /* The root's other output columns whose pages are already in
              * HBM are indexed (and decoded, if they must be) now, while the
@@ -389,27 +456,10 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         DevPtr dir, tuples, nlk, nlr, nlc, slots;
         int log2_slots = 0;
         bool inline_dir = true;
-        unsigned long long *d_params = &ctx.d_status->aux[0];
-        bool direct = false; /* direct-mapped table tried (the device decides) */
-        bool open = false;   /* open-addressing table tried (the device decides) */
-        DevPtr open_slots;
-        uint64_t open_n = 0;
-        /* Unique INT32 keys too spread out for the direct-mapped table: an
-         * open-addressing table (one slot walk per probe row, against a
-         * directory entry and a tuple range). Tried only after the
-         * direct-mapped table turned out unusable; a repeated key sends the
-         * join on to the hash table. */
-        auto build_open = [&]() -> bool {
-            if (bk.type != CJ_INT32 || B.rows > kOpenMaxRows) return false;
-            open_n = (std::max<uint64_t>(2 * B.rows, 1024) + 3) & ~3ull; /* groups of 4 slots */
-            open_slots = ctx.alloc(open_n * 8);
-            ck(cudaMemsetAsync(d_params + kOpenDup, 0, 8, ctx.stream), "memset");
-            KScope k(*this, "open_build");
-            ck(launch_open_build(L, bv, (uint32_t)B.rows, open_slots->as<unsigned long long>(), open_n,
-                                 d_params + kOpenDup),
-               "open_build");
-            return true;
-        };
+        bool unique = false; /* a table of unique keys tried (the device decides) */
+        const bool words_clear = join_words_clear;
+        join_words_clear = false; /* every join counts its matches there */
+        UniqueTable table{};
         auto build_hash = [&]() {
             BuildPlan bp;
             bp.num_rows = (uint32_t)B.rows;
@@ -448,32 +498,35 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             if (ctx.opt.dense_keys > 0) {
                 /* Unique keys spread over at most dense_keys x rows values get
                  * a direct-mapped table: one random access per probe row
-                 * instead of a directory entry and a tuple. The device works
-                 * out the key range and whether the table is usable; the
-                 * host learns it at the probe's own synchronisation and then,
-                 * if it was not, builds the hash table. */
-                /* 4 bytes per slot: at 8 x rows, 32 B per build row, against
-                 * about 16-24 B for the hash table, for one random access
-                 * per probe row instead of two; at most 2^28 slots (1 GiB) */
-                const uint64_t max_span = std::min<uint64_t>((uint64_t)ctx.opt.dense_keys * B.rows, 1ull << 28);
-                ck(cudaMemsetAsync(d_params, 0xFF, 8, ctx.stream), "memset");
-                ck(cudaMemsetAsync(d_params + 1, 0, (kDirectParams - 1) * 8, ctx.stream), "memset");
-                slots = ctx.alloc(max_span * 4);
-                KScope k(*this, "direct_build");
-                ck(launch_direct_build(L, bv, (uint32_t)B.rows, max_span, slots->as<uint32_t>(), d_params),
-                   "direct_build");
-                direct = true;
+                 * instead of a directory entry and a tuple; unique INT32 keys
+                 * that span more an open-addressing table: one sector. The
+                 * device works out the key range and which table it is, if
+                 * any; the host learns it at the probe's own synchronisation
+                 * and then, if neither, builds the hash table. Direct-mapped:
+                 * 4 bytes per slot, at 8 x rows 32 B per build row, at most
+                 * 2^28 slots (1 GiB); open-addressing: 16 B per build row.
+                 * One buffer serves both. */
+                table.max_span = std::min<uint64_t>((uint64_t)ctx.opt.dense_keys * B.rows, 1ull << 28);
+                if (bk.type == CJ_INT32 && B.rows <= kOpenMaxRows)
+                    table.open_slots = (uint32_t)std::max<uint64_t>(2 * B.rows, 1024);
+                table.params = ctx.d_status->table;
+                slots = ctx.alloc((std::max<uint64_t>(table.max_span * 4, table.open_slots * 8ull) + 15) & ~15ull);
+                table.slots = slots->ptr;
+                if (!words_clear) clear_join_words();
+                KScope k(*this, "unique_build");
+                ck(launch_unique_build(L, bv, (uint32_t)B.rows, table), "unique_build");
+                unique = true;
             }
-            if (!direct) build_hash();
+            if (!unique) build_hash();
         }
         /* Allocates the match outputs for `cap` pairs and launches the probe
          * of the table built above. */
         auto launch_probe = [&](uint64_t cap) {
-            mb = need_b ? ctx.alloc(cap * 4) : nullptr;
-            mp = need_p ? ctx.alloc(cap * 4) : nullptr;
             /* the key columns' result pages, sized for the capacity */
             const uint32_t key_rpp = rows_per_page_fixed(pk.type);
             mk = emit_keys ? ctx.alloc((cap + key_rpp - 1) / key_rpp * kPageSize) : nullptr;
+            mb = need_b ? ctx.alloc(cap * 4) : nullptr;
+            mp = need_p ? ctx.alloc(cap * 4) : nullptr;
             MatchOut mo;
             mo.build_rids = mb ? mb->as<uint32_t>() : nullptr;
             mo.probe_rids = mp ? mp->as<uint32_t>() : nullptr;
@@ -481,6 +534,48 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             mo.key_bytes = key_bytes;
             mo.capacity = collect ? cap : 0;
             mo.counter = &ctx.d_status->counter;
+            if (unique) {
+                /* The root's fixed-width columns whose pages are in HBM are
+                 * written by the probe itself where they hold no NULL; row
+                 * ids are collected for the others only. */
+                UniqueOut uo{};
+                uo.match = mo;
+                for (auto &o : outs) {
+                    if (!is_root || o.from_keys) continue;
+                    const auto it = decoded.find({o.col.input, o.col.col});
+                    if (o.col.type != CJ_VARCHAR && it != decoded.end() && it->second.ready && uo.n < kEmitColumns) {
+                        const uint32_t R = rows_per_page_fixed(o.col.type);
+                        o.pages = ctx.alloc((cap + R - 1) / R * kPageSize);
+                        o.direct_only = o.from_build && table.open_slots && table.open_slots * 8ull +
+                                                        it->second.src.num_pages * kPageSize > kEmitBesideOpen;
+                        uo.cols[uo.n++] = {view(*o.rel, o.col, nullptr), o.pages->as<uint8_t>(), o.from_build ? 1 : 0,
+                                           o.direct_only ? 1 : 0};
+                    } else {
+                        (o.from_build ? uo.need_b : uo.need_p) = true;
+                    }
+                }
+                if (!is_root) {
+                    uo.need_b = need_b;
+                    uo.need_p = need_p;
+                }
+                ProbeKey key{};
+                if (pk.vec < 0) {
+                    /* a scan: the probe reads the key's pages themselves */
+                    const Decoded &d = indexed(pk.input, pk.col);
+                    key.col = make_view(d, P, pk, nullptr);
+                    key.base = d.task.base;
+                    key.loc = d.task.loc;
+                    key.num_pages = d.src.num_pages;
+                    key.err = d.task.err;
+                } else {
+                    key.col = view(P, pk, nullptr);
+                }
+                PhaseScope ph(*this, PH_PROBE);
+                KScope k(*this, "probe_unique");
+                ck(launch_probe_unique(L, key, (uint32_t)P.rows, table, uo), "probe_unique");
+                return;
+            }
+            const ColView pv = view(P, pk, nullptr);
             DevPtr sched = ctx.alloc(probe_sched_bytes((uint32_t)P.rows));
             {
                 PhaseScope ph(*this, nl ? PH_NL : PH_PROBE);
@@ -489,16 +584,6 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                     ck(launch_nl_probe_tiles(L, pv, (uint32_t)P.rows, nlk->as<int64_t>(), nlr->as<uint32_t>(),
                                              nlc->as<uint32_t>(), mo, sched->ptr),
                        "nl_probe");
-                } else if (open) {
-                    KScope k(*this, "probe_open");
-                    ck(launch_probe_tiles_open(L, pv, (uint32_t)P.rows, open_slots->as<unsigned long long>(), open_n,
-                                               d_params + kOpenDup, mo, sched->ptr),
-                       "probe_open");
-                } else if (direct) {
-                    KScope k(*this, "probe_array");
-                    ck(launch_probe_tiles_array(L, pv, (uint32_t)P.rows, slots->as<uint32_t>(), d_params, mo,
-                                                sched->ptr),
-                       "probe_array");
                 } else {
                     KScope k(*this, "probe_hash");
                     ck(launch_probe_tiles_hash(probe_launch(ctx, P.rows), pv, (uint32_t)P.rows, bk.type,
@@ -508,67 +593,63 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 }
             }
         };
-        /* keys too spread out (aux[3] = 1) or a key repeats (2): the
-         * direct-mapped table is unusable (its probe did nothing); an
-         * open-addressing table for spread-out keys, else the hash table */
-        auto replace_direct = [&]() {
-            direct = false;
+        /* The device refused the table of unique keys (its probe did
+         * nothing): the hash table. */
+        auto replace_unique = [&]() {
+            unique = false;
             slots.reset();
+            for (auto &o : outs) o.pages.reset();
             PhaseScope ph(*this, PH_BUILD);
-            open = ctx.h_status->aux[3] == 1 && build_open();
-            if (!open) build_hash();
+            build_hash();
+        };
+        auto count_join = [&]() {
+            const int kind = table_kind(ctx.h_status->table, table.open_slots);
+            stats.num_direct_joins += kind == 1;
+            stats.num_open_joins += kind == 2;
         };
         uint64_t cap = P.rows;
         bool all_fixed = true;
         for (const auto &o : outs) all_fixed &= o.col.type != CJ_VARCHAR;
-        if (is_root && direct && collect && all_fixed && (flags & CJ_EXEC_RESULT_ON_DEVICE) && ctx.opt.defer_count) {
+        if (is_root && unique && collect && all_fixed && (flags & CJ_EXEC_RESULT_ON_DEVICE) && ctx.opt.defer_count) {
             /* Unique build keys at the root, result left in HBM, no VARCHAR
              * output: at most one match per probe row, so the result is sized
              * for P.rows and its pages are written with the match count read
              * on the device. The execution's one host synchronisation comes
-             * last; only if the device refused the direct-mapped table does
-             * the join go on as below. */
+             * last; only if the device refused the table does the join go on
+             * as below. */
             launch_probe(cap);
             std::vector<OutCol> cols;
             std::vector<int32_t> types;
             root_columns(cols, types);
             std::unique_ptr<cj_result> r(materialize(cols, types, cap, &ctx.d_status->counter));
             sync();
-            if (!ctx.h_status->aux[3]) {
+            if (table_kind(ctx.h_status->table, table.open_slots)) {
                 M = ctx.h_status->counter;
                 finish_counted(*r, M);
-                stats.num_direct_joins++;
+                count_join();
                 stats.matches += M;
                 synced_last = true;
                 *out = r.release();
                 return Relation{};
             }
             r.reset();
-            replace_direct();
+            replace_unique();
         }
         for (;;) {
             launch_probe(cap);
             sync();
-            if (direct && ctx.h_status->aux[3]) {
-                replace_direct();
-                continue;
-            }
-            if (open && ctx.h_status->aux[kOpenDup]) {
-                /* a key repeats: the probe did nothing; hash table */
-                open = false;
-                open_slots.reset();
-                PhaseScope ph(*this, PH_BUILD);
-                build_hash();
+            if (unique && !table_kind(ctx.h_status->table, table.open_slots)) {
+                replace_unique();
                 continue;
             }
             M = ctx.h_status->counter;
             if (M <= cap || !collect) break;
+            if (unique) fail(CJ_ERR_INTERNAL, "more matches than probe rows over unique keys");
             if (M > 0xFFFFFFFFull) fail(CJ_ERR_LIMIT, "join result exceeds 2^32-1 rows");
             stats.probe_reruns++;
             cap = M;
         }
-        if (direct) stats.num_direct_joins++;
-        if (open) stats.num_open_joins++;
+        if (unique) count_join();
     }
     if (M > 0xFFFFFFFFull) fail(CJ_ERR_LIMIT, "join result exceeds 2^32-1 rows");
     stats.matches += M;
@@ -735,8 +816,10 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
                 /* values already in place: headers and bitmaps, once per
                  * shared page array */
                 res->dev_pages[c] = cols[c].pages;
-                t.col.type = types[c];
-                t.finish = 1;
+                if (cols[c].rel) t.col = out_view(cols[c]);
+                else t.col.type = types[c];
+                t.finish = cols[c].rel ? 2 : 1;
+                t.table = cols[c].direct_only ? ctx.d_status->table : nullptr;
             } else {
                 /* decoded here, not before the loop: the kernel stream waits
                  * for a column's upload only when its pages are written */

@@ -50,6 +50,8 @@ struct Decoded {
     DevPtr own_state;                   /* the state, unless the status block's */
     ColumnState *state = nullptr;       /* COL_* flags and errors (device)    */
     int status_col = -1;                /* its place in the status block      */
+    bool ready = false;                 /* values / valid / desc written      */
+    ColumnTask task{};
 };
 
 /* Allocates a column's arrays and describes its index and decode. `state`
@@ -80,6 +82,7 @@ inline ColumnTask column_task(Context &ctx, Decoded &d, ColumnState *state) {
     t.desc = d.desc ? d.desc->as<uint64_t>() : nullptr;
     t.valid = d.valid->as<uint32_t>();
     t.type = d.type;
+    d.task = t;
     return t;
 }
 

@@ -278,11 +278,11 @@ class Filter {
             check_cuda(scan_u32_to_u64(L, cnt->as<uint32_t>(), off->as<uint64_t>(), words, tmp->ptr), "scan");
             /* the count goes back with the status block (sync_status copies
              * all of it to the host) */
-            check_cuda(cudaMemcpyAsync(&ctx.d_status->aux[7], off->as<uint64_t>() + words, 8,
+            check_cuda(cudaMemcpyAsync(&ctx.d_status->aux, off->as<uint64_t>() + words, 8,
                                        cudaMemcpyDeviceToDevice, ctx.stream),
                        "copy");
             ctx.sync_status();
-            count = ctx.h_status->aux[7];
+            count = ctx.h_status->aux;
             sel = ctx.alloc(std::max<uint64_t>(count, 1) * 4);
             k_word_emit<<<grid_for(ctx, words, 256), 256, 0, ctx.stream>>>(bits->as<uint32_t>(), off->as<uint64_t>(),
                                                                              words, sel->as<uint32_t>());
@@ -312,10 +312,10 @@ class Filter {
                 } else {
                     DevPtr temp = ctx.alloc(varchar_temp_bytes(count, TR));
                     check_cuda(launch_varchar_plan(L, v, count, TR, temp->ptr,
-                                                   reinterpret_cast<unsigned long long *>(&ctx.d_status->aux[7])),
+                                                   reinterpret_cast<unsigned long long *>(&ctx.d_status->aux)),
                                "varchar_plan");
-                    ctx.sync_status(); /* brings the page count back in aux[7] */
-                    cp.num_pages = ctx.h_status->aux[7];
+                    ctx.sync_status(); /* brings the page count back in aux */
+                    cp.num_pages = ctx.h_status->aux;
                     cp.owner = ctx.alloc(cp.num_pages * kPageSize);
                     check_cuda(launch_varchar_write(L, v, count, TR, temp->ptr, cp.owner->as<uint8_t>()),
                                "varchar_write");

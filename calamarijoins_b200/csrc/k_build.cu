@@ -448,7 +448,8 @@ cudaError_t build_impl(const Launch &L, const BuildPlan &bp, const ColView &key,
     return cudaGetLastError();
 }
 
-/* ---- direct-mapped table (unique keys over a dense range) ---- */
+/* ---- direct-mapped tables of a batch (unique keys over a dense range; a
+ * plan by itself: k_unique.cu) ---- */
 CJ_DEV unsigned long long warp_min_u64(unsigned long long v) {
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, d));
@@ -498,47 +499,6 @@ CJ_DEV void key_range_rows(const ColView &key, uint64_t i0, uint64_t i1, uint64_
             atomicMax(range + 1, mx);
             atomicAdd(range + 2, (unsigned long long)cnt);
         }
-    }
-}
-
-__global__ void __launch_bounds__(kBuildThreads)
-    k_key_range(ColView key, uint32_t n, unsigned long long *range) {
-    key_range_rows(key, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, n, (uint64_t)gridDim.x * blockDim.x,
-                   range);
-}
-
-/* params: [0] min ^ 2^63, [1] max ^ 2^63, [2] count (from k_key_range),
- * [3] unusable (1: span too wide, 2: a key repeats), [4] lo, [5] span. */
-__global__ void k_array_prep(unsigned long long *p, uint64_t max_span) {
-    if (p[2] == 0) return; /* no non-NULL key: span 0, nothing matches */
-    const unsigned long long width = p[1] - p[0]; /* max - min: the bias cancels */
-    if (width >= max_span) {
-        p[3] = 1ull;
-        return;
-    }
-    if (p[2] > width + 1) { /* more keys than values in their range: one repeats */
-        p[3] = 2ull;
-        return;
-    }
-    p[4] = p[0] ^ (1ull << 63);
-    p[5] = width + 1;
-}
-
-__global__ void k_array_fill(uint32_t *__restrict__ slots, const unsigned long long *p) {
-    const uint64_t span = p[5];
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < span; i += (uint64_t)gridDim.x * blockDim.x)
-        slots[i] = kArrayEmpty;
-}
-
-__global__ void k_array_build(ColView key, uint32_t n, uint32_t *__restrict__ slots, unsigned long long *p) {
-    if (p[3]) return;
-    const uint64_t lo = p[4], span = p[5];
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        int64_t k;
-        if (!load_key(key, (uint32_t)i, &k)) continue;
-        const uint64_t off = (uint64_t)k - lo;
-        if (off >= span) continue; /* cannot happen: lo and span come from these keys */
-        if (atomicCAS(slots + off, kArrayEmpty, (uint32_t)i) != kArrayEmpty) p[3] = 2ull; /* a key repeats */
     }
 }
 
@@ -611,44 +571,6 @@ __global__ void __launch_bounds__(kBuildThreads)
         const uint64_t off = (uint64_t)k - lo;
         if (off >= span) continue;
         if (atomicCAS(T.slots + off, kArrayEmpty, (uint32_t)i) != kArrayEmpty) p[3] = 2ull;
-    }
-}
-
-/* ---- open-addressing table (unique INT32 keys, any spread) ---- */
-constexpr unsigned long long kOpenEmpty = ~0ull; /* row 2^32-1 never exists */
-
-__global__ void k_open_fill(unsigned long long *__restrict__ slots, uint64_t nslots) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < nslots;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        slots[i] = kOpenEmpty;
-}
-
-/* Each non-NULL key claims the first empty slot from its hash on (at most
- * half the slots fill, so a free one is always found); meeting its own key
- * on the way means the key repeats. A slot is read before it is CASed
- * (slots only go from empty to full, so a full one read from L2 is final):
- * the copies of a heavily repeated key see it taken without hammering one
- * address with atomics, and once a repeat is flagged every thread stops. */
-__global__ void k_open_insert(ColView key, uint32_t n, unsigned long long *__restrict__ slots, uint32_t nslots,
-                              unsigned long long *dup) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-        if (*reinterpret_cast<volatile unsigned long long *>(dup)) return;
-        int64_t k;
-        if (!load_key(key, (uint32_t)i, &k)) continue;
-        const unsigned long long v = ((unsigned long long)(uint32_t)k << 32) | (unsigned long long)i;
-        uint32_t h = open_slot(k, nslots);
-        for (uint32_t step = 0; step < nslots; ++step) {
-            unsigned long long cur = __ldcg(slots + h);
-            if (cur == kOpenEmpty) {
-                cur = atomicCAS(slots + h, kOpenEmpty, v);
-                if (cur == kOpenEmpty) break;
-            }
-            if ((uint32_t)(cur >> 32) == (uint32_t)k) {
-                *dup = 1ull;
-                break;
-            }
-            if (++h == nslots) h = 0;
-        }
     }
 }
 
@@ -734,21 +656,6 @@ size_t build_grouped_temp_bytes(uint64_t total_cells) {
     return align256(total_cells * 4) + align256((total_cells + 1) * 8) + scan_temp_bytes(total_cells) + 256;
 }
 
-cudaError_t launch_direct_build(const Launch &L, const ColView &key, uint32_t n, uint64_t max_span, uint32_t *slots,
-                                unsigned long long *params) {
-    if (n == 0) return cudaSuccess;
-    uint64_t g = ((uint64_t)n + kBuildThreads * 8 - 1) / (kBuildThreads * 8);
-    g = std::min<uint64_t>(std::max<uint64_t>(g, 1), (uint64_t)L.num_sms * 8);
-    k_key_range<<<(unsigned)g, kBuildThreads, 0, L.stream>>>(key, n, params);
-    k_array_prep<<<1, 1, 0, L.stream>>>(params, max_span);
-    g = std::min<uint64_t>(std::max<uint64_t>((max_span + 255) / 256, 1), (uint64_t)L.num_sms * 8);
-    k_array_fill<<<(unsigned)g, 256, 0, L.stream>>>(slots, params);
-    g = std::min<uint64_t>(((uint64_t)n + 255) / 256, (uint64_t)L.num_sms * 8);
-    k_array_build<<<(unsigned)g, 256, 0, L.stream>>>(key, n, slots, params);
-    count_launches(4);
-    return cudaGetLastError();
-}
-
 cudaError_t launch_direct_build_grouped(const Launch &L, const DirectTask *tasks_dev, uint32_t ntasks,
                                         uint32_t total_key_blocks, uint32_t total_fill_blocks) {
     if (!ntasks) return cudaSuccess;
@@ -757,17 +664,6 @@ cudaError_t launch_direct_build_grouped(const Launch &L, const DirectTask *tasks
     if (total_fill_blocks) k_array_fill_grouped<<<total_fill_blocks, kBuildThreads, 0, L.stream>>>(tasks_dev, ntasks);
     if (total_key_blocks) k_array_build_grouped<<<total_key_blocks, kBuildThreads, 0, L.stream>>>(tasks_dev, ntasks);
     count_launches(4);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_open_build(const Launch &L, const ColView &key, uint32_t n, unsigned long long *slots,
-                              uint64_t nslots, unsigned long long *dup) {
-    if (nslots < 2ull * n || nslots > 0xFFFFFFFFull) return cudaErrorInvalidValue; /* free slots; u32 indices */
-    uint64_t g = std::min<uint64_t>(std::max<uint64_t>((nslots + 255) / 256, 1), (uint64_t)L.num_sms * 8);
-    k_open_fill<<<(unsigned)g, 256, 0, L.stream>>>(slots, nslots);
-    g = std::min<uint64_t>(std::max<uint64_t>(((uint64_t)n + 255) / 256, 1), (uint64_t)L.num_sms * 8);
-    k_open_insert<<<(unsigned)g, 256, 0, L.stream>>>(key, n, slots, (uint32_t)nslots, dup);
-    count_launches(2);
     return cudaGetLastError();
 }
 

@@ -194,24 +194,28 @@ CJ_DEV uint64_t live_rows(uint64_t rows, const unsigned long long *rows_dev) {
 }
 
 /* Finishes a page whose values are in place (a NULL-free column written by
- * the probe): header, zero gap after the values, bitmap of nr ones. */
+ * the probe): header, zero gap after the values, bitmap of nr ones. One warp
+ * per page, whole words (byte by byte by a block per page: 54 us for the
+ * 110,000 pages of a 43.9M-row result). */
 template <typename T> CJ_DEV void finish_dense_page(uint8_t *__restrict__ pages, uint64_t rows, uint64_t pg) {
     constexpr uint32_t R = sizeof(T) == 4 ? kRowsPerPageInt32 : kRowsPerPage8B;
     constexpr uint32_t DB = sizeof(T) == 4 ? 4u : 8u;
-    uint8_t *dst = pages + pg * kPageSize;
+    uint32_t *dst = reinterpret_cast<uint32_t *>(pages + pg * kPageSize);
     const uint32_t nr = (uint32_t)min((uint64_t)R, rows - pg * R);
-    if (threadIdx.x == 0) {
-        if (DB == 8) __stcs(reinterpret_cast<unsigned long long *>(dst), (unsigned long long)nr * 0x10001ull);
-        else __stcs(reinterpret_cast<unsigned int *>(dst), nr * 0x10001u);
-    }
-    const uint32_t bm_bytes = (nr + 7) / 8, bm0 = kPageSize - bm_bytes;
-    for (uint32_t b = DB + nr * (uint32_t)sizeof(T) + threadIdx.x; b < kPageSize; b += blockDim.x) {
-        uint8_t v = 0;
-        if (b >= bm0) {
-            const uint32_t i = b - bm0;
-            v = (i + 1) * 8 <= nr ? 0xFFu : (uint8_t)((1u << (nr - i * 8)) - 1u);
+    if (lane_id() < DB / 4) __stcs(dst + lane_id(), lane_id() == 0 ? nr * 0x10001u : 0u);
+    const uint32_t bm0 = kPageSize - (nr + 7) / 8;
+    for (uint32_t k = (DB + nr * (uint32_t)sizeof(T)) / 4 + lane_id(); k < kPageSize / 4; k += 32) {
+        uint32_t v = 0;
+        if (4 * k >= bm0 && (4 * k + 4 - bm0) * 8 <= nr) {
+            v = ~0u;
+        } else if (4 * k + 4 > bm0) {
+            for (uint32_t j = 0; j < 4; ++j) {
+                if (4 * k + j < bm0) continue;
+                const uint32_t i = 4 * k + j - bm0;
+                v |= ((i + 1) * 8 <= nr ? 0xFFu : (1u << (nr - i * 8)) - 1u) << (8 * j);
+            }
         }
-        dst[b] = v;
+        __stcs(dst + k, v);
     }
 }
 
@@ -224,8 +228,10 @@ CJ_DEV void write_page_blocks(const PageTask &T, uint32_t b, PageSmem &sm) {
     const uint32_t R = rows_per_page_dev(T.col.type);
     const uint64_t num_pages = (rows + R - 1) / R;
     if (b >= num_pages) return;
-    if (T.finish) {
-        for (uint64_t pg = b; pg < num_pages; pg += T.blocks) {
+    if (T.finish == 1 ||
+        (T.finish == 2 && col_null_free(T.col) && !(T.table && T.table[kTableRefused] == kTableSpread))) {
+        constexpr uint32_t kWarps = kMatThreads / 32;
+        for (uint64_t pg = b * kWarps + (threadIdx.x >> 5); pg < num_pages; pg += (uint64_t)T.blocks * kWarps) {
             if (T.col.type == CJ_INT32) finish_dense_page<int32_t>(T.out, rows, pg);
             else finish_dense_page<long long>(T.out, rows, pg);
         }

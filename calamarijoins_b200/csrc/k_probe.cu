@@ -252,67 +252,6 @@ template <int kItemsT> struct ArrayMatcherT {
     }
 };
 
-/* One light chain per row: 4 rows per thread fit 32 registers (387 us vs
- * 434 us for 2 on 64M probe rows). The grouped kernel's tiles are 2 rows
- * per thread for every matcher (ArrayMatcherT<kProbeItems>). */
-using ArrayMatcher = ArrayMatcherT<4>;
-
-/* Open-addressing table of unique INT32 keys (launch_open_build): walk the
- * slots from the key's hash until the key or an empty slot. The walk reads
- * the aligned group of four slots (one 32-byte sector) around its position
- * with two independent 16-byte loads and examines the group's slots from
- * there on, so most rows are answered by one round trip instead of one per
- * slot (the slot count is a multiple of 4: a group never runs past the
- * end). */
-struct OpenMatcher {
-    static constexpr bool kAtMostOne = true; /* unique keys */
-    static constexpr bool kHeavy = false;
-    static constexpr int kItems = 4;
-    static constexpr int kMinBlocks = kProbeMinBlocks;
-    const unsigned long long *slots;
-    uint32_t nslots; /* < 2^32 and a multiple of 4 (launch_probe_tiles_open checks) */
-    const unsigned long long *dup;
-    struct Shared {
-        uint32_t unused;
-    };
-    CJ_DEV bool skip() const { return *dup != 0ull; }
-    CJ_DEV OpenMatcher resolved() const { return *this; }
-    CJ_DEV void init(Shared &) const {}
-    CJ_DEV uint32_t count(const Shared &, int64_t key, uint32_t &first) const {
-        if (key != (int64_t)(int32_t)key) return 0; /* no INT32 build key equals it */
-        const uint32_t k32 = (uint32_t)(int32_t)key;
-        uint32_t h = open_slot(key, nslots);
-        for (uint32_t step = 0; step < nslots;) {
-            const uint32_t g0 = h & ~3u;
-            const ulonglong2 *grp = reinterpret_cast<const ulonglong2 *>(slots + g0);
-            const ulonglong2 a = __ldg(grp), b = __ldg(grp + 1);
-#pragma unroll
-            for (uint32_t q = 0; q < 4; ++q) {
-                if (q < (h & 3u)) continue;
-                const unsigned long long v = q == 0 ? a.x : q == 1 ? a.y : q == 2 ? b.x : b.y;
-                if (v == ~0ull) return 0;
-                if ((uint32_t)(v >> 32) == k32) {
-                    first = (uint32_t)v;
-                    return 1;
-                }
-                ++step;
-            }
-            h = g0 + 4;
-            if (h >= nslots) h = 0;
-        }
-        return 0;
-    }
-    CJ_DEV void write_all(const Shared &sh, int64_t key, unsigned long long pos, uint32_t prow,
-                          const MatchOut &out) const {
-        uint32_t r;
-        if (count(sh, key, r) && pos < out.capacity) {
-            if (out.build_rids) out.build_rids[pos] = r;
-            if (out.probe_rids) out.probe_rids[pos] = prow;
-            put_key(out, pos, key);
-        }
-    }
-};
-
 struct LoopMatcher {
     static constexpr bool kAtMostOne = false;
     static constexpr bool kHeavy = false;
@@ -646,20 +585,6 @@ cudaError_t launch_probe_tiles_hash(const Launch &L, const ColView &pkey, uint32
         return run_tiles(L, pkey, n_probe, m, out, sched_mem);
     }
     HashMatcher<int64_t> m{{dir, reinterpret_cast<const Tuple<int64_t> *>(tuples), log2_slots}, bloom};
-    return run_tiles(L, pkey, n_probe, m, out, sched_mem);
-}
-
-cudaError_t launch_probe_tiles_array(const Launch &L, const ColView &pkey, uint32_t n_probe, const uint32_t *slots,
-                                     const unsigned long long *params, const MatchOut &out, void *sched_mem) {
-    ArrayMatcher m{slots, params};
-    return run_tiles(L, pkey, n_probe, m, out, sched_mem);
-}
-
-cudaError_t launch_probe_tiles_open(const Launch &L, const ColView &pkey, uint32_t n_probe,
-                                    const unsigned long long *slots, uint64_t nslots,
-                                    const unsigned long long *dup, const MatchOut &out, void *sched_mem) {
-    if (nslots > 0xFFFFFFFFull || nslots % 4 || reinterpret_cast<uintptr_t>(slots) % 16) return cudaErrorInvalidValue;
-    OpenMatcher m{slots, (uint32_t)nslots, dup};
     return run_tiles(L, pkey, n_probe, m, out, sched_mem);
 }
 

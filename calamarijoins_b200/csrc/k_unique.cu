@@ -1,0 +1,658 @@
+/*
+ * k_unique.cu — joins over unique build keys: the table's build and a probe
+ * that reads the key column's pages and writes the result's pages.
+ *
+ * The table (launch_unique_build) is direct-mapped when the keys lie densely
+ * (slots[key - lo] = build row), else, for INT32 keys, open-addressing
+ * (8-byte slots key << 32 | build row, linear probing from the key's hash,
+ * at most half full). Which one, and whether the keys are unique at all, is
+ * decided on the device: `params` says so to the kernels that follow and,
+ * at the next synchronisation, to the host. Both kinds share one buffer.
+ *
+ * The probe (k_probe_unique) takes up to 2,048 probe rows per CTA and step:
+ * a page of the key column when the probe side is a scan (NULLs resolved
+ * from the page's own bitmap: no decoded copy of the column is written or
+ * read back), else 2,048 rows of an intermediate. A lane has eight
+ * independent rows: their keys are all requested before any is used, then
+ * all their slots, then (for a result column without NULLs) their values.
+ * One atomicAdd per step places the matches, and the values of the root's
+ * fixed-width columns without NULLs go straight to their places in the
+ * result pages: no match row ids are written and read back for them.
+ * Columns with NULLs (known on the device only) get their row ids and are
+ * written by k_write_pages.
+ *
+ * Bound: requests from L1 to L2, about one per clock and SM whatever their
+ * size (every random slot or value is one), then the 128-byte lines of L1
+ * that the requests in flight hold. 64M x 4M rows, 43.9M matches, two
+ * 8-byte result columns, direct-mapped: 605 us, where decode, probe and
+ * page writers took 945 us (152 + 390 + 403).
+ */
+#include <algorithm>
+#include <atomic>
+
+#include "cj_device.cuh"
+
+namespace cj {
+namespace {
+
+constexpr unsigned long long kOpenEmpty = ~0ull; /* row 2^32-1 never exists */
+
+/* ---------------- build ---------------- */
+constexpr int kUniqueThreads = 256;
+constexpr int kUniqueRows = 4; /* build rows a thread has in flight */
+
+/* Smallest / largest key (as unsigned order: XOR 2^63; the smallest as its
+ * complement, so that zeroed words are the identity) and count of the
+ * non-NULL keys, folded over the block into p[0..2]. */
+CJ_DEV void fold_range(const ColView &key, uint64_t first, uint64_t n, uint64_t stride, unsigned long long *p) {
+    __shared__ unsigned long long s_lo[32], s_hi[32];
+    __shared__ uint32_t s_cnt[32];
+    unsigned long long lo = 0, hi = 0;
+    uint32_t cnt = 0;
+    for (uint64_t i0 = first; i0 < n; i0 += stride * kUniqueRows) {
+        int64_t k[kUniqueRows];
+        bool v[kUniqueRows];
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) {
+            const uint64_t i = i0 + q * stride;
+            v[q] = i < n && load_key(key, (uint32_t)i, &k[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q)
+            if (v[q]) {
+                const unsigned long long b = (unsigned long long)k[q] ^ (1ull << 63);
+                lo = max(lo, ~b);
+                hi = max(hi, b);
+                ++cnt;
+            }
+    }
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) {
+        lo = max(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+    }
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    const uint32_t warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+    if (lane_id() == 0) {
+        s_lo[warp] = lo;
+        s_hi[warp] = hi;
+        s_cnt[warp] = cnt;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        lo = lane_id() < nwarps ? s_lo[lane_id()] : 0;
+        hi = lane_id() < nwarps ? s_hi[lane_id()] : 0;
+        cnt = lane_id() < nwarps ? s_cnt[lane_id()] : 0;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) {
+            lo = max(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+            hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+        }
+        cnt = __reduce_add_sync(0xffffffffu, cnt);
+        if (lane_id() == 0 && cnt) {
+            atomicMax(p, lo);
+            atomicMax(p + 1, hi);
+            atomicAdd(p + 2, (unsigned long long)cnt);
+        }
+    }
+}
+
+/* Reads the folded range (from L2: other blocks wrote it) and decides. */
+CJ_DEV void decide_table(unsigned long long *p, uint64_t max_span) {
+    const unsigned long long cnt = __ldcg(p + 2);
+    if (cnt == 0) return; /* no non-NULL key: span 0, nothing matches */
+    const unsigned long long b = ~__ldcg(p), width = __ldcg(p + 1) - b; /* max - min: the bias cancels */
+    if (width >= max_span) p[kTableRefused] = kTableSpread;
+    else if (cnt > width + 1) p[kTableRefused] = kTableRepeats; /* more keys than values in their range */
+    p[kTableLo] = b ^ (1ull << 63);
+    p[kTableSpan] = width + 1;
+}
+
+/* Empty slots are all ones in either kind of table. */
+CJ_DEV uint64_t table_bytes(const UniqueTable &t) {
+    const unsigned long long refused = t.params[kTableRefused];
+    if (refused == kTableSpread) return t.open_slots * 8ull;
+    return refused ? 0ull : t.params[kTableSpan] * 4ull;
+}
+CJ_DEV void fill_table(const UniqueTable &t, uint64_t first, uint64_t stride) {
+    const uint64_t bytes = table_bytes(t), n16 = (bytes + 15) / 16; /* the buffer is a multiple of 16 bytes */
+    const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
+    for (uint64_t i = first; i < n16; i += stride) reinterpret_cast<uint4 *>(t.slots)[i] = ones;
+}
+
+/* Each key claims its slot; meeting its own key there means that the keys
+ * repeat, and the table cannot be used. kUniqueRows rows per thread and
+ * step, their compare-and-swaps all in flight together. */
+CJ_DEV void insert_rows(const ColView &key, const UniqueTable &t, uint64_t first, uint64_t n, uint64_t stride) {
+    const unsigned long long refused = t.params[kTableRefused];
+    if (refused == 0) {
+        uint32_t *slots = reinterpret_cast<uint32_t *>(t.slots);
+        const uint64_t lo = t.params[kTableLo], span = t.params[kTableSpan];
+        for (uint64_t i0 = first; i0 < n; i0 += stride * kUniqueRows) {
+            uint64_t off[kUniqueRows];
+#pragma unroll
+            for (int q = 0; q < kUniqueRows; ++q) {
+                const uint64_t i = i0 + q * stride;
+                int64_t k;
+                off[q] = i < n && load_key(key, (uint32_t)i, &k) ? (uint64_t)k - lo : ~0ull;
+            }
+            uint32_t was[kUniqueRows];
+#pragma unroll
+            for (int q = 0; q < kUniqueRows; ++q)
+                was[q] = off[q] < span ? atomicCAS(slots + off[q], kArrayEmpty, (uint32_t)(i0 + q * stride))
+                                       : kArrayEmpty;
+            bool dup = false;
+#pragma unroll
+            for (int q = 0; q < kUniqueRows; ++q) dup |= was[q] != kArrayEmpty;
+            if (dup) t.params[kTableDup] = 1ull;
+        }
+        return;
+    }
+    if (refused != kTableSpread || !t.open_slots) return;
+    unsigned long long *slots = reinterpret_cast<unsigned long long *>(t.slots);
+    for (uint64_t i = first; i < n; i += stride) {
+        /* a repeat is flagged once; every thread then stops */
+        if (*reinterpret_cast<volatile unsigned long long *>(t.params + kTableDup)) return;
+        int64_t k;
+        if (!load_key(key, (uint32_t)i, &k)) continue;
+        const unsigned long long v = ((unsigned long long)(uint32_t)k << 32) | (unsigned long long)i;
+        uint32_t h = open_slot(k, t.open_slots);
+        for (uint32_t step = 0; step < t.open_slots; ++step) {
+            unsigned long long cur = __ldcg(slots + h); /* slots only fill: a full one is final */
+            if (cur == kOpenEmpty) {
+                cur = atomicCAS(slots + h, kOpenEmpty, v);
+                if (cur == kOpenEmpty) break;
+            }
+            if ((uint32_t)(cur >> 32) == (uint32_t)k) {
+                t.params[kTableDup] = 1ull;
+                break;
+            }
+            if (++h == t.open_slots) h = 0;
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kUniqueThreads)
+    k_unique_range(ColView key_arg, uint32_t n, UniqueTable t) {
+    const ColView key = resolve_view(key_arg);
+    fold_range(key, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, n, (uint64_t)gridDim.x * blockDim.x, t.params);
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(t.params + kTableDone, 1ull) == gridDim.x - 1) {
+            __threadfence();
+            decide_table(t.params, t.max_span);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kUniqueThreads) k_unique_fill(UniqueTable t) {
+    fill_table(t, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, (uint64_t)gridDim.x * blockDim.x);
+}
+
+__global__ void __launch_bounds__(kUniqueThreads)
+    k_unique_insert(ColView key_arg, uint32_t n, UniqueTable t) {
+    const ColView key = resolve_view(key_arg);
+    insert_rows(key, t, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, n, (uint64_t)gridDim.x * blockDim.x);
+}
+
+/* A small build side: the three passes by one block, one launch. */
+constexpr int kSmallThreads = 1024;
+constexpr uint32_t kSmallRows = 8192;
+__global__ void __launch_bounds__(kSmallThreads)
+    k_unique_small(ColView key_arg, uint32_t n, UniqueTable t) {
+    const ColView key = resolve_view(key_arg);
+    fold_range(key, threadIdx.x, n, kSmallThreads, t.params);
+    __syncthreads();
+    if (threadIdx.x == 0) decide_table(t.params, t.max_span);
+    __syncthreads();
+    fill_table(t, threadIdx.x, kSmallThreads);
+    __syncthreads();
+    insert_rows(key, t, threadIdx.x, n, kSmallThreads);
+}
+
+/* ---------------- probe ---------------- */
+/* 256 threads, 48 registers and 10 KB of shared memory: five CTAs per SM.
+ * Measured at 64M x 4M rows (probe alone): five 605 us, four with 64
+ * registers 619, six with 40 (spills) 620. */
+constexpr int kProbeBlocks = 5;
+constexpr int kItems = 8;                              /* rows per lane and step       */
+constexpr int kProbeThreads = 2048 / kItems;
+constexpr int kParts = kProbeThreads / 32;
+constexpr uint32_t kWarpRows = 32 * kItems;            /* 256                          */
+constexpr uint32_t kTileRows = kWarpRows * kProbeThreads / 32; /* 2048: a full page */
+
+/* A row's key as the table sees it (direct-mapped: key - lo; open
+ * addressing: the key's 32 bits), its build row (kArrayEmpty: no match).
+ * For INT32 probe keys the table's range is cut to INT32's first, so that a
+ * 32-bit difference says all. */
+template <typename T> struct DirectLookup {
+    const uint32_t *slots;
+    int64_t lo;
+    uint32_t span; /* at most 2^28 */
+    CJ_DEV DirectLookup(const UniqueTable &t) {
+        slots = reinterpret_cast<const uint32_t *>(t.slots);
+        lo = (int64_t)t.params[kTableLo];
+        span = (uint32_t)t.params[kTableSpan];
+        if constexpr (sizeof(T) == 4) {
+            const int64_t first = max(lo, (int64_t)INT32_MIN), end = min(lo + (int64_t)span, (int64_t)INT32_MAX + 1);
+            span = end > first ? (uint32_t)(end - first) : 0u;
+            if (span) slots += first - lo;
+            lo = first;
+        }
+    }
+    static constexpr bool kMask = false; /* a code says by itself whether it may be in the table */
+    CJ_DEV uint32_t code(T key, bool present, bool *in) const {
+        *in = true;
+        uint32_t c;
+        if constexpr (sizeof(T) == 4) {
+            c = (uint32_t)key - (uint32_t)lo;
+        } else {
+            const uint64_t off = (uint64_t)key - (uint64_t)lo; /* keys below lo wrap past span */
+            c = off < span ? (uint32_t)off : ~0u;
+        }
+        return present ? c : ~0u;
+    }
+    CJ_DEV T key_of(uint32_t c) const { return (T)(lo + c); }
+    CJ_DEV void find(const uint32_t *c, uint32_t, uint32_t *rid) const {
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            rid[it] = kArrayEmpty;
+            if (c[it] < span) rid[it] = __ldg(slots + c[it]);
+        }
+    }
+};
+
+/* Open addressing: the first slots of all of a lane's rows in flight
+ * together, then slot by slot (a neighbour is mostly in the sector that just
+ * came) until the key or an empty slot. Keys outside the build keys' range
+ * are not looked up at all. The bound is the requests that L1 sends out,
+ * about one per clock and SM: reading the slot's aligned 32 bytes at once
+ * took 858 us where this takes 797 (64M rows, without the range), whatever
+ * the table's size between 1.3 and 2 slots a row. */
+template <typename T> struct OpenLookup {
+    const unsigned long long *slots;
+    uint32_t nslots, lo, width; /* of the INT32 build keys */
+    CJ_DEV OpenLookup(const UniqueTable &t)
+        : slots(reinterpret_cast<const unsigned long long *>(t.slots)), nslots(t.open_slots),
+          lo((uint32_t)t.params[kTableLo]), width((uint32_t)(t.params[kTableSpan] - 1)) {}
+    static constexpr bool kMask = true;
+    CJ_DEV uint32_t code(T key, bool present, bool *in) const {
+        /* an INT64 key that is no INT32 value equals no build key */
+        *in = present && key == (T)(int32_t)key && (uint32_t)key - lo <= width;
+        return (uint32_t)key;
+    }
+    CJ_DEV T key_of(uint32_t c) const { return (T)(int32_t)c; }
+    CJ_DEV void find(const uint32_t *c, uint32_t ok, uint32_t *rid) const {
+        unsigned long long v[kItems];
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            v[it] = kOpenEmpty;
+            if ((ok >> it) & 1u) v[it] = __ldg(slots + open_slot((int64_t)(int32_t)c[it], nslots));
+        }
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            rid[it] = kArrayEmpty;
+            uint32_t h = open_slot((int64_t)(int32_t)c[it], nslots);
+            for (uint32_t step = 0; v[it] != kOpenEmpty && step < nslots; ++step) {
+                if ((uint32_t)(v[it] >> 32) == c[it]) {
+                    rid[it] = (uint32_t)v[it];
+                    break;
+                }
+                if (++h == nslots) h = 0;
+                v[it] = __ldg(slots + h);
+            }
+        }
+    }
+};
+
+/* The keys of 256 rows of a page, from row s0 + part * 256 on, as the table
+ * sees them: bit `it` of the result set when row it * 32 + lane of them is
+ * non-NULL and may be in the table. The value positions come from the
+ * bitmap: the 64 words of rows [s0, s0 + 2048) two per lane, a warp scan of
+ * their popcounts; *before: the page's values before row s0, moved on. */
+template <typename T, class LK>
+CJ_DEV uint32_t page_keys(const uint8_t *pg, uint32_t nr, uint32_t nv, uint32_t s0, uint32_t part, uint32_t *before,
+                          const LK &lk, uint32_t *code, unsigned int *err) {
+    constexpr uint32_t DB = sizeof(T) == 4 ? 4u : 8u;
+    const T *vals = reinterpret_cast<const T *>(pg + DB);
+    const uint32_t lane = lane_id(), r0 = s0 + part * kWarpRows + lane;
+    uint32_t present = 0;
+    T v[kItems];
+    if (nr == nv) {
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            v[it] = T(0);
+            if (r0 + it * 32 < nr) {
+                v[it] = __ldcs(vals + r0 + it * 32);
+                present |= 1u << it;
+            }
+        }
+    } else {
+        const uint32_t nb = (nr + 7) / 8, bm0 = kPageSize - nb;
+        const uint32_t *words = reinterpret_cast<const uint32_t *>(pg);
+        uint32_t w[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) { /* word s0 / 32 + j * 32 + lane of the bitmap */
+            const uint32_t first = s0 + (j * 32 + lane) * 32;
+            w[j] = 0;
+            if (first < nr) {
+                const uint32_t b = bm0 + first / 8, al = b >> 2, sh = (b & 3u) * 8;
+                const uint32_t lo = __ldg(words + al), hi = al + 1 < kPageSize / 4 ? __ldg(words + al + 1) : 0u;
+                w[j] = __funnelshift_r(lo, hi, sh);
+                if (nr - first < 32) w[j] &= (1u << (nr - first)) - 1u;
+            }
+        }
+        const uint32_t c0 = __popc(w[0]), c1 = __popc(w[1]);
+        const uint32_t t0 = __reduce_add_sync(0xffffffffu, c0);
+        /* this part's words and the values before each: lanes of one of the
+         * two halves */
+        const bool low = part < kParts / 2;
+        const uint32_t word = low ? w[0] : w[1], cnt = low ? c0 : c1;
+        const uint32_t pre = *before + (low ? 0u : t0) + warp_inclusive_scan(cnt) - cnt;
+        if (s0 + kTileRows < nr) *before += t0 + __reduce_add_sync(0xffffffffu, c1);
+        const uint32_t lt = lanemask_lt(), bit = 1u << lane;
+        uint32_t most = 0;
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            const int src = (int)(part * kItems + it) & 31;
+            const uint32_t bits = __shfl_sync(0xffffffffu, word, src);
+            const uint32_t k = __shfl_sync(0xffffffffu, pre, src) + __popc(bits & lt);
+            v[it] = T(0);
+            const bool here = (bits & bit) != 0;
+            most = max(most, here ? k : 0u);
+            if (here && k < nv) {
+                v[it] = __ldcs(vals + k);
+                present |= 1u << it;
+            }
+        }
+        if (nv && most >= nv) atomicOr(err, DEV_ERR_PAGE_HEADER); /* bitmap holds > n_values bits */
+        if (!nv && word) atomicOr(err, DEV_ERR_PAGE_HEADER);
+    }
+    uint32_t ok = 0;
+#pragma unroll
+    for (int it = 0; it < kItems; ++it) {
+        bool in;
+        code[it] = lk.code(v[it], (present >> it) & 1u, &in);
+        if (LK::kMask && in) ok |= 1u << it;
+    }
+    return ok;
+}
+
+/* 256 consecutive values of a column's full pages touch two pages at most:
+ * the first one's values and the place of the run in it are the warp's, a
+ * value's offset from there fits 32 bits. */
+template <typename T> struct PageRun {
+    static constexpr uint32_t R = sizeof(T) == 4 ? kRowsPerPageInt32 : kRowsPerPage8B;
+    static constexpr uint32_t kGap = kPageSize - R * (uint32_t)sizeof(T); /* bytes of a page that hold no values */
+    uint8_t *base;
+    uint32_t k0;
+    CJ_DEV PageRun(const uint8_t *pages, uint32_t first) {
+        const uint32_t p = first / R;
+        k0 = first - p * R;
+        base = const_cast<uint8_t *>(pages) + (uint64_t)p * kPageSize + (sizeof(T) == 4 ? 4 : 8);
+    }
+    CJ_DEV T *at(uint32_t i) const {
+        const uint32_t k = k0 + i;
+        return reinterpret_cast<T *>(base + (k * (uint32_t)sizeof(T) + (k >= R ? kGap : 0u)));
+    }
+};
+
+/* A warp's matches, packed: what the columns are written from, by full
+ * warps and without predicates on the rows that did not match. Kept small:
+ * shared memory is taken from L1, and every random load in flight holds a
+ * 128-byte line of L1 until it returns. At 64M rows a variant with 37 KB per
+ * CTA ran 880 us at five CTAs per SM and 1587 at six. */
+struct WarpMatches {
+    uint32_t rid[kWarpRows];
+    uint8_t row[kWarpRows];
+};
+constexpr int kEmit = 3; /* matches a lane has in flight */
+
+/* The values of result column c of the warp's n matches, to their places
+ * from output position `at` on. */
+template <typename T>
+CJ_DEV void emit_column(const EmitColumn &c, bool direct, const WarpMatches &w, uint32_t n, uint32_t at, uint32_t row0) {
+    const PageRun<T> out(c.pages, at);
+    const bool in_order = !c.from_build && direct && !c.col.rid_b;
+    const PageRun<T> in(c.col.pages, row0); /* used when in_order */
+    for (uint32_t i0 = lane_id(); i0 < n; i0 += 32 * kEmit) {
+        T v[kEmit];
+#pragma unroll
+        for (int j = 0; j < kEmit; ++j) {
+            const uint32_t i = i0 + j * 32;
+            if (i >= n) break;
+            if (in_order) {
+                v[j] = __ldcs(in.at(w.row[i]));
+            } else {
+                uint32_t r = c.from_build ? w.rid[i] : row0 + w.row[i];
+                if (c.col.rid_b) r = __ldg(c.col.rid_b + r);
+                v[j] = direct ? page_value<T>(c.col.pages, r) : __ldg(reinterpret_cast<const T *>(c.col.values) + r);
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kEmit; ++j)
+            if (i0 + j * 32 < n) __stcs(out.at(i0 + j * 32), v[j]);
+    }
+}
+
+/* What the kernel writes, worked out once per warp: the result columns that
+ * hold no NULL, and the match row ids that the others need. */
+struct EmitPlan {
+    uint32_t active = 0, direct = 0;
+    bool want_b, want_p;
+    CJ_DEV EmitPlan(const UniqueOut &out, bool open) : want_b(out.need_b), want_p(out.need_p) {
+        for (int c = 0; c < out.n; ++c) {
+            const EmitColumn &e = out.cols[c];
+            if (col_null_free(e.col) && !(open && e.direct_only)) {
+                active |= 1u << c;
+                if (col_direct(e.col)) direct |= 1u << c;
+            } else if (e.from_build) {
+                want_b = true;
+            } else {
+                want_p = true;
+            }
+        }
+    }
+};
+
+struct StepShared {
+    WarpMatches matches[kParts];
+    uint32_t count[2][kParts];
+    unsigned long long base[2];
+};
+
+/* A CTA's step: every warp looks up its 256 rows and packs their matches,
+ * one atomicAdd reserves the step's output (one per warp instead made the
+ * counter the bound: 592 us at 64M rows, 800 us with half the rows per
+ * warp), and the warps write it. row0: the relation row of the warp's first;
+ * ok: a lane's items to look up; buf alternates between steps. Block-wide. */
+template <typename T, class LK>
+CJ_DEV void probe_step(const LK &lk, const uint32_t *code, uint32_t ok, uint32_t row0, const UniqueOut &out,
+                       const EmitPlan &plan, StepShared &sh, uint32_t part, uint32_t buf) {
+    const uint32_t lane = lane_id(), lt = lanemask_lt();
+    WarpMatches &w = sh.matches[part];
+    uint32_t rid[kItems], n = 0, m = 0;
+    uint32_t place[(kItems + 3) / 4] = {}; /* of the lane's matches among the warp's: a byte per item */
+    lk.find(code, ok, rid);
+#pragma unroll
+    for (int it = 0; it < kItems; ++it) {
+        const bool hit = rid[it] != kArrayEmpty;
+        const uint32_t b = __ballot_sync(0xffffffffu, hit);
+        const uint32_t i = n + __popc(b & lt);
+        if (hit) {
+            w.rid[i] = rid[it];
+            w.row[i] = (uint8_t)(it * 32 + lane);
+            m |= 1u << it;
+        }
+        place[it / 4] |= (i & 0xFFu) << (8 * (it % 4));
+        n += __popc(b);
+    }
+    if (lane == 0) sh.count[buf][part] = n;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t total = 0;
+#pragma unroll
+        for (int p = 0; p < kParts; ++p) total += sh.count[buf][p];
+        sh.base[buf] = total ? atomicAdd(out.match.counter, (unsigned long long)total) : 0ull;
+    }
+    __syncthreads();
+    if (!n) return;
+    uint32_t before = 0;
+    for (uint32_t p = 0; p < part; ++p) before += sh.count[buf][p];
+    /* at most one match per row: positions stay below the probe rows, which
+     * the capacity covers */
+    const unsigned long long base = sh.base[buf] + before;
+    if (base + n > out.match.capacity) return;
+    const uint32_t at = (uint32_t)base;
+    if (out.match.key_pages) { /* of the probe key's type */
+        const PageRun<T> keys(out.match.key_pages, at);
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            T *to = keys.at((place[it / 4] >> (8 * (it % 4))) & 0xFFu);
+            if ((m >> it) & 1u) __stcs(to, lk.key_of(code[it]));
+        }
+    }
+    if (plan.want_b)
+        for (uint32_t i = lane; i < n; i += 32) __stcs(out.match.build_rids + at + i, w.rid[i]);
+    if (plan.want_p)
+        for (uint32_t i = lane; i < n; i += 32) __stcs(out.match.probe_rids + at + i, row0 + w.row[i]);
+    for (int c = 0; c < out.n; ++c) {
+        if (!((plan.active >> c) & 1u)) continue;
+        const EmitColumn &e = out.cols[c];
+        if (e.col.type == CJ_INT32) emit_column<int32_t>(e, (plan.direct >> c) & 1u, w, n, at, row0);
+        else emit_column<long long>(e, (plan.direct >> c) & 1u, w, n, at, row0);
+    }
+    __syncwarp(); /* done with w before the next step packs */
+}
+
+/* Asks L2 for a warp's eighth of a page that it reads next: its keys then
+ * cost an L2 round trip, not one to HBM. */
+CJ_DEV void prefetch_part(const uint8_t *pg, uint32_t part) {
+    constexpr uint32_t kLines = kPageSize / 128 / kParts;
+    if (lane_id() < kLines) asm volatile("prefetch.global.L2 [%0];" ::"l"(pg + (part * kLines + lane_id()) * 128));
+}
+
+/* One key of a relation row, typed. */
+template <typename T> CJ_DEV bool row_key(const ColView &c, uint32_t i, T *key) {
+    int64_t k;
+    if (!load_key_stream(c, i, &k)) return false;
+    *key = (T)k;
+    return true;
+}
+
+template <bool kPages, typename T, class LK>
+CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const UniqueTable &t, const UniqueOut &out, StepShared &sh) {
+    const LK lk(t);
+    const EmitPlan plan(out, LK::kMask);
+    const uint32_t part = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); /* warp-uniform */
+    uint32_t buf = 0;
+    if constexpr (kPages) {
+        for (uint64_t p = blockIdx.x; p < k.num_pages; p += gridDim.x) {
+            const uint8_t *pg = k.col.pages + p * kPageSize;
+            const uint32_t head = __ldg(reinterpret_cast<const uint32_t *>(pg));
+            const uint32_t nr = head & 0xFFFFu, nv = head >> 16;
+            const uint64_t rs = page_first_row(k.base, k.loc, p);
+            if (p + gridDim.x < k.num_pages) prefetch_part(pg + (uint64_t)gridDim.x * kPageSize, part);
+            if (nv > nr || sizeof(T) + sizeof(T) * nv + (nr + 7) / 8 > kPageSize)
+                continue; /* the index has raised the error */
+            if (rs + nr > n) {
+                if (threadIdx.x == 0) atomicOr(k.err, DEV_ERR_ROW_COUNT);
+                continue;
+            }
+            uint32_t before = 0;
+            for (uint32_t s0 = 0; s0 < nr; s0 += kTileRows) {
+                uint32_t code[kItems] = {};
+                const uint32_t ok = page_keys<T>(pg, nr, nv, s0, part, &before, lk, code, k.err);
+                probe_step<T>(lk, code, ok, (uint32_t)rs + s0 + part * kWarpRows, out, plan, sh, part, buf);
+                buf ^= 1u;
+            }
+        }
+    } else {
+        const ColView col = resolve_view(k.col);
+        for (uint64_t t0 = (uint64_t)blockIdx.x * kTileRows; t0 < n; t0 += (uint64_t)gridDim.x * kTileRows) {
+            uint32_t code[kItems] = {}, ok = 0;
+            const uint64_t r0 = t0 + part * kWarpRows;
+#pragma unroll
+            for (int it = 0; it < kItems; ++it) {
+                const uint64_t i = r0 + it * 32 + lane_id();
+                T key = T(0);
+                bool in;
+                const bool present = i < n && row_key<T>(col, (uint32_t)i, &key);
+                code[it] = lk.code(key, present, &in);
+                if (LK::kMask && in) ok |= 1u << it;
+            }
+            probe_step<T>(lk, code, ok, (uint32_t)r0, out, plan, sh, part, buf);
+            buf ^= 1u;
+        }
+    }
+}
+
+template <bool kPages, typename T>
+__global__ void __launch_bounds__(kProbeThreads, kProbeBlocks)
+    k_probe_unique(const __grid_constant__ ProbeKey k, uint32_t n, const __grid_constant__ UniqueTable t,
+                   const __grid_constant__ UniqueOut out) {
+    __shared__ StepShared sh;
+    const unsigned long long refused = t.params[kTableRefused];
+    if (t.params[kTableDup]) return;
+    if (refused == 0) probe_all<kPages, T, DirectLookup<T>>(k, n, t, out, sh);
+    else if (refused == kTableSpread && t.open_slots) probe_all<kPages, T, OpenLookup<T>>(k, n, t, out, sh);
+}
+
+/* Random loads in flight are held in L1: as little of it as possible goes to
+ * shared memory (default split 628 us, this one 605). Once per kernel and
+ * device. */
+template <class K> void prefer_l1(K kernel) {
+    constexpr int kDevices = 64;
+    static std::atomic<const void *> done[kDevices][4];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) {
+        cudaGetLastError();
+        return;
+    }
+    for (auto &slot : done[dev]) {
+        const void *seen = slot.load(std::memory_order_acquire);
+        if (seen == reinterpret_cast<const void *>(kernel)) return;
+        if (seen) continue;
+        cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 25);
+        slot.store(reinterpret_cast<const void *>(kernel), std::memory_order_release);
+        return;
+    }
+}
+
+} // namespace
+
+cudaError_t launch_unique_build(const Launch &L, const ColView &key, uint32_t n, const UniqueTable &t) {
+    if (n == 0) return cudaSuccess;
+    if (t.open_slots && t.open_slots < 2ull * n) return cudaErrorInvalidValue; /* half empty */
+    if (reinterpret_cast<uintptr_t>(t.slots) % 16) return cudaErrorInvalidValue;
+    if (n <= kSmallRows) {
+        k_unique_small<<<1, kSmallThreads, 0, L.stream>>>(key, n, t);
+        count_launches(1);
+        return cudaGetLastError();
+    }
+    const uint64_t wave = (uint64_t)L.num_sms * 8;
+    const uint64_t rows_per_block = kUniqueThreads * kUniqueRows;
+    const unsigned g = (unsigned)std::min<uint64_t>((n + rows_per_block - 1) / rows_per_block, wave);
+    k_unique_range<<<g, kUniqueThreads, 0, L.stream>>>(key, n, t);
+    const uint64_t most = std::max<uint64_t>(t.max_span * 4, t.open_slots * 8ull) / 16 + 1;
+    k_unique_fill<<<(unsigned)std::min<uint64_t>((most + 255) / 256, wave), kUniqueThreads, 0, L.stream>>>(t);
+    k_unique_insert<<<g, kUniqueThreads, 0, L.stream>>>(key, n, t);
+    count_launches(3);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_probe_unique(const Launch &L, const ProbeKey &k, uint32_t n, const UniqueTable &t,
+                                const UniqueOut &out) {
+    if (n == 0) return cudaSuccess;
+    const bool pages = k.base != nullptr;
+    const uint64_t tiles = pages ? k.num_pages : ((uint64_t)n + kTileRows - 1) / kTileRows;
+    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * kProbeBlocks));
+    const auto kernel = k.col.type == CJ_INT32 ? (pages ? k_probe_unique<true, int32_t> : k_probe_unique<false, int32_t>)
+                                               : (pages ? k_probe_unique<true, long long> : k_probe_unique<false, long long>);
+    prefer_l1(kernel);
+    kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+} // namespace cj

@@ -12,11 +12,15 @@ pytestmark = pytest.mark.gpu
 I, L, F, V = DataType.INT32, DataType.INT64, DataType.FP64, DataType.VARCHAR
 
 
-def _resident(plan, ctx):
+def _run_resident(plan, ctx, flags=_lib.CJ_EXEC_RESULT_ON_DEVICE):
     rp = Plan()
     rp.nodes, rp.root = plan.nodes, plan.root
     rp.inputs = [ResidentTable(ctx, t) for t in plan.inputs]
-    return rp
+    try:
+        return run_product(rp, ctx, flags)[0]
+    finally:
+        for t in rp.inputs:
+            t.free()
 
 
 def _scan(columns, rows):
@@ -36,7 +40,7 @@ def test_index_chunks(gpu_ctx, pages):
             encode_column(L, rng.integers(0, 1 << 50, n), valid)]
     plan = _scan(cols, n)
     for flags in (0, _lib.CJ_EXEC_RESULT_ON_DEVICE):
-        got, _ = run_product(_resident(plan, gpu_ctx), gpu_ctx, flags)
+        got = _run_resident(plan, gpu_ctx, flags)
         assert_same(got, run_oracle(plan), f"{pages} pages")
 
 
@@ -53,7 +57,7 @@ def test_many_columns(gpu_ctx, ncols):
         else:
             cols.append(encode_column(t, rng.integers(0, 10 ** 6, n), valid))
     plan = _scan(cols, n)
-    got, _ = run_product(_resident(plan, gpu_ctx), gpu_ctx, _lib.CJ_EXEC_RESULT_ON_DEVICE)
+    got = _run_resident(plan, gpu_ctx)
     assert_same(got, run_oracle(plan), f"{ncols} columns")
 
 
@@ -74,14 +78,12 @@ def test_errors_of_unread_columns(gpu_ctx, empty):
     s = [plan.new_scan_node(0, [(0, I)]), plan.new_scan_node(1, [(0, I)]), plan.new_scan_node(2, [(0, I), (1, I)])]
     j = plan.new_join_node(True, s[0], s[1], 0, 0, [(0, I)])
     plan.root = plan.new_join_node(True, j, s[2], 0, 0, [(0, I), (2, I)])
-    rp = _resident(plan, gpu_ctx)
     if empty:
-        got, _ = run_product(rp, gpu_ctx, _lib.CJ_EXEC_RESULT_ON_DEVICE)
-        assert got.num_rows == 0
+        assert _run_resident(plan, gpu_ctx).num_rows == 0
     else:
         with pytest.raises(CJError) as ei:
-            run_product(rp, gpu_ctx, _lib.CJ_EXEC_RESULT_ON_DEVICE)
+            _run_resident(plan, gpu_ctx)
         assert ei.value.status == 3
     plan.inputs[2] = ColumnarTable(n, [c.columns[0], c.columns[0]])
-    got, _ = run_product(_resident(plan, gpu_ctx), gpu_ctx, _lib.CJ_EXEC_RESULT_ON_DEVICE)
+    got = _run_resident(plan, gpu_ctx)
     assert got.num_rows == (0 if empty else n)  # the context is as usable as before
