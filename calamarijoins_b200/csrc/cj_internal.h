@@ -350,6 +350,21 @@ struct UniqueOut {
 cudaError_t launch_probe_unique(const Launch &L, const ProbeKey &k, uint32_t n, const UniqueTable &t,
                                 const UniqueOut &out);
 
+/* Table of build keys that repeat, over a dense range: entries[key - lo] is
+ * the key's build row count (high word) and, for one, the row itself, for
+ * more, the end of its rows in `rows` (low word). */
+struct MultiTable {
+    unsigned long long *entries; /* span + 1 */
+    uint32_t *rows;              /* build rows */
+    int64_t lo;
+    uint32_t span;
+};
+cudaError_t launch_multi_build(const Launch &L, const ColView &key, uint32_t n, const MultiTable &t);
+/* Probe of it; the match counter must be zero before. When the count ends
+ * above out.match.capacity the output is incomplete: run again with room. */
+cudaError_t launch_probe_multi(const Launch &L, const ProbeKey &k, uint32_t n, const MultiTable &t,
+                               const UniqueOut &out);
+
 constexpr int kDirectParams = 6; /* words of a grouped direct-mapped table */
 
 /* Probe and nested loop share one tiled kernel; `sched` is scratch of

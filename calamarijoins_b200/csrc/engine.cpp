@@ -28,6 +28,8 @@
 namespace cj {
 namespace {
 
+constexpr uint64_t kMultiSpan = 4; /* values of the range per build row */
+
 /* A probe of an open-addressing table reads a build column's values beside
  * it while both stay in L2 (126 MB on two dies, each keeping its own copy of
  * what it reads); a larger pair is read one after the other, through the
@@ -457,6 +459,9 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         int log2_slots = 0;
         bool inline_dir = true;
         bool unique = false; /* a table of unique keys tried (the device decides) */
+        bool multi = false;  /* the table of repeated dense keys */
+        MultiTable multi_table{};
+        DevPtr multi_rows;
         const bool words_clear = join_words_clear;
         join_words_clear = false; /* every join counts its matches there */
         UniqueTable table{};
@@ -534,7 +539,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             mo.key_bytes = key_bytes;
             mo.capacity = collect ? cap : 0;
             mo.counter = &ctx.d_status->counter;
-            if (unique) {
+            if (unique || multi) {
                 /* The root's fixed-width columns whose pages are in HBM are
                  * written by the probe itself where they hold no NULL; row
                  * ids are collected for the others only. */
@@ -543,10 +548,14 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 for (auto &o : outs) {
                     if (!is_root || o.from_keys) continue;
                     const auto it = decoded.find({o.col.input, o.col.col});
-                    if (o.col.type != CJ_VARCHAR && it != decoded.end() && it->second.ready && uo.n < kEmitColumns) {
+                    const bool beside = /* the table and the column stay in L2 together */
+                        !o.from_build || !multi || it == decoded.end() ||
+                        (multi_table.span * 2ull + B.rows) * 4 + it->second.src.num_pages * kPageSize <= kEmitBesideOpen;
+                    if (o.col.type != CJ_VARCHAR && it != decoded.end() && it->second.ready && uo.n < kEmitColumns &&
+                        beside) {
                         const uint32_t R = rows_per_page_fixed(o.col.type);
                         o.pages = ctx.alloc((cap + R - 1) / R * kPageSize);
-                        o.direct_only = o.from_build && table.open_slots && table.open_slots * 8ull +
+                        o.direct_only = unique && o.from_build && table.open_slots && table.open_slots * 8ull +
                                                         it->second.src.num_pages * kPageSize > kEmitBesideOpen;
                         uo.cols[uo.n++] = {view(*o.rel, o.col, nullptr), o.pages->as<uint8_t>(), o.from_build ? 1 : 0,
                                            o.direct_only ? 1 : 0};
@@ -571,6 +580,11 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                     key.col = view(P, pk, nullptr);
                 }
                 PhaseScope ph(*this, PH_PROBE);
+                if (multi) {
+                    KScope k(*this, "probe_multi");
+                    ck(launch_probe_multi(L, key, (uint32_t)P.rows, multi_table, uo), "probe_multi");
+                    return;
+                }
                 KScope k(*this, "probe_unique");
                 ck(launch_probe_unique(L, key, (uint32_t)P.rows, table, uo), "probe_unique");
                 return;
@@ -593,21 +607,47 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 }
             }
         };
+        uint64_t cap = P.rows;
         /* The device refused the table of unique keys (its probe did
-         * nothing): the hash table. */
+         * nothing). Keys that repeat over a dense range get the table of
+         * repeated keys: one random access per probe row and one per further
+         * match (64M x 4M rows over 3M keys: hash build, probe and page
+         * writers 235 + 1004 + 570 us, 130 + 956 + 344 here, the probe with
+         * one of the columns written beside it); 8 bytes per value of the
+         * range, at most kMultiSpan values per build row so that it stays
+         * near the hash table's 24 bytes per row. Else the hash table. */
         auto replace_unique = [&]() {
             unique = false;
             slots.reset();
-            for (auto &o : outs) o.pages.reset();
+            for (auto &o : outs) {
+                o.pages.reset();
+                o.direct_only = false;
+            }
             PhaseScope ph(*this, PH_BUILD);
-            build_hash();
+            const unsigned long long *tp = ctx.h_status->table;
+            if (tp[kTableRefused] != kTableSpread && tp[kTableSpan] <= kMultiSpan * B.rows) {
+                multi = true;
+                multi_table.lo = (int64_t)tp[kTableLo];
+                multi_table.span = (uint32_t)tp[kTableSpan];
+                slots = ctx.alloc((tp[kTableSpan] + 1) * 8);
+                multi_rows = ctx.alloc(B.rows * 4);
+                multi_table.entries = slots->as<unsigned long long>();
+                multi_table.rows = multi_rows->as<uint32_t>();
+                /* room for the keys' mean number of rows per match, up to 4;
+                 * a result above it runs the probe again */
+                const uint64_t mean = P.rows * (uint64_t)tp[kTableCount] / (uint64_t)tp[kTableSpan];
+                cap = std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(cap, mean), 4 * P.rows), 0xFFFFFFFFull);
+                KScope k(*this, "multi_build");
+                ck(launch_multi_build(L, bv, (uint32_t)B.rows, multi_table), "multi_build");
+            } else {
+                build_hash();
+            }
         };
         auto count_join = [&]() {
             const int kind = table_kind(ctx.h_status->table, table.open_slots);
             stats.num_direct_joins += kind == 1;
             stats.num_open_joins += kind == 2;
         };
-        uint64_t cap = P.rows;
         bool all_fixed = true;
         for (const auto &o : outs) all_fixed &= o.col.type != CJ_VARCHAR;
         if (is_root && unique && collect && all_fixed && (flags & CJ_EXEC_RESULT_ON_DEVICE) && ctx.opt.defer_count) {
@@ -636,6 +676,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             replace_unique();
         }
         for (;;) {
+            if (multi) clear_join_words(); /* the match counter */
             launch_probe(cap);
             sync();
             if (unique && !table_kind(ctx.h_status->table, table.open_slots)) {

@@ -1,6 +1,7 @@
 /*
- * k_unique.cu — joins over unique build keys: the table's build and a probe
- * that reads the key column's pages and writes the result's pages.
+ * k_unique.cu — joins over unique build keys, and over repeated ones of a
+ * dense range: the tables' builds and a probe that reads the key column's
+ * pages and writes the result's pages.
  *
  * The table (launch_unique_build) is direct-mapped when the keys lie densely
  * (slots[key - lo] = build row), else, for INT32 keys, open-addressing
@@ -20,6 +21,10 @@
  * result pages: no match row ids are written and read back for them.
  * Columns with NULLs (known on the device only) get their row ids and are
  * written by k_write_pages.
+ *
+ * Keys that repeat over a dense range get a table of their own
+ * (launch_multi_build: a count, and the row or where the key's rows lie, per
+ * value) and the same probe with room for several matches a row.
  *
  * Bound: requests from L1 to L2, about one per clock and SM whatever their
  * size (every random slot or value is one), then the 128-byte lines of L1
@@ -210,11 +215,91 @@ __global__ void __launch_bounds__(kSmallThreads)
     insert_rows(key, t, threadIdx.x, n, kSmallThreads);
 }
 
+/* Build of a table of repeated keys: count, place, scatter (launch_multi_build). */
+__global__ void __launch_bounds__(kUniqueThreads) k_multi_count(ColView key_arg, uint32_t n, MultiTable t) {
+    const ColView key = resolve_view(key_arg);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += stride * kUniqueRows) {
+        uint64_t off[kUniqueRows];
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) {
+            const uint64_t i = i0 + q * stride;
+            int64_t k;
+            off[q] = i < n && load_key(key, (uint32_t)i, &k) ? (uint64_t)k - (uint64_t)t.lo : ~0ull;
+        }
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q)
+            if (off[q] < t.span) atomicAdd(reinterpret_cast<uint32_t *>(t.entries + off[q]) + 1, 1u);
+    }
+}
+
+/* A place in `rows` for every value with two build rows or more. One
+ * atomicAdd per 2,048 values: the places' order does not matter. */
+constexpr int kPlaceItems = 8;
+__global__ void __launch_bounds__(kUniqueThreads) k_multi_place(MultiTable t) {
+    __shared__ uint32_t wbuf[kUniqueThreads / 32 + 1];
+    __shared__ uint32_t s_base;
+    uint32_t *cursor = reinterpret_cast<uint32_t *>(t.entries + t.span);
+    for (uint64_t v0 = (uint64_t)blockIdx.x * kUniqueThreads * kPlaceItems; v0 < t.span;
+         v0 += (uint64_t)gridDim.x * kUniqueThreads * kPlaceItems) {
+        uint32_t c[kPlaceItems], sum = 0, total;
+#pragma unroll
+        for (int q = 0; q < kPlaceItems; ++q) {
+            const uint64_t v = v0 + q * kUniqueThreads + threadIdx.x;
+            c[q] = v < t.span ? (uint32_t)(t.entries[v] >> 32) : 0u;
+            if (c[q] > 1) sum += c[q];
+        }
+        const uint32_t pre = block_exclusive_scan<uint32_t>(sum, wbuf, &total);
+        if (threadIdx.x == 0) s_base = total ? atomicAdd(cursor, total) : 0u;
+        __syncthreads();
+        uint32_t at = s_base + pre;
+#pragma unroll
+        for (int q = 0; q < kPlaceItems; ++q) {
+            const uint64_t v = v0 + q * kUniqueThreads + threadIdx.x;
+            if (c[q] < 2) continue;
+            *reinterpret_cast<uint32_t *>(t.entries + v) = at;
+            at += c[q];
+        }
+        __syncthreads();
+    }
+}
+
+/* A single row goes into its entry; rows of a repeated key to their places,
+ * which moves the entry's low word on to the end of the key's rows. */
+__global__ void __launch_bounds__(kUniqueThreads) k_multi_scatter(ColView key_arg, uint32_t n, MultiTable t) {
+    const ColView key = resolve_view(key_arg);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += stride * kUniqueRows) {
+        uint64_t off[kUniqueRows];
+        uint32_t c[kUniqueRows];
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) {
+            const uint64_t i = i0 + q * stride;
+            int64_t k;
+            off[q] = i < n && load_key(key, (uint32_t)i, &k) ? (uint64_t)k - (uint64_t)t.lo : ~0ull;
+        }
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) /* counts no longer change */
+            c[q] = off[q] < t.span ? reinterpret_cast<const uint32_t *>(t.entries + off[q])[1] : 0u;
+        uint32_t at[kUniqueRows];
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) {
+            uint32_t *low = reinterpret_cast<uint32_t *>(t.entries + (c[q] ? off[q] : 0));
+            if (c[q] == 1) *low = (uint32_t)(i0 + q * stride);
+            else if (c[q]) at[q] = atomicAdd(low, 1u);
+        }
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q)
+            if (c[q] > 1) t.rows[at[q]] = (uint32_t)(i0 + q * stride);
+    }
+}
+
 /* ---------------- probe ---------------- */
 /* 256 threads, 48 registers and 10 KB of shared memory: five CTAs per SM.
  * Measured at 64M x 4M rows (probe alone): five 605 us, four with 64
  * registers 619, six with 40 (spills) 620. */
 constexpr int kProbeBlocks = 5;
+constexpr int kMultiBlocks = 4; /* 64 registers; three with 80 1467 us, five with 48 2343 */
 constexpr int kItems = 8;                              /* rows per lane and step       */
 constexpr int kProbeThreads = 2048 / kItems;
 constexpr int kParts = kProbeThreads / 32;
@@ -229,16 +314,16 @@ template <typename T> struct DirectLookup {
     const uint32_t *slots;
     int64_t lo;
     uint32_t span; /* at most 2^28 */
-    CJ_DEV DirectLookup(const UniqueTable &t) {
-        slots = reinterpret_cast<const uint32_t *>(t.slots);
-        lo = (int64_t)t.params[kTableLo];
-        span = (uint32_t)t.params[kTableSpan];
+    CJ_DEV DirectLookup(const uint32_t *table, int64_t first, uint32_t values) {
+        int64_t skip = 0;
         if constexpr (sizeof(T) == 4) {
-            const int64_t first = max(lo, (int64_t)INT32_MIN), end = min(lo + (int64_t)span, (int64_t)INT32_MAX + 1);
-            span = end > first ? (uint32_t)(end - first) : 0u;
-            if (span) slots += first - lo;
-            lo = first;
+            const int64_t end = min(first + (int64_t)values, (int64_t)INT32_MAX + 1), cut = max(first, (int64_t)INT32_MIN);
+            values = end > cut ? (uint32_t)(end - cut) : 0u;
+            skip = values ? cut - first : 0;
         }
+        slots = table + skip;
+        lo = first + skip;
+        span = values;
     }
     static constexpr bool kMask = false; /* a code says by itself whether it may be in the table */
     CJ_DEV uint32_t code(T key, bool present, bool *in) const {
@@ -410,8 +495,8 @@ constexpr int kEmit = 3; /* matches a lane has in flight */
 
 /* The values of result column c of the warp's n matches, to their places
  * from output position `at` on. */
-template <typename T>
-CJ_DEV void emit_column(const EmitColumn &c, bool direct, const WarpMatches &w, uint32_t n, uint32_t at, uint32_t row0) {
+template <typename T, class W>
+CJ_DEV void emit_column(const EmitColumn &c, bool direct, const W &w, uint32_t n, uint32_t at, uint32_t row0) {
     const PageRun<T> out(c.pages, at);
     const bool in_order = !c.from_build && direct && !c.col.rid_b;
     const PageRun<T> in(c.col.pages, row0); /* used when in_order */
@@ -460,6 +545,24 @@ struct StepShared {
     uint32_t count[2][kParts];
     unsigned long long base[2];
 };
+
+/* Writes a warp's n packed matches from output position `at` on, but for
+ * the key column. */
+template <class W>
+CJ_DEV void emit_packed(const UniqueOut &out, const EmitPlan &plan, const W &w, uint32_t n, uint32_t at,
+                        uint32_t row0) {
+    const uint32_t lane = lane_id();
+    if (plan.want_b)
+        for (uint32_t i = lane; i < n; i += 32) __stcs(out.match.build_rids + at + i, w.rid[i]);
+    if (plan.want_p)
+        for (uint32_t i = lane; i < n; i += 32) __stcs(out.match.probe_rids + at + i, row0 + w.row[i]);
+    for (int c = 0; c < out.n; ++c) {
+        if (!((plan.active >> c) & 1u)) continue;
+        const EmitColumn &e = out.cols[c];
+        if (e.col.type == CJ_INT32) emit_column<int32_t>(e, (plan.direct >> c) & 1u, w, n, at, row0);
+        else emit_column<long long>(e, (plan.direct >> c) & 1u, w, n, at, row0);
+    }
+}
 
 /* A CTA's step: every warp looks up its 256 rows and packs their matches,
  * one atomicAdd reserves the step's output (one per warp instead made the
@@ -512,17 +615,177 @@ CJ_DEV void probe_step(const LK &lk, const uint32_t *code, uint32_t ok, uint32_t
             if ((m >> it) & 1u) __stcs(to, lk.key_of(code[it]));
         }
     }
-    if (plan.want_b)
-        for (uint32_t i = lane; i < n; i += 32) __stcs(out.match.build_rids + at + i, w.rid[i]);
-    if (plan.want_p)
-        for (uint32_t i = lane; i < n; i += 32) __stcs(out.match.probe_rids + at + i, row0 + w.row[i]);
-    for (int c = 0; c < out.n; ++c) {
-        if (!((plan.active >> c) & 1u)) continue;
-        const EmitColumn &e = out.cols[c];
-        if (e.col.type == CJ_INT32) emit_column<int32_t>(e, (plan.direct >> c) & 1u, w, n, at, row0);
-        else emit_column<long long>(e, (plan.direct >> c) & 1u, w, n, at, row0);
-    }
+    emit_packed(out, plan, w, n, at, row0);
     __syncwarp(); /* done with w before the next step packs */
+}
+
+/* The same over a table of repeated keys. The matches of rows with up to
+ * three are packed and written together; those of rows with more in rounds,
+ * the j-th matches of all of them; the rows of a key with more than kHeavyRun
+ * build rows one after the other. 64M x 4M rows over 3M keys, 58.6M matches:
+ * 956 us with one result column of two written beside it (bound by the
+ * registers of its many paths: 64, some spilled; a separate function for the
+ * rare ones cost more in the common one, 1141 us; every match of a row in
+ * rounds 1458). */
+constexpr uint32_t kHeavyRun = 32;
+constexpr uint32_t kMultiRoom = 320; /* matches packed at once: 256 rows and a quarter more */
+struct MultiMatches {
+    uint32_t rid[kMultiRoom]; /* the keys first, then the build rows */
+    uint8_t row[kMultiRoom];
+};
+struct MultiShared {
+    MultiMatches matches[kParts];
+    unsigned long long count[2][kParts];
+    unsigned long long base[2];
+};
+template <typename T> struct MultiLookup {
+    DirectLookup<T> d;
+    const unsigned long long *entries;
+    const uint32_t *rows;
+    static constexpr bool kMask = false;
+    CJ_DEV MultiLookup(const MultiTable &t)
+        : d(nullptr, t.lo, t.span), entries(t.entries + (d.lo - t.lo)), rows(t.rows) {}
+    CJ_DEV uint32_t code(T key, bool present, bool *in) const { return d.code(key, present, in); }
+    CJ_DEV T key_of(uint32_t c) const { return d.key_of(c); }
+};
+
+/* The lanes' items of one packing: item `it`'s matches go to places first(it)
+ * on, `count(it)` of them (at most three); the packed total is returned. */
+template <class C, class F> CJ_DEV uint32_t pack_few(C count, F put) {
+    const uint32_t lt = lanemask_lt();
+    uint32_t n = 0;
+#pragma unroll
+    for (int it = 0; it < kItems; ++it) {
+        const uint32_t c = count(it);
+        const uint32_t b0 = __ballot_sync(0xffffffffu, c & 1u), b1 = __ballot_sync(0xffffffffu, c & 2u);
+        const uint32_t i = n + __popc(b0 & lt) + 2 * __popc(b1 & lt);
+        n += __popc(b0) + 2 * __popc(b1);
+        if (c && i + c <= kMultiRoom) put(it, i, c);
+    }
+    return n;
+}
+template <typename T>
+CJ_DEV void emit_keys(const MultiLookup<T> &lk, const UniqueOut &out, const MultiMatches &w, uint32_t n, uint32_t at) {
+    __syncwarp();
+    const PageRun<T> keys(out.match.key_pages, at);
+    for (uint32_t i = lane_id(); i < n; i += 32) __stcs(keys.at(i), lk.key_of(w.rid[i]));
+    __syncwarp();
+}
+
+template <typename T>
+CJ_DEV void probe_step(const MultiLookup<T> &lk, const uint32_t *code, uint32_t, uint32_t row0, const UniqueOut &out,
+                       const EmitPlan &plan, MultiShared &sh, uint32_t part, uint32_t buf) {
+    const uint32_t lane = lane_id(), lt = lanemask_lt();
+    MultiMatches &w = sh.matches[part];
+    uint32_t low[kItems], cnt[kItems];
+#pragma unroll
+    for (int it = 0; it < kItems; ++it) {
+        unsigned long long e = 0;
+        if (code[it] < lk.d.span) e = __ldg(lk.entries + code[it]);
+        low[it] = (uint32_t)e;
+        cnt[it] = (uint32_t)(e >> 32);
+    }
+    unsigned long long many = 0; /* matches of rows with more than three */
+#pragma unroll
+    for (int it = 0; it < kItems; ++it)
+        if (cnt[it] > 3) many += cnt[it];
+    many = warp_sum(many);
+    const auto few_of = [&](int it) { return cnt[it] <= 3 ? cnt[it] : 0u; };
+    const uint32_t few = pack_few(few_of, [&](int it, uint32_t i, uint32_t c) {
+#pragma unroll
+        for (uint32_t j = 0; j < 3; ++j)
+            if (j < c) {
+                w.rid[i + j] = code[it];
+                w.row[i + j] = (uint8_t)(it * 32 + lane);
+            }
+    });
+    const bool packed = few <= kMultiRoom; /* else all of them in rounds */
+    const unsigned long long total = few + many;
+    if (lane == 0) sh.count[buf][part] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        unsigned long long all = 0;
+#pragma unroll
+        for (int p = 0; p < kParts; ++p) all += sh.count[buf][p];
+        sh.base[buf] = all ? atomicAdd(out.match.counter, all) : 0ull;
+    }
+    __syncthreads();
+    if (!total) return;
+    unsigned long long base = sh.base[buf];
+    for (uint32_t p = 0; p < part; ++p) base += sh.count[buf][p];
+    /* past the capacity nothing is written: the caller runs the probe again
+     * with room for the whole count */
+    if (base + total > out.match.capacity) return;
+    uint32_t at = (uint32_t)base;
+    if (packed && few) {
+        if (out.match.key_pages) emit_keys(lk, out, w, few, at);
+        pack_few(few_of, [&](int it, uint32_t i, uint32_t c) {
+            if (c == 1) {
+                w.rid[i] = low[it];
+            } else {
+                const uint32_t *r = lk.rows + (low[it] - c);
+                const uint32_t r0 = __ldg(r), r1 = __ldg(r + 1);
+                if (c == 3) w.rid[i + 2] = __ldg(r + 2);
+                w.rid[i] = r0;
+                w.rid[i + 1] = r1;
+            }
+        });
+        __syncwarp();
+        emit_packed(out, plan, w, few, at, row0);
+        at += few;
+    }
+    __syncwarp(); /* done with w before it is packed again */
+    if (packed && !many) return;
+    for (uint32_t j = 0;; ++j) {
+        const auto hit_of = [&](int it) {
+            return cnt[it] > j && cnt[it] <= kHeavyRun && (!packed || cnt[it] > 3) ? 1u : 0u;
+        };
+        const uint32_t n = pack_few(hit_of, [&](int it, uint32_t i, uint32_t) {
+            w.rid[i] = code[it];
+            w.row[i] = (uint8_t)(it * 32 + lane);
+        });
+        if (!n) break;
+        if (out.match.key_pages) emit_keys(lk, out, w, n, at);
+        pack_few(hit_of, [&](int it, uint32_t i, uint32_t) {
+            w.rid[i] = cnt[it] == 1 ? low[it] : __ldg(lk.rows + (low[it] - cnt[it] + j));
+        });
+        __syncwarp();
+        emit_packed(out, plan, w, n, at, row0);
+        __syncwarp();
+        at += n;
+    }
+    for (int it = 0; it < kItems; ++it) {
+        uint32_t c = 0, lo = 0, cd = 0; /* item `it`, without indexing registers */
+#pragma unroll
+        for (int q = 0; q < kItems; ++q)
+            if (q == it) {
+                c = cnt[q];
+                lo = low[q];
+                cd = code[q];
+            }
+        uint32_t heavy = __ballot_sync(0xffffffffu, c > kHeavyRun);
+        while (heavy) {
+            const int src = __ffs(heavy) - 1;
+            heavy &= heavy - 1;
+            const uint32_t rows_n = __shfl_sync(0xffffffffu, c, src);
+            const uint32_t first = __shfl_sync(0xffffffffu, lo, src) - rows_n, kc = __shfl_sync(0xffffffffu, cd, src);
+            for (uint32_t k0 = 0; k0 < rows_n; k0 += kWarpRows) {
+                const uint32_t n = min(kWarpRows, rows_n - k0);
+                for (uint32_t i = lane; i < n; i += 32) {
+                    w.rid[i] = __ldg(lk.rows + (first + k0 + i));
+                    w.row[i] = (uint8_t)(it * 32 + src);
+                }
+                __syncwarp();
+                if (out.match.key_pages) {
+                    const PageRun<T> keys(out.match.key_pages, at);
+                    for (uint32_t i = lane; i < n; i += 32) __stcs(keys.at(i), lk.key_of(kc));
+                }
+                emit_packed(out, plan, w, n, at, row0);
+                __syncwarp();
+                at += n;
+            }
+        }
+    }
 }
 
 /* Asks L2 for a warp's eighth of a page that it reads next: its keys then
@@ -540,9 +803,8 @@ template <typename T> CJ_DEV bool row_key(const ColView &c, uint32_t i, T *key) 
     return true;
 }
 
-template <bool kPages, typename T, class LK>
-CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const UniqueTable &t, const UniqueOut &out, StepShared &sh) {
-    const LK lk(t);
+template <bool kPages, typename T, class LK, class SH>
+CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueOut &out, SH &sh) {
     const EmitPlan plan(out, LK::kMask);
     const uint32_t part = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); /* warp-uniform */
     uint32_t buf = 0;
@@ -594,8 +856,20 @@ __global__ void __launch_bounds__(kProbeThreads, kProbeBlocks)
     __shared__ StepShared sh;
     const unsigned long long refused = t.params[kTableRefused];
     if (t.params[kTableDup]) return;
-    if (refused == 0) probe_all<kPages, T, DirectLookup<T>>(k, n, t, out, sh);
-    else if (refused == kTableSpread && t.open_slots) probe_all<kPages, T, OpenLookup<T>>(k, n, t, out, sh);
+    if (refused == 0) {
+        const DirectLookup<T> lk(reinterpret_cast<const uint32_t *>(t.slots), (int64_t)t.params[kTableLo],
+                                 (uint32_t)t.params[kTableSpan]);
+        probe_all<kPages, T>(k, n, lk, out, sh);
+    }
+    if (refused == kTableSpread && t.open_slots) probe_all<kPages, T>(k, n, OpenLookup<T>(t), out, sh);
+}
+
+template <bool kPages, typename T>
+__global__ void __launch_bounds__(kProbeThreads, kMultiBlocks)
+    k_probe_multi(const __grid_constant__ ProbeKey k, uint32_t n, const __grid_constant__ MultiTable t,
+                  const __grid_constant__ UniqueOut out) {
+    __shared__ MultiShared sh;
+    probe_all<kPages, T>(k, n, MultiLookup<T>(t), out, sh);
 }
 
 /* Random loads in flight are held in L1: as little of it as possible goes to
@@ -649,6 +923,35 @@ cudaError_t launch_probe_unique(const Launch &L, const ProbeKey &k, uint32_t n, 
     const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * kProbeBlocks));
     const auto kernel = k.col.type == CJ_INT32 ? (pages ? k_probe_unique<true, int32_t> : k_probe_unique<false, int32_t>)
                                                : (pages ? k_probe_unique<true, long long> : k_probe_unique<false, long long>);
+    prefer_l1(kernel);
+    kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_multi_build(const Launch &L, const ColView &key, uint32_t n, const MultiTable &t) {
+    if (!n || !t.span) return cudaErrorInvalidValue;
+    const uint64_t wave = (uint64_t)L.num_sms * 8;
+    cudaError_t e = cudaMemsetAsync(t.entries, 0, ((uint64_t)t.span + 1) * 8, L.stream);
+    if (e != cudaSuccess) return e;
+    const uint64_t rows_per_block = kUniqueThreads * kUniqueRows, values_per_block = kUniqueThreads * kPlaceItems;
+    const unsigned g = (unsigned)std::min<uint64_t>((n + rows_per_block - 1) / rows_per_block, wave);
+    k_multi_count<<<g, kUniqueThreads, 0, L.stream>>>(key, n, t);
+    k_multi_place<<<(unsigned)std::min<uint64_t>((t.span + values_per_block - 1) / values_per_block, wave),
+                    kUniqueThreads, 0, L.stream>>>(t);
+    k_multi_scatter<<<g, kUniqueThreads, 0, L.stream>>>(key, n, t);
+    count_launches(3);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_probe_multi(const Launch &L, const ProbeKey &k, uint32_t n, const MultiTable &t,
+                               const UniqueOut &out) {
+    if (n == 0) return cudaSuccess;
+    const bool pages = k.base != nullptr;
+    const uint64_t tiles = pages ? k.num_pages : ((uint64_t)n + kTileRows - 1) / kTileRows;
+    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * kMultiBlocks));
+    const auto kernel = k.col.type == CJ_INT32 ? (pages ? k_probe_multi<true, int32_t> : k_probe_multi<false, int32_t>)
+                                               : (pages ? k_probe_multi<true, long long> : k_probe_multi<false, long long>);
     prefer_l1(kernel);
     kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out);
     count_launches(1);

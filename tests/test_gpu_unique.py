@@ -1,6 +1,6 @@
 """GPU: joins over unique build keys (k_unique.cu) against the oracle: the
 probe that reads the key column's pages and writes the result's, at the
-edges of its pages and steps, and both kinds of table at the edges of the
+edges of its pages and steps, and every kind of table at the edges of the
 key range."""
 import numpy as np
 import pytest
@@ -149,6 +149,68 @@ def test_joins_in_a_row(gpu_ctx):
         scan = plan.new_scan_node(k + 1, [(0, I), (1, I)])
         left = plan.new_join_node(True, left, scan, k, 0, list(enumerate(types)) + [(len(types) + 1, I)])
         types = types + [I]
+    plan.root = left
+    want = run_oracle(plan)
+    for flags in (0, _lib.CJ_EXEC_RESULT_ON_DEVICE):
+        got, _ = run_product(plan, gpu_ctx, flags)
+        assert_same(got, want)
+
+
+def _multi_case(case, rng):
+    nb = 20_000
+    if case == "twice":
+        k = np.concatenate([np.arange(nb // 2)] * 2)
+    elif case == "heavy":  # runs of 1, 32, 33, 300 and 5,000 rows
+        k = np.concatenate([np.arange(nb - 5365), np.full(32, 7), np.full(33, 8), np.full(300, 9), np.full(5000, 10)])
+    elif case == "sparse":  # one repeat over a range of 3.9 values per row
+        k = rng.choice(int(3.9 * nb), nb, replace=False)
+        k[5] = k[6]
+    elif case == "edge":  # at the top of INT32
+        k = HI - rng.integers(0, nb // 2, nb)
+    else:  # all rows one key
+        k = np.full(3000, 42)
+    return rng.permutation(k)
+
+
+@pytest.mark.parametrize("case", ["twice", "heavy", "sparse", "edge", "one_key"])
+@pytest.mark.parametrize("bt,pt", [(I, I), (L, I), (I, L)])
+def test_repeated_dense_keys(gpu_ctx, case, bt, pt):
+    """The table of repeated dense keys: keys of one row, a few and many
+    (above and below a warp's rounds), NULLs on both sides, results larger
+    than the room made for them, payloads written by the probe and through
+    row ids."""
+    rng = np.random.default_rng(len(case))
+    bkeys = _multi_case(case, rng)
+    nb, n = len(bkeys), 25_000
+    pkeys = np.clip(bkeys[rng.integers(0, nb, n)] + rng.integers(0, 2, n) * rng.integers(0, nb, n), LO, HI)
+    if case == "heavy":
+        pkeys[rng.random(n) < 0.9] = 100  # keep the 5,000-row key rare
+    if case == "one_key":
+        pkeys[100:] = 41
+    bok = (rng.random(nb) >= 0.05).astype(np.uint8)
+    pok = (rng.random(n) >= 0.05).astype(np.uint8)
+    plan = _plan(bkeys, pkeys, bt, pt, bok, pok,
+                 bpay=[(L, np.arange(nb), None), (I, rng.integers(0, 99, nb), (rng.random(nb) > 0.5).astype(np.uint8))],
+                 ppay=[(F, rng.random(n), None)])
+    _check(plan, gpu_ctx, "hash")
+
+
+def test_repeated_dense_keys_in_a_chain(gpu_ctx):
+    """Repeated keys below the root: row ids only, and rows of an
+    intermediate as the probe side."""
+    rng = np.random.default_rng(6)
+    n, d = 30_000, [np.concatenate([rng.permutation(400)] * 3), np.concatenate([rng.permutation(900)] * 2)]
+    plan = Plan()
+    plan.inputs = [ColumnarTable(n, [encode_column(I, x[rng.integers(0, len(x), n)].astype(np.int32),
+                                                   (rng.random(n) > 0.1).astype(np.uint8)) for x in d])]
+    left = plan.new_scan_node(0, [(0, I), (1, I)])
+    types = [I, I]
+    for k, x in enumerate(d):
+        plan.inputs.append(ColumnarTable(len(x), [encode_column(I, x.astype(np.int32)),
+                                                  encode_column(L, np.arange(len(x)))]))
+        scan = plan.new_scan_node(k + 1, [(0, I), (1, L)])
+        left = plan.new_join_node(True, left, scan, k, 0, list(enumerate(types)) + [(len(types) + 1, L)])
+        types = types + [L]
     plan.root = left
     want = run_oracle(plan)
     for flags in (0, _lib.CJ_EXEC_RESULT_ON_DEVICE):
