@@ -571,13 +571,19 @@ void BatchExecutor::materialize_roots() {
     DevPtr pt = upload_tasks(ptasks);
     ck(launch_write_pages_grouped(L, pt->as<PageTask>(), (uint32_t)ptasks.size(), page_grid), "write_pages_grouped");
     if (!var.empty()) {
-        DevPtr totals = ctx.alloc(var.size() * 8);
+        DevPtr totals = ctx.alloc(var.size() * 12); /* page counts, then finished-tile counts */
+        ck(cudaMemsetAsync(totals->ptr, 0, var.size() * 12, ctx.stream), "memset");
+        std::vector<VarcharTask> vtasks(var.size());
         for (size_t k = 0; k < var.size(); ++k) {
             PlanState &p = ps[var[k].plan];
-            ck(launch_varchar_plan(L, p.root_cols[var[k].col], p.root_rows, TR, var[k].temp->ptr,
-                                   totals->as<unsigned long long>() + k),
-               "varchar_plan");
+            VarcharTask &t = vtasks[k];
+            t.col = p.root_cols[var[k].col];
+            t.rows = p.root_rows;
+            t.total_pages = totals->as<unsigned long long>() + k;
+            t.done = reinterpret_cast<unsigned int *>(totals->as<unsigned long long>() + var.size()) + k;
+            place_varchar(t, TR, var[k].temp->ptr);
         }
+        ck(launch_varchar(L, vtasks.data(), vtasks.size(), true), "varchar_plan");
         std::vector<unsigned long long> host(var.size());
         if (mode == Mode::Capture) {
             if (learned->var_pages.size() != var.size())
@@ -598,10 +604,9 @@ void BatchExecutor::materialize_roots() {
             const size_t c = var[k].col;
             res->num_pages[c] = host[k];
             res->dev_pages[c] = ctx.alloc(host[k] * kPageSize);
-            ck(launch_varchar_write(L, p.root_cols[c], p.root_rows, TR, var[k].temp->ptr,
-                                    res->dev_pages[c]->as<uint8_t>()),
-               "varchar_write");
+            vtasks[k].out = res->dev_pages[c]->as<uint8_t>();
         }
+        ck(launch_varchar(L, vtasks.data(), vtasks.size(), false), "varchar_write");
     }
     if (flags & CJ_EXEC_RESULT_ON_DEVICE) return;
     for (auto &p : ps) {

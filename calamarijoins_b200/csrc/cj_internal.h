@@ -485,13 +485,23 @@ cudaError_t launch_write_pages_grouped(const Launch &L, const PageTask *tasks_de
 
 /* Output pages */
 uint32_t rows_per_page_fixed(int32_t type);
+/* One VARCHAR result column. launch_varchar with `plan` cuts its rows into
+ * pages and leaves their number in *total_pages (done and total_pages zero
+ * before); without it the pages are written to `out`, sized by that number. */
+struct VarcharTask {
+    ColView col;
+    uint64_t rows;
+    unsigned int *done;
+    unsigned long long *total_pages;
+    uint8_t *out;
+    uint32_t tile_rows, tiles; /* from here on: place_varchar */
+    uint32_t *tile_pages, *nseg, *seg, *seg_page;
+    uint64_t *tile_base, *row_desc;
+    uint32_t tile_first;
+};
+constexpr int kVarcharArgs = 16; /* tasks passed by value */
 size_t varchar_temp_bytes(uint64_t rows, uint32_t tile_rows);
-/* Pass 1: page count per tile; total pages into *total_pages_dev. */
-cudaError_t launch_varchar_plan(const Launch &L, const ColView &col, uint64_t rows,
-                                uint32_t tile_rows, void *temp,
-                                unsigned long long *total_pages_dev);
-/* Pass 2: write pages (out_pages sized by pass 1's total). */
-cudaError_t launch_varchar_write(const Launch &L, const ColView &col, uint64_t rows,
-                                 uint32_t tile_rows, void *temp, uint8_t *out_pages);
+void place_varchar(VarcharTask &t, uint32_t tile_rows, void *temp);
+cudaError_t launch_varchar(const Launch &L, const VarcharTask *tasks, size_t n, bool plan);
 
 } // namespace cj

@@ -783,30 +783,38 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
     {
         PhaseScope ph(*this, PH_MAT);
         const uint32_t TR = (uint32_t)std::max<int64_t>(64, std::min<int64_t>(ctx.opt.varchar_tile_rows, 8192));
-        std::vector<DevPtr> vtemp(nc);
+        std::vector<DevPtr> vtemp;
+        std::vector<VarcharTask> vtasks;
+        std::vector<int> vtask_of(nc, -1); /* a VARCHAR column's task */
         DevPtr totals;
         size_t nvar = 0;
         for (size_t c = 0; c < nc; ++c)
             if (types[c] == CJ_VARCHAR) ++nvar;
         if (rows && nvar) {
-            totals = ctx.alloc(nvar * 8);
-            size_t k = 0;
+            totals = ctx.alloc(nvar * 12); /* page counts, then finished-tile counts */
+            ck(cudaMemsetAsync(totals->ptr, 0, nvar * 12, ctx.stream), "memset");
             for (size_t c = 0; c < nc; ++c) {
                 if (types[c] != CJ_VARCHAR) continue;
-                vtemp[c] = ctx.alloc(varchar_temp_bytes(rows, TR));
-                const ColView cv = out_view(cols[c]);
+                const size_t k = vtasks.size();
+                vtask_of[c] = (int)k;
+                vtemp.push_back(ctx.alloc(varchar_temp_bytes(rows, TR)));
+                VarcharTask t{};
+                t.col = out_view(cols[c]);
+                t.rows = rows;
+                t.total_pages = totals->as<unsigned long long>() + k;
+                t.done = reinterpret_cast<unsigned int *>(totals->as<unsigned long long>() + nvar) + k;
+                place_varchar(t, TR, vtemp.back()->ptr);
+                vtasks.push_back(t);
+            }
+            {
                 KScope ks(*this, "varchar_plan");
-                ck(launch_varchar_plan(L, cv, rows, TR, vtemp[c]->ptr,
-                                       totals->as<unsigned long long>() + k),
-                   "varchar_plan");
-                ++k;
+                ck(launch_varchar(L, vtasks.data(), vtasks.size(), true), "varchar_plan");
             }
             std::vector<unsigned long long> host(nvar);
             ck(cudaMemcpyAsync(host.data(), totals->ptr, nvar * 8, cudaMemcpyDeviceToHost, ctx.stream), "copy");
             sync();
-            k = 0;
             for (size_t c = 0; c < nc; ++c)
-                if (types[c] == CJ_VARCHAR) res->num_pages[c] = host[k++];
+                if (types[c] == CJ_VARCHAR) res->num_pages[c] = host[vtask_of[c]];
         }
         uint64_t total_pages = 0;
         for (size_t c = 0; c < nc; ++c) {
@@ -869,8 +877,12 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
             }
             t.out = res->dev_pages[c]->as<uint8_t>();
             if (types[c] == CJ_VARCHAR) {
-                KScope ks(*this, "varchar_write");
-                ck(launch_varchar_write(L, t.col, rows, TR, vtemp[c]->ptr, t.out), "varchar_write");
+                VarcharTask &v = vtasks[vtask_of[c]];
+                v.out = t.out;
+                if (to_host) {
+                    KScope ks(*this, "varchar_write");
+                    ck(launch_varchar(L, &v, 1, false), "varchar_write");
+                }
             } else if (alias[c] < 0) {
                 ptasks.push_back(t);
                 if (to_host) write_pages();
@@ -892,6 +904,10 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
             }
         }
         if (!ptasks.empty()) write_pages();
+        if (!to_host && !vtasks.empty()) {
+            KScope ks(*this, "varchar_write");
+            ck(launch_varchar(L, vtasks.data(), vtasks.size(), false), "varchar_write");
+        }
     }
     if (dl.first) {
         dl.last = ctx.get_event();

@@ -310,15 +310,20 @@ class Filter {
                     pt.out = cp.owner->as<uint8_t>();
                     check_cuda(launch_write_pages(L, &pt, 1), "write_pages");
                 } else {
-                    DevPtr temp = ctx.alloc(varchar_temp_bytes(count, TR));
-                    check_cuda(launch_varchar_plan(L, v, count, TR, temp->ptr,
-                                                   reinterpret_cast<unsigned long long *>(&ctx.d_status->aux)),
-                               "varchar_plan");
+                    DevPtr temp = ctx.alloc(varchar_temp_bytes(count, TR)), done = ctx.alloc(4);
+                    check_cuda(cudaMemsetAsync(done->ptr, 0, 4, ctx.stream), "memset");
+                    VarcharTask vt{};
+                    vt.col = v;
+                    vt.rows = count;
+                    vt.done = done->as<unsigned int>();
+                    vt.total_pages = &ctx.d_status->aux;
+                    place_varchar(vt, TR, temp->ptr);
+                    check_cuda(launch_varchar(L, &vt, 1, true), "varchar_plan");
                     ctx.sync_status(); /* brings the page count back in aux */
                     cp.num_pages = ctx.h_status->aux;
                     cp.owner = ctx.alloc(cp.num_pages * kPageSize);
-                    check_cuda(launch_varchar_write(L, v, count, TR, temp->ptr, cp.owner->as<uint8_t>()),
-                               "varchar_write");
+                    vt.out = cp.owner->as<uint8_t>();
+                    check_cuda(launch_varchar(L, &vt, 1, false), "varchar_write");
                 }
                 cp.dev = cp.owner->as<uint8_t>();
             }

@@ -22,11 +22,11 @@
  * VARCHAR pages (k_varchar_plan / k_varchar_write): rows are cut into tiles;
  * within a tile pages are packed greedily in row order like
  * ColumnInserter<std::string> (plan.h:340-369): a page takes rows while
- * 4 + 2*n_values + chars + ceil(n_rows/8) <= 8192, found by binary search on
- * the tile's prefix sums. A string longer than 8185 bytes arrives as a chain
- * of long-string pages and is copied verbatim, as VarcharPageBuilder::
- * copy_long_string_pages does (page_builders.h:345-362). Pass 1 counts each
- * tile's pages, a scan places them, pass 2 writes them.
+ * 4 + 2*n_values + chars + ceil(n_rows/8) <= 8192. A string longer than 8185
+ * bytes arrives as a chain of long-string pages and is copied verbatim, as
+ * VarcharPageBuilder::copy_long_string_pages does (page_builders.h:345-362).
+ * Pass 1 cuts every tile into segments (a page, or a long string's chain) and
+ * places the tiles' pages, pass 2 writes a segment per CTA.
  */
 #include <algorithm>
 
@@ -294,217 +294,262 @@ __global__ void k_gather_grouped(const GatherTask *__restrict__ tasks, uint32_t 
     }
 }
 
-/* ---------------- VARCHAR ---------------- */
-struct VarSmem {
-    uint64_t *desc;     /* TR   row descriptors (0 = NULL)                 */
-    uint32_t *lpre;     /* TR+1 prefix of short-string bytes               */
-    uint32_t *vpre;     /* TR+1 prefix of short non-NULL rows              */
-    uint32_t *longpre;  /* TR+1 prefix of long-string rows                 */
-    uint32_t *seg;      /* TR+1 first row of each segment                  */
-    uint32_t *segpg;    /* TR+1 first output page of each segment          */
-};
+/* ---------------- VARCHAR ----------------
+ * Weights: a page holds rows a..b-1 when 8 (2 values + characters) + rows <=
+ * 8 * 8188, so a row weighs 1, plus 16 and 8 a character when it is not NULL,
+ * and a page's rows weigh kPageWeight at most. A long string's row weighs
+ * more than a page by itself, which ends the segment before it. */
+constexpr uint32_t kPageWeight = 8 * (kPageSize - 4);
 
-CJ_DEV VarSmem carve(uint8_t *base, uint32_t TR) {
-    VarSmem s;
-    s.desc = reinterpret_cast<uint64_t *>(base);
-    uint32_t *u = reinterpret_cast<uint32_t *>(base + (size_t)TR * 8);
-    s.lpre = u;
-    s.vpre = u + (TR + 1);
-    s.longpre = u + 2 * (TR + 1);
-    s.seg = u + 3 * (TR + 1);
-    s.segpg = u + 4 * (TR + 1);
-    return s;
+CJ_DEV uint32_t row_weight(uint64_t d) {
+    if (!d) return 1u;
+    return desc_is_long(d) ? kPageWeight + 1u : 17u + 8u * desc_len(d);
 }
 
-/* Loads the tile's descriptors, builds the prefix sums and cuts the tile
- * into segments (one normal page, or one long string's chain). Returns the
- * segment count; the page count is in s.segpg[nseg]. Block-wide. */
-CJ_DEV uint32_t plan_tile(const ColView &col, uint64_t r0, uint32_t nt, uint32_t TR,
-                          const VarSmem &s, uint32_t *wbuf, uint32_t *s_nseg) {
-    const bool all_valid = col_all_valid(col);
-    for (uint32_t r = threadIdx.x; r < nt; r += blockDim.x) {
-        uint32_t br = base_row(col, (uint32_t)(r0 + r));
-        s.desc[r] = (all_valid || valid_bit(col.valid, br)) ? __ldg(col.str_desc + br) : 0ull;
-    }
-    __syncthreads();
-    const uint32_t per = (TR + blockDim.x - 1) / blockDim.x;
-    const uint32_t q0 = threadIdx.x * per;
-    uint32_t lsum = 0, vsum = 0, gsum = 0;
-    for (uint32_t k = 0; k < per; ++k) {
-        uint32_t r = q0 + k;
-        if (r >= nt) break;
-        uint64_t d = s.desc[r];
-        if (!d) continue;
-        if (desc_is_long(d)) ++gsum;
-        else {
-            lsum += desc_len(d);
-            ++vsum;
+/* Cuts tile t of a column into segments: the rows' descriptors (through the
+ * row ids, eight a thread in flight) go to row_desc in row order, a block
+ * scan of the weights to shared memory, and the first warp walks the
+ * segments, 32 candidate ends a step. The last tile of the column to finish
+ * turns the tiles' page counts into their first pages. Bound by the random
+ * descriptor loads (32 bytes of L2 each). 1.8M rows: 20 us, before 60 us
+ * with a thread walking 11 dependent steps a segment. */
+CJ_DEV void plan_tile(const VarcharTask &T, uint32_t t, uint32_t *s_pre, uint32_t *wbuf, uint64_t *wbuf64,
+                      bool *s_last) {
+    const uint32_t TR = T.tile_rows;
+    const uint64_t r0 = (uint64_t)t * TR;
+    const uint32_t nt = (uint32_t)min((uint64_t)TR, T.rows - r0);
+    const bool all_valid = col_all_valid(T.col);
+    constexpr int kBatch = 8;
+    for (uint32_t b0 = threadIdx.x; b0 < nt; b0 += kMatThreads * kBatch) {
+        uint32_t br[kBatch];
+        uint64_t d[kBatch];
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const uint32_t r = b0 + k * kMatThreads;
+            br[k] = (uint32_t)(r0 + r);
+            if (r < nt && T.col.rid_a) br[k] = __ldg(T.col.rid_a + br[k]);
+        }
+        if (T.col.rid_b) {
+#pragma unroll
+            for (int k = 0; k < kBatch; ++k)
+                if (b0 + k * kMatThreads < nt) br[k] = __ldg(T.col.rid_b + br[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            d[k] = 0;
+            if (b0 + k * kMatThreads < nt && (all_valid || valid_bit(T.col.valid, br[k])))
+                d[k] = __ldg(T.col.str_desc + br[k]);
+        }
+#pragma unroll
+        for (int k = 0; k < kBatch; ++k) {
+            const uint32_t r = b0 + k * kMatThreads;
+            if (r >= nt) continue;
+            T.row_desc[r0 + r] = d[k];
+            s_pre[r] = row_weight(d[k]);
         }
     }
-    uint32_t ltot, vtot, gtot;
-    uint32_t lp = block_exclusive_scan<uint32_t>(lsum, wbuf, &ltot);
-    uint32_t vp = block_exclusive_scan<uint32_t>(vsum, wbuf, &vtot);
-    uint32_t gp = block_exclusive_scan<uint32_t>(gsum, wbuf, &gtot);
-    for (uint32_t k = 0; k < per; ++k) {
-        uint32_t r = q0 + k;
-        if (r >= nt) break;
-        s.lpre[r] = lp;
-        s.vpre[r] = vp;
-        s.longpre[r] = gp;
-        uint64_t d = s.desc[r];
-        if (d) {
-            if (desc_is_long(d)) ++gp;
-            else {
-                lp += desc_len(d);
-                ++vp;
-            }
-        }
-    }
-    if (threadIdx.x == 0) {
-        s.lpre[nt] = ltot;
-        s.vpre[nt] = vtot;
-        s.longpre[nt] = gtot;
-    }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    /* exclusive prefix of the weights, each thread a run of rows */
+    const uint32_t per = (nt + kMatThreads - 1) / kMatThreads, q0 = min(threadIdx.x * per, nt), q1 = min(q0 + per, nt);
+    uint32_t sum = 0, total;
+    for (uint32_t r = q0; r < q1; ++r) sum += s_pre[r];
+    uint32_t pre = block_exclusive_scan<uint32_t>(sum, wbuf, &total);
+    for (uint32_t r = q0; r < q1; ++r) {
+        const uint32_t w = s_pre[r];
+        s_pre[r] = pre;
+        pre += w;
+    }
+    if (threadIdx.x == 0) s_pre[nt] = total;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint32_t lane = lane_id();
+        uint32_t *seg = T.seg + (uint64_t)t * (TR + 1), *seg_page = T.seg_page + (uint64_t)t * (TR + 1);
         uint32_t a = 0, ns = 0, np = 0;
         while (a < nt) {
-            s.seg[ns] = a;
-            s.segpg[ns] = np;
-            uint64_t d = s.desc[a];
-            if (d && desc_is_long(d)) {
-                np += desc_len(d);
-                a += 1;
+            if (lane == 0) {
+                seg[ns] = a;
+                seg_page[ns] = np;
+            }
+            uint32_t end, pages = 1;
+            if (s_pre[a + 1] - s_pre[a] > kPageWeight) { /* a long string */
+                end = a + 1;
+                pages = desc_len(T.row_desc[r0 + a]);
             } else {
+                /* the largest end with s_pre[end] - s_pre[a] <= kPageWeight,
+                 * at least a + 1 */
                 uint32_t lo = a + 1, hi = nt;
                 while (lo < hi) {
-                    uint32_t mid = (lo + hi + 1) >> 1;
-                    uint32_t n = mid - a;
-                    bool ok = s.longpre[mid] == s.longpre[a] && n <= 65533u &&
-                              4u + 2u * (s.vpre[mid] - s.vpre[a]) + (s.lpre[mid] - s.lpre[a]) +
-                                      (n + 7) / 8 <= kPageSize;
-                    if (ok) lo = mid;
-                    else hi = mid - 1;
+                    const uint32_t step = (hi - lo + 31) / 32, e = lo + step * (lane + 1);
+                    const bool ok = e <= hi && s_pre[e] - s_pre[a] <= kPageWeight;
+                    const uint32_t n = __popc(__ballot_sync(0xffffffffu, ok)); /* a prefix of the lanes */
+                    const uint32_t next = lo + step * n;
+                    hi = min(hi, next + step - 1);
+                    lo = next;
                 }
-                np += 1;
-                a = lo;
+                end = lo;
             }
+            np += pages;
             ++ns;
+            a = end;
         }
-        s.seg[ns] = nt;
-        s.segpg[ns] = np;
-        *s_nseg = ns;
+        if (lane == 0) {
+            seg[ns] = nt;
+            T.nseg[t] = ns;
+            T.tile_pages[t] = np;
+            __threadfence();
+            *s_last = atomicAdd(T.done, 1u) == T.tiles - 1;
+        }
     }
     __syncthreads();
-    return *s_nseg;
-}
-
-__global__ void __launch_bounds__(kMatThreads)
-    k_varchar_plan(ColView col, uint64_t rows, uint32_t TR, uint32_t *__restrict__ tile_pages) {
-    extern __shared__ __align__(16) uint8_t dsm[];
-    __shared__ uint32_t wbuf[kMatThreads / 32 + 1];
-    __shared__ uint32_t s_nseg;
-    VarSmem s = carve(dsm, TR);
-    const uint64_t tiles = (rows + TR - 1) / TR;
-    for (uint64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const uint64_t r0 = t * TR;
-        const uint32_t nt = (uint32_t)min((uint64_t)TR, rows - r0);
-        uint32_t ns = plan_tile(col, r0, nt, TR, s, wbuf, &s_nseg);
-        if (threadIdx.x == 0) tile_pages[t] = s.segpg[ns];
-        __syncthreads();
-    }
-}
-
-__global__ void __launch_bounds__(kMatThreads)
-    k_varchar_write(ColView col, uint64_t rows, uint32_t TR, const uint64_t *__restrict__ tile_base,
-                    uint8_t *__restrict__ out) {
-    extern __shared__ __align__(16) uint8_t dsm[];
-    __shared__ uint4 s_page[kPageSize / 16];
-    __shared__ uint32_t wbuf[kMatThreads / 32 + 1];
-    __shared__ uint32_t s_nseg;
-    VarSmem s = carve(dsm, TR);
-    uint8_t *sp = reinterpret_cast<uint8_t *>(s_page);
-    const uint32_t warp = threadIdx.x >> 5, lane = lane_id(), nwarps = blockDim.x >> 5;
-    const uint64_t tiles = (rows + TR - 1) / TR;
-    for (uint64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
-        const uint64_t r0 = t * TR;
-        const uint32_t nt = (uint32_t)min((uint64_t)TR, rows - r0);
-        const uint32_t ns = plan_tile(col, r0, nt, TR, s, wbuf, &s_nseg);
-        const uint64_t base = tile_base[t];
-        for (uint32_t g = 0; g < ns; ++g) {
-            const uint32_t a = s.seg[g], b = s.seg[g + 1];
-            const uint64_t opg = base + s.segpg[g];
-            const uint64_t d0 = s.desc[a];
-            if (d0 && desc_is_long(d0)) {
-                const uint4 *src = reinterpret_cast<const uint4 *>(col.pages + desc_pos(d0) * kPageSize);
-                uint4 *dst = reinterpret_cast<uint4 *>(out + opg * kPageSize);
-                const uint64_t n16 = (uint64_t)desc_len(d0) * (kPageSize / 16);
-                for (uint64_t k = threadIdx.x; k < n16; k += blockDim.x) dst[k] = __ldg(src + k);
-                continue;
-            }
-            for (uint32_t k = threadIdx.x; k < kPageSize / 16; k += blockDim.x) s_page[k] = make_uint4(0, 0, 0, 0);
-            __syncthreads();
-            const uint32_t n = b - a, nv = s.vpre[b] - s.vpre[a];
-            const uint32_t chars_at = 4u + 2u * nv;
-            const uint32_t bm_bytes = (n + 7) / 8;
-            uint8_t *bm = sp + kPageSize - bm_bytes;
-            uint16_t *offs = reinterpret_cast<uint16_t *>(sp + 4);
-            /* offsets, bitmap and short strings */
-            for (uint32_t j0 = 0; j0 < n; j0 += blockDim.x) {
-                const uint32_t j = j0 + threadIdx.x;
-                bool v = false;
-                if (j < n) {
-                    const uint32_t r = a + j;
-                    const uint64_t d = s.desc[r];
-                    if (d) {
-                        v = true;
-                        const uint32_t k = s.vpre[r] - s.vpre[a];
-                        const uint32_t beg = s.lpre[r] - s.lpre[a];
-                        const uint32_t len = desc_len(d);
-                        offs[k] = (uint16_t)(beg + len);
-                        if (len <= 32) {
-                            const uint8_t *src = col.pages + desc_pos(d);
-                            uint8_t *dst = sp + chars_at + beg;
-                            for (uint32_t q = 0; q < len; ++q) dst[q] = __ldg(src + q);
-                        }
-                    }
-                }
-                uint32_t ball = __ballot_sync(0xffffffffu, v);
-                if (lane < 4) {
-                    uint32_t byte = (j0 + warp * 32) / 8 + lane;
-                    if (byte < bm_bytes) bm[byte] = (uint8_t)(ball >> (8 * lane));
-                }
-            }
-            /* longer strings: one warp per string */
-            for (uint32_t r = a + warp; r < b; r += nwarps) {
-                const uint64_t d = s.desc[r];
-                if (!d || desc_len(d) <= 32) continue;
-                const uint8_t *src = col.pages + desc_pos(d);
-                uint8_t *dst = sp + chars_at + (s.lpre[r] - s.lpre[a]);
-                const uint32_t len = desc_len(d);
-                for (uint32_t q = lane; q < len; q += 32) dst[q] = __ldg(src + q);
-            }
-            if (threadIdx.x == 0) {
-                reinterpret_cast<uint16_t *>(sp)[0] = (uint16_t)n;
-                reinterpret_cast<uint16_t *>(sp)[1] = (uint16_t)nv;
-            }
-            __syncthreads();
-            uint4 *dst = reinterpret_cast<uint4 *>(out + opg * kPageSize);
-            for (uint32_t k = threadIdx.x; k < kPageSize / 16; k += blockDim.x) dst[k] = s_page[k];
-            __syncthreads();
+    if (!*s_last) return;
+    __threadfence();
+    uint64_t off = 0;
+    constexpr uint32_t kRun = 8;
+    for (uint32_t c0 = 0; c0 < T.tiles; c0 += kMatThreads * kRun) {
+        uint32_t v[kRun];
+        uint64_t s = 0, tot;
+#pragma unroll
+        for (uint32_t k = 0; k < kRun; ++k) {
+            const uint32_t c = c0 + threadIdx.x * kRun + k;
+            v[k] = c < T.tiles ? __ldcg(T.tile_pages + c) : 0u;
+            s += v[k];
         }
-        __syncthreads();
+        uint64_t e = off + block_exclusive_scan<uint64_t>(s, wbuf64, &tot);
+#pragma unroll
+        for (uint32_t k = 0; k < kRun; ++k) {
+            const uint32_t c = c0 + threadIdx.x * kRun + k;
+            if (c < T.tiles) T.tile_base[c] = e;
+            e += v[k];
+        }
+        off += tot;
     }
+    if (threadIdx.x == 0) *T.total_pages = off;
 }
 
-size_t var_dyn_smem(uint32_t TR) { return (size_t)TR * 8 + 5 * ((size_t)TR + 1) * 4; }
+/* Writes segment g of tile t. Block-wide. */
+struct VarcharShared {
+    uint4 page[kPageSize / 16];
+    uint64_t src[kMatThreads]; /* a string's first character, by row of the chunk */
+    uint16_t dst[kMatThreads], len[kMatThreads];
+    uint32_t wbuf[kMatThreads / 32 + 1];
+};
+constexpr uint32_t kCopyLanes = 8;    /* lanes that copy a string together      */
+constexpr uint32_t kBlockCopy = 256;  /* longer strings are copied by the block */
 
-bool g_var_attrs = false;
-void set_var_attrs() {
-    if (g_var_attrs) return;
-    cudaFuncSetAttribute(k_varchar_plan, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    cudaFuncSetAttribute(k_varchar_write, cudaFuncAttributeMaxDynamicSharedMemorySize, 190 * 1024);
-    g_var_attrs = true;
+/* Characters q .. q + 3 of a string at src (fewer at its end) to shared
+ * memory: one or two aligned words, no byte outside the string's words. */
+CJ_DEV void copy4(const uint8_t *src, uint8_t *dst, uint32_t q, uint32_t len) {
+    const uint32_t n = min(4u, len - q);
+    const uintptr_t s = reinterpret_cast<uintptr_t>(src + q);
+    const uint32_t sh = (uint32_t)(s & 3u);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(s & ~(uintptr_t)3);
+    const uint32_t lo = __ldg(w), hi = sh + n > 4 ? __ldg(w + 1) : 0u;
+    const uint32_t v = __funnelshift_r(lo, hi, 8 * sh);
+    dst[q] = (uint8_t)v;
+    if (n > 1) dst[q + 1] = (uint8_t)(v >> 8);
+    if (n > 2) dst[q + 2] = (uint8_t)(v >> 16);
+    if (n > 3) dst[q + 3] = (uint8_t)(v >> 24);
+}
+
+CJ_DEV void write_segment(const VarcharTask &T, uint32_t t, uint32_t g, VarcharShared &sh) {
+    const uint64_t r0 = (uint64_t)t * T.tile_rows, s0 = (uint64_t)t * (T.tile_rows + 1);
+    const uint32_t a = T.seg[s0 + g], n = T.seg[s0 + g + 1] - a;
+    uint8_t *out = T.out + (T.tile_base[t] + T.seg_page[s0 + g]) * kPageSize;
+    const uint64_t *desc = T.row_desc + r0 + a;
+    const uint64_t d0 = desc[0];
+    if (d0 && desc_is_long(d0)) {
+        const uint4 *src = reinterpret_cast<const uint4 *>(T.col.pages + desc_pos(d0) * kPageSize);
+        uint4 *dst = reinterpret_cast<uint4 *>(out);
+        const uint64_t n16 = (uint64_t)desc_len(d0) * (kPageSize / 16);
+        for (uint64_t k = threadIdx.x; k < n16; k += kMatThreads) dst[k] = __ldg(src + k);
+        return;
+    }
+    const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
+    uint8_t *sp = reinterpret_cast<uint8_t *>(sh.page);
+    /* the number of values says where the characters begin */
+    uint32_t mine = 0, nv;
+    for (uint32_t j = threadIdx.x; j < n; j += kMatThreads) mine += desc[j] != 0;
+    for (uint32_t k = threadIdx.x; k < kPageSize / 16; k += kMatThreads) sh.page[k] = make_uint4(0, 0, 0, 0);
+    block_exclusive_scan<uint32_t>(mine, sh.wbuf, &nv);
+    const uint32_t chars_at = 4u + 2u * nv, bm_bytes = (n + 7) / 8;
+    uint8_t *bm = sp + kPageSize - bm_bytes;
+    uint16_t *offs = reinterpret_cast<uint16_t *>(sp + 4);
+    uint32_t before = 0; /* characters (low half) and values (high half) of earlier chunks */
+    for (uint32_t j0 = 0; j0 < n; j0 += kMatThreads) {
+        const uint32_t j = j0 + threadIdx.x;
+        const uint64_t d = j < n ? desc[j] : 0ull;
+        const uint32_t len = d ? desc_len(d) : 0u;
+        uint32_t total;
+        /* at most 8188 characters and 4094 values a page: no carry between the halves */
+        const uint32_t pre = before + block_exclusive_scan<uint32_t>(len | (d ? 1u << 16 : 0u), sh.wbuf, &total);
+        before += total;
+        const uint32_t beg = pre & 0xFFFFu;
+        if (d) offs[pre >> 16] = (uint16_t)(beg + len);
+        sh.src[threadIdx.x] = d ? desc_pos(d) : 0ull;
+        sh.dst[threadIdx.x] = (uint16_t)(chars_at + beg);
+        sh.len[threadIdx.x] = (uint16_t)len;
+        const uint32_t ball = __ballot_sync(0xffffffffu, d != 0);
+        if (lane < 4) {
+            const uint32_t byte = (j0 + warp * 32) / 8 + lane;
+            if (byte < bm_bytes) bm[byte] = (uint8_t)(ball >> (8 * lane));
+        }
+        const bool long_ones = __syncthreads_or(len > kBlockCopy);
+        const uint32_t rows = min((uint32_t)kMatThreads, n - j0);
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x / kCopyLanes; i < rows; i += kMatThreads / kCopyLanes) {
+            const uint32_t l = sh.len[i];
+            if (l > kBlockCopy) continue;
+            const uint8_t *src = T.col.pages + sh.src[i];
+            for (uint32_t q = (threadIdx.x % kCopyLanes) * 4; q < l; q += kCopyLanes * 4)
+                copy4(src, sp + sh.dst[i], q, l);
+        }
+        if (long_ones)
+            for (uint32_t i = 0; i < rows; ++i) {
+                const uint32_t l = sh.len[i];
+                if (l <= kBlockCopy) continue;
+                for (uint32_t q = threadIdx.x * 4; q < l; q += kMatThreads * 4)
+                    copy4(T.col.pages + sh.src[i], sp + sh.dst[i], q, l);
+            }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *reinterpret_cast<uint32_t *>(sp) = n | (nv << 16);
+    __syncthreads();
+    uint4 *dst = reinterpret_cast<uint4 *>(out);
+    for (uint32_t k = threadIdx.x; k < kPageSize / 16; k += kMatThreads) __stcs(dst + k, sh.page[k]);
+    __syncthreads();
+}
+
+/* Columns of a result, by value. Pass 1: a block per tile; pass 2:
+ * kSegBlocks blocks per tile, which share its segments (about six at 22
+ * bytes a string and 2,048 rows). */
+constexpr uint32_t kSegBlocks = 8;
+struct VarcharArgs {
+    VarcharTask t[kVarcharArgs];
+    uint32_t n;
+};
+CJ_DEV uint32_t find_varchar(const VarcharArgs &a, uint32_t tile) {
+    uint32_t c = 0;
+    while (c + 1 < a.n && a.t[c + 1].tile_first <= tile) ++c;
+    return c;
+}
+
+__global__ void __launch_bounds__(kMatThreads) k_varchar_plan(const __grid_constant__ VarcharArgs a) {
+    extern __shared__ uint32_t s_pre[];
+    __shared__ uint32_t wbuf[kMatThreads / 32 + 1];
+    __shared__ uint64_t wbuf64[kMatThreads / 32 + 1];
+    __shared__ bool s_last;
+    const VarcharTask &T = a.t[find_varchar(a, blockIdx.x)];
+    plan_tile(T, blockIdx.x - T.tile_first, s_pre, wbuf, wbuf64, &s_last);
+}
+
+/* 1.8M strings of 20 characters on average: 74 us, before 212 us with a
+ * block per tile that planned it again and a lane per string, byte by byte. */
+__global__ void __launch_bounds__(kMatThreads, 6) k_varchar_write(const __grid_constant__ VarcharArgs a) {
+    __shared__ VarcharShared sh;
+    const uint32_t tile = blockIdx.x / kSegBlocks;
+    const VarcharTask &T = a.t[find_varchar(a, tile)];
+    const uint32_t t = tile - T.tile_first, ns = T.nseg[t];
+    for (uint32_t g = blockIdx.x % kSegBlocks; g < ns; g += kSegBlocks) write_segment(T, t, g, sh);
 }
 
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -568,45 +613,53 @@ uint32_t rows_per_page_fixed(int32_t type) {
     return type == CJ_INT32 ? kRowsPerPageInt32 : kRowsPerPage8B;
 }
 
+/* temp: page counts and first pages of the tiles, segment counts, the
+ * segments' first rows and pages, the rows' descriptors */
 size_t varchar_temp_bytes(uint64_t rows, uint32_t TR) {
-    uint64_t tiles = (rows + TR - 1) / TR;
-    return align256(tiles * 4) + align256((tiles + 1) * 8) + scan_temp_bytes(tiles) + 256;
+    const uint64_t tiles = (rows + TR - 1) / TR, segs = tiles * (TR + 1ull);
+    return align256(tiles * 4) * 2 + align256(tiles * 8) + align256(segs * 4) * 2 + align256(rows * 8);
 }
 
-cudaError_t launch_varchar_plan(const Launch &L, const ColView &col, uint64_t rows, uint32_t TR,
-                                void *temp, unsigned long long *total_pages_dev) {
-    set_var_attrs();
-    const uint64_t tiles = (rows + TR - 1) / TR;
-    char *t = reinterpret_cast<char *>(temp);
-    uint32_t *tile_pages = reinterpret_cast<uint32_t *>(t);
-    uint64_t *tile_base = reinterpret_cast<uint64_t *>(t + align256(tiles * 4));
-    void *scan_tmp = t + align256(tiles * 4) + align256((tiles + 1) * 8);
-    if (tiles) {
-        uint64_t g = tiles, cap = (uint64_t)L.num_sms * 2;
-        if (g > cap) g = cap;
-        k_varchar_plan<<<(unsigned)g, kMatThreads, var_dyn_smem(TR), L.stream>>>(col, rows, TR, tile_pages);
+void place_varchar(VarcharTask &t, uint32_t TR, void *temp) {
+    const uint64_t tiles = (t.rows + TR - 1) / TR, segs = tiles * (TR + 1ull);
+    char *p = reinterpret_cast<char *>(temp);
+    auto take = [&](uint64_t bytes) {
+        char *q = p;
+        p += align256(bytes);
+        return q;
+    };
+    t.tile_rows = TR;
+    t.tiles = (uint32_t)tiles;
+    t.tile_pages = reinterpret_cast<uint32_t *>(take(tiles * 4));
+    t.nseg = reinterpret_cast<uint32_t *>(take(tiles * 4));
+    t.tile_base = reinterpret_cast<uint64_t *>(take(tiles * 8));
+    t.seg = reinterpret_cast<uint32_t *>(take(segs * 4));
+    t.seg_page = reinterpret_cast<uint32_t *>(take(segs * 4));
+    t.row_desc = reinterpret_cast<uint64_t *>(take(t.rows * 8));
+}
+
+cudaError_t launch_varchar(const Launch &L, const VarcharTask *tasks, size_t n, bool plan) {
+    for (size_t k = 0; k < n;) {
+        VarcharArgs a;
+        a.n = 0;
+        uint64_t tiles = 0;
+        size_t smem = 0;
+        while (k < n && a.n < kVarcharArgs && (tiles + tasks[k].tiles) * kSegBlocks < (1ull << 31)) {
+            a.t[a.n] = tasks[k++];
+            a.t[a.n].tile_first = (uint32_t)tiles;
+            tiles += a.t[a.n].tiles;
+            smem = std::max(smem, ((size_t)a.t[a.n].tile_rows + 1) * 4);
+            ++a.n;
+        }
+        if (!a.n) return cudaErrorInvalidValue;
+        if (!tiles) continue;
+        if (plan) k_varchar_plan<<<(unsigned)tiles, kMatThreads, smem, L.stream>>>(a);
+        else k_varchar_write<<<(unsigned)(tiles * kSegBlocks), kMatThreads, 0, L.stream>>>(a);
         count_launches(1);
-        cudaError_t e = cudaGetLastError();
+        const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    cudaError_t e = scan_u32_to_u64(L, tile_pages, tile_base, tiles, scan_tmp);
-    if (e != cudaSuccess) return e;
-    return cudaMemcpyAsync(total_pages_dev, tile_base + tiles, sizeof(unsigned long long),
-                           cudaMemcpyDeviceToDevice, L.stream);
-}
-
-cudaError_t launch_varchar_write(const Launch &L, const ColView &col, uint64_t rows, uint32_t TR,
-                                 void *temp, uint8_t *out) {
-    set_var_attrs();
-    const uint64_t tiles = (rows + TR - 1) / TR;
-    if (!tiles) return cudaSuccess;
-    const uint64_t *tile_base =
-        reinterpret_cast<const uint64_t *>(reinterpret_cast<char *>(temp) + align256(tiles * 4));
-    uint64_t g = tiles, cap = (uint64_t)L.num_sms * 2;
-    if (g > cap) g = cap;
-    k_varchar_write<<<(unsigned)g, kMatThreads, var_dyn_smem(TR), L.stream>>>(col, rows, TR, tile_base, out);
-    count_launches(1);
-    return cudaGetLastError();
+    return cudaSuccess;
 }
 
 } // namespace cj
