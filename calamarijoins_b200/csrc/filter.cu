@@ -30,6 +30,7 @@
  */
 #include <algorithm>
 #include <functional>
+#include <map>
 #include <set>
 #include <string>
 #include <vector>
@@ -73,6 +74,7 @@ struct StrView {
         cur_start = 0;
         cur_count = page_count(pg + first * kPageSize);
     }
+    CJ_DEV uint32_t skip_to(uint32_t i, uint32_t, uint32_t) { return i; }
     CJ_DEV uint8_t at(uint32_t i) {
         if (!is_long) return p[i];
         while (i >= cur_start + cur_count && cur_page + 1 < chain) {
@@ -89,8 +91,84 @@ struct StrView {
     }
 };
 
+/* A short string read forwards and back by bytes: the aligned word around
+ * the last byte stays in a register, so a string costs a load per four
+ * characters, not one per character looked at (32 lanes' bytes are 32
+ * sectors). */
+struct ShortStr {
+    const uint8_t *p;
+    uint32_t len;
+    uintptr_t at_word = 0;
+    uint32_t word = 0;
+    CJ_DEV ShortStr(const uint8_t *pg, uint64_t desc) : p(pg + desc_pos(desc)), len(desc_len(desc)) {}
+    CJ_DEV uint32_t aligned(uintptr_t w) {
+        if (w != at_word) {
+            at_word = w;
+            word = __ldg(reinterpret_cast<const uint32_t *>(w));
+        }
+        return word;
+    }
+    CJ_DEV uint8_t at(uint32_t i) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p) + i;
+        return (uint8_t)(aligned(a & ~(uintptr_t)3) >> (8 * (uint32_t)(a & 3u)));
+    }
+    /* The first position from i on that a search for byte c followed by byte
+     * c2 (256: any, or none) has to look at: skips four positions at once
+     * whose characters are ASCII (code points of their own), no newline, and
+     * do not begin with c and c2. */
+    CJ_DEV uint32_t skip_to(uint32_t i, uint32_t c, uint32_t c2) {
+        if (i >= len) return i;
+        const uint32_t cc = (c & 0xFFu) * 0x01010101u, cc2 = (c2 & 0xFFu) * 0x01010101u, nl = 0x0A0A0A0Au;
+        if (i + 5 <= len) {
+            /* one aligned word a step, the same turns for every lane */
+            const uintptr_t a = reinterpret_cast<uintptr_t>(p) + i;
+            const uint32_t *next = reinterpret_cast<const uint32_t *>(a & ~(uintptr_t)3);
+            const uint32_t sh = 8 * (uint32_t)(a & 3u);
+            uint32_t lo = __ldg(next);
+            do {
+                const uint32_t hi = __ldg(++next); /* holds byte i + 4 at least */
+                const unsigned long long both = ((unsigned long long)hi << 32 | lo) >> sh;
+                const uint32_t w = (uint32_t)both, x = w ^ nl;
+                /* a zero byte of x (or, of both keys' differences, below), or
+                 * a byte above 0x7F */
+                uint32_t stop = ((x - 0x01010101u) & ~x) | w;
+                if (c < 256) {
+                    uint32_t y = w ^ cc;
+                    if (c2 < 256) y |= (uint32_t)(both >> 8) ^ cc2;
+                    stop |= (y - 0x01010101u) & ~y;
+                }
+                if (stop & 0x80808080u) return i;
+                i += 4;
+                lo = hi;
+            } while (i + 5 <= len);
+        }
+        if (i >= len) return i;
+        /* the last one to four positions; the second byte has one fewer */
+        const uint32_t r = len - i, live = 0x80808080u >> (8 * (4 - r));
+        const uint32_t w = tail(i), x = w ^ nl;
+        uint32_t stop = (((x - 0x01010101u) & ~x) | w) & live;
+        if (c < 256) {
+            uint32_t y = w ^ cc, yl = live;
+            if (c2 < 256) {
+                y |= (w >> 8) ^ cc2;
+                yl >>= 8;
+            }
+            stop |= (y - 0x01010101u) & ~y & yl;
+        }
+        return stop ? i : len;
+    }
+    /* The string's last bytes from i on, one to four; what follows them in
+     * the word is anything. */
+    CJ_DEV uint32_t tail(uint32_t i) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p) + i, w = a & ~(uintptr_t)3;
+        const uint32_t lo = aligned(w);
+        const uint32_t hi = w + 4 < reinterpret_cast<uintptr_t>(p) + len ? aligned(w + 4) : 0u;
+        return __funnelshift_r(lo, hi, 8 * (uint32_t)(a & 3u));
+    }
+};
+
 /* Three-way bytewise comparison with the literal (std::string_view order). */
-CJ_DEV int str_compare(StrView &s, const uint8_t *lit, uint32_t lit_len) {
+template <class S> CJ_DEV int str_compare(S &s, const uint8_t *lit, uint32_t lit_len) {
     const uint32_t m = s.len < lit_len ? s.len : lit_len;
     for (uint32_t i = 0; i < m; ++i) {
         const uint8_t a = s.at(i), b = lit[i];
@@ -112,35 +190,56 @@ CJ_DEV uint32_t cp_len(uint8_t b) {
 /* Whole-string LIKE: '%' matches any run of code points and '_' one code
  * point, neither a newline; other pattern bytes match themselves. Greedy
  * with backtracking to the last '%': each '%' extends one code point at a
- * time and never over a newline. */
-CJ_DEV bool like_match(StrView &s, const uint8_t *pat, uint32_t m) {
+ * time and never over a newline.
+ *
+ * Bound by instructions: the lanes of a warp take different turns at every
+ * byte (5.6 of 32 active over 10M strings of 20 characters against '%qz%':
+ * 1766 us). So after a '%' the lanes skip together, four positions a step,
+ * what cannot begin the two bytes that follow it (with one byte a lane of
+ * the 32 stopped at nearly every step: 1226 us), the pattern's bytes at j
+ * and after the last '%' stay in registers, and a string too short for the
+ * rest of the pattern is given up at once: 407 us. */
+template <class S> CJ_DEV bool like_match(S &s, const uint8_t *pat, uint32_t m) {
+    constexpr uint32_t kEnd = 256; /* past the pattern's last byte */
     const uint32_t n = s.len;
-    uint32_t i = 0, j = 0;
-    int64_t star_j = -1;
-    uint32_t star_i = 0;
+    uint32_t need = 0; /* bytes that the pattern from j on takes at least */
+    for (uint32_t k = 0; k < m; ++k) need += pat[k] != '%';
+    if (n < need) return false;
+    uint32_t i = 0, j = 0, pc = m ? pat[0] : kEnd;
+    /* the position after the last '%', its byte and, where both are literal,
+     * the next one */
+    uint32_t star_j = 0, star_i = 0, star_pc = 0, star_next = kEnd, star_need = 0;
+    bool star = false;
     while (i < n) {
-        if (j < m && pat[j] == '%') {
-            star_j = j++;
+        if (pc == '%') {
+            star = true;
+            star_j = ++j;
             star_i = i;
+            star_need = need;
+            star_pc = pc = j < m ? pat[j] : kEnd;
+            star_next = pc != kEnd && j + 1 < m ? pat[j + 1] : kEnd;
+            if (star_next == '%' || star_next == '_') star_next = kEnd;
+            if (pc != '%' && pc != '_') i = star_i = s.skip_to(star_i, star_pc, star_next);
             continue;
         }
         const uint8_t c = s.at(i);
-        if (j < m && pat[j] == '_' && c != '\n') {
-            i += cp_len(c);
+        if (pc == '_' ? c != '\n' : pc == c) {
+            i += pc == '_' ? cp_len(c) : 1u;
             ++j;
+            --need;
+            pc = j < m ? pat[j] : kEnd;
             continue;
         }
-        if (j < m && pat[j] != '_' && pat[j] == c) {
-            ++i;
-            ++j;
-            continue;
-        }
-        if (star_j < 0) return false;
-        const uint8_t sc = s.at(star_i);
+        if (!star) return false;
+        const uint8_t sc = i == star_i ? c : s.at(star_i);
         if (sc == '\n') return false;
         star_i += cp_len(sc);
+        if (star_i + star_need > n) return false;
+        if (star_pc != '_') star_i = s.skip_to(star_i, star_pc, star_next);
         i = star_i;
-        j = (uint32_t)star_j + 1;
+        j = star_j;
+        pc = star_pc;
+        need = star_need;
     }
     while (j < m && pat[j] == '%') ++j;
     return j == m && i == n;
@@ -167,6 +266,12 @@ template <typename T> CJ_DEV bool cmp_num(int op, T a, T b) {
     case CJ_CMP_GEQ: return a >= b;
     default: return false;
     }
+}
+
+template <class S> CJ_DEV bool cmp_str(S &s, const CmpArgs &a) {
+    if (a.op == CJ_CMP_LIKE) return like_match(s, a.lit, a.lit_len);
+    if (a.op == CJ_CMP_NOT_LIKE) return !like_match(s, a.lit, a.lit_len);
+    return cmp_num<int>(a.op, str_compare(s, a.lit, a.lit_len), 0);
 }
 
 /* Value of base row r of a fixed-width column and whether it is present. */
@@ -203,13 +308,14 @@ __global__ void __launch_bounds__(kFilterThreads) k_compare(CmpArgs a) {
                 double v;
                 bit = fixed_value<double>(c, r, &v) && cmp_num<double>(a.op, v, a.f64);
             } else if (valid_bit(c.valid, r)) { /* VARCHAR */
-                StrView s;
-                s.init(c.pages, __ldg(c.str_desc + r));
-                if (a.op == CJ_CMP_LIKE) bit = like_match(s, a.lit, a.lit_len);
-                else if (a.op == CJ_CMP_NOT_LIKE) bit = !like_match(s, a.lit, a.lit_len);
-                else {
-                    const int d = str_compare(s, a.lit, a.lit_len);
-                    bit = cmp_num<int>(a.op, d, 0);
+                const uint64_t d = __ldg(c.str_desc + r);
+                if (desc_is_long(d)) {
+                    StrView s;
+                    s.init(c.pages, d);
+                    bit = cmp_str(s, a);
+                } else {
+                    ShortStr s(c.pages, d);
+                    bit = cmp_str(s, a);
                 }
             }
         }
@@ -268,6 +374,7 @@ class Filter {
         DevPtr sel;
         uint64_t count = rows;
         if (pred && rows) {
+            decode(pred_columns());
             DevPtr bits = eval(pred->root, words, 0);
             DevPtr cnt = ctx.alloc(words * 4), off = ctx.alloc((words + 1) * 8);
             DevPtr tmp = ctx.alloc(scan_temp_bytes(words));
@@ -293,6 +400,7 @@ class Filter {
         tab->ctx = &ctx;
         tab->num_rows = count;
         const uint32_t TR = 2048;
+        if (count) decode(std::set<uint64_t>(cols, cols + ncols));
         for (uint64_t k = 0; k < ncols; ++k) {
             const uint64_t c = cols[k];
             ColumnPages cp;
@@ -374,21 +482,45 @@ class Filter {
         }
     }
 
-    const Decoded &decode(uint64_t c) {
-        auto it = decoded.find(c);
-        if (it != decoded.end()) return it->second;
-        Decoded d;
-        d.type = in.cols[c].type;
-        d.rows = in.num_rows;
-        d.src = in.cols[c];
-        ColumnTask task = column_task(ctx, d, nullptr);
-        check_cuda(launch_columns(L, &task, 1, true), "page_index");
-        check_cuda(launch_columns(L, &task, 1, false), "decode");
-        return decoded.emplace(c, std::move(d)).first->second;
+    /* The columns that the predicate reads. */
+    std::set<uint64_t> pred_columns() const {
+        std::set<uint64_t> need;
+        std::function<void(uint64_t, int)> walk = [&](uint64_t node, int depth) {
+            if (depth > (int)pred->num_nodes) fail(CJ_ERR_INVALID_PLAN, "predicate has a cycle");
+            const cj_pred_node &n = pred->nodes[node];
+            if (n.kind == CJ_PRED_CMP) {
+                need.insert(n.column);
+                return;
+            }
+            walk(n.left, depth + 1);
+            if (n.kind != CJ_PRED_NOT) walk(n.right, depth + 1);
+        };
+        walk(pred->root, 0);
+        return need;
+    }
+    /* Indexes and decodes columns, one launch each for all of them. */
+    void decode(const std::set<uint64_t> &need) {
+        std::vector<ColumnTask> tasks;
+        DevPtr states = ctx.alloc(std::max<size_t>(need.size(), 1) * sizeof(ColumnState));
+        check_cuda(cudaMemsetAsync(states->ptr, 0, states->bytes, ctx.stream), "memset");
+        keep.push_back(states);
+        for (uint64_t c : need) {
+            if (decoded.count(c)) continue;
+            Decoded d;
+            d.type = in.cols[c].type;
+            d.rows = in.num_rows;
+            d.src = in.cols[c];
+            tasks.push_back(column_task(ctx, d, states->as<ColumnState>() + tasks.size()));
+            tasks.back().err = &ctx.d_status->errors;
+            decoded.emplace(c, std::move(d));
+        }
+        if (tasks.empty()) return;
+        check_cuda(launch_columns(L, tasks.data(), tasks.size(), true), "page_index");
+        check_cuda(launch_columns(L, tasks.data(), tasks.size(), false), "decode");
     }
 
     ColView view(uint64_t c) {
-        const Decoded &d = decode(c);
+        const Decoded &d = decoded.at(c);
         Relation R;
         RelCol rc{d.type, 0, c, -1, false};
         return make_view(d, R, rc, nullptr);
