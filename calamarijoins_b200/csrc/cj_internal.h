@@ -230,6 +230,42 @@ cudaError_t launch_columns(const Launch &L, ColumnTask *tasks, size_t n, bool in
 /* Index and decode of the columns of a batch, placed by place_columns. */
 cudaError_t launch_columns_grouped(const Launch &L, const ColumnTask *tasks_dev, uint32_t n, const ColumnGrid &g);
 
+/* Table of unique build keys (k_unique.cu): direct-mapped when their range is
+ * at most max_span, else, for INT32 keys (open_slots > 0), open-addressing.
+ * `slots` holds max(4 max_span, 8 open_slots) bytes rounded up to 16,
+ * 16-byte aligned; open_slots is at least twice the build rows. `params` (kTableWords words, zero before the build) receives what the
+ * device found. */
+constexpr uint32_t kArrayEmpty = 0xFFFFFFFFu;
+constexpr uint64_t kOpenMaxRows = 1ull << 28;
+enum TableWord { /* of params */
+    kTableMinC = 0,    /* ~min, max of the non-NULL keys (XOR 2^63: unsigned
+                          order is signed order) and their count           */
+    kTableMax = 1,
+    kTableCount = 2,
+    kTableRefused = 3, /* not direct-mapped: a TableRefusal                */
+    kTableLo = 4,      /* smallest key, values in the range                */
+    kTableSpan = 5,
+    kTableDup = 6,     /* the build met a repeated key: the table is unusable */
+    kTableDone = 7,    /* blocks of the range pass that have finished      */
+    kTableWords = 8
+};
+enum TableRefusal : unsigned long long {
+    kTableSpread = 1,  /* the keys' range is above max_span           */
+    kTableRepeats = 2  /* more keys than values in their range        */
+};
+struct UniqueTable {
+    void *slots;
+    unsigned long long *params;
+    uint64_t max_span;
+    uint32_t open_slots; /* 0: no open-addressing table */
+};
+/* What the params say (host copy or device): 0 unusable, 1 direct-mapped,
+ * 2 open-addressing. */
+__host__ __device__ inline int table_kind(const unsigned long long *p, uint32_t open_slots) {
+    if (p[kTableDup]) return 0;
+    if (!p[kTableRefused]) return 1;
+    return p[kTableRefused] == kTableSpread && open_slots ? 2 : 0;
+}
 /* Build */
 struct BuildPlan {
     int log2_slots;      /* directory = 2^log2_slots entries + 1          */
@@ -275,48 +311,13 @@ struct BuildTask {
     uint64_t *dir;
     void *tuples;
     void *part_buf; /* n tuples of scratch */
+    UniqueTable unique; /* nothing is built when this table (params set) is usable */
 };
 size_t build_grouped_temp_bytes(uint64_t total_cells);
 cudaError_t launch_build_grouped(const Launch &L, const BuildTask *tasks_dev, uint32_t ntasks, uint32_t total_chunks,
                                  uint32_t total_parts, uint64_t total_cells, uint32_t max_parts, uint32_t max_slots,
                                  const uint16_t *bloom, void *temp);
 
-/* Table of unique build keys (k_unique.cu): direct-mapped when their range is
- * at most max_span, else, for INT32 keys (open_slots > 0), open-addressing.
- * `slots` holds max(4 max_span, 8 open_slots) bytes rounded up to 16,
- * 16-byte aligned; open_slots is at least twice the build rows. `params` (kTableWords words, zero before the build) receives what the
- * device found. */
-constexpr uint32_t kArrayEmpty = 0xFFFFFFFFu;
-constexpr uint64_t kOpenMaxRows = 1ull << 28;
-enum TableWord { /* of params */
-    kTableMinC = 0,    /* ~min, max of the non-NULL keys (XOR 2^63: unsigned
-                          order is signed order) and their count           */
-    kTableMax = 1,
-    kTableCount = 2,
-    kTableRefused = 3, /* not direct-mapped: a TableRefusal                */
-    kTableLo = 4,      /* smallest key, values in the range                */
-    kTableSpan = 5,
-    kTableDup = 6,     /* the build met a repeated key: the table is unusable */
-    kTableDone = 7,    /* blocks of the range pass that have finished      */
-    kTableWords = 8
-};
-enum TableRefusal : unsigned long long {
-    kTableSpread = 1,  /* the keys' range is above max_span           */
-    kTableRepeats = 2  /* more keys than values in their range        */
-};
-struct UniqueTable {
-    void *slots;
-    unsigned long long *params;
-    uint64_t max_span;
-    uint32_t open_slots; /* 0: no open-addressing table */
-};
-/* What the params say (host copy or device): 0 unusable, 1 direct-mapped,
- * 2 open-addressing. */
-inline int table_kind(const unsigned long long *p, uint32_t open_slots) {
-    if (p[kTableDup]) return 0;
-    if (!p[kTableRefused]) return 1;
-    return p[kTableRefused] == kTableSpread && open_slots ? 2 : 0;
-}
 cudaError_t launch_unique_build(const Launch &L, const ColView &key, uint32_t n, const UniqueTable &t);
 
 /* The probe's key column: a scan read page by page (base and loc of its page
@@ -365,7 +366,21 @@ cudaError_t launch_multi_build(const Launch &L, const ColView &key, uint32_t n, 
 cudaError_t launch_probe_multi(const Launch &L, const ProbeKey &k, uint32_t n, const MultiTable &t,
                                const UniqueOut &out);
 
-constexpr int kDirectParams = 6; /* words of a grouped direct-mapped table */
+/* The build for the joins of a batch level: task k owns blocks [key_base,
+ * key_base + key_blocks) of the passes over its rows and [fill_base, ...) of
+ * the fill. */
+struct UniqueBuildTask {
+    ColView key;
+    UniqueTable table;
+    uint32_t n;
+    uint32_t key_base, key_blocks, fill_base, fill_blocks; /* place_unique */
+};
+struct UniqueGrid {
+    uint32_t key = 0, fill = 0;
+};
+UniqueGrid place_unique(const Launch &L, UniqueBuildTask *tasks, size_t n);
+cudaError_t launch_unique_build_grouped(const Launch &L, const UniqueBuildTask *tasks_dev, uint32_t n,
+                                        const UniqueGrid &g);
 
 /* Probe and nested loop share one tiled kernel; `sched` is scratch of
  * probe_sched_bytes(n_probe) bytes (the tile ticket). */
@@ -389,8 +404,8 @@ cudaError_t launch_nl_probe_tiles(const Launch &L, const ColView &pkey, uint32_t
 struct ProbeTask {
     ColView pkey;
     uint32_t n_probe;
-    int32_t kind;           /* 0 hash, 1 nested loop, 2 direct-mapped table
-                               when usable (params[3] == 0), else hash     */
+    int32_t kind;           /* 0 hash, 1 nested loop, 2 the direct-mapped table
+                               `unique` when it is usable, else hash       */
     int32_t build_key_type; /* hash: CJ_INT32 / CJ_INT64 tuples            */
     int32_t log2_slots;
     const uint64_t *dir;
@@ -398,34 +413,11 @@ struct ProbeTask {
     const int64_t *nl_keys;
     const uint32_t *nl_rids;
     const uint32_t *nl_count;
-    const uint32_t *slots;              /* kind 2: direct-mapped table      */
-    const unsigned long long *params;   /* kind 2: its kDirectParams words  */
+    UniqueTable unique;         /* kind 2 (open_slots 0) */
     MatchOut out;               /* out.counter zeroed before launch         */
     uint32_t num_tiles;
     uint32_t tile_base;         /* first global tile of this task           */
 };
-/* Grouped direct-mapped builds: slots[key - lo] = build row for every task
- * whose keys are unique and span at most max_span values; task k owns blocks
- * [block_base, block_base + blocks) of each pass. params hold kDirectParams
- * words per task, set to {~0, 0, 0, 0, 0, 0} before, and receive [0] min and
- * [1] max of the non-NULL keys (XOR 2^63), [2] their count, [3] non-zero when
- * the table cannot be used (1: span above max_span, 2: a repeated key), [4]
- * lo, [5] span. */
-struct DirectTask {
-    ColView key;
-    uint32_t n;
-    uint32_t key_blocks;   /* blocks over the keys                         */
-    uint32_t key_base;
-    uint32_t fill_blocks;  /* blocks over max_span slots                   */
-    uint32_t fill_base;
-    uint64_t max_span;
-    uint32_t *slots;
-    unsigned long long *params;
-};
-cudaError_t launch_direct_build_grouped(const Launch &L, const DirectTask *tasks_dev, uint32_t ntasks,
-                                        uint32_t total_key_blocks, uint32_t total_fill_blocks);
-constexpr uint32_t kDirectBlockRows = 256 * 8; /* key rows per block of the grouped passes */
-constexpr uint32_t kDirectFillSlots = 256 * 16; /* slots per block of the grouped fill     */
 uint32_t probe_tiles(uint32_t n_probe);
 /* `ticket` must be zeroed, and each task's counter. */
 cudaError_t launch_probe_grouped(const Launch &L, const ProbeTask *tasks_dev, uint32_t ntasks,
@@ -473,9 +465,11 @@ struct PageTask {
     const unsigned long long *rows_dev;
     uint8_t *out;
     int32_t finish;
-    const unsigned long long *table; /* finish 2: also written through the row
-                                        ids when set and these table words say
-                                        open-addressing (EmitColumn::direct_only) */
+    const unsigned long long *table; /* finish 2, with the table words set: also
+                                        written through the row ids unless the
+                                        table is direct-mapped or, with
+                                        open_slots, open-addressing            */
+    uint32_t open_slots;
     uint32_t block_base, blocks; /* place_pages */
 };
 constexpr int kPageArgs = 24; /* tasks passed by value */

@@ -309,6 +309,13 @@ CJ_DEV uint32_t find_task(const BuildTask *tasks, uint32_t ntasks, uint32_t unit
     return lo;
 }
 
+/* A task whose unique table is usable builds nothing (its cells of the
+ * histogram matrix stay as they were: other tasks' offsets are taken relative
+ * to their own first cell). */
+CJ_DEV bool task_idle(const BuildTask &T) {
+    return T.unique.params && table_kind(T.unique.params, T.unique.open_slots) != 0;
+}
+
 CJ_DEV PartGeom task_geom(const BuildTask &T) {
     PartGeom g;
     g.n = T.n;
@@ -326,6 +333,7 @@ __global__ void __launch_bounds__(kPartThreads)
     if (threadIdx.x == 0) s_task = find_task(tasks, ntasks, blockIdx.x, false);
     __syncthreads();
     const BuildTask &T = tasks[s_task];
+    if (task_idle(T)) return;
     hist_chunk(T.key, task_geom(T), blockIdx.x - T.chunk_base, matrix + T.cell_base, s_hist);
 }
 
@@ -337,6 +345,7 @@ __global__ void __launch_bounds__(kPartThreads)
     if (threadIdx.x == 0) s_task = find_task(tasks, ntasks, blockIdx.x, false);
     __syncthreads();
     const BuildTask &T = tasks[s_task];
+    if (task_idle(T)) return;
     const uint64_t *off = offsets + T.cell_base;
     if (T.key.type == CJ_INT32)
         scatter_chunk<int32_t>(T.key, task_geom(T), blockIdx.x - T.chunk_base, off, off[0],
@@ -359,6 +368,7 @@ __global__ void __launch_bounds__(kBuildThreads)
         if (threadIdx.x == 0) s_task = find_task(tasks, ntasks, u, true);
         __syncthreads();
         const BuildTask &T = tasks[s_task];
+        if (task_idle(T)) continue;
         const uint32_t S = 1u << (T.log2_slots - T.log2_parts);
         const uint64_t *off = offsets + T.cell_base;
         if (T.key.type == CJ_INT32)
@@ -448,132 +458,6 @@ cudaError_t build_impl(const Launch &L, const BuildPlan &bp, const ColView &key,
     return cudaGetLastError();
 }
 
-/* ---- direct-mapped tables of a batch (unique keys over a dense range; a
- * plan by itself: k_unique.cu) ---- */
-CJ_DEV unsigned long long warp_min_u64(unsigned long long v) {
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, d));
-    return v;
-}
-CJ_DEV unsigned long long warp_max_u64(unsigned long long v) {
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, d));
-    return v;
-}
-
-/* Block-wide min / max / count of the non-NULL keys of rows i0, i0 +
- * stride, ... below i1, folded into range[0..2] by atomics. */
-CJ_DEV void key_range_rows(const ColView &key, uint64_t i0, uint64_t i1, uint64_t stride,
-                           unsigned long long *range) {
-    __shared__ unsigned long long s_min[kBuildThreads / 32], s_max[kBuildThreads / 32];
-    __shared__ unsigned int s_cnt[kBuildThreads / 32];
-    unsigned long long mn = ~0ull, mx = 0ull;
-    unsigned int cnt = 0;
-    for (uint64_t i = i0; i < i1; i += stride) {
-        int64_t k;
-        if (load_key(key, (uint32_t)i, &k)) {
-            const unsigned long long b = (unsigned long long)k ^ (1ull << 63);
-            mn = min(mn, b);
-            mx = max(mx, b);
-            ++cnt;
-        }
-    }
-    mn = warp_min_u64(mn);
-    mx = warp_max_u64(mx);
-    cnt = __reduce_add_sync(0xffffffffu, cnt);
-    const uint32_t warp = threadIdx.x >> 5;
-    if (lane_id() == 0) {
-        s_min[warp] = mn;
-        s_max[warp] = mx;
-        s_cnt[warp] = cnt;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < kBuildThreads / 32; ++w) {
-            mn = min(mn, s_min[w]);
-            mx = max(mx, s_max[w]);
-            cnt += s_cnt[w];
-        }
-        if (cnt) {
-            atomicMin(range, mn);
-            atomicMax(range + 1, mx);
-            atomicAdd(range + 2, (unsigned long long)cnt);
-        }
-    }
-}
-
-/* ---- grouped direct-mapped builds (every candidate join of a batch level) ---- */
-CJ_DEV uint32_t find_direct_task(const DirectTask *tasks, uint32_t ntasks, uint32_t block, bool fill) {
-    uint32_t lo = 0, hi = ntasks;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if ((fill ? tasks[mid].fill_base : tasks[mid].key_base) <= block) lo = mid;
-        else hi = mid;
-    }
-    return lo;
-}
-
-__global__ void __launch_bounds__(kBuildThreads)
-    k_key_range_grouped(const DirectTask *__restrict__ tasks, uint32_t ntasks) {
-    __shared__ uint32_t s_task;
-    if (threadIdx.x == 0) s_task = find_direct_task(tasks, ntasks, blockIdx.x, false);
-    __syncthreads();
-    const DirectTask &T = tasks[s_task];
-    const uint64_t r0 = (uint64_t)(blockIdx.x - T.key_base) * kDirectBlockRows;
-    const uint64_t r1 = min((uint64_t)T.n, r0 + kDirectBlockRows);
-    key_range_rows(T.key, r0 + threadIdx.x, r1, blockDim.x, T.params);
-}
-
-__global__ void k_array_prep_grouped(const DirectTask *__restrict__ tasks, uint32_t ntasks) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= ntasks) return;
-    unsigned long long *p = tasks[t].params;
-    if (p[2] == 0) return;
-    const unsigned long long width = p[1] - p[0];
-    if (width >= tasks[t].max_span) {
-        p[3] = 1ull;
-        return;
-    }
-    if (p[2] > width + 1) { /* more keys than values in their range: one repeats */
-        p[3] = 2ull;
-        return;
-    }
-    p[4] = p[0] ^ (1ull << 63);
-    p[5] = width + 1;
-}
-
-__global__ void __launch_bounds__(kBuildThreads)
-    k_array_fill_grouped(const DirectTask *__restrict__ tasks, uint32_t ntasks) {
-    __shared__ uint32_t s_task;
-    if (threadIdx.x == 0) s_task = find_direct_task(tasks, ntasks, blockIdx.x, true);
-    __syncthreads();
-    const DirectTask &T = tasks[s_task];
-    const uint64_t span = T.params[3] ? 0ull : T.params[5];
-    const uint64_t i0 = (uint64_t)(blockIdx.x - T.fill_base) * kDirectFillSlots;
-    const uint64_t i1 = min(span, i0 + kDirectFillSlots);
-    for (uint64_t i = i0 + threadIdx.x; i < i1; i += blockDim.x) T.slots[i] = kArrayEmpty;
-}
-
-__global__ void __launch_bounds__(kBuildThreads)
-    k_array_build_grouped(const DirectTask *__restrict__ tasks, uint32_t ntasks) {
-    __shared__ uint32_t s_task;
-    if (threadIdx.x == 0) s_task = find_direct_task(tasks, ntasks, blockIdx.x, false);
-    __syncthreads();
-    const DirectTask &T = tasks[s_task];
-    unsigned long long *p = T.params;
-    if (p[3]) return;
-    const uint64_t lo = p[4], span = p[5];
-    const uint64_t r0 = (uint64_t)(blockIdx.x - T.key_base) * kDirectBlockRows;
-    const uint64_t r1 = min((uint64_t)T.n, r0 + kDirectBlockRows);
-    for (uint64_t i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
-        int64_t k;
-        if (!load_key(T.key, (uint32_t)i, &k)) continue;
-        const uint64_t off = (uint64_t)k - lo;
-        if (off >= span) continue;
-        if (atomicCAS(T.slots + off, kArrayEmpty, (uint32_t)i) != kArrayEmpty) p[3] = 2ull;
-    }
-}
-
 /* cudaFuncSetAttribute applies to the current device only: track which
  * devices have had the limits raised. */
 constexpr int kMaxAttrDevices = 64;
@@ -654,17 +538,6 @@ cudaError_t launch_build_grouped(const Launch &L, const BuildTask *tasks_dev, ui
 
 size_t build_grouped_temp_bytes(uint64_t total_cells) {
     return align256(total_cells * 4) + align256((total_cells + 1) * 8) + scan_temp_bytes(total_cells) + 256;
-}
-
-cudaError_t launch_direct_build_grouped(const Launch &L, const DirectTask *tasks_dev, uint32_t ntasks,
-                                        uint32_t total_key_blocks, uint32_t total_fill_blocks) {
-    if (!ntasks) return cudaSuccess;
-    if (total_key_blocks) k_key_range_grouped<<<total_key_blocks, kBuildThreads, 0, L.stream>>>(tasks_dev, ntasks);
-    k_array_prep_grouped<<<(ntasks + 127) / 128, 128, 0, L.stream>>>(tasks_dev, ntasks);
-    if (total_fill_blocks) k_array_fill_grouped<<<total_fill_blocks, kBuildThreads, 0, L.stream>>>(tasks_dev, ntasks);
-    if (total_key_blocks) k_array_build_grouped<<<total_key_blocks, kBuildThreads, 0, L.stream>>>(tasks_dev, ntasks);
-    count_launches(4);
-    return cudaGetLastError();
 }
 
 size_t build_tuple_bytes(int key_bytes) {

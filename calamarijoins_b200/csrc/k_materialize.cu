@@ -39,11 +39,28 @@ constexpr int kMatThreads = 256;
 
 CJ_DEV uint32_t rows_per_page_dev(int32_t type) { return type == CJ_INT32 ? kRowsPerPageInt32 : kRowsPerPage8B; }
 
+/* out[i] = src[idx[i]] for i = first, first + stride, ...: four rows a thread
+ * in flight (one at a time left each waiting for two round trips a row). */
+CJ_DEV void gather_rows(const uint32_t *__restrict__ src, const uint32_t *__restrict__ idx, uint32_t *__restrict__ out,
+                        uint64_t first, uint64_t n, uint64_t stride) {
+    constexpr int kRows = 4;
+    for (uint64_t i0 = first; i0 < n; i0 += stride * kRows) {
+        uint32_t v[kRows];
+#pragma unroll
+        for (int k = 0; k < kRows; ++k)
+            if (i0 + k * stride < n) v[k] = __ldcs(idx + i0 + k * stride);
+#pragma unroll
+        for (int k = 0; k < kRows; ++k)
+            if (i0 + k * stride < n) v[k] = __ldg(src + v[k]);
+#pragma unroll
+        for (int k = 0; k < kRows; ++k)
+            if (i0 + k * stride < n) out[i0 + k * stride] = v[k];
+    }
+}
+
 __global__ void k_gather_u32(const uint32_t *__restrict__ src, const uint32_t *__restrict__ idx,
                              uint64_t n, uint32_t *__restrict__ out) {
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        out[i] = __ldg(src + __ldcs(idx + i));
+    gather_rows(src, idx, out, (uint64_t)blockIdx.x * blockDim.x + threadIdx.x, n, (uint64_t)gridDim.x * blockDim.x);
 }
 
 constexpr int kMatMinBlocks = 8; /* page writers: 8 x 256 threads per SM */
@@ -228,8 +245,7 @@ CJ_DEV void write_page_blocks(const PageTask &T, uint32_t b, PageSmem &sm) {
     const uint32_t R = rows_per_page_dev(T.col.type);
     const uint64_t num_pages = (rows + R - 1) / R;
     if (b >= num_pages) return;
-    if (T.finish == 1 ||
-        (T.finish == 2 && col_null_free(T.col) && !(T.table && T.table[kTableRefused] == kTableSpread))) {
+    if (T.finish == 1 || (T.finish == 2 && col_null_free(T.col) && !(T.table && !table_kind(T.table, T.open_slots)))) {
         constexpr uint32_t kWarps = kMatThreads / 32;
         for (uint64_t pg = b * kWarps + (threadIdx.x >> 5); pg < num_pages; pg += (uint64_t)T.blocks * kWarps) {
             if (T.col.type == CJ_INT32) finish_dense_page<int32_t>(T.out, rows, pg);
@@ -289,7 +305,7 @@ __global__ void k_gather_grouped(const GatherTask *__restrict__ tasks, uint32_t 
         const GatherTask &T = tasks[s_task];
         const uint64_t r0 = (gc - T.chunk_base) * kGatherChunk;
         const uint64_t r1 = min(T.n, r0 + kGatherChunk);
-        for (uint64_t i = r0 + threadIdx.x; i < r1; i += blockDim.x) T.out[i] = __ldg(T.src + __ldcs(T.idx + i));
+        gather_rows(T.src, T.idx, T.out, r0 + threadIdx.x, r1, blockDim.x);
         __syncthreads();
     }
 }

@@ -220,16 +220,15 @@ template <int kItemsT> struct ArrayMatcherT {
     static constexpr int kMinBlocks = kProbeMinBlocks;
     static constexpr int kItems = kItemsT;
     const uint32_t *slots;
-    const unsigned long long *params; /* [3] unusable, [4] lo, [5] span */
+    const unsigned long long *params; /* TableWord */
     uint64_t lo = 0, span = 0;        /* read from params by resolved() */
     struct Shared {
         uint32_t unused;
     };
-    CJ_DEV bool skip() const { return params[3] != 0ull; }
     CJ_DEV ArrayMatcherT resolved() const {
         ArrayMatcherT m = *this;
-        m.lo = params[4];
-        m.span = params[5];
+        m.lo = params[kTableLo];
+        m.span = params[kTableSpan];
         return m;
     }
     CJ_DEV void init(Shared &) const {}
@@ -309,7 +308,6 @@ template <int kItemsT> struct ProbeSmemT {
     uint32_t pre[kRows];   /* row's match offset within its warp        */
     uint32_t warp[kProbeThreads / 32 + 1];
     uint32_t tile;
-    uint32_t task;
     unsigned long long base;
 };
 
@@ -446,8 +444,14 @@ __global__ void __launch_bounds__(kProbeThreads, CJ_GROUPED_MIN_BLOCKS)
     k_probe_grouped(const ProbeTask *__restrict__ tasks, uint32_t ntasks, uint32_t total_tiles,
                     unsigned int *ticket, const uint16_t *__restrict__ g_bloom) {
     __shared__ GroupedShared sh;
-    __shared__ ProbeSmemT<kProbeItems> ps;   /* ticket, task, and the halves' row state */
-    __shared__ ProbeSmemT<kGroupedItems> pw; /* row state of a whole-tile direct probe   */
+    /* row state of a half tile, or of a whole one probed directly: never
+     * both (together they took 10 KB per CTA of L1) */
+    __shared__ union Rows {
+        ProbeSmemT<kProbeItems> half;
+        ProbeSmemT<kGroupedItems> whole;
+    } rows;
+    ProbeSmemT<kProbeItems> &ps = rows.half;
+    __shared__ uint32_t s_tile, s_task;
     static_assert(HashMatcher<int32_t>::kItems == kProbeItems && LoopMatcher::kItems == kProbeItems,
                   "hash and nested-loop tasks probe half tiles");
     __shared__ uint32_t loaded_task;
@@ -458,33 +462,34 @@ __global__ void __launch_bounds__(kProbeThreads, CJ_GROUPED_MIN_BLOCKS)
     for (;;) {
         if (threadIdx.x == 0) {
             const uint32_t t = atomicAdd(ticket, 1u);
-            ps.tile = t;
+            s_tile = t;
             uint32_t lo = 0, hi = ntasks;
             while (hi - lo > 1) {
                 const uint32_t mid = (lo + hi) >> 1;
                 if (tasks[mid].tile_base <= t) lo = mid;
                 else hi = mid;
             }
-            ps.task = lo;
+            s_task = lo;
         }
         __syncthreads();
-        const uint32_t gt = ps.tile;
+        const uint32_t gt = s_tile, task = s_task;
         if (gt >= total_tiles) break;
-        const ProbeTask &T = tasks[ps.task];
+        const ProbeTask &T = tasks[task];
         const uint32_t tile = gt - T.tile_base;
-        if (T.kind == 2 && T.params[3] == 0ull) {
+        if (T.kind == 2 && table_kind(T.unique.params, 0)) {
             /* a direct-mapped table the build found usable (unique keys
              * over a dense range); otherwise the task's hash table below */
-            const ArrayMatcherT<kGroupedItems> m = ArrayMatcherT<kGroupedItems>{T.slots, T.params}.resolved();
+            const ArrayMatcherT<kGroupedItems> m = ArrayMatcherT<kGroupedItems>{
+                reinterpret_cast<const uint32_t *>(T.unique.slots), T.unique.params}.resolved();
             ArrayMatcherT<kGroupedItems>::Shared none;
-            probe_tile(T.pkey, T.n_probe, m, none, T.out, tile, pw);
+            probe_tile(T.pkey, T.n_probe, m, none, T.out, tile, rows.whole);
         } else if (T.kind == 1) {
             LoopMatcher m{T.nl_keys, T.nl_rids, T.nl_count};
-            if (loaded_task != ps.task) {
+            if (loaded_task != task) {
                 __syncthreads();
                 m.init(sh.l);
                 __syncthreads();
-                if (threadIdx.x == 0) loaded_task = ps.task;
+                if (threadIdx.x == 0) loaded_task = task;
                 bloom_live = false;
                 __syncthreads();
             }

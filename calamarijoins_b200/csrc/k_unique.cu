@@ -215,6 +215,45 @@ __global__ void __launch_bounds__(kSmallThreads)
     insert_rows(key, t, threadIdx.x, n, kSmallThreads);
 }
 
+/* The three passes for every candidate join of a batch level (one launch
+ * less than with a pass of its own for the decision). */
+CJ_DEV uint32_t find_build(const UniqueBuildTask *tasks, uint32_t ntasks, uint32_t block, bool fill) {
+    uint32_t lo = 0, hi = ntasks;
+    while (hi - lo > 1) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if ((fill ? tasks[mid].fill_base : tasks[mid].key_base) <= block) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+__global__ void __launch_bounds__(kUniqueThreads)
+    k_unique_range_grouped(const UniqueBuildTask *__restrict__ tasks, uint32_t ntasks) {
+    const UniqueBuildTask &T = tasks[find_build(tasks, ntasks, blockIdx.x, false)];
+    const ColView key = resolve_view(T.key);
+    const uint64_t b = blockIdx.x - T.key_base;
+    fold_range(key, b * blockDim.x + threadIdx.x, T.n, (uint64_t)T.key_blocks * blockDim.x, T.table.params);
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(T.table.params + kTableDone, 1ull) == T.key_blocks - 1) {
+            __threadfence();
+            decide_table(T.table.params, T.table.max_span);
+        }
+    }
+}
+__global__ void __launch_bounds__(kUniqueThreads)
+    k_unique_fill_grouped(const UniqueBuildTask *__restrict__ tasks, uint32_t ntasks) {
+    const UniqueBuildTask &T = tasks[find_build(tasks, ntasks, blockIdx.x, true)];
+    const uint64_t b = blockIdx.x - T.fill_base;
+    fill_table(T.table, b * blockDim.x + threadIdx.x, (uint64_t)T.fill_blocks * blockDim.x);
+}
+__global__ void __launch_bounds__(kUniqueThreads)
+    k_unique_insert_grouped(const UniqueBuildTask *__restrict__ tasks, uint32_t ntasks) {
+    const UniqueBuildTask &T = tasks[find_build(tasks, ntasks, blockIdx.x, false)];
+    const ColView key = resolve_view(T.key);
+    const uint64_t b = blockIdx.x - T.key_base;
+    insert_rows(key, T.table, b * blockDim.x + threadIdx.x, T.n, (uint64_t)T.key_blocks * blockDim.x);
+}
+
 /* Build of a table of repeated keys: count, place, scatter (launch_multi_build). */
 __global__ void __launch_bounds__(kUniqueThreads) k_multi_count(ColView key_arg, uint32_t n, MultiTable t) {
     const ColView key = resolve_view(key_arg);
@@ -803,6 +842,24 @@ template <typename T> CJ_DEV bool row_key(const ColView &c, uint32_t i, T *key) 
     return true;
 }
 
+/* A step over relation rows t0 ... t0 + 2047. Block-wide. */
+template <typename T, class LK, class SH>
+CJ_DEV void probe_rows(const ColView &col, uint32_t n, uint64_t t0, const LK &lk, const UniqueOut &out,
+                       const EmitPlan &plan, SH &sh, uint32_t part, uint32_t buf) {
+    uint32_t code[kItems] = {}, ok = 0;
+    const uint64_t r0 = t0 + part * kWarpRows;
+#pragma unroll
+    for (int it = 0; it < kItems; ++it) {
+        const uint64_t i = r0 + it * 32 + lane_id();
+        T key = T(0);
+        bool in;
+        const bool present = i < n && row_key<T>(col, (uint32_t)i, &key);
+        code[it] = lk.code(key, present, &in);
+        if (LK::kMask && in) ok |= 1u << it;
+    }
+    probe_step<T>(lk, code, ok, (uint32_t)r0, out, plan, sh, part, buf);
+}
+
 template <bool kPages, typename T, class LK, class SH>
 CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueOut &out, SH &sh) {
     const EmitPlan plan(out, LK::kMask);
@@ -832,18 +889,7 @@ CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueO
     } else {
         const ColView col = resolve_view(k.col);
         for (uint64_t t0 = (uint64_t)blockIdx.x * kTileRows; t0 < n; t0 += (uint64_t)gridDim.x * kTileRows) {
-            uint32_t code[kItems] = {}, ok = 0;
-            const uint64_t r0 = t0 + part * kWarpRows;
-#pragma unroll
-            for (int it = 0; it < kItems; ++it) {
-                const uint64_t i = r0 + it * 32 + lane_id();
-                T key = T(0);
-                bool in;
-                const bool present = i < n && row_key<T>(col, (uint32_t)i, &key);
-                code[it] = lk.code(key, present, &in);
-                if (LK::kMask && in) ok |= 1u << it;
-            }
-            probe_step<T>(lk, code, ok, (uint32_t)r0, out, plan, sh, part, buf);
+            probe_rows<T>(col, n, t0, lk, out, plan, sh, part, buf);
             buf ^= 1u;
         }
     }
@@ -926,6 +972,32 @@ cudaError_t launch_probe_unique(const Launch &L, const ProbeKey &k, uint32_t n, 
     prefer_l1(kernel);
     kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out);
     count_launches(1);
+    return cudaGetLastError();
+}
+
+UniqueGrid place_unique(const Launch &L, UniqueBuildTask *tasks, size_t n) {
+    UniqueGrid g;
+    const uint64_t wave = (uint64_t)L.num_sms * 8, rows = kUniqueThreads * kUniqueRows;
+    for (size_t k = 0; k < n; ++k) {
+        UniqueBuildTask &t = tasks[k];
+        const uint64_t most = std::max<uint64_t>(t.table.max_span * 4, t.table.open_slots * 8ull) / 16 + 1;
+        t.key_blocks = (uint32_t)std::min<uint64_t>((t.n + rows - 1) / rows, wave);
+        t.key_base = g.key;
+        t.fill_blocks = (uint32_t)std::min<uint64_t>((most + kUniqueThreads * 8 - 1) / (kUniqueThreads * 8), wave);
+        t.fill_base = g.fill;
+        g.key += t.key_blocks;
+        g.fill += t.fill_blocks;
+    }
+    return g;
+}
+
+cudaError_t launch_unique_build_grouped(const Launch &L, const UniqueBuildTask *tasks_dev, uint32_t n,
+                                        const UniqueGrid &g) {
+    if (!n) return cudaSuccess;
+    k_unique_range_grouped<<<g.key, kUniqueThreads, 0, L.stream>>>(tasks_dev, n);
+    k_unique_fill_grouped<<<g.fill, kUniqueThreads, 0, L.stream>>>(tasks_dev, n);
+    k_unique_insert_grouped<<<g.key, kUniqueThreads, 0, L.stream>>>(tasks_dev, n);
+    count_launches(3);
     return cudaGetLastError();
 }
 
