@@ -58,7 +58,11 @@ struct JoinWork {
         RelCol col;
     };
     std::vector<Out> outs;
-    DevPtr dir, tuples, part_buf, nlk, nlr, nlc, mb, mp, status, slots;
+    uint64_t *dir = nullptr; /* this and the next four: in the level's slab */
+    void *tuples = nullptr, *part_buf = nullptr;
+    int64_t *nlk = nullptr;
+    uint32_t *nlr = nullptr, *nlc = nullptr;
+    DevPtr mb, mp;
     UniqueTable unique{}; /* direct-mapped table (params null: none) */
     int log2_slots = 0, log2_parts = 0;
     uint64_t M = 0;
@@ -163,7 +167,7 @@ class BatchExecutor {
     }
     uint32_t num_checks = 0; /* checks captured so far (levels, then VARCHAR totals) */
     std::vector<DevPtr> keep_checks;
-    DevPtr col_states; /* ColumnState of every decoded column */
+    DevPtr col_mem; /* arrays and ColumnState of every decoded column */
     int levels(PlanState &p, uint64_t node, int depth);
     void decode_all();
     Decoded &dec(size_t plan, uint64_t t, uint64_t c) { return decoded.at({plan, t, c}); }
@@ -218,13 +222,20 @@ void BatchExecutor::decode_all() {
         }
     }
     if (keys.empty()) return;
-    col_states = ctx.alloc(keys.size() * sizeof(ColumnState));
-    ck(cudaMemsetAsync(col_states->ptr, 0, keys.size() * sizeof(ColumnState), ctx.stream), "memset");
-    std::vector<ColumnTask> tasks;
-    for (size_t k = 0; k < keys.size(); ++k) {
-        tasks.push_back(column_task(ctx, decoded.at(keys[k]), col_states->as<ColumnState>() + k));
-        tasks.back().err = &ctx.d_status->errors;
+    std::vector<Decoded *> cols;
+    Slab slab;
+    for (const auto &key : keys) {
+        cols.push_back(&decoded.at(key));
+        cols.back()->reserve(slab);
     }
+    slab.reserve(keys.size() * sizeof(ColumnState));
+    slab.open(ctx);
+    col_mem = slab.mem;
+    ColumnState *states = slab.take_as<ColumnState>(keys.size() * sizeof(ColumnState));
+    ck(cudaMemsetAsync(states, 0, keys.size() * sizeof(ColumnState), ctx.stream), "memset");
+    std::vector<ColumnTask> tasks;
+    for (size_t k = 0; k < keys.size(); ++k)
+        tasks.push_back(column_task(*cols[k], slab, states + k, &ctx.d_status->errors));
     const ColumnGrid grid = place_columns(L, tasks.data(), tasks.size());
     DevPtr td = upload_tasks(tasks);
     ck(launch_columns_grouped(L, td->as<ColumnTask>(), (uint32_t)tasks.size(), grid), "decode_grouped");
@@ -291,28 +302,52 @@ void BatchExecutor::run_level(int lvl) {
     std::vector<NlCollectTask> ntasks;
     uint32_t chunks = 0, parts = 0, max_parts = 1, max_slots = 1;
     uint64_t cells = 0;
-    for (auto &w : work) {
-        if (!w.B->rows || !w.P->rows) continue;
-        const ColView bv = view(w.plan, *w.B, w.bk, nullptr);
-        if (w.nl) {
-            w.nlk = ctx.alloc(kNestedLoopMax * 8);
-            w.nlr = ctx.alloc(kNestedLoopMax * 4);
-            w.nlc = ctx.alloc(4);
-            ntasks.push_back({bv, (uint32_t)w.B->rows, w.nlk->as<int64_t>(), w.nlr->as<uint32_t>(), w.nlc->as<uint32_t>()});
-            continue;
-        }
+    /* one allocation for the build structures of the level's joins */
+    Slab level;
+    auto build_plan = [&](const JoinWork &w) {
         BuildPlan bp;
         bp.num_rows = (uint32_t)w.B->rows;
         bp.log2_slots = std::max(11, ceil_log2(w.B->rows));
         const int spp = std::min(build_log2_spp(ctx, w.B->rows), bp.log2_slots);
         bp.log2_parts = std::min(bp.log2_slots - spp, 12);
         if (bp.log2_slots - bp.log2_parts > 14) fail(CJ_ERR_LIMIT, "build side too large for one radix pass");
+        return bp;
+    };
+    auto span_of = [&](const JoinWork &w) {
+        return std::min<uint64_t>((uint64_t)ctx.opt.dense_keys * w.B->rows, 1ull << 28);
+    };
+    for (const auto &w : work) {
+        if (!w.B->rows || !w.P->rows) continue;
+        if (w.nl) {
+            level.reserve(kNestedLoopMax * 8);
+            level.reserve(kNestedLoopMax * 4);
+            level.reserve(4);
+            continue;
+        }
+        const int kb = w.bk.type == CJ_INT32 ? 4 : 8;
+        level.reserve(build_dir_bytes(build_plan(w).log2_slots, kb));
+        level.reserve(w.B->rows * build_tuple_bytes(kb));
+        level.reserve(w.B->rows * build_tuple_bytes(kb));
+        if (ctx.opt.dense_keys > 0) level.reserve(span_of(w) * 4);
+    }
+    level.open(ctx);
+    for (auto &w : work) {
+        if (!w.B->rows || !w.P->rows) continue;
+        const ColView bv = view(w.plan, *w.B, w.bk, nullptr);
+        if (w.nl) {
+            w.nlk = level.take_as<int64_t>(kNestedLoopMax * 8);
+            w.nlr = level.take_as<uint32_t>(kNestedLoopMax * 4);
+            w.nlc = level.take_as<uint32_t>(4);
+            ntasks.push_back({bv, (uint32_t)w.B->rows, w.nlk, w.nlr, w.nlc});
+            continue;
+        }
+        const BuildPlan bp = build_plan(w);
         w.log2_slots = bp.log2_slots;
         w.log2_parts = bp.log2_parts;
         const int kb = w.bk.type == CJ_INT32 ? 4 : 8;
-        w.dir = ctx.alloc(build_dir_bytes(bp.log2_slots, kb));
-        w.tuples = ctx.alloc(w.B->rows * build_tuple_bytes(kb));
-        w.part_buf = ctx.alloc(w.B->rows * build_tuple_bytes(kb));
+        w.dir = level.take_as<uint64_t>(build_dir_bytes(bp.log2_slots, kb));
+        w.tuples = level.take(w.B->rows * build_tuple_bytes(kb));
+        w.part_buf = level.take(w.B->rows * build_tuple_bytes(kb));
         BuildGeometry g = build_geometry(build_launch(ctx, w.B->rows), bp);
         BuildTask t{};
         t.key = bv;
@@ -324,9 +359,9 @@ void BatchExecutor::run_level(int lvl) {
         t.chunk_base = chunks;
         t.part_base = parts;
         t.cell_base = cells;
-        t.dir = w.dir->as<uint64_t>();
-        t.tuples = w.tuples->ptr;
-        t.part_buf = w.part_buf->ptr;
+        t.dir = w.dir;
+        t.tuples = w.tuples;
+        t.part_buf = w.part_buf;
         chunks += g.grid;
         parts += 1u << bp.log2_parts;
         cells += g.cells;
@@ -344,9 +379,8 @@ void BatchExecutor::run_level(int lvl) {
     for (size_t k = 0; k < work.size(); ++k) {
         auto &w = work[k];
         if (w.nl || !w.B->rows || !w.P->rows || ctx.opt.dense_keys <= 0) continue;
-        w.unique.max_span = std::min<uint64_t>((uint64_t)ctx.opt.dense_keys * w.B->rows, 1ull << 28);
-        w.slots = ctx.alloc((w.unique.max_span * 4 + 15) & ~15ull);
-        w.unique.slots = w.slots->ptr;
+        w.unique.max_span = span_of(w);
+        w.unique.slots = level.take(w.unique.max_span * 4); /* 256-byte multiples: whole 16-byte fills */
         uidx.push_back(k);
     }
     if (!uidx.empty()) {
@@ -408,10 +442,17 @@ void BatchExecutor::run_level(int lvl) {
         unsigned long long *wp = words->as<unsigned long long>();
         unsigned int *ticket = reinterpret_cast<unsigned int *>(wp);
         size_t off = 1;
+        Slab matches;
+        for (size_t k : pidx) {
+            if (work[k].need_b) matches.reserve(work[k].cap * 4);
+            if (work[k].need_p) matches.reserve(work[k].cap * 4);
+        }
+        matches.open(ctx);
+        keep_checks.push_back(matches.mem);
         for (size_t k : pidx) {
             auto &w = work[k];
-            w.mb = w.need_b ? ctx.alloc(w.cap * 4) : nullptr;
-            w.mp = w.need_p ? ctx.alloc(w.cap * 4) : nullptr;
+            w.mb = w.need_b ? matches.part(w.cap * 4) : nullptr;
+            w.mp = w.need_p ? matches.part(w.cap * 4) : nullptr;
             ProbeTask t{};
             t.pkey = view(w.plan, *w.P, w.pk, nullptr);
             t.n_probe = (uint32_t)w.P->rows;
@@ -419,11 +460,11 @@ void BatchExecutor::run_level(int lvl) {
             t.unique = w.unique;
             t.build_key_type = w.bk.type;
             t.log2_slots = w.log2_slots;
-            t.dir = w.dir ? w.dir->as<uint64_t>() : nullptr;
-            t.tuples = w.tuples ? w.tuples->ptr : nullptr;
-            t.nl_keys = w.nlk ? w.nlk->as<int64_t>() : nullptr;
-            t.nl_rids = w.nlr ? w.nlr->as<uint32_t>() : nullptr;
-            t.nl_count = w.nlc ? w.nlc->as<uint32_t>() : nullptr;
+            t.dir = w.dir;
+            t.tuples = w.tuples;
+            t.nl_keys = w.nlk;
+            t.nl_rids = w.nlr;
+            t.nl_count = w.nlc;
             t.out.build_rids = w.mb ? w.mb->as<uint32_t>() : nullptr;
             t.out.probe_rids = w.mp ? w.mp->as<uint32_t>() : nullptr;
             t.out.capacity = (w.need_b || w.need_p) ? w.cap : 0;
@@ -466,11 +507,8 @@ void BatchExecutor::run_level(int lvl) {
         learned->level_M.push_back(std::move(Ms));
     }
     ++level_ix;
+    level.mem.reset();
     for (auto &w : work) {
-        w.dir.reset();
-        w.tuples.reset();
-        w.part_buf.reset();
-        w.slots.reset();
         stats.probe_rows += w.P->rows;
         stats.matches += w.M;
     }
@@ -547,6 +585,16 @@ void BatchExecutor::materialize_roots() {
         res->dev_pages.resize(nc);
         res->host_cols.assign(nc, nullptr);
         if (!p.root_rows) continue;
+        Slab pages; /* the plan's fixed-width result pages */
+        for (size_t c = 0; c < nc; ++c) {
+            if (p.root_types[c] == CJ_VARCHAR) continue;
+            const uint32_t R = rows_per_page_fixed(p.root_types[c]);
+            pages.reserve((p.root_rows + R - 1) / R * kPageSize);
+        }
+        if (pages.size) {
+            pages.open(ctx);
+            res->keep = pages.mem;
+        }
         for (size_t c = 0; c < nc; ++c) {
             if (p.root_types[c] == CJ_VARCHAR) {
                 var.push_back({i, c, ctx.alloc(varchar_temp_bytes(p.root_rows, TR))});
@@ -554,7 +602,7 @@ void BatchExecutor::materialize_roots() {
             }
             const uint32_t R = rows_per_page_fixed(p.root_types[c]);
             res->num_pages[c] = (p.root_rows + R - 1) / R;
-            res->dev_pages[c] = ctx.alloc(res->num_pages[c] * kPageSize);
+            res->dev_pages[c] = pages.part(res->num_pages[c] * kPageSize);
             PageTask t{};
             t.col = p.root_cols[c];
             t.rows = p.root_rows;

@@ -164,6 +164,8 @@ class Executor {
     int32_t column_type(uint64_t t, uint64_t c) const { return input_col_type(plan, t, c); }
 
     void validate();
+    using TC = std::pair<uint64_t, uint64_t>;
+    std::map<TC, ColumnPages> upload_small(const std::vector<TC> &order);
     void prefetch();
     void launch_tasks(std::vector<ColumnTask> &tasks, bool index);
     Decoded &indexed(uint64_t t, uint64_t c);
@@ -190,6 +192,49 @@ class Executor {
 
 void Executor::validate() { validate_plan(ctx, plan); }
 
+/* Host columns that together are small: their pages are gathered in one
+ * staging buffer and go up in one copy on the kernel stream, so that they are
+ * indexed and decoded like resident ones. Above kSmallUpload the gathering
+ * costs more than it saves (copies straight from page-locked pages, each on
+ * its way while kernels run, take over). Empty: the columns go one by one. */
+std::map<Executor::TC, ColumnPages> Executor::upload_small(const std::vector<TC> &order) {
+    constexpr uint64_t kSmallUpload = 1u << 20;
+    uint64_t pages = 0;
+    std::vector<TC> host;
+    for (const TC &tc : order)
+        if (!resident(tc.first)) {
+            host.push_back(tc);
+            pages += plan.inputs[tc.first].columns[tc.second].num_pages;
+        }
+    std::map<TC, ColumnPages> out;
+    if (host.empty() || !pages || pages * kPageSize > std::min<uint64_t>(kSmallUpload, ctx.staging_bytes)) return out;
+    PhaseScope ph(*this, PH_UPLOAD);
+    DevPtr dev = ctx.alloc(pages * kPageSize);
+    ck(cudaEventSynchronize(ctx.staging_ev[0]), "staging wait");
+    uint8_t *to = static_cast<uint8_t *>(ctx.staging[0]);
+    uint64_t at = 0;
+    for (const TC &tc : host) {
+        const cj_column_desc &cd = plan.inputs[tc.first].columns[tc.second];
+        ColumnPages cp;
+        cp.type = cd.type;
+        cp.num_pages = cd.num_pages;
+        if (cd.num_pages && !cd.pages) fail(CJ_ERR_INVALID_ARGUMENT, "column has pages but no page array");
+        if (cd.num_pages) {
+            cp.owner = dev;
+            cp.dev = dev->as<uint8_t>() + at * kPageSize;
+        }
+        for (uint64_t k = 0; k < cd.num_pages; ++k, ++at) {
+            if (!cd.pages[k]) fail(CJ_ERR_INVALID_ARGUMENT, "null page pointer");
+            std::memcpy(to + at * kPageSize, cd.pages[k], kPageSize);
+        }
+        out.emplace(tc, std::move(cp));
+    }
+    ck(cudaMemcpyAsync(dev->ptr, to, pages * kPageSize, cudaMemcpyHostToDevice, ctx.stream), "page upload");
+    ck(cudaEventRecord(ctx.staging_ev[0], ctx.stream), "event record");
+    stats.h2d_bytes += pages * kPageSize;
+    return out;
+}
+
 /* Starts the upload of every host column the plan will decode, on the
  * context's upload stream, in the order the kernels need them: join keys
  * bottom-up, then the root's outputs. The kernel stream waits for a
@@ -202,7 +247,6 @@ void Executor::validate() { validate_plan(ctx, plan); }
  * until the plan reads it: a plan that never gets to a malformed column
  * (an empty join below) still runs. */
 void Executor::prefetch() {
-    using TC = std::pair<uint64_t, uint64_t>;
     std::vector<TC> order;
     std::set<TC> seen;
     auto add = [&](const TC &tc) {
@@ -226,24 +270,36 @@ void Executor::prefetch() {
         return out;
     };
     for (const TC &tc : cols(plan.root, 0)) add(tc);
-    std::vector<ColumnTask> tasks, decodes;
-    TC streamed;
-    const bool stream = streamed_key(&streamed);
+    ck(cudaMemsetAsync(ctx.d_status, 0, sizeof(StatusBlock), ctx.stream), "memset");
+    std::map<TC, ColumnPages> small = upload_small(order);
+    std::vector<std::pair<TC, Decoded>> now;
+    Slab slab;
     for (const TC &tc : order) {
         const cj_table *r = resident(tc.first);
-        if (!r || r->num_rows > 0xFFFFFFFFull || tasks.size() == kStatusColumns) continue;
+        const auto up = small.find(tc);
+        if ((!r && up == small.end()) || table_rows(tc.first) > 0xFFFFFFFFull || now.size() == kStatusColumns) continue;
         Decoded d;
         d.type = column_type(tc.first, tc.second);
-        d.rows = r->num_rows;
-        d.src = r->cols[tc.second];
-        d.status_col = (int)tasks.size();
-        tasks.push_back(column_task(ctx, d, &ctx.d_status->cols[tasks.size()]));
-        d.ready = !(stream && tc == streamed);
-        if (d.ready) decodes.push_back(tasks.back());
-        decoded.emplace(tc, std::move(d));
+        d.rows = table_rows(tc.first);
+        d.src = r ? r->cols[tc.second] : up->second;
+        d.status_col = (int)now.size();
+        d.reserve(slab);
+        now.emplace_back(tc, std::move(d));
     }
-    ck(cudaMemsetAsync(ctx.d_status, 0, sizeof(StatusBlock), ctx.stream), "memset");
-    if (!tasks.empty()) {
+    if (!now.empty()) {
+        std::vector<ColumnTask> tasks, decodes;
+        TC streamed;
+        const bool stream = streamed_key(&streamed);
+        slab.open(ctx);
+        for (auto &kv : now) {
+            Decoded &d = kv.second;
+            d.mem = slab.mem;
+            ColumnState *state = &ctx.d_status->cols[d.status_col];
+            tasks.push_back(column_task(d, slab, state, &state->err));
+            d.ready = !(stream && kv.first == streamed);
+            if (d.ready) decodes.push_back(tasks.back());
+            decoded.emplace(kv.first, std::move(d));
+        }
         PhaseScope ph(*this, PH_DECODE);
         launch_tasks(tasks, true);
         if (!decodes.empty()) launch_tasks(decodes, false);
@@ -251,6 +307,16 @@ void Executor::prefetch() {
     cudaEvent_t first = nullptr;
     for (const TC &tc : order) {
         if (resident(tc.first)) continue;
+        const auto up = small.find(tc);
+        if (up != small.end()) {
+            if (decoded.count(tc)) continue;
+            Prefetched pf; /* more columns than the status block tracks */
+            pf.pages = up->second;
+            pf.done = ctx.get_event();
+            ck(cudaEventRecord(pf.done, ctx.stream), "event record");
+            prefetched.emplace(tc, std::move(pf));
+            continue;
+        }
         if (!first) {
             first = ctx.get_event();
             ck(cudaEventRecord(first, ctx.h2d_stream), "event record");
@@ -327,7 +393,14 @@ Decoded &Executor::indexed(uint64_t t, uint64_t c) {
         upload_pages(ctx, plan.inputs[t].columns[c], d.src, &stats.h2d_bytes);
     }
     PhaseScope ph(*this, PH_DECODE);
-    std::vector<ColumnTask> tasks{column_task(ctx, d, nullptr)};
+    Slab slab;
+    d.reserve(slab);
+    slab.reserve(sizeof(ColumnState));
+    slab.open(ctx);
+    d.mem = slab.mem;
+    ColumnState *state = slab.take_as<ColumnState>(sizeof(ColumnState));
+    ck(cudaMemsetAsync(state, 0, sizeof(ColumnState), ctx.stream), "memset");
+    std::vector<ColumnTask> tasks{column_task(d, slab, state, &ctx.d_status->errors)};
     launch_tasks(tasks, true);
     return decoded.emplace(key, std::move(d)).first->second;
 }
@@ -780,6 +853,9 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
             }
         }
     } dl{ctx};
+    constexpr uint64_t kSmallDownload = 4u << 20; /* copied in 80 us; nothing worth overlapping */
+    bool small_download = false;
+    std::vector<int64_t> alias(nc, -1);
     {
         PhaseScope ph(*this, PH_MAT);
         const uint32_t TR = (uint32_t)std::max<int64_t>(64, std::min<int64_t>(ctx.opt.varchar_tile_rows, 8192));
@@ -828,7 +904,6 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
         stats.output_pages = total_pages;
         /* Columns that share device pages (the join keys written by the
          * probe) share one host copy too: downloaded once. */
-        std::vector<int64_t> alias(nc, -1);
         for (size_t c = 0; c < nc; ++c)
             for (size_t k = 0; k < c && alias[c] < 0; ++k)
                 if (cols[c].pages && cols[k].pages == cols[c].pages) alias[c] = (int64_t)k;
@@ -849,7 +924,9 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
         }
         /* A host result's columns are written one by one, each downloaded
          * while the next is written (and still uploaded); a result left in
-         * HBM has its fixed-width columns written by one launch. */
+         * HBM, or a small one, has its columns written by one launch of each
+         * kind, and a small one is then copied on the kernel stream. */
+        const bool overlap = to_host && host_pages * kPageSize > kSmallDownload;
         std::vector<PageTask> ptasks;
         auto write_pages = [&]() {
             KScope ks(*this, "write_pages");
@@ -879,16 +956,16 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
             if (types[c] == CJ_VARCHAR) {
                 VarcharTask &v = vtasks[vtask_of[c]];
                 v.out = t.out;
-                if (to_host) {
+                if (overlap) {
                     KScope ks(*this, "varchar_write");
                     ck(launch_varchar(L, &v, 1, false), "varchar_write");
                 }
             } else if (alias[c] < 0) {
                 ptasks.push_back(t);
-                if (to_host) write_pages();
+                if (overlap) write_pages();
             }
             const size_t bytes = res->num_pages[c] * kPageSize;
-            if (to_host && bytes && alias[c] < 0) {
+            if (overlap && bytes && alias[c] < 0) {
                 cudaEvent_t written = ctx.get_event();
                 ck(cudaEventRecord(written, ctx.stream), "event record");
                 ck(cudaStreamWaitEvent(ctx.d2h_stream, written, 0), "stream wait");
@@ -904,9 +981,20 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
             }
         }
         if (!ptasks.empty()) write_pages();
-        if (!to_host && !vtasks.empty()) {
+        if (!overlap && rows && !vtasks.empty()) {
             KScope ks(*this, "varchar_write");
             ck(launch_varchar(L, vtasks.data(), vtasks.size(), false), "varchar_write");
+        }
+        small_download = to_host && !overlap;
+    }
+    if (small_download) {
+        PhaseScope ph(*this, PH_DOWNLOAD);
+        for (size_t c = 0; c < nc; ++c) {
+            const size_t bytes = res->num_pages[c] * kPageSize;
+            if (!bytes || alias[c] >= 0) continue;
+            ck(cudaMemcpyAsync(res->host_cols[c], res->dev_pages[c]->ptr, bytes, cudaMemcpyDeviceToHost, ctx.stream),
+               "download");
+            stats.d2h_bytes += bytes;
         }
     }
     if (dl.first) {

@@ -40,47 +40,70 @@ inline Launch probe_launch(const Context &ctx, uint64_t rows) {
     return L;
 }
 
-/* A base column decoded into dense device arrays. */
+/* One device allocation that many buffers are carved from, 256-byte aligned:
+ * a batch of 48 plans made 1,300 allocations for its columns and 600 for its
+ * joins, about 0.4 us of host time each with the release. reserve() all of
+ * them, open(), then take() each; they live as long as `mem`. */
+struct Slab {
+    DevPtr mem;
+    size_t size = 0, used = 0;
+    static size_t align(size_t bytes) { return (bytes + 255) & ~size_t(255); }
+    void reserve(size_t bytes) { size += align(bytes); }
+    void open(Context &ctx) { mem = ctx.alloc(size); }
+    void *take(size_t bytes) {
+        if (used + align(bytes) > size) fail(CJ_ERR_INTERNAL, "slab exhausted");
+        void *p = bytes ? mem->as<uint8_t>() + used : nullptr;
+        used += align(bytes);
+        return p;
+    }
+    template <typename T> T *take_as(size_t bytes) { return reinterpret_cast<T *>(take(bytes)); }
+    /* a buffer object over a part: the slab's owner keeps the memory */
+    DevPtr part(size_t bytes) {
+        auto b = std::make_shared<DevBuf>();
+        b->bytes = bytes;
+        b->arena = true;
+        b->ptr = take(bytes);
+        return b;
+    }
+};
+
+/* A base column decoded into dense device arrays (task's pointers, in `mem`
+ * or a slab of its executor). */
 struct Decoded {
     int32_t type = CJ_INT32;
     uint64_t rows = 0;
     ColumnPages src;
-    DevPtr values, valid, desc;
-    DevPtr loc, base;                   /* page index (page_first_row)        */
-    DevPtr own_state;                   /* the state, unless the status block's */
-    ColumnState *state = nullptr;       /* COL_* flags and errors (device)    */
-    int status_col = -1;                /* its place in the status block      */
-    bool ready = false;                 /* values / valid / desc written      */
+    DevPtr mem;
+    int status_col = -1; /* place of its state in the status block */
+    bool ready = false;  /* values / valid / desc written          */
     ColumnTask task{};
+
+    uint64_t value_bytes() const { return std::max<uint64_t>(rows, 1) * (type == CJ_INT32 ? 4 : 8); }
+    uint64_t valid_bytes() const { return std::max<uint64_t>((rows + 31) / 32, 1) * 4; }
+    uint64_t loc_bytes() const { return std::max<uint64_t>(src.num_pages, 1) * 4; }
+    uint64_t base_bytes() const { return (uint64_t)index_blocks(src.num_pages) * 8; }
+    void reserve(Slab &s) const {
+        s.reserve(loc_bytes());
+        s.reserve(base_bytes());
+        s.reserve(valid_bytes());
+        s.reserve(value_bytes());
+    }
 };
 
-/* Allocates a column's arrays and describes its index and decode. `state`
- * (device, zero before the launches) null: one of its own, errors then go
- * straight to the status word. */
-inline ColumnTask column_task(Context &ctx, Decoded &d, ColumnState *state) {
-    const uint64_t np = d.src.num_pages;
-    d.loc = ctx.alloc(std::max<uint64_t>(np, 1) * 4);
-    d.base = ctx.alloc(index_blocks(np) * 8);
-    d.valid = ctx.alloc(std::max<uint64_t>((d.rows + 31) / 32, 1) * 4);
-    if (d.type == CJ_VARCHAR) d.desc = ctx.alloc(std::max<uint64_t>(d.rows, 1) * 8);
-    else d.values = ctx.alloc(std::max<uint64_t>(d.rows, 1) * (d.type == CJ_INT32 ? 4 : 8));
+/* Describes a column's index and decode over arrays taken from `slab`. */
+inline ColumnTask column_task(Decoded &d, Slab &slab, ColumnState *state, unsigned int *err) {
     ColumnTask t{};
-    t.err = state ? &state->err : &ctx.d_status->errors;
-    if (!state) {
-        d.own_state = ctx.alloc(sizeof(ColumnState));
-        check_cuda(cudaMemsetAsync(d.own_state->ptr, 0, sizeof(ColumnState), ctx.stream), "memset");
-        state = d.own_state->as<ColumnState>();
-    }
-    d.state = state;
-    t.pages = d.src.dev;
-    t.num_pages = np;
-    t.rows = d.rows;
-    t.loc = d.loc->as<uint32_t>();
-    t.base = d.base->as<uint64_t>();
+    t.err = err;
     t.state = state;
-    t.values = d.values ? d.values->ptr : nullptr;
-    t.desc = d.desc ? d.desc->as<uint64_t>() : nullptr;
-    t.valid = d.valid->as<uint32_t>();
+    t.pages = d.src.dev;
+    t.num_pages = d.src.num_pages;
+    t.rows = d.rows;
+    t.loc = slab.take_as<uint32_t>(d.loc_bytes());
+    t.base = slab.take_as<uint64_t>(d.base_bytes());
+    t.valid = slab.take_as<uint32_t>(d.valid_bytes());
+    void *values = slab.take(d.value_bytes());
+    if (d.type == CJ_VARCHAR) t.desc = reinterpret_cast<uint64_t *>(values);
+    else t.values = values;
     t.type = d.type;
     d.task = t;
     return t;
@@ -145,14 +168,14 @@ inline Relation scan_relation(const cj_plan_desc &plan, const cj_plan_node &n) {
 inline ColView make_view(const Decoded &d, const Relation &R, const RelCol &c, const uint32_t *rid_a) {
     ColView v{};
     v.type = c.type;
-    v.values = d.values ? d.values->ptr : nullptr;
-    v.valid = d.valid->as<uint32_t>();
-    v.str_desc = d.desc ? d.desc->as<uint64_t>() : nullptr;
+    v.values = d.task.values;
+    v.valid = d.task.valid;
+    v.str_desc = d.task.desc;
     v.pages = d.src.dev;
     v.rid_a = rid_a;
     v.rid_b = c.vec >= 0 ? R.vecs[c.vec]->as<uint32_t>() : nullptr;
     v.null_sentinel = (c.sentinel && c.type == CJ_INT32) ? 1 : 0;
-    v.col_flags = &d.state->flags;
+    v.col_flags = &d.task.state->flags;
     return v;
 }
 

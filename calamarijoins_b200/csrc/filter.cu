@@ -501,17 +501,28 @@ class Filter {
     /* Indexes and decodes columns, one launch each for all of them. */
     void decode(const std::set<uint64_t> &need) {
         std::vector<ColumnTask> tasks;
-        DevPtr states = ctx.alloc(std::max<size_t>(need.size(), 1) * sizeof(ColumnState));
-        check_cuda(cudaMemsetAsync(states->ptr, 0, states->bytes, ctx.stream), "memset");
-        keep.push_back(states);
+        Slab slab;
         for (uint64_t c : need) {
             if (decoded.count(c)) continue;
             Decoded d;
             d.type = in.cols[c].type;
             d.rows = in.num_rows;
             d.src = in.cols[c];
-            tasks.push_back(column_task(ctx, d, states->as<ColumnState>() + tasks.size()));
-            tasks.back().err = &ctx.d_status->errors;
+            d.reserve(slab);
+            slab.reserve(sizeof(ColumnState));
+        }
+        if (!slab.size) return;
+        slab.open(ctx);
+        keep.push_back(slab.mem);
+        for (uint64_t c : need) {
+            if (decoded.count(c)) continue;
+            Decoded d;
+            d.type = in.cols[c].type;
+            d.rows = in.num_rows;
+            d.src = in.cols[c];
+            ColumnState *state = slab.take_as<ColumnState>(sizeof(ColumnState));
+            check_cuda(cudaMemsetAsync(state, 0, sizeof(ColumnState), ctx.stream), "memset");
+            tasks.push_back(column_task(d, slab, state, &ctx.d_status->errors));
             decoded.emplace(c, std::move(d));
         }
         if (tasks.empty()) return;
