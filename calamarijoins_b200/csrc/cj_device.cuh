@@ -47,6 +47,12 @@ CJ_DEV uint32_t open_slot(int64_t key, uint32_t nslots) {
     return __umulhi((uint32_t)key * 0x9E3779B9u, nslots);
 }
 
+/* The same for INT64 keys, the high word folded in as in hash_key. */
+CJ_DEV uint32_t open_slot_wide(int64_t key, uint32_t nslots) {
+    const uint32_t m = (uint32_t)key ^ ((uint32_t)((uint64_t)key >> 32) * 0x2545F491u);
+    return __umulhi((m ^ (m >> 15)) * 0x9E3779B9u, nslots);
+}
+
 /* Loads the 2048-entry Bloom tag table into shared memory. */
 CJ_DEV void load_bloom(uint16_t *s_bloom, const uint16_t *g_bloom) {
     const uint32_t *src = reinterpret_cast<const uint32_t *>(g_bloom);

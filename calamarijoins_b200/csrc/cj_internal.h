@@ -79,7 +79,7 @@ struct StatusBlock {
     unsigned int errors;          /* DevError bits                          */
     unsigned int pad;
     unsigned long long counter;   /* match counter of the last probe        */
-    unsigned long long table[8];  /* kTableWords of the last unique table   */
+    unsigned long long table[9];  /* kTableWords of the last unique table   */
     unsigned long long aux;       /* a count on its way to the host (filter) */
     unsigned long long stale[3];  /* DEV_ERR_STALE: check index, count found,
                                      count recorded (one of the mismatches) */
@@ -231,9 +231,10 @@ cudaError_t launch_columns(const Launch &L, ColumnTask *tasks, size_t n, bool in
 cudaError_t launch_columns_grouped(const Launch &L, const ColumnTask *tasks_dev, uint32_t n, const ColumnGrid &g);
 
 /* Table of unique build keys (k_unique.cu): direct-mapped when their range is
- * at most max_span, else, for INT32 keys (open_slots > 0), open-addressing.
- * `slots` holds max(4 max_span, 8 open_slots) bytes rounded up to 16,
- * 16-byte aligned; open_slots is at least twice the build rows. `params` (kTableWords words, zero before the build) receives what the
+ * at most max_span, else (open_slots > 0) open-addressing, with 8-byte slots
+ * for INT32 keys and 16-byte ones for INT64 keys (wide). `slots` holds
+ * unique_table_bytes, 16-byte aligned; open_slots is at least twice the build
+ * rows. `params` (kTableWords words, zero before the build) receives what the
  * device found. */
 constexpr uint32_t kArrayEmpty = 0xFFFFFFFFu;
 constexpr uint64_t kOpenMaxRows = 1ull << 28;
@@ -247,18 +248,26 @@ enum TableWord { /* of params */
     kTableSpan = 5,
     kTableDup = 6,     /* the build met a repeated key: the table is unusable */
     kTableDone = 7,    /* blocks of the range pass that have finished      */
-    kTableWords = 8
+    kTableEmpty = 8,   /* wide: a key next to the range, that of an empty slot */
+    kTableWords = 9
 };
 enum TableRefusal : unsigned long long {
     kTableSpread = 1,  /* the keys' range is above max_span           */
-    kTableRepeats = 2  /* more keys than values in their range        */
+    kTableRepeats = 2, /* more keys than values in their range        */
+    kTableWhole = 3    /* wide: the keys span all of INT64: no key is
+                          free to mark empty slots                    */
 };
 struct UniqueTable {
     void *slots;
     unsigned long long *params;
     uint64_t max_span;
     uint32_t open_slots; /* 0: no open-addressing table */
+    uint32_t wide;       /* 16-byte slots: INT64 build keys */
 };
+inline uint64_t unique_table_bytes(const UniqueTable &t) {
+    const uint64_t direct = t.max_span * 4, open = (uint64_t)t.open_slots * (t.wide ? 16 : 8);
+    return ((direct > open ? direct : open) + 15) & ~15ull;
+}
 /* What the params say (host copy or device): 0 unusable, 1 direct-mapped,
  * 2 open-addressing. */
 __host__ __device__ inline int table_kind(const unsigned long long *p, uint32_t open_slots) {

@@ -576,19 +576,20 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             if (ctx.opt.dense_keys > 0) {
                 /* Unique keys spread over at most dense_keys x rows values get
                  * a direct-mapped table: one random access per probe row
-                 * instead of a directory entry and a tuple; unique INT32 keys
-                 * that span more an open-addressing table: one sector. The
-                 * device works out the key range and which table it is, if
-                 * any; the host learns it at the probe's own synchronisation
-                 * and then, if neither, builds the hash table. Direct-mapped:
-                 * 4 bytes per slot, at 8 x rows 32 B per build row, at most
-                 * 2^28 slots (1 GiB); open-addressing: 16 B per build row.
-                 * One buffer serves both. */
+                 * instead of a directory entry and a tuple; unique keys that
+                 * span more an open-addressing table: one sector. The device
+                 * works out the key range and which table it is, if any; the
+                 * host learns it at the probe's own synchronisation and then,
+                 * if neither, builds another. Direct-mapped: 4 bytes per
+                 * slot, at 8 x rows 32 B per build row, at most 2^28 slots (1
+                 * GiB); open-addressing: 16 B per build row, 32 for INT64
+                 * keys. One buffer serves both. */
                 table.max_span = std::min<uint64_t>((uint64_t)ctx.opt.dense_keys * B.rows, 1ull << 28);
-                if (bk.type == CJ_INT32 && B.rows <= kOpenMaxRows)
+                table.wide = bk.type == CJ_INT64;
+                if (B.rows <= kOpenMaxRows)
                     table.open_slots = (uint32_t)std::max<uint64_t>(2 * B.rows, 1024);
                 table.params = ctx.d_status->table;
-                slots = ctx.alloc((std::max<uint64_t>(table.max_span * 4, table.open_slots * 8ull) + 15) & ~15ull);
+                slots = ctx.alloc(unique_table_bytes(table));
                 table.slots = slots->ptr;
                 if (!words_clear) clear_join_words();
                 KScope k(*this, "unique_build");
@@ -628,7 +629,8 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                         beside) {
                         const uint32_t R = rows_per_page_fixed(o.col.type);
                         o.pages = ctx.alloc((cap + R - 1) / R * kPageSize);
-                        o.direct_only = unique && o.from_build && table.open_slots && table.open_slots * 8ull +
+                        o.direct_only = unique && o.from_build && table.open_slots &&
+                                        table.open_slots * (table.wide ? 16ull : 8ull) +
                                                         it->second.src.num_pages * kPageSize > kEmitBesideOpen;
                         uo.cols[uo.n++] = {view(*o.rel, o.col, nullptr), o.pages->as<uint8_t>(), o.from_build ? 1 : 0,
                                            o.direct_only ? 1 : 0};
@@ -698,7 +700,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             }
             PhaseScope ph(*this, PH_BUILD);
             const unsigned long long *tp = ctx.h_status->table;
-            if (tp[kTableRefused] != kTableSpread && tp[kTableSpan] <= kMultiSpan * B.rows) {
+            if ((!tp[kTableRefused] || tp[kTableRefused] == kTableRepeats) && tp[kTableSpan] <= kMultiSpan * B.rows) {
                 multi = true;
                 multi_table.lo = (int64_t)tp[kTableLo];
                 multi_table.span = (uint32_t)tp[kTableSpan];
@@ -719,7 +721,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         auto count_join = [&]() {
             const int kind = table_kind(ctx.h_status->table, table.open_slots);
             stats.num_direct_joins += kind == 1;
-            stats.num_open_joins += kind == 2;
+            stats.num_open_joins += kind == 2 && !table.wide; /* INT32 keys, as documented */
         };
         bool all_fixed = true;
         for (const auto &o : outs) all_fixed &= o.col.type != CJ_VARCHAR;

@@ -4,9 +4,9 @@
  * pages and writes the result's pages.
  *
  * The table (launch_unique_build) is direct-mapped when the keys lie densely
- * (slots[key - lo] = build row), else, for INT32 keys, open-addressing
- * (8-byte slots key << 32 | build row, linear probing from the key's hash,
- * at most half full). Which one, and whether the keys are unique at all, is
+ * (slots[key - lo] = build row), else open-addressing (slots of 8 bytes, key
+ * << 32 | build row, or for INT64 keys of 16, key and build row; linear
+ * probing from the key's hash, at most half full). Which one, and whether the keys are unique at all, is
  * decided on the device: `params` says so to the kernels that follow and,
  * at the next synchronisation, to the host. Both kinds share one buffer.
  *
@@ -103,26 +103,39 @@ CJ_DEV void fold_range(const ColView &key, uint64_t first, uint64_t n, uint64_t 
 }
 
 /* Reads the folded range (from L2: other blocks wrote it) and decides. */
-CJ_DEV void decide_table(unsigned long long *p, uint64_t max_span) {
+CJ_DEV void decide_table(unsigned long long *p, uint64_t max_span, bool wide) {
     const unsigned long long cnt = __ldcg(p + 2);
     if (cnt == 0) return; /* no non-NULL key: span 0, nothing matches */
-    const unsigned long long b = ~__ldcg(p), width = __ldcg(p + 1) - b; /* max - min: the bias cancels */
-    if (width >= max_span) p[kTableRefused] = kTableSpread;
+    const unsigned long long b = ~__ldcg(p), e = __ldcg(p + 1), width = e - b; /* max - min: the bias cancels */
+    if (width >= max_span) {
+        p[kTableRefused] = wide && b == 0 && e == ~0ull ? kTableWhole : kTableSpread;
+        p[kTableEmpty] = (e != ~0ull ? e + 1 : b - 1) ^ (1ull << 63);
+    }
     else if (cnt > width + 1) p[kTableRefused] = kTableRepeats; /* more keys than values in their range */
     p[kTableLo] = b ^ (1ull << 63);
     p[kTableSpan] = width + 1;
 }
 
-/* Empty slots are all ones in either kind of table. */
+/* A slot of an open-addressing table of INT64 keys. */
+struct alignas(16) WideSlot {
+    unsigned long long key;
+    uint32_t rid, pad;
+};
+
+/* Empty slots are all ones, but for wide ones, whose key is kTableEmpty. */
 CJ_DEV uint64_t table_bytes(const UniqueTable &t) {
     const unsigned long long refused = t.params[kTableRefused];
-    if (refused == kTableSpread) return t.open_slots * 8ull;
+    if (refused == kTableSpread) return (uint64_t)t.open_slots * (t.wide ? 16 : 8);
     return refused ? 0ull : t.params[kTableSpan] * 4ull;
 }
 CJ_DEV void fill_table(const UniqueTable &t, uint64_t first, uint64_t stride) {
     const uint64_t bytes = table_bytes(t), n16 = (bytes + 15) / 16; /* the buffer is a multiple of 16 bytes */
-    const uint4 ones = make_uint4(~0u, ~0u, ~0u, ~0u);
-    for (uint64_t i = first; i < n16; i += stride) reinterpret_cast<uint4 *>(t.slots)[i] = ones;
+    uint4 empty = make_uint4(~0u, ~0u, ~0u, ~0u);
+    if (t.wide && t.params[kTableRefused] == kTableSpread) {
+        empty.x = (uint32_t)t.params[kTableEmpty];
+        empty.y = (uint32_t)(t.params[kTableEmpty] >> 32);
+    }
+    for (uint64_t i = first; i < n16; i += stride) reinterpret_cast<uint4 *>(t.slots)[i] = empty;
 }
 
 /* Each key claims its slot; meeting its own key there means that the keys
@@ -154,6 +167,32 @@ CJ_DEV void insert_rows(const ColView &key, const UniqueTable &t, uint64_t first
         return;
     }
     if (refused != kTableSpread || !t.open_slots) return;
+    if (t.wide) {
+        WideSlot *slots = reinterpret_cast<WideSlot *>(t.slots);
+        const unsigned long long empty = t.params[kTableEmpty];
+        for (uint64_t i = first; i < n; i += stride) {
+            if (*reinterpret_cast<volatile unsigned long long *>(t.params + kTableDup)) return;
+            int64_t k;
+            if (!load_key(key, (uint32_t)i, &k)) continue;
+            uint32_t h = open_slot_wide(k, t.open_slots);
+            for (uint32_t step = 0; step < t.open_slots; ++step) {
+                unsigned long long cur = __ldcg(&slots[h].key);
+                if (cur == empty) {
+                    cur = atomicCAS(&slots[h].key, empty, (unsigned long long)k);
+                    if (cur == empty) {
+                        slots[h].rid = (uint32_t)i;
+                        break;
+                    }
+                }
+                if (cur == (unsigned long long)k) {
+                    t.params[kTableDup] = 1ull;
+                    break;
+                }
+                if (++h == t.open_slots) h = 0;
+            }
+        }
+        return;
+    }
     unsigned long long *slots = reinterpret_cast<unsigned long long *>(t.slots);
     for (uint64_t i = first; i < n; i += stride) {
         /* a repeat is flagged once; every thread then stops */
@@ -185,7 +224,7 @@ __global__ void __launch_bounds__(kUniqueThreads)
         __threadfence();
         if (atomicAdd(t.params + kTableDone, 1ull) == gridDim.x - 1) {
             __threadfence();
-            decide_table(t.params, t.max_span);
+            decide_table(t.params, t.max_span, t.wide);
         }
     }
 }
@@ -208,7 +247,7 @@ __global__ void __launch_bounds__(kSmallThreads)
     const ColView key = resolve_view(key_arg);
     fold_range(key, threadIdx.x, n, kSmallThreads, t.params);
     __syncthreads();
-    if (threadIdx.x == 0) decide_table(t.params, t.max_span);
+    if (threadIdx.x == 0) decide_table(t.params, t.max_span, t.wide);
     __syncthreads();
     fill_table(t, threadIdx.x, kSmallThreads);
     __syncthreads();
@@ -236,7 +275,7 @@ __global__ void __launch_bounds__(kUniqueThreads)
         __threadfence();
         if (atomicAdd(T.table.params + kTableDone, 1ull) == T.key_blocks - 1) {
             __threadfence();
-            decide_table(T.table.params, T.table.max_span);
+            decide_table(T.table.params, T.table.max_span, T.table.wide);
         }
     }
 }
@@ -338,6 +377,7 @@ __global__ void __launch_bounds__(kUniqueThreads) k_multi_scatter(ColView key_ar
  * Measured at 64M x 4M rows (probe alone): five 605 us, four with 64
  * registers 619, six with 40 (spills) 620. */
 constexpr int kProbeBlocks = 5;
+constexpr int kWideBlocks = 4; /* 64 registers: the codes are 64-bit keys */
 constexpr int kMultiBlocks = 4; /* 64 registers; three with 80 1467 us, five with 48 2343 */
 constexpr int kItems = 8;                              /* rows per lane and step       */
 constexpr int kProbeThreads = 2048 / kItems;
@@ -364,6 +404,7 @@ template <typename T> struct DirectLookup {
         lo = first + skip;
         span = values;
     }
+    using Code = uint32_t;
     static constexpr bool kMask = false; /* a code says by itself whether it may be in the table */
     CJ_DEV uint32_t code(T key, bool present, bool *in) const {
         *in = true;
@@ -399,6 +440,7 @@ template <typename T> struct OpenLookup {
     CJ_DEV OpenLookup(const UniqueTable &t)
         : slots(reinterpret_cast<const unsigned long long *>(t.slots)), nslots(t.open_slots),
           lo((uint32_t)t.params[kTableLo]), width((uint32_t)(t.params[kTableSpan] - 1)) {}
+    using Code = uint32_t;
     static constexpr bool kMask = true;
     CJ_DEV uint32_t code(T key, bool present, bool *in) const {
         /* an INT64 key that is no INT32 value equals no build key */
@@ -429,6 +471,48 @@ template <typename T> struct OpenLookup {
     }
 };
 
+/* The same over INT64 build keys: a slot is one 16-byte load. */
+template <typename T> struct WideLookup {
+    const WideSlot *slots;
+    uint32_t nslots;
+    unsigned long long lo, width, empty;
+    using Code = T;
+    static constexpr bool kMask = true;
+    CJ_DEV WideLookup(const UniqueTable &t)
+        : slots(reinterpret_cast<const WideSlot *>(t.slots)), nslots(t.open_slots), lo(t.params[kTableLo]),
+          width(t.params[kTableSpan] - 1), empty(t.params[kTableEmpty]) {}
+    CJ_DEV T code(T key, bool present, bool *in) const {
+        *in = present && (unsigned long long)(int64_t)key - lo <= width;
+        return key;
+    }
+    CJ_DEV T key_of(T c) const { return c; }
+    CJ_DEV ulonglong2 slot(uint32_t h) const { return __ldg(reinterpret_cast<const ulonglong2 *>(slots + h)); }
+    CJ_DEV void find(const T *c, uint32_t ok, uint32_t *rid) const {
+#pragma unroll
+        for (int it = 0; it < kItems; it += 4) { /* four rows' slots in flight: 16 registers */
+            ulonglong2 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[j].x = empty;
+                if ((ok >> (it + j)) & 1u) v[j] = slot(open_slot_wide(c[it + j], nslots));
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                rid[it + j] = kArrayEmpty;
+                uint32_t h = open_slot_wide(c[it + j], nslots);
+                for (uint32_t step = 0; v[j].x != empty && step < nslots; ++step) {
+                    if (v[j].x == (unsigned long long)(int64_t)c[it + j]) {
+                        rid[it + j] = (uint32_t)v[j].y;
+                        break;
+                    }
+                    if (++h == nslots) h = 0;
+                    v[j] = slot(h);
+                }
+            }
+        }
+    }
+};
+
 /* The keys of 256 rows of a page, from row s0 + part * 256 on, as the table
  * sees them: bit `it` of the result set when row it * 32 + lane of them is
  * non-NULL and may be in the table. The value positions come from the
@@ -436,7 +520,7 @@ template <typename T> struct OpenLookup {
  * their popcounts; *before: the page's values before row s0, moved on. */
 template <typename T, class LK>
 CJ_DEV uint32_t page_keys(const uint8_t *pg, uint32_t nr, uint32_t nv, uint32_t s0, uint32_t part, uint32_t *before,
-                          const LK &lk, uint32_t *code, unsigned int *err) {
+                          const LK &lk, typename LK::Code *code, unsigned int *err) {
     constexpr uint32_t DB = sizeof(T) == 4 ? 4u : 8u;
     const T *vals = reinterpret_cast<const T *>(pg + DB);
     const uint32_t lane = lane_id(), r0 = s0 + part * kWarpRows + lane;
@@ -609,7 +693,7 @@ CJ_DEV void emit_packed(const UniqueOut &out, const EmitPlan &plan, const W &w, 
  * warp), and the warps write it. row0: the relation row of the warp's first;
  * ok: a lane's items to look up; buf alternates between steps. Block-wide. */
 template <typename T, class LK>
-CJ_DEV void probe_step(const LK &lk, const uint32_t *code, uint32_t ok, uint32_t row0, const UniqueOut &out,
+CJ_DEV void probe_step(const LK &lk, const typename LK::Code *code, uint32_t ok, uint32_t row0, const UniqueOut &out,
                        const EmitPlan &plan, StepShared &sh, uint32_t part, uint32_t buf) {
     const uint32_t lane = lane_id(), lt = lanemask_lt();
     WarpMatches &w = sh.matches[part];
@@ -681,6 +765,7 @@ template <typename T> struct MultiLookup {
     DirectLookup<T> d;
     const unsigned long long *entries;
     const uint32_t *rows;
+    using Code = uint32_t;
     static constexpr bool kMask = false;
     CJ_DEV MultiLookup(const MultiTable &t)
         : d(nullptr, t.lo, t.span), entries(t.entries + (d.lo - t.lo)), rows(t.rows) {}
@@ -846,7 +931,8 @@ template <typename T> CJ_DEV bool row_key(const ColView &c, uint32_t i, T *key) 
 template <typename T, class LK, class SH>
 CJ_DEV void probe_rows(const ColView &col, uint32_t n, uint64_t t0, const LK &lk, const UniqueOut &out,
                        const EmitPlan &plan, SH &sh, uint32_t part, uint32_t buf) {
-    uint32_t code[kItems] = {}, ok = 0;
+    typename LK::Code code[kItems] = {};
+    uint32_t ok = 0;
     const uint64_t r0 = t0 + part * kWarpRows;
 #pragma unroll
     for (int it = 0; it < kItems; ++it) {
@@ -880,7 +966,7 @@ CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueO
             }
             uint32_t before = 0;
             for (uint32_t s0 = 0; s0 < nr; s0 += kTileRows) {
-                uint32_t code[kItems] = {};
+                typename LK::Code code[kItems] = {};
                 const uint32_t ok = page_keys<T>(pg, nr, nv, s0, part, &before, lk, code, k.err);
                 probe_step<T>(lk, code, ok, (uint32_t)rs + s0 + part * kWarpRows, out, plan, sh, part, buf);
                 buf ^= 1u;
@@ -910,6 +996,23 @@ __global__ void __launch_bounds__(kProbeThreads, kProbeBlocks)
     if (refused == kTableSpread && t.open_slots) probe_all<kPages, T>(k, n, OpenLookup<T>(t), out, sh);
 }
 
+/* A table that may have wide slots: a kernel of its own, so that their
+ * registers are not the other's. */
+template <bool kPages, typename T>
+__global__ void __launch_bounds__(kProbeThreads, kWideBlocks)
+    k_probe_wide(const __grid_constant__ ProbeKey k, uint32_t n, const __grid_constant__ UniqueTable t,
+                 const __grid_constant__ UniqueOut out) {
+    __shared__ StepShared sh;
+    const unsigned long long refused = t.params[kTableRefused];
+    if (t.params[kTableDup]) return;
+    if (refused == 0) {
+        const DirectLookup<T> lk(reinterpret_cast<const uint32_t *>(t.slots), (int64_t)t.params[kTableLo],
+                                 (uint32_t)t.params[kTableSpan]);
+        probe_all<kPages, T>(k, n, lk, out, sh);
+    }
+    if (refused == kTableSpread && t.open_slots) probe_all<kPages, T>(k, n, WideLookup<T>(t), out, sh);
+}
+
 template <bool kPages, typename T>
 __global__ void __launch_bounds__(kProbeThreads, kMultiBlocks)
     k_probe_multi(const __grid_constant__ ProbeKey k, uint32_t n, const __grid_constant__ MultiTable t,
@@ -923,7 +1026,7 @@ __global__ void __launch_bounds__(kProbeThreads, kMultiBlocks)
  * device. */
 template <class K> void prefer_l1(K kernel) {
     constexpr int kDevices = 64;
-    static std::atomic<const void *> done[kDevices][4];
+    static std::atomic<const void *> done[kDevices][12];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) {
         cudaGetLastError();
@@ -954,7 +1057,7 @@ cudaError_t launch_unique_build(const Launch &L, const ColView &key, uint32_t n,
     const uint64_t rows_per_block = kUniqueThreads * kUniqueRows;
     const unsigned g = (unsigned)std::min<uint64_t>((n + rows_per_block - 1) / rows_per_block, wave);
     k_unique_range<<<g, kUniqueThreads, 0, L.stream>>>(key, n, t);
-    const uint64_t most = std::max<uint64_t>(t.max_span * 4, t.open_slots * 8ull) / 16 + 1;
+    const uint64_t most = unique_table_bytes(t) / 16 + 1;
     k_unique_fill<<<(unsigned)std::min<uint64_t>((most + 255) / 256, wave), kUniqueThreads, 0, L.stream>>>(t);
     k_unique_insert<<<g, kUniqueThreads, 0, L.stream>>>(key, n, t);
     count_launches(3);
@@ -966,9 +1069,12 @@ cudaError_t launch_probe_unique(const Launch &L, const ProbeKey &k, uint32_t n, 
     if (n == 0) return cudaSuccess;
     const bool pages = k.base != nullptr;
     const uint64_t tiles = pages ? k.num_pages : ((uint64_t)n + kTileRows - 1) / kTileRows;
-    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * kProbeBlocks));
-    const auto kernel = k.col.type == CJ_INT32 ? (pages ? k_probe_unique<true, int32_t> : k_probe_unique<false, int32_t>)
+    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * (t.wide ? kWideBlocks : kProbeBlocks)));
+    const auto narrow = k.col.type == CJ_INT32 ? (pages ? k_probe_unique<true, int32_t> : k_probe_unique<false, int32_t>)
                                                : (pages ? k_probe_unique<true, long long> : k_probe_unique<false, long long>);
+    const auto wide = k.col.type == CJ_INT32 ? (pages ? k_probe_wide<true, int32_t> : k_probe_wide<false, int32_t>)
+                                             : (pages ? k_probe_wide<true, long long> : k_probe_wide<false, long long>);
+    const auto kernel = t.wide ? wide : narrow;
     prefer_l1(kernel);
     kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out);
     count_launches(1);
@@ -980,7 +1086,7 @@ UniqueGrid place_unique(const Launch &L, UniqueBuildTask *tasks, size_t n) {
     const uint64_t wave = (uint64_t)L.num_sms * 8, rows = kUniqueThreads * kUniqueRows;
     for (size_t k = 0; k < n; ++k) {
         UniqueBuildTask &t = tasks[k];
-        const uint64_t most = std::max<uint64_t>(t.table.max_span * 4, t.table.open_slots * 8ull) / 16 + 1;
+        const uint64_t most = unique_table_bytes(t.table) / 16 + 1;
         t.key_blocks = (uint32_t)std::min<uint64_t>((t.n + rows - 1) / rows, wave);
         t.key_base = g.key;
         t.fill_blocks = (uint32_t)std::min<uint64_t>((most + kUniqueThreads * 8 - 1) / (kUniqueThreads * 8), wave);

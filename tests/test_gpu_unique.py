@@ -216,3 +216,36 @@ def test_repeated_dense_keys_in_a_chain(gpu_ctx):
     for flags in (0, _lib.CJ_EXEC_RESULT_ON_DEVICE):
         got, _ = run_product(plan, gpu_ctx, flags)
         assert_same(got, want)
+
+
+@pytest.mark.parametrize("nb", [65, 1000, 8193, 40_000])
+@pytest.mark.parametrize("case", ["random", "top", "bottom", "whole", "repeat", "minus_one"])
+@pytest.mark.parametrize("pt", [I, L])
+def test_wide_open_addressing(gpu_ctx, nb, case, pt):
+    """Spread INT64 keys: 16-byte slots whose empty key lies next to the
+    keys' range, which may end at either end of INT64 (at both: the hash
+    table), hold -1 and the slots' fill pattern, or repeat."""
+    rng = np.random.default_rng(nb)
+    bkeys = np.unique(rng.integers(-(2 ** 62), 2 ** 62, nb))
+    bkeys[0], bkeys[-1] = -(2 ** 62) - 5, 2 ** 62 + 5
+    if case in ("top", "whole"):
+        bkeys[-1] = 2 ** 63 - 1
+    if case in ("bottom", "whole"):
+        bkeys[0] = -(2 ** 63)
+    if case == "minus_one":
+        bkeys[1:4] = [-1, 0, 5]
+    if case == "repeat":
+        bkeys[7] = bkeys[9]
+    if pt == I:
+        bkeys[4:40] = np.arange(36) * 1000 - 7000
+    bkeys = rng.permutation(bkeys)
+    n = 2 * nb + 5000
+    pkeys = bkeys[rng.integers(0, len(bkeys), n)].copy()
+    miss = rng.random(n) < 0.3
+    pkeys[miss] ^= 1 << 20
+    if pt == I:
+        pkeys = np.where(rng.random(n) < 0.5, rng.integers(-20, 60, n) * 500, np.clip(pkeys, LO, HI))
+    plan = _plan(bkeys, pkeys, L, pt, (rng.random(len(bkeys)) > 0.02).astype(np.uint8),
+                 (rng.random(n) > 0.02).astype(np.uint8), bpay=[(I, np.arange(len(bkeys)), None)],
+                 ppay=[(F, rng.random(n), None)])
+    _check(plan, gpu_ctx, "hash")
