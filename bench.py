@@ -299,6 +299,21 @@ def algorithmic_bytes(kernel: str, st: dict, plan_info: dict):
         # slots, 2 per build row) once; per match 2 x 4 B row ids and the
         # 4 B key the probe emits for the root's key columns
         return npr * (4 + 1 / 8) + nb * 2 * 8 + m * 12
+    if kernel == "probe_unique" and WL["name"] in ("c2", "c2s"):
+        # probe keys (4 B + validity bit) and the table once; per match the
+        # probe FP64 value read and written and the 4 B key. Direct-mapped (4 B
+        # per slot): the build INT64 column read once, a value written per
+        # match; open addressing (2 slots of 8 B per build row): a 4 B row id
+        # per match for the page writer
+        if st.get("num_direct_joins"):
+            return npr * (4 + 1 / 8) + nb * (4 + 8) + m * (8 + 8 + 4 + 8)
+        if st.get("num_open_joins"):
+            return npr * (4 + 1 / 8) + nb * 2 * 8 + m * (8 + 8 + 4 + 4)
+        return None  # the launch found the table unusable and returned at once
+    if kernel == "probe_multi" and WL["name"] == "c2h":
+        # as above over 8 B per distinct key (3/4 of the build rows) and 4 B
+        # per build row; a row id per match for the build column
+        return npr * (4 + 1 / 8) + nb * (0.75 * 8 + 4) + m * (8 + 8 + 4 + 4)
     if kernel == "write_pages_int32":
         # per output row: 4 B match row id + 4 B value + validity bit read; page bytes written
         pages = (m + 1983) // 1984

@@ -37,6 +37,10 @@ constexpr uint64_t kMultiSpan = 4; /* values of the range per build row */
  * apart (64M probe rows). A direct-mapped table is 16 MB there. */
 constexpr uint64_t kEmitBesideOpen = 48ull << 20;
 
+/* Memory taken for matches that may not come is not asked about up to this
+ * size (a query of the free memory takes tens of us). */
+constexpr uint64_t kAmpleRoom = 4ull << 30;
+
 enum Phase { PH_UPLOAD, PH_DECODE, PH_BUILD, PH_PROBE, PH_NL, PH_INTER, PH_MAT, PH_DOWNLOAD, PH_COUNT };
 /* NVTX range names of the phases (host-side ranges around the enqueueing of
  * each phase; visible in Nsight Systems timelines). */
@@ -157,6 +161,20 @@ class Executor {
         }
         stats.output_rows = rows;
         stats.output_pages = pages;
+    }
+
+    /* Whether `bytes` may be set aside for matches that may not come: above
+     * kAmpleRoom, half of what is left. A selective join whose matches would
+     * fit does not fail for room it would not have used. */
+    bool room_for(uint64_t bytes) {
+        if (bytes <= kAmpleRoom) return true;
+        size_t left = 0, total = 0;
+        uint64_t used = 0, reserved = 0;
+        ck(cudaMemGetInfo(&left, &total), "cudaMemGetInfo");
+        ck(cudaMemPoolGetAttribute(ctx.pool, cudaMemPoolAttrUsedMemCurrent, &used), "pool attr");
+        ck(cudaMemPoolGetAttribute(ctx.pool, cudaMemPoolAttrReservedMemCurrent, &reserved), "pool attr");
+        std::lock_guard<std::mutex> g(ctx.dev_mu); /* frees of other threads touch the cache too */
+        return bytes <= (left + (reserved - std::min(reserved, used)) + ctx.dev_cached) / 2;
     }
 
     const cj_table *resident(uint64_t t) const { return resident_input(plan, t); }
@@ -619,6 +637,11 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                  * ids are collected for the others only. */
                 UniqueOut uo{};
                 uo.match = mo;
+                uint64_t beside_bytes = 0; /* at most: a column's pages for `cap` rows */
+                for (const auto &o : outs)
+                    if (is_root && !o.from_keys && o.col.type != CJ_VARCHAR)
+                        beside_bytes += cap * (o.col.type == CJ_INT32 ? 5 : 9);
+                const bool room = room_for(beside_bytes);
                 for (auto &o : outs) {
                     if (!is_root || o.from_keys) continue;
                     const auto it = decoded.find({o.col.input, o.col.col});
@@ -626,7 +649,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                         !o.from_build || !multi || it == decoded.end() ||
                         (multi_table.span * 2ull + B.rows) * 4 + it->second.src.num_pages * kPageSize <= kEmitBesideOpen;
                     if (o.col.type != CJ_VARCHAR && it != decoded.end() && it->second.ready && uo.n < kEmitColumns &&
-                        beside) {
+                        beside && room) {
                         const uint32_t R = rows_per_page_fixed(o.col.type);
                         o.pages = ctx.alloc((cap + R - 1) / R * kPageSize);
                         o.direct_only = unique && o.from_build && table.open_slots &&
@@ -711,7 +734,10 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 /* room for the keys' mean number of rows per match, up to 4;
                  * a result above it runs the probe again */
                 const uint64_t mean = P.rows * (uint64_t)tp[kTableCount] / (uint64_t)tp[kTableSpan];
-                cap = std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(cap, mean), 4 * P.rows), 0xFFFFFFFFull);
+                const uint64_t more = std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(cap, mean), 4 * P.rows),
+                                                         0xFFFFFFFFull);
+                /* a match: two row ids and a key at most, here */
+                if (more > cap && room_for(more * 17)) cap = more;
                 KScope k(*this, "multi_build");
                 ck(launch_multi_build(L, bv, (uint32_t)B.rows, multi_table), "multi_build");
             } else {
