@@ -513,15 +513,25 @@ template <typename T> struct WideLookup {
     }
 };
 
+/* A CTA's step takes one page of an INT32 key column (2,048 rows or fewer at
+ * a time), or two of an INT64 one side by side: a full page of 8-byte keys
+ * has 1,007 rows, and one page a step left half of the warps without any
+ * (300K x 5M INT64 rows, the whole join: 352 us, 306 with two). */
+template <typename T> constexpr uint32_t kStepPages = sizeof(T) == 4 ? 1 : 2;
+template <typename T> constexpr uint32_t kPageParts = kParts / kStepPages<T>; /* warps of a page */
+template <typename T> constexpr uint32_t kPageRows = kTileRows / kStepPages<T>;
+
 /* The keys of 256 rows of a page, from row s0 + part * 256 on, as the table
  * sees them: bit `it` of the result set when row it * 32 + lane of them is
  * non-NULL and may be in the table. The value positions come from the
- * bitmap: the 64 words of rows [s0, s0 + 2048) two per lane, a warp scan of
- * their popcounts; *before: the page's values before row s0, moved on. */
+ * bitmap: the words of rows [s0, s0 + kPageRows), one or two per lane, a warp
+ * scan of their popcounts; *before: the page's values before row s0, moved
+ * on. */
 template <typename T, class LK>
 CJ_DEV uint32_t page_keys(const uint8_t *pg, uint32_t nr, uint32_t nv, uint32_t s0, uint32_t part, uint32_t *before,
                           const LK &lk, typename LK::Code *code, unsigned int *err) {
     constexpr uint32_t DB = sizeof(T) == 4 ? 4u : 8u;
+    constexpr int kWords = kPageRows<T> / 1024;
     const T *vals = reinterpret_cast<const T *>(pg + DB);
     const uint32_t lane = lane_id(), r0 = s0 + part * kWarpRows + lane;
     uint32_t present = 0;
@@ -538,9 +548,9 @@ CJ_DEV uint32_t page_keys(const uint8_t *pg, uint32_t nr, uint32_t nv, uint32_t 
     } else {
         const uint32_t nb = (nr + 7) / 8, bm0 = kPageSize - nb;
         const uint32_t *words = reinterpret_cast<const uint32_t *>(pg);
-        uint32_t w[2];
+        uint32_t w[kWords], cnt[kWords];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) { /* word s0 / 32 + j * 32 + lane of the bitmap */
+        for (int j = 0; j < kWords; ++j) { /* word s0 / 32 + j * 32 + lane of the bitmap */
             const uint32_t first = s0 + (j * 32 + lane) * 32;
             w[j] = 0;
             if (first < nr) {
@@ -549,15 +559,22 @@ CJ_DEV uint32_t page_keys(const uint8_t *pg, uint32_t nr, uint32_t nv, uint32_t 
                 w[j] = __funnelshift_r(lo, hi, sh);
                 if (nr - first < 32) w[j] &= (1u << (nr - first)) - 1u;
             }
+            cnt[j] = __popc(w[j]);
         }
-        const uint32_t c0 = __popc(w[0]), c1 = __popc(w[1]);
-        const uint32_t t0 = __reduce_add_sync(0xffffffffu, c0);
-        /* this part's words and the values before each: lanes of one of the
-         * two halves */
-        const bool low = part < kParts / 2;
-        const uint32_t word = low ? w[0] : w[1], cnt = low ? c0 : c1;
-        const uint32_t pre = *before + (low ? 0u : t0) + warp_inclusive_scan(cnt) - cnt;
-        if (s0 + kTileRows < nr) *before += t0 + __reduce_add_sync(0xffffffffu, c1);
+        /* this part's words and the values before each */
+        uint32_t word, pre;
+        if constexpr (kWords == 2) { /* lanes of one of the two halves */
+            const uint32_t t0 = __reduce_add_sync(0xffffffffu, cnt[0]);
+            const bool low = part < kParts / 2;
+            const uint32_t mine = low ? cnt[0] : cnt[1];
+            word = low ? w[0] : w[1];
+            pre = *before + (low ? 0u : t0) + warp_inclusive_scan(mine) - mine;
+            if (s0 + kPageRows<T> < nr) *before += t0 + __reduce_add_sync(0xffffffffu, cnt[1]);
+        } else {
+            word = w[0];
+            pre = *before + warp_inclusive_scan(cnt[0]) - cnt[0];
+            if (s0 + kPageRows<T> < nr) *before += __reduce_add_sync(0xffffffffu, cnt[0]);
+        }
         const uint32_t lt = lanemask_lt(), bit = 1u << lane;
         uint32_t most = 0;
 #pragma unroll
@@ -912,10 +929,10 @@ CJ_DEV void probe_step(const MultiLookup<T> &lk, const uint32_t *code, uint32_t,
     }
 }
 
-/* Asks L2 for a warp's eighth of a page that it reads next: its keys then
- * cost an L2 round trip, not one to HBM. */
-CJ_DEV void prefetch_part(const uint8_t *pg, uint32_t part) {
-    constexpr uint32_t kLines = kPageSize / 128 / kParts;
+/* Asks L2 for a warp's part of a page that it reads next: its keys then cost
+ * an L2 round trip, not one to HBM. */
+template <typename T> CJ_DEV void prefetch_part(const uint8_t *pg, uint32_t part) {
+    constexpr uint32_t kLines = kPageSize / 128 / kPageParts<T>;
     if (lane_id() < kLines) asm volatile("prefetch.global.L2 [%0];" ::"l"(pg + (part * kLines + lane_id()) * 128));
 }
 
@@ -946,18 +963,18 @@ CJ_DEV void probe_rows(const ColView &col, uint32_t n, uint64_t t0, const LK &lk
     probe_step<T>(lk, code, ok, (uint32_t)r0, out, plan, sh, part, buf);
 }
 
-template <bool kPages, typename T, class LK, class SH>
-CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueOut &out, SH &sh) {
-    const EmitPlan plan(out, LK::kMask);
-    const uint32_t part = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); /* warp-uniform */
+/* The key column's pages, one a step (INT32) or two (INT64). Block-wide. */
+template <typename T, class LK, class SH>
+CJ_DEV void probe_pages(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueOut &out, const EmitPlan &plan, SH &sh,
+                        uint32_t part) {
     uint32_t buf = 0;
-    if constexpr (kPages) {
+    if constexpr (kStepPages<T> == 1) {
         for (uint64_t p = blockIdx.x; p < k.num_pages; p += gridDim.x) {
             const uint8_t *pg = k.col.pages + p * kPageSize;
             const uint32_t head = __ldg(reinterpret_cast<const uint32_t *>(pg));
             const uint32_t nr = head & 0xFFFFu, nv = head >> 16;
             const uint64_t rs = page_first_row(k.base, k.loc, p);
-            if (p + gridDim.x < k.num_pages) prefetch_part(pg + (uint64_t)gridDim.x * kPageSize, part);
+            if (p + gridDim.x < k.num_pages) prefetch_part<T>(pg + (uint64_t)gridDim.x * kPageSize, part);
             if (nv > nr || sizeof(T) + sizeof(T) * nv + (nr + 7) / 8 > kPageSize)
                 continue; /* the index has raised the error */
             if (rs + nr > n) {
@@ -965,7 +982,7 @@ CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueO
                 continue;
             }
             uint32_t before = 0;
-            for (uint32_t s0 = 0; s0 < nr; s0 += kTileRows) {
+            for (uint32_t s0 = 0; s0 < nr; s0 += kPageRows<T>) {
                 typename LK::Code code[kItems] = {};
                 const uint32_t ok = page_keys<T>(pg, nr, nv, s0, part, &before, lk, code, k.err);
                 probe_step<T>(lk, code, ok, (uint32_t)rs + s0 + part * kWarpRows, out, plan, sh, part, buf);
@@ -973,7 +990,57 @@ CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueO
             }
         }
     } else {
+        const uint64_t stride = (uint64_t)gridDim.x * 2;
+        const uint32_t ppart = part % kPageParts<T>;
+        for (uint64_t p0 = (uint64_t)blockIdx.x * 2; p0 < k.num_pages; p0 += stride) {
+            const uint64_t p = p0 + part / kPageParts<T>, q = p ^ 1; /* p0 is even */
+            const uint8_t *pg = k.col.pages + p * kPageSize;
+            uint32_t nr = 0, nv = 0, other = 0;
+            uint64_t rs = 0;
+            if (q < k.num_pages) other = __ldg(reinterpret_cast<const uint32_t *>(k.col.pages + q * kPageSize)) & 0xFFFFu;
+            if (p < k.num_pages) {
+                const uint32_t head = __ldg(reinterpret_cast<const uint32_t *>(pg));
+                nr = head & 0xFFFFu;
+                nv = head >> 16;
+                rs = page_first_row(k.base, k.loc, p);
+            }
+            const uint32_t turns = max(nr, other); /* as many as the page with more rows takes */
+            if (p + stride < k.num_pages) prefetch_part<T>(pg + stride * kPageSize, ppart);
+            if (nv > nr || sizeof(T) + sizeof(T) * nv + (nr + 7) / 8 > kPageSize) {
+                nr = 0; /* the index has raised the error */
+            } else if (rs + nr > n) {
+                if (lane_id() == 0) atomicOr(k.err, DEV_ERR_ROW_COUNT);
+                nr = 0;
+            }
+            uint32_t before = 0;
+            for (uint32_t s0 = 0; s0 < turns; s0 += kPageRows<T>) {
+                typename LK::Code code[kItems] = {};
+                uint32_t ok = 0;
+                if (s0 < nr) {
+                    ok = page_keys<T>(pg, nr, nv, s0, ppart, &before, lk, code, k.err);
+                } else {
+#pragma unroll
+                    for (int it = 0; it < kItems; ++it) {
+                        bool in;
+                        code[it] = lk.code(T(0), false, &in);
+                    }
+                }
+                probe_step<T>(lk, code, ok, (uint32_t)rs + s0 + ppart * kWarpRows, out, plan, sh, part, buf);
+                buf ^= 1u;
+            }
+        }
+    }
+}
+
+template <bool kPages, typename T, class LK, class SH>
+CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueOut &out, SH &sh) {
+    const EmitPlan plan(out, LK::kMask);
+    const uint32_t part = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); /* warp-uniform */
+    if constexpr (kPages) {
+        probe_pages<T>(k, n, lk, out, plan, sh, part);
+    } else {
         const ColView col = resolve_view(k.col);
+        uint32_t buf = 0;
         for (uint64_t t0 = (uint64_t)blockIdx.x * kTileRows; t0 < n; t0 += (uint64_t)gridDim.x * kTileRows) {
             probe_rows<T>(col, n, t0, lk, out, plan, sh, part, buf);
             buf ^= 1u;
@@ -1019,6 +1086,12 @@ __global__ void __launch_bounds__(kProbeThreads, kMultiBlocks)
                   const __grid_constant__ UniqueOut out) {
     __shared__ MultiShared sh;
     probe_all<kPages, T>(k, n, MultiLookup<T>(t), out, sh);
+}
+
+/* Steps of a probe's CTAs. */
+uint64_t probe_tiles(const ProbeKey &k, uint32_t n) {
+    if (!k.base) return ((uint64_t)n + kTileRows - 1) / kTileRows;
+    return k.col.type == CJ_INT32 ? k.num_pages : (k.num_pages + 1) / 2;
 }
 
 /* Random loads in flight are held in L1: as little of it as possible goes to
@@ -1068,7 +1141,7 @@ cudaError_t launch_probe_unique(const Launch &L, const ProbeKey &k, uint32_t n, 
                                 const UniqueOut &out) {
     if (n == 0) return cudaSuccess;
     const bool pages = k.base != nullptr;
-    const uint64_t tiles = pages ? k.num_pages : ((uint64_t)n + kTileRows - 1) / kTileRows;
+    const uint64_t tiles = probe_tiles(k, n);
     const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * (t.wide ? kWideBlocks : kProbeBlocks)));
     const auto narrow = k.col.type == CJ_INT32 ? (pages ? k_probe_unique<true, int32_t> : k_probe_unique<false, int32_t>)
                                                : (pages ? k_probe_unique<true, long long> : k_probe_unique<false, long long>);
@@ -1126,7 +1199,7 @@ cudaError_t launch_probe_multi(const Launch &L, const ProbeKey &k, uint32_t n, c
                                const UniqueOut &out) {
     if (n == 0) return cudaSuccess;
     const bool pages = k.base != nullptr;
-    const uint64_t tiles = pages ? k.num_pages : ((uint64_t)n + kTileRows - 1) / kTileRows;
+    const uint64_t tiles = probe_tiles(k, n);
     const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * kMultiBlocks));
     const auto kernel = k.col.type == CJ_INT32 ? (pages ? k_probe_multi<true, int32_t> : k_probe_multi<false, int32_t>)
                                                : (pages ? k_probe_multi<true, long long> : k_probe_multi<false, long long>);
