@@ -246,17 +246,23 @@ enum TableWord { /* of params */
     kTableRefused = 3, /* not direct-mapped: a TableRefusal                */
     kTableLo = 4,      /* smallest key, values in the range                */
     kTableSpan = 5,
-    kTableDup = 6,     /* the build met a repeated key: the table is unusable */
+    kTableDup = 6,     /* the build met a repeated key, or a walk of kMaxWalk
+                          slots: the table is unusable                     */
     kTableDone = 7,    /* blocks of the range pass that have finished      */
-    kTableEmpty = 8,   /* wide: a key next to the range, that of an empty slot */
+    kTableEmpty = 8,   /* a key next to the range, that of an empty slot (but
+                          for kTableWhole)                                 */
     kTableWords = 9
 };
 enum TableRefusal : unsigned long long {
     kTableSpread = 1,  /* the keys' range is above max_span           */
     kTableRepeats = 2, /* more keys than values in their range        */
-    kTableWhole = 3    /* wide: the keys span all of INT64: no key is
-                          free to mark empty slots                    */
+    kTableWhole = 3    /* the keys span all of INT64: no key is free to
+                          mark empty slots                            */
 };
+/* An insert walks at most this many slots of an open-addressing table (at
+ * most half full: about one on average); keys whose hashes pile up, on which
+ * the walks' sum would be quadratic, go on to the hash table. */
+constexpr uint32_t kMaxWalk = 512;
 struct UniqueTable {
     void *slots;
     unsigned long long *params;
@@ -374,6 +380,32 @@ cudaError_t launch_multi_build(const Launch &L, const ColView &key, uint32_t n, 
  * above out.match.capacity the output is incomplete: run again with room. */
 cudaError_t launch_probe_multi(const Launch &L, const ProbeKey &k, uint32_t n, const MultiTable &t,
                                const UniqueOut &out);
+
+/* The same over any range that leaves a key free for the empty slots: open
+ * addressing, a slot per key with its count and its row or the end of its
+ * rows. `found` (zero before the build) receives what the device found. */
+struct alignas(16) MultiSlot {
+    unsigned long long key;
+    uint32_t low, count;
+};
+struct OpenMultiTable {
+    MultiSlot *slots;
+    uint32_t *rows;              /* build rows                              */
+    uint32_t *slot_of;           /* build rows: scratch of the build        */
+    unsigned long long *found;   /* kMultiWords words                       */
+    unsigned long long lo, width, empty; /* smallest key, largest - smallest,
+                                    the key of an empty slot                */
+    uint32_t nslots;             /* at least twice the build rows           */
+};
+enum MultiWord {
+    kMultiKeys = 0,   /* different keys                                      */
+    kMultiGaveUp = 1, /* a key's walk reached kMaxWalk: the table is unusable */
+    kMultiCursor = 2,
+    kMultiWords = 3
+};
+cudaError_t launch_open_multi_build(const Launch &L, const ColView &key, uint32_t n, const OpenMultiTable &t);
+cudaError_t launch_probe_open_multi(const Launch &L, const ProbeKey &k, uint32_t n, const OpenMultiTable &t,
+                                    const UniqueOut &out);
 
 /* The build for the joins of a batch level: task k owns blocks [key_base,
  * key_base + key_blocks) of the passes over its rows and [fill_base, ...) of

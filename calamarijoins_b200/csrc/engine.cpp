@@ -552,6 +552,8 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         bool unique = false; /* a table of unique keys tried (the device decides) */
         bool multi = false;  /* the table of repeated dense keys */
         MultiTable multi_table{};
+        bool open_multi = false; /* multi: the keys are not dense */
+        OpenMultiTable open_table{};
         DevPtr multi_rows;
         const bool words_clear = join_words_clear;
         join_words_clear = false; /* every join counts its matches there */
@@ -647,7 +649,8 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                     const auto it = decoded.find({o.col.input, o.col.col});
                     const bool beside = /* the table and the column stay in L2 together */
                         !o.from_build || !multi || it == decoded.end() ||
-                        (multi_table.span * 2ull + B.rows) * 4 + it->second.src.num_pages * kPageSize <= kEmitBesideOpen;
+                        (open_multi ? open_table.nslots * 16ull : multi_table.span * 8ull) + B.rows * 4 +
+                                it->second.src.num_pages * kPageSize <= kEmitBesideOpen;
                     if (o.col.type != CJ_VARCHAR && it != decoded.end() && it->second.ready && uo.n < kEmitColumns &&
                         beside && room) {
                         const uint32_t R = rows_per_page_fixed(o.col.type);
@@ -678,6 +681,11 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                     key.col = view(P, pk, nullptr);
                 }
                 PhaseScope ph(*this, PH_PROBE);
+                if (multi && open_multi) {
+                    KScope k(*this, "probe_open_multi");
+                    ck(launch_probe_open_multi(L, key, (uint32_t)P.rows, open_table, uo), "probe_open_multi");
+                    return;
+                }
                 if (multi) {
                     KScope k(*this, "probe_multi");
                     ck(launch_probe_multi(L, key, (uint32_t)P.rows, multi_table, uo), "probe_multi");
@@ -707,13 +715,20 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         };
         uint64_t cap = P.rows;
         /* The device refused the table of unique keys (its probe did
-         * nothing). Keys that repeat over a dense range get the table of
-         * repeated keys: one random access per probe row and one per further
-         * match (64M x 4M rows over 3M keys: hash build, probe and page
-         * writers 235 + 1004 + 570 us, 130 + 956 + 344 here, the probe with
-         * one of the columns written beside it); 8 bytes per value of the
-         * range, at most kMultiSpan values per build row so that it stays
-         * near the hash table's 24 bytes per row. Else the hash table. */
+         * nothing). Keys that repeat get a table of repeated keys: one random
+         * access per probe row and one per further match.
+         * Over a dense range (64M x 4M rows over 3M keys): hash build, probe
+         * and page writers 235 + 1004 + 570 us, 130 + 956 + 344 here, the
+         * probe with one of the columns written beside it; 8 bytes per value
+         * of the range, at most kMultiSpan values per build row so that it
+         * stays near the hash table's 24 bytes per row.
+         * Over any other range, open addressing, 36 bytes per build row
+         * (30M x 3M rows over 2.25M keys, the whole join, hash table and
+         * this: INT32 keys 2094 and 1599 us, INT64 2312 and 1940; 100K x 5K
+         * INT64 345 and 248).
+         * The hash table is left for keys that span all of INT64 or pile up
+         * in the table, and for more build rows than fit kOpenMaxRows or the
+         * memory. */
         auto replace_unique = [&]() {
             unique = false;
             slots.reset();
@@ -722,7 +737,17 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 o.direct_only = false;
             }
             PhaseScope ph(*this, PH_BUILD);
-            const unsigned long long *tp = ctx.h_status->table;
+            unsigned long long tp[kTableWords];
+            std::copy(ctx.h_status->table, ctx.h_status->table + kTableWords, tp);
+            /* room for the keys' mean number of rows per match, up to 4; a
+             * result above it runs the probe again */
+            auto widen = [&](uint64_t keys) {
+                const uint64_t mean = P.rows * (uint64_t)tp[kTableCount] / std::max<uint64_t>(keys, 1);
+                const uint64_t more = std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(cap, mean), 4 * P.rows),
+                                                         0xFFFFFFFFull);
+                /* a match: two row ids and a key at most, here */
+                if (more > cap && room_for(more * 17)) cap = more;
+            };
             if ((!tp[kTableRefused] || tp[kTableRefused] == kTableRepeats) && tp[kTableSpan] <= kMultiSpan * B.rows) {
                 multi = true;
                 multi_table.lo = (int64_t)tp[kTableLo];
@@ -731,18 +756,40 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 multi_rows = ctx.alloc(B.rows * 4);
                 multi_table.entries = slots->as<unsigned long long>();
                 multi_table.rows = multi_rows->as<uint32_t>();
-                /* room for the keys' mean number of rows per match, up to 4;
-                 * a result above it runs the probe again */
-                const uint64_t mean = P.rows * (uint64_t)tp[kTableCount] / (uint64_t)tp[kTableSpan];
-                const uint64_t more = std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(cap, mean), 4 * P.rows),
-                                                         0xFFFFFFFFull);
-                /* a match: two row ids and a key at most, here */
-                if (more > cap && room_for(more * 17)) cap = more;
+                widen(tp[kTableSpan]);
                 KScope k(*this, "multi_build");
                 ck(launch_multi_build(L, bv, (uint32_t)B.rows, multi_table), "multi_build");
-            } else {
-                build_hash();
+                return;
             }
+            if (tp[kTableRefused] != kTableWhole && B.rows <= kOpenMaxRows &&
+                room_for(B.rows * (2 * sizeof(MultiSlot) + 8))) {
+                open_table.nslots = (uint32_t)std::max<uint64_t>(2 * B.rows, 1024);
+                open_table.lo = tp[kTableLo];
+                open_table.width = tp[kTableSpan] - 1;
+                open_table.empty = tp[kTableEmpty];
+                open_table.found = ctx.d_status->table;
+                slots = ctx.alloc(open_table.nslots * sizeof(MultiSlot));
+                multi_rows = ctx.alloc(B.rows * 4);
+                DevPtr slot_of = ctx.alloc(B.rows * 4);
+                open_table.slots = slots->as<MultiSlot>();
+                open_table.rows = multi_rows->as<uint32_t>();
+                open_table.slot_of = slot_of->as<uint32_t>();
+                clear_join_words();
+                {
+                    KScope k(*this, "open_multi_build");
+                    ck(launch_open_multi_build(L, bv, (uint32_t)B.rows, open_table), "open_multi_build");
+                }
+                sync(); /* the number of keys, before a probe that might run twice without it */
+                if (!ctx.h_status->table[kMultiGaveUp]) {
+                    multi = open_multi = true;
+                    widen(ctx.h_status->table[kMultiKeys]);
+                    return;
+                }
+                slots.reset();
+                multi_rows.reset();
+            }
+            clear_join_words(); /* the match counter, and words no longer read */
+            build_hash();
         };
         auto count_join = [&]() {
             const int kind = table_kind(ctx.h_status->table, table.open_slots);

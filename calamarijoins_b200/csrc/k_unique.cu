@@ -22,9 +22,10 @@
  * Columns with NULLs (known on the device only) get their row ids and are
  * written by k_write_pages.
  *
- * Keys that repeat over a dense range get a table of their own
- * (launch_multi_build: a count, and the row or where the key's rows lie, per
- * value) and the same probe with room for several matches a row.
+ * Keys that repeat get a table of their own (a count, and the row or where
+ * the key's rows lie: per value of a dense range, launch_multi_build, else in
+ * an open-addressing slot per key, launch_open_multi_build) and the same probe
+ * with room for several matches a row.
  *
  * Bound: requests from L1 to L2, about one per clock and SM whatever their
  * size (every random slot or value is one), then the 128-byte lines of L1
@@ -107,10 +108,8 @@ CJ_DEV void decide_table(unsigned long long *p, uint64_t max_span, bool wide) {
     const unsigned long long cnt = __ldcg(p + 2);
     if (cnt == 0) return; /* no non-NULL key: span 0, nothing matches */
     const unsigned long long b = ~__ldcg(p), e = __ldcg(p + 1), width = e - b; /* max - min: the bias cancels */
-    if (width >= max_span) {
-        p[kTableRefused] = wide && b == 0 && e == ~0ull ? kTableWhole : kTableSpread;
-        p[kTableEmpty] = (e != ~0ull ? e + 1 : b - 1) ^ (1ull << 63);
-    }
+    p[kTableEmpty] = (e != ~0ull ? e + 1 : b - 1) ^ (1ull << 63);
+    if (width >= max_span) p[kTableRefused] = wide && b == 0 && e == ~0ull ? kTableWhole : kTableSpread;
     else if (cnt > width + 1) p[kTableRefused] = kTableRepeats; /* more keys than values in their range */
     p[kTableLo] = b ^ (1ull << 63);
     p[kTableSpan] = width + 1;
@@ -138,6 +137,13 @@ CJ_DEV void fill_table(const UniqueTable &t, uint64_t first, uint64_t stride) {
     for (uint64_t i = first; i < n16; i += stride) reinterpret_cast<uint4 *>(t.slots)[i] = empty;
 }
 
+/* The keys repeat, or pile up. Written once, or nearly: thousands of stores
+ * to the one word that every thread also reads took 310 of the insert's 435
+ * us (3M rows, a quarter of the keys twice). */
+CJ_DEV void flag_once(unsigned long long *word) {
+    if (!*reinterpret_cast<volatile unsigned long long *>(word)) *reinterpret_cast<volatile unsigned long long *>(word) = 1ull;
+}
+
 /* Each key claims its slot; meeting its own key there means that the keys
  * repeat, and the table cannot be used. kUniqueRows rows per thread and
  * step, their compare-and-swaps all in flight together. */
@@ -162,7 +168,7 @@ CJ_DEV void insert_rows(const ColView &key, const UniqueTable &t, uint64_t first
             bool dup = false;
 #pragma unroll
             for (int q = 0; q < kUniqueRows; ++q) dup |= was[q] != kArrayEmpty;
-            if (dup) t.params[kTableDup] = 1ull;
+            if (dup) flag_once(t.params + kTableDup);
         }
         return;
     }
@@ -175,7 +181,7 @@ CJ_DEV void insert_rows(const ColView &key, const UniqueTable &t, uint64_t first
             int64_t k;
             if (!load_key(key, (uint32_t)i, &k)) continue;
             uint32_t h = open_slot_wide(k, t.open_slots);
-            for (uint32_t step = 0; step < t.open_slots; ++step) {
+            for (uint32_t step = 0;; ++step) {
                 unsigned long long cur = __ldcg(&slots[h].key);
                 if (cur == empty) {
                     cur = atomicCAS(&slots[h].key, empty, (unsigned long long)k);
@@ -184,8 +190,8 @@ CJ_DEV void insert_rows(const ColView &key, const UniqueTable &t, uint64_t first
                         break;
                     }
                 }
-                if (cur == (unsigned long long)k) {
-                    t.params[kTableDup] = 1ull;
+                if (cur == (unsigned long long)k || step == kMaxWalk) {
+                    flag_once(t.params + kTableDup);
                     break;
                 }
                 if (++h == t.open_slots) h = 0;
@@ -201,14 +207,14 @@ CJ_DEV void insert_rows(const ColView &key, const UniqueTable &t, uint64_t first
         if (!load_key(key, (uint32_t)i, &k)) continue;
         const unsigned long long v = ((unsigned long long)(uint32_t)k << 32) | (unsigned long long)i;
         uint32_t h = open_slot(k, t.open_slots);
-        for (uint32_t step = 0; step < t.open_slots; ++step) {
+        for (uint32_t step = 0;; ++step) {
             unsigned long long cur = __ldcg(slots + h); /* slots only fill: a full one is final */
             if (cur == kOpenEmpty) {
                 cur = atomicCAS(slots + h, kOpenEmpty, v);
                 if (cur == kOpenEmpty) break;
             }
-            if ((uint32_t)(cur >> 32) == (uint32_t)k) {
-                t.params[kTableDup] = 1ull;
+            if ((uint32_t)(cur >> 32) == (uint32_t)k || step == kMaxWalk) {
+                flag_once(t.params + kTableDup);
                 break;
             }
             if (++h == t.open_slots) h = 0;
@@ -372,12 +378,110 @@ __global__ void __launch_bounds__(kUniqueThreads) k_multi_scatter(ColView key_ar
     }
 }
 
+/* Build of the open-addressing one: claim a slot per key and count, place,
+ * scatter. The slot of each row is kept for the scatter (4 bytes a row, a
+ * walk less). Bound by the random accesses: two to the table per row in the
+ * claim (a read and the count's add), two in the scatter. */
+__global__ void __launch_bounds__(kUniqueThreads) k_open_multi_fill(OpenMultiTable t) {
+    const uint4 empty = make_uint4((uint32_t)t.empty, (uint32_t)(t.empty >> 32), 0u, 0u);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < t.nslots; i += stride)
+        reinterpret_cast<uint4 *>(t.slots)[i] = empty;
+}
+__global__ void __launch_bounds__(kUniqueThreads) k_open_multi_claim(ColView key_arg, uint32_t n, OpenMultiTable t) {
+    const ColView key = resolve_view(key_arg);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += stride * kUniqueRows) {
+        unsigned long long k[kUniqueRows], cur[kUniqueRows];
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) {
+            const uint64_t i = i0 + q * stride;
+            int64_t v;
+            k[q] = i < n && load_key(key, (uint32_t)i, &v) ? (unsigned long long)v : t.empty; /* no row's key */
+        }
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q)
+            cur[q] = k[q] != t.empty ? __ldcg(&t.slots[open_slot_wide((int64_t)k[q], t.nslots)].key) : t.empty;
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) {
+            uint32_t at = ~0u;
+            if (k[q] != t.empty) {
+                uint32_t h = open_slot_wide((int64_t)k[q], t.nslots);
+                unsigned long long c = cur[q];
+                for (uint32_t step = 0; step <= kMaxWalk; ++step) {
+                    if (c == t.empty) {
+                        c = atomicCAS(&t.slots[h].key, t.empty, k[q]);
+                        if (c == t.empty) c = k[q];
+                    }
+                    if (c == k[q]) {
+                        at = h;
+                        break;
+                    }
+                    if (++h == t.nslots) h = 0;
+                    c = __ldcg(&t.slots[h].key); /* slots only fill: a full one is final */
+                }
+                if (at != ~0u) atomicAdd(&t.slots[at].count, 1u);
+                else flag_once(t.found + kMultiGaveUp);
+            }
+            if (i0 + q * stride < n) t.slot_of[i0 + q * stride] = at;
+        }
+    }
+}
+__global__ void __launch_bounds__(kUniqueThreads) k_open_multi_place(OpenMultiTable t) {
+    __shared__ uint32_t wbuf[kUniqueThreads / 32 + 1];
+    __shared__ unsigned long long s_base;
+    uint32_t keys = 0;
+    for (uint64_t v0 = (uint64_t)blockIdx.x * kUniqueThreads * kPlaceItems; v0 < t.nslots;
+         v0 += (uint64_t)gridDim.x * kUniqueThreads * kPlaceItems) {
+        uint32_t c[kPlaceItems], sum = 0, total;
+#pragma unroll
+        for (int q = 0; q < kPlaceItems; ++q) {
+            const uint64_t v = v0 + q * kUniqueThreads + threadIdx.x;
+            c[q] = v < t.nslots ? t.slots[v].count : 0u;
+            keys += c[q] > 0;
+            if (c[q] > 1) sum += c[q];
+        }
+        const uint32_t pre = block_exclusive_scan<uint32_t>(sum, wbuf, &total);
+        if (threadIdx.x == 0) s_base = total ? atomicAdd(t.found + kMultiCursor, (unsigned long long)total) : 0ull;
+        __syncthreads();
+        uint32_t at = (uint32_t)s_base + pre;
+#pragma unroll
+        for (int q = 0; q < kPlaceItems; ++q) {
+            if (c[q] < 2) continue;
+            t.slots[v0 + q * kUniqueThreads + threadIdx.x].low = at;
+            at += c[q];
+        }
+        __syncthreads();
+    }
+    keys = __reduce_add_sync(0xffffffffu, keys);
+    if (lane_id() == 0 && keys) atomicAdd(t.found + kMultiKeys, (unsigned long long)keys);
+}
+__global__ void __launch_bounds__(kUniqueThreads) k_open_multi_scatter(uint32_t n, OpenMultiTable t) {
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += stride * kUniqueRows) {
+        uint32_t h[kUniqueRows], c[kUniqueRows], at[kUniqueRows];
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) h[q] = i0 + q * stride < n ? __ldcs(t.slot_of + i0 + q * stride) : ~0u;
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) c[q] = h[q] != ~0u ? t.slots[h[q]].count : 0u; /* no longer change */
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) {
+            if (c[q] == 1) t.slots[h[q]].low = (uint32_t)(i0 + q * stride);
+            else if (c[q]) at[q] = atomicAdd(&t.slots[h[q]].low, 1u);
+        }
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q)
+            if (c[q] > 1) t.rows[at[q]] = (uint32_t)(i0 + q * stride);
+    }
+}
+
 /* ---------------- probe ---------------- */
 /* 256 threads, 48 registers and 10 KB of shared memory: five CTAs per SM.
  * Measured at 64M x 4M rows (probe alone): five 605 us, four with 64
  * registers 619, six with 40 (spills) 620. */
 constexpr int kProbeBlocks = 5;
 constexpr int kWideBlocks = 4; /* 64 registers: the codes are 64-bit keys */
+constexpr int kOpenMultiBlocks = 3; /* 80 registers; four with 64: 1291 us where three take 1277 (INT64 keys, below) */
 constexpr int kMultiBlocks = 4; /* 64 registers; three with 80 1467 us, five with 48 2343 */
 constexpr int kItems = 8;                              /* rows per lane and step       */
 constexpr int kProbeThreads = 2048 / kItems;
@@ -759,14 +863,17 @@ CJ_DEV void probe_step(const LK &lk, const typename LK::Code *code, uint32_t ok,
     __syncwarp(); /* done with w before the next step packs */
 }
 
-/* The same over a table of repeated keys. The matches of rows with up to
+/* The same over a table of repeated keys, of either kind. The matches of rows with up to
  * three are packed and written together; those of rows with more in rounds,
  * the j-th matches of all of them; the rows of a key with more than kHeavyRun
  * build rows one after the other. 64M x 4M rows over 3M keys, 58.6M matches:
  * 956 us with one result column of two written beside it (bound by the
  * registers of its many paths: 64, some spilled; a separate function for the
  * rare ones cost more in the common one, 1141 us; every match of a row in
- * rounds 1458). */
+ * rounds 1458; warps without rows of more than three on a path of their own
+ * 1150). Open addressing, 30M x 3M rows, 31M matches: 955 us with INT32 keys,
+ * 1282 with INT64 ones (a 96 MB table); the hash probe takes 455 and 685, but
+ * runs twice, having no number of keys to size the result by. */
 constexpr uint32_t kHeavyRun = 32;
 constexpr uint32_t kMultiRoom = 320; /* matches packed at once: 256 rows and a quarter more */
 struct MultiMatches {
@@ -784,10 +891,65 @@ template <typename T> struct MultiLookup {
     const uint32_t *rows;
     using Code = uint32_t;
     static constexpr bool kMask = false;
+    static constexpr bool kStage = true; /* codes fit the packed matches: keys are written by full warps */
     CJ_DEV MultiLookup(const MultiTable &t)
         : d(nullptr, t.lo, t.span), entries(t.entries + (d.lo - t.lo)), rows(t.rows) {}
     CJ_DEV uint32_t code(T key, bool present, bool *in) const { return d.code(key, present, in); }
     CJ_DEV T key_of(uint32_t c) const { return d.key_of(c); }
+    CJ_DEV void find(const uint32_t *c, uint32_t, uint32_t *low, uint32_t *cnt) const {
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            unsigned long long e = 0;
+            if (c[it] < d.span) e = __ldg(entries + c[it]);
+            low[it] = (uint32_t)e;
+            cnt[it] = (uint32_t)(e >> 32);
+        }
+    }
+};
+
+/* Open addressing: a slot is one 16-byte load; its keys, which need not fit
+ * 32 bits, go to their places straight from the lanes. */
+template <typename T> struct OpenMultiLookup {
+    const MultiSlot *slots;
+    const uint32_t *rows;
+    uint32_t nslots;
+    unsigned long long lo, width, empty;
+    using Code = T;
+    static constexpr bool kMask = true;
+    static constexpr bool kStage = false;
+    CJ_DEV OpenMultiLookup(const OpenMultiTable &t)
+        : slots(t.slots), rows(t.rows), nslots(t.nslots), lo(t.lo), width(t.width), empty(t.empty) {}
+    CJ_DEV T code(T key, bool present, bool *in) const {
+        *in = present && (unsigned long long)(int64_t)key - lo <= width;
+        return key;
+    }
+    CJ_DEV T key_of(T c) const { return c; }
+    CJ_DEV ulonglong2 slot(uint32_t h) const { return __ldg(reinterpret_cast<const ulonglong2 *>(slots + h)); }
+    CJ_DEV void find(const T *c, uint32_t ok, uint32_t *low, uint32_t *cnt) const {
+#pragma unroll
+        for (int it = 0; it < kItems; it += 4) { /* four rows' slots in flight: 16 registers */
+            ulonglong2 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                v[j].x = empty;
+                if ((ok >> (it + j)) & 1u) v[j] = slot(open_slot_wide((int64_t)c[it + j], nslots));
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                low[it + j] = cnt[it + j] = 0;
+                uint32_t h = open_slot_wide((int64_t)c[it + j], nslots);
+                for (uint32_t step = 0; v[j].x != empty && step < nslots; ++step) {
+                    if (v[j].x == (unsigned long long)(int64_t)c[it + j]) {
+                        low[it + j] = (uint32_t)v[j].y;
+                        cnt[it + j] = (uint32_t)(v[j].y >> 32);
+                        break;
+                    }
+                    if (++h == nslots) h = 0;
+                    v[j] = slot(h);
+                }
+            }
+        }
+    }
 };
 
 /* The lanes' items of one packing: item `it`'s matches go to places first(it)
@@ -805,27 +967,21 @@ template <class C, class F> CJ_DEV uint32_t pack_few(C count, F put) {
     }
     return n;
 }
-template <typename T>
-CJ_DEV void emit_keys(const MultiLookup<T> &lk, const UniqueOut &out, const MultiMatches &w, uint32_t n, uint32_t at) {
+template <typename T, class LK>
+CJ_DEV void emit_keys(const LK &lk, const UniqueOut &out, const MultiMatches &w, uint32_t n, uint32_t at) {
     __syncwarp();
     const PageRun<T> keys(out.match.key_pages, at);
     for (uint32_t i = lane_id(); i < n; i += 32) __stcs(keys.at(i), lk.key_of(w.rid[i]));
     __syncwarp();
 }
 
-template <typename T>
-CJ_DEV void probe_step(const MultiLookup<T> &lk, const uint32_t *code, uint32_t, uint32_t row0, const UniqueOut &out,
+template <typename T, class LK>
+CJ_DEV void probe_step(const LK &lk, const typename LK::Code *code, uint32_t ok, uint32_t row0, const UniqueOut &out,
                        const EmitPlan &plan, MultiShared &sh, uint32_t part, uint32_t buf) {
     const uint32_t lane = lane_id(), lt = lanemask_lt();
     MultiMatches &w = sh.matches[part];
     uint32_t low[kItems], cnt[kItems];
-#pragma unroll
-    for (int it = 0; it < kItems; ++it) {
-        unsigned long long e = 0;
-        if (code[it] < lk.d.span) e = __ldg(lk.entries + code[it]);
-        low[it] = (uint32_t)e;
-        cnt[it] = (uint32_t)(e >> 32);
-    }
+    lk.find(code, ok, low, cnt);
     unsigned long long many = 0; /* matches of rows with more than three */
 #pragma unroll
     for (int it = 0; it < kItems; ++it)
@@ -836,7 +992,7 @@ CJ_DEV void probe_step(const MultiLookup<T> &lk, const uint32_t *code, uint32_t,
 #pragma unroll
         for (uint32_t j = 0; j < 3; ++j)
             if (j < c) {
-                w.rid[i + j] = code[it];
+                if constexpr (LK::kStage) w.rid[i + j] = code[it];
                 w.row[i + j] = (uint8_t)(it * 32 + lane);
             }
     });
@@ -859,8 +1015,15 @@ CJ_DEV void probe_step(const MultiLookup<T> &lk, const uint32_t *code, uint32_t,
     if (base + total > out.match.capacity) return;
     uint32_t at = (uint32_t)base;
     if (packed && few) {
-        if (out.match.key_pages) emit_keys(lk, out, w, few, at);
+        if constexpr (LK::kStage) {
+            if (out.match.key_pages) emit_keys<T>(lk, out, w, few, at);
+        }
+        const PageRun<T> keys(out.match.key_pages, at);
         pack_few(few_of, [&](int it, uint32_t i, uint32_t c) {
+            if constexpr (!LK::kStage) {
+                if (out.match.key_pages)
+                    for (uint32_t j = 0; j < c; ++j) __stcs(keys.at(i + j), lk.key_of(code[it]));
+            }
             if (c == 1) {
                 w.rid[i] = low[it];
             } else {
@@ -882,12 +1045,18 @@ CJ_DEV void probe_step(const MultiLookup<T> &lk, const uint32_t *code, uint32_t,
             return cnt[it] > j && cnt[it] <= kHeavyRun && (!packed || cnt[it] > 3) ? 1u : 0u;
         };
         const uint32_t n = pack_few(hit_of, [&](int it, uint32_t i, uint32_t) {
-            w.rid[i] = code[it];
+            if constexpr (LK::kStage) w.rid[i] = code[it];
             w.row[i] = (uint8_t)(it * 32 + lane);
         });
         if (!n) break;
-        if (out.match.key_pages) emit_keys(lk, out, w, n, at);
+        if constexpr (LK::kStage) {
+            if (out.match.key_pages) emit_keys<T>(lk, out, w, n, at);
+        }
+        const PageRun<T> keys(out.match.key_pages, at);
         pack_few(hit_of, [&](int it, uint32_t i, uint32_t) {
+            if constexpr (!LK::kStage) {
+                if (out.match.key_pages) __stcs(keys.at(i), lk.key_of(code[it]));
+            }
             w.rid[i] = cnt[it] == 1 ? low[it] : __ldg(lk.rows + (low[it] - cnt[it] + j));
         });
         __syncwarp();
@@ -896,7 +1065,8 @@ CJ_DEV void probe_step(const MultiLookup<T> &lk, const uint32_t *code, uint32_t,
         at += n;
     }
     for (int it = 0; it < kItems; ++it) {
-        uint32_t c = 0, lo = 0, cd = 0; /* item `it`, without indexing registers */
+        uint32_t c = 0, lo = 0; /* item `it`, without indexing registers */
+        typename LK::Code cd = 0;
 #pragma unroll
         for (int q = 0; q < kItems; ++q)
             if (q == it) {
@@ -909,7 +1079,8 @@ CJ_DEV void probe_step(const MultiLookup<T> &lk, const uint32_t *code, uint32_t,
             const int src = __ffs(heavy) - 1;
             heavy &= heavy - 1;
             const uint32_t rows_n = __shfl_sync(0xffffffffu, c, src);
-            const uint32_t first = __shfl_sync(0xffffffffu, lo, src) - rows_n, kc = __shfl_sync(0xffffffffu, cd, src);
+            const uint32_t first = __shfl_sync(0xffffffffu, lo, src) - rows_n;
+            const typename LK::Code kc = __shfl_sync(0xffffffffu, cd, src);
             for (uint32_t k0 = 0; k0 < rows_n; k0 += kWarpRows) {
                 const uint32_t n = min(kWarpRows, rows_n - k0);
                 for (uint32_t i = lane; i < n; i += 32) {
@@ -1088,6 +1259,14 @@ __global__ void __launch_bounds__(kProbeThreads, kMultiBlocks)
     probe_all<kPages, T>(k, n, MultiLookup<T>(t), out, sh);
 }
 
+template <bool kPages, typename T>
+__global__ void __launch_bounds__(kProbeThreads, kOpenMultiBlocks)
+    k_probe_open_multi(const __grid_constant__ ProbeKey k, uint32_t n, const __grid_constant__ OpenMultiTable t,
+                       const __grid_constant__ UniqueOut out) {
+    __shared__ MultiShared sh;
+    probe_all<kPages, T>(k, n, OpenMultiLookup<T>(t), out, sh);
+}
+
 /* Steps of a probe's CTAs. */
 uint64_t probe_tiles(const ProbeKey &k, uint32_t n) {
     if (!k.base) return ((uint64_t)n + kTileRows - 1) / kTileRows;
@@ -1099,7 +1278,7 @@ uint64_t probe_tiles(const ProbeKey &k, uint32_t n) {
  * device. */
 template <class K> void prefer_l1(K kernel) {
     constexpr int kDevices = 64;
-    static std::atomic<const void *> done[kDevices][12];
+    static std::atomic<const void *> done[kDevices][16];
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kDevices) {
         cudaGetLastError();
@@ -1203,6 +1382,35 @@ cudaError_t launch_probe_multi(const Launch &L, const ProbeKey &k, uint32_t n, c
     const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * kMultiBlocks));
     const auto kernel = k.col.type == CJ_INT32 ? (pages ? k_probe_multi<true, int32_t> : k_probe_multi<false, int32_t>)
                                                : (pages ? k_probe_multi<true, long long> : k_probe_multi<false, long long>);
+    prefer_l1(kernel);
+    kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_open_multi_build(const Launch &L, const ColView &key, uint32_t n, const OpenMultiTable &t) {
+    if (!n || t.nslots < 2ull * n || reinterpret_cast<uintptr_t>(t.slots) % 16) return cudaErrorInvalidValue;
+    const uint64_t wave = (uint64_t)L.num_sms * 8;
+    const uint64_t rows_per_block = kUniqueThreads * kUniqueRows, slots_per_block = kUniqueThreads * kPlaceItems;
+    const unsigned g = (unsigned)std::min<uint64_t>((n + rows_per_block - 1) / rows_per_block, wave);
+    const unsigned gs = (unsigned)std::min<uint64_t>((t.nslots + slots_per_block - 1) / slots_per_block, wave);
+    k_open_multi_fill<<<gs, kUniqueThreads, 0, L.stream>>>(t);
+    k_open_multi_claim<<<g, kUniqueThreads, 0, L.stream>>>(key, n, t);
+    k_open_multi_place<<<gs, kUniqueThreads, 0, L.stream>>>(t);
+    k_open_multi_scatter<<<g, kUniqueThreads, 0, L.stream>>>(n, t);
+    count_launches(4);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_probe_open_multi(const Launch &L, const ProbeKey &k, uint32_t n, const OpenMultiTable &t,
+                                    const UniqueOut &out) {
+    if (n == 0) return cudaSuccess;
+    const bool pages = k.base != nullptr;
+    const uint64_t tiles = probe_tiles(k, n);
+    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * kOpenMultiBlocks));
+    const auto kernel = k.col.type == CJ_INT32
+                            ? (pages ? k_probe_open_multi<true, int32_t> : k_probe_open_multi<false, int32_t>)
+                            : (pages ? k_probe_open_multi<true, long long> : k_probe_open_multi<false, long long>);
     prefer_l1(kernel);
     kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out);
     count_launches(1);
