@@ -307,20 +307,75 @@ __global__ void __launch_bounds__(kFilterThreads) k_compare(CmpArgs a) {
             } else if (c.type == CJ_FP64) {
                 double v;
                 bit = fixed_value<double>(c, r, &v) && cmp_num<double>(a.op, v, a.f64);
-            } else if (valid_bit(c.valid, r)) { /* VARCHAR */
-                const uint64_t d = __ldg(c.str_desc + r);
-                if (desc_is_long(d)) {
-                    StrView s;
-                    s.init(c.pages, d);
-                    bit = cmp_str(s, a);
-                } else {
-                    ShortStr s(c.pages, d);
-                    bit = cmp_str(s, a);
-                }
             }
         }
         const uint32_t w = __ballot_sync(0xffffffffu, bit);
         if (lane_id() == 0 && base + threadIdx.x < a.rows) a.out[(base + threadIdx.x) >> 5] = w;
+    }
+}
+
+/* A VARCHAR column compared with the literal, for the rows whose bit of `mask`
+ * is set (null: all); the bits of other rows are 0. A block takes 2,048 rows
+ * at a time, packs those that are non-NULL and in the mask, and its threads
+ * compare them side by side: a comparison costs tens of instructions a
+ * character step for the whole warp however few of its rows are still in
+ * question. 10M strings of 20 characters against '%qz%' beside two conditions
+ * that leave a quarter of the rows: the filter 1006 us, 715 so. */
+constexpr uint32_t kTextWords = 64;
+__global__ void __launch_bounds__(kFilterThreads) k_compare_text(CmpArgs a, const uint32_t *__restrict__ mask) {
+    static_assert(kFilterThreads == kTextWords * 4, "a thread lists a byte of the words");
+    __shared__ uint32_t s_live[kTextWords], s_pre[kTextWords], s_out[kTextWords];
+    __shared__ uint16_t s_row[kTextWords * 32];
+    __shared__ uint32_t s_total;
+    const ColView c = resolve_view(a.col);
+    const uint64_t words = (a.rows + 31) / 32;
+    for (uint64_t w0 = (uint64_t)blockIdx.x * kTextWords; w0 < words; w0 += (uint64_t)gridDim.x * kTextWords) {
+        if (threadIdx.x < 32) {
+            uint32_t v[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const uint64_t w = w0 + 2 * threadIdx.x + j;
+                v[j] = 0;
+                if (w >= words) continue;
+                v[j] = __ldg(c.valid + w); /* no bits past the last row */
+                if (mask) v[j] &= __ldg(mask + w);
+            }
+            const uint32_t n0 = __popc(v[0]), n = n0 + __popc(v[1]);
+            const uint32_t incl = warp_inclusive_scan(n);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                s_live[2 * threadIdx.x + j] = v[j];
+                s_pre[2 * threadIdx.x + j] = incl - n + (j ? n0 : 0u);
+                s_out[2 * threadIdx.x + j] = 0;
+            }
+            if (threadIdx.x == 31) s_total = incl;
+        }
+        __syncthreads();
+        {
+            const uint32_t w = threadIdx.x >> 2, b0 = (threadIdx.x & 3u) * 8, live = s_live[w];
+            uint32_t at = s_pre[w] + __popc(live & ((1u << b0) - 1u));
+            for (uint32_t bits = (live >> b0) & 0xFFu; bits; bits &= bits - 1)
+                s_row[at++] = (uint16_t)(w * 32 + b0 + __ffs(bits) - 1);
+        }
+        __syncthreads();
+        const uint32_t total = s_total;
+        for (uint32_t k = threadIdx.x; k < total; k += kFilterThreads) {
+            const uint32_t q = s_row[k];
+            const uint64_t d = __ldg(c.str_desc + w0 * 32 + q);
+            bool bit;
+            if (desc_is_long(d)) {
+                StrView s;
+                s.init(c.pages, d);
+                bit = cmp_str(s, a);
+            } else {
+                ShortStr s(c.pages, d);
+                bit = cmp_str(s, a);
+            }
+            if (bit) atomicOr(&s_out[q >> 5], 1u << (q & 31u));
+        }
+        __syncthreads();
+        if (threadIdx.x < kTextWords && w0 + threadIdx.x < words) a.out[w0 + threadIdx.x] = s_out[threadIdx.x];
+        __syncthreads();
     }
 }
 
@@ -375,7 +430,7 @@ class Filter {
         uint64_t count = rows;
         if (pred && rows) {
             decode(pred_columns());
-            DevPtr bits = eval(pred->root, words, 0);
+            DevPtr bits = eval(pred->root, words, 0, nullptr);
             DevPtr cnt = ctx.alloc(words * 4), off = ctx.alloc((words + 1) * 8);
             DevPtr tmp = ctx.alloc(scan_temp_bytes(words));
             k_word_popc<<<grid_for(ctx, words, 256), 256, 0, ctx.stream>>>(bits->as<uint32_t>(), words,
@@ -449,6 +504,7 @@ class Filter {
     Launch L;
     std::map<uint64_t, Decoded> decoded;
     std::vector<DevPtr> keep;
+    std::vector<int8_t> text_of; /* has_text, by node; -1 not known yet */
 
     void validate(uint64_t ncols, const uint64_t *cols) {
         if (ncols && !cols) fail(CJ_ERR_INVALID_ARGUMENT, "null column list");
@@ -537,7 +593,26 @@ class Filter {
         return make_view(d, R, rc, nullptr);
     }
 
-    DevPtr eval(uint64_t node, uint64_t words, int depth) {
+    /* Whether a node's subtree compares text (worked out once a node). */
+    bool has_text(uint64_t node, int depth) {
+        if (depth > (int)pred->num_nodes) fail(CJ_ERR_INVALID_PLAN, "predicate has a cycle");
+        text_of.resize(pred->num_nodes, -1);
+        if (text_of[node] < 0) {
+            const cj_pred_node &n = pred->nodes[node];
+            bool t;
+            if (n.kind == CJ_PRED_CMP)
+                t = in.cols[n.column].type == CJ_VARCHAR && n.op != CJ_CMP_IS_NULL && n.op != CJ_CMP_IS_NOT_NULL;
+            else t = has_text(n.left, depth + 1) || (n.kind != CJ_PRED_NOT && has_text(n.right, depth + 1));
+            text_of[node] = t;
+        }
+        return text_of[node];
+    }
+
+    /* The node's bit for the rows whose bit of `mask` is set (null: all); the
+     * other rows' bits are anything. Text is compared last: of the children
+     * of an AND the one without text comes first, and the second is asked for
+     * the rows that the first lets through only. */
+    DevPtr eval(uint64_t node, uint64_t words, int depth, const uint32_t *mask) {
         if (depth > (int)pred->num_nodes) fail(CJ_ERR_INVALID_PLAN, "predicate has a cycle");
         const cj_pred_node &n = pred->nodes[node];
         DevPtr out = ctx.alloc(words * 4);
@@ -549,7 +624,8 @@ class Filter {
             a.i64 = n.i64;
             a.f64 = n.literal_type == CJ_INT64 ? (double)n.i64 : n.f64;
             a.out = out->as<uint32_t>();
-            if (in.cols[n.column].type == CJ_VARCHAR && n.op != CJ_CMP_IS_NULL && n.op != CJ_CMP_IS_NOT_NULL) {
+            const bool text = has_text(node, depth);
+            if (text) {
                 DevPtr lit = ctx.alloc(std::max<uint64_t>(n.str_len, 1));
                 if (n.str_len)
                     check_cuda(cudaMemcpyAsync(lit->ptr, n.str, n.str_len, cudaMemcpyHostToDevice, ctx.stream),
@@ -558,13 +634,17 @@ class Filter {
                 a.lit_len = (uint32_t)n.str_len;
                 keep.push_back(lit);
             }
-            const unsigned grid = grid_for(ctx, in.num_rows, kFilterThreads);
-            k_compare<<<grid, kFilterThreads, 0, ctx.stream>>>(a);
+            const unsigned grid = grid_for(ctx, in.num_rows, text ? kTextWords * 32 : kFilterThreads);
+            if (text) k_compare_text<<<grid, kFilterThreads, 0, ctx.stream>>>(a, mask);
+            else k_compare<<<grid, kFilterThreads, 0, ctx.stream>>>(a);
             count_launches(1);
             check_cuda(cudaGetLastError(), "compare");
         } else {
-            DevPtr l = eval(n.left, words, depth + 1);
-            DevPtr r = n.kind == CJ_PRED_NOT ? nullptr : eval(n.right, words, depth + 1);
+            const bool swap = n.kind == CJ_PRED_AND && has_text(n.left, depth + 1) && !has_text(n.right, depth + 1);
+            DevPtr l = eval(swap ? n.right : n.left, words, depth + 1, mask);
+            DevPtr r;
+            if (n.kind != CJ_PRED_NOT)
+                r = eval(swap ? n.left : n.right, words, depth + 1, n.kind == CJ_PRED_AND ? l->as<uint32_t>() : mask);
             k_bitmap_logic<<<grid_for(ctx, words, 256), 256, 0, ctx.stream>>>(
                 l->as<uint32_t>(), r ? r->as<uint32_t>() : nullptr, out->as<uint32_t>(), words, in.num_rows, n.kind);
             count_launches(1);

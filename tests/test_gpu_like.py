@@ -5,7 +5,7 @@ string's end."""
 import numpy as np
 import pytest
 
-from calamarijoins_b200 import ColumnarTable, Comparison, DataType, encode_column
+from calamarijoins_b200 import ColumnarTable, Comparison, DataType, LogicalOperation, encode_column
 from oracle import oracle_api as oa
 from tests.helpers import assert_same
 from tests.test_gpu_filter import gpu_filter
@@ -32,3 +32,23 @@ def test_like_skips(gpu_ctx, pattern):
         got = gpu_filter(gpu_ctx, t, pred, [0])
         assert got.num_rows == int(sel.sum()), pattern
         assert_same(got, want, pattern)
+
+
+@pytest.mark.parametrize("rows", [1, 31, 33, 2047, 2048, 2049, 5000])
+@pytest.mark.parametrize("keep", [0, 1, 50, 100])
+def test_text_beside_other_conditions(gpu_ctx, rows, keep):
+    """Text is compared for the rows that the other side of an AND leaves,
+    around the 2,048 rows of a block: any order and nesting, under NOT and OR."""
+    rng = np.random.default_rng(rows + keep)
+    texts = [None if rng.random() < 0.1 else "ab"[int(rng.integers(2))] * int(rng.integers(0, 9)) for _ in range(rows)]
+    texts = [t if t is None else (t * (2000 if rng.random() < 0.002 else 1)).encode() for t in texts]
+    t = ColumnarTable(rows, [encode_column(DataType.INT32, rng.integers(0, 100, rows).astype(np.int32)),
+                             encode_column(DataType.VARCHAR, texts)])
+    A, O, N = LogicalOperation.makeAnd, LogicalOperation.makeOr, LogicalOperation.makeNot
+    num, like, eq = Comparison(0, Comparison.LT, keep), Comparison(1, Comparison.LIKE, "%bb%"), Comparison(1, Comparison.GEQ, "ab")
+    for pred in (A(num, like), A(like, num), A(A(eq, num), N(like)), N(A(num, N(like))), O(A(num, like), eq),
+                 A(O(like, num), N(O(eq, like))), A(num, A(Comparison(1, Comparison.IS_NOT_NULL), N(N(like))))):
+        want, sel = oa.oracle_filter(t, pred, [0, 1])
+        got = gpu_filter(gpu_ctx, t, pred, [0, 1])
+        assert got.num_rows == int(sel.sum())
+        assert_same(got, want)
