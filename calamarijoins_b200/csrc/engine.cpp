@@ -30,6 +30,15 @@ namespace {
 
 constexpr uint64_t kMultiSpan = 4; /* values of the range per build row */
 
+/* Probe rows per build row from which repeated keys that are not dense get
+ * their open-addressing table. Its probe is the cheaper one per row, its build
+ * dearer than the hash table's and followed by a synchronisation: 3M x 6M
+ * INT64 rows 506 us and 470 on the hash table (sums of the kernels), 3M x 30M
+ * 1953 and 2280 (the whole join);
+ * a five-join star whose last build side is an intermediate of 86K rows
+ * against 105K probe rows 828 us and 766. */
+constexpr uint64_t kOpenMultiProbe = 4;
+
 /* A probe of an open-addressing table reads a build column's values beside
  * it while both stay in L2 (126 MB on two dies, each keeping its own copy of
  * what it reads); a larger pair is read one after the other, through the
@@ -726,9 +735,9 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
          * (30M x 3M rows over 2.25M keys, the whole join, hash table and
          * this: INT32 keys 2094 and 1599 us, INT64 2312 and 1940; 100K x 5K
          * INT64 345 and 248).
-         * The hash table is left for keys that span all of INT64 or pile up
-         * in the table, and for more build rows than fit kOpenMaxRows or the
-         * memory. */
+         * The hash table is left for fewer probe rows than kOpenMultiProbe
+         * per build row, for keys that span all of INT64 or pile up in the
+         * table, and for more build rows than fit kOpenMaxRows or the memory. */
         auto replace_unique = [&]() {
             unique = false;
             slots.reset();
@@ -761,7 +770,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 ck(launch_multi_build(L, bv, (uint32_t)B.rows, multi_table), "multi_build");
                 return;
             }
-            if (tp[kTableRefused] != kTableWhole && B.rows <= kOpenMaxRows &&
+            if (tp[kTableRefused] != kTableWhole && B.rows <= kOpenMaxRows && P.rows / kOpenMultiProbe >= B.rows &&
                 room_for(B.rows * (2 * sizeof(MultiSlot) + 8))) {
                 open_table.nslots = (uint32_t)std::max<uint64_t>(2 * B.rows, 1024);
                 open_table.lo = tp[kTableLo];

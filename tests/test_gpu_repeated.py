@@ -30,7 +30,7 @@ def test_rows_per_key(gpu_ctx, bt, pt, per_key):
     k = _keys(rng, 3000 if per_key < 10 else 400, bt)
     bkeys = np.concatenate([np.repeat(k[:len(k) // 5], per_key), k[len(k) // 5:], k[:2]])
     rng.shuffle(bkeys)
-    n = len(bkeys) + 2500
+    n = 4 * len(bkeys) + 2500  # a quarter of that, and the hash table serves it
     src = k if (bt, pt) != (L, I) else np.concatenate([k, rng.integers(-(2 ** 31) + 1, 2 ** 31, 50)])
     if (bt, pt) == (L, I):
         bkeys[:200] = rng.integers(-50, 50, 200)  # some that INT32 probe keys meet
@@ -47,7 +47,7 @@ def test_rows_per_key(gpu_ctx, bt, pt, per_key):
 @pytest.mark.parametrize("cols", ["nulls", "text"])
 def test_result_columns(gpu_ctx, cols):
     rng = np.random.default_rng(6)
-    nb, n = 9000, 30_000
+    nb, n = 9000, 36_001
     bkeys = (rng.permutation(nb) // 2) * 777_777
     pkeys = bkeys[rng.integers(0, nb, n)] + (rng.random(n) < 0.3)
     ok = lambda rows: (rng.random(rows) >= 0.2).astype(np.uint8)
@@ -72,7 +72,7 @@ def test_keys_that_go_on(gpu_ctx, case):
         if case == "piled_up_repeats":
             bkeys = np.concatenate([bkeys, bkeys[:50]])
     rng.shuffle(bkeys)
-    pkeys = np.concatenate([bkeys[rng.integers(0, len(bkeys), 4000)], bkeys + 1 if case != "whole" else bkeys])
+    pkeys = np.concatenate([bkeys[rng.integers(0, len(bkeys), 13_000)], bkeys + 1 if case != "whole" else bkeys])
     _check(_plan(bkeys, pkeys, L, L, bpay=[(I, rng.integers(0, 99, len(bkeys)), None)]), gpu_ctx, "hash")
 
 
@@ -83,7 +83,7 @@ def test_large_and_rerun(gpu_ctx):
     k = np.unique(rng.integers(-(2 ** 62), 2 ** 62, 150_000))
     bkeys = np.concatenate([k, k[:60_000], np.repeat(k[:3], 40)])
     rng.shuffle(bkeys)
-    pkeys = np.concatenate([k[rng.integers(0, len(k), 200_000)], np.repeat(k[0], 40_000), np.repeat(k[1], 3000)])
+    pkeys = np.concatenate([k[rng.integers(0, len(k), 850_000)], np.repeat(k[0], 60_000), np.repeat(k[1], 3000)])
     rng.shuffle(pkeys)
     plan = _plan(bkeys, pkeys, L, L, bpay=[(L, np.arange(len(bkeys)), None)], ppay=[(I, np.arange(len(pkeys)), None)])
     want = run_oracle(plan)
