@@ -365,6 +365,7 @@ Context *create_context(int device, cudaMemPool_t shared_pool, std::shared_ptr<P
     c->opt.buffer_cache_bytes = std::max<int64_t>(0, env_opt("CJ_BUFFER_CACHE_BYTES", c->opt.buffer_cache_bytes));
     c->opt.inline_dir_max_bytes = std::max<int64_t>(0, env_opt("CJ_INLINE_DIR_MAX_BYTES", c->opt.inline_dir_max_bytes));
     c->opt.defer_count = env_opt("CJ_DEFER_COUNT", c->opt.defer_count);
+    c->opt.spare_room = env_opt("CJ_SPARE_ROOM_BYTES", c->opt.spare_room);
     if (shared_pool) c->opt.buffer_cache_bytes = 0; /* contexts sharing a pool share through it */
     if (const char *tf = std::getenv("CJ_TUNING_FILE"); tf && *tf) c->tuning = load_tuning_file(tf, c->num_sms);
     return c.release();

@@ -173,9 +173,11 @@ class Executor {
     }
 
     /* Whether `bytes` may be set aside for matches that may not come: above
-     * kAmpleRoom, half of what is left. A selective join whose matches would
-     * fit does not fail for room it would not have used. */
+     * kAmpleRoom, half of what is left (or the context's own bound). A
+     * selective join whose matches would fit does not fail for room it would
+     * not have used. */
     bool room_for(uint64_t bytes) {
+        if (ctx.opt.spare_room >= 0) return bytes <= (uint64_t)ctx.opt.spare_room;
         if (bytes <= kAmpleRoom) return true;
         size_t left = 0, total = 0;
         uint64_t used = 0, reserved = 0;
@@ -627,9 +629,18 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             }
             if (!unique) build_hash();
         }
+        /* Result pages of an earlier probe: a table that was refused, or a
+         * capacity that the matches outgrew. */
+        auto drop_pages = [&]() {
+            for (auto &o : outs) {
+                o.pages.reset();
+                o.direct_only = false;
+            }
+        };
         /* Allocates the match outputs for `cap` pairs and launches the probe
          * of the table built above. */
         auto launch_probe = [&](uint64_t cap) {
+            drop_pages();
             /* the key columns' result pages, sized for the capacity */
             const uint32_t key_rpp = rows_per_page_fixed(pk.type);
             mk = emit_keys ? ctx.alloc((cap + key_rpp - 1) / key_rpp * kPageSize) : nullptr;
@@ -741,10 +752,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         auto replace_unique = [&]() {
             unique = false;
             slots.reset();
-            for (auto &o : outs) {
-                o.pages.reset();
-                o.direct_only = false;
-            }
+            drop_pages();
             PhaseScope ph(*this, PH_BUILD);
             unsigned long long tp[kTableWords];
             std::copy(ctx.h_status->table, ctx.h_status->table + kTableWords, tp);
@@ -1025,6 +1033,8 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
             if (cols[c].pages) {
                 /* values already in place: headers and bitmaps, once per
                  * shared page array */
+                if (cols[c].pages->bytes < res->num_pages[c] * kPageSize)
+                    fail(CJ_ERR_INTERNAL, "result pages smaller than the result");
                 res->dev_pages[c] = cols[c].pages;
                 if (cols[c].rel) t.col = out_view(cols[c]);
                 else t.col.type = types[c];

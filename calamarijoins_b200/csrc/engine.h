@@ -57,6 +57,10 @@ struct Options {
      * result with the match count read on the device, without a host
      * synchronisation after the probe (environment CJ_DEFER_COUNT=0: off) */
     int64_t defer_count = 1;
+    /* most bytes that a plan sets aside for matches that may not come;
+     * negative: 4 GiB, and above that half of the memory that is left
+     * (environment CJ_SPARE_ROOM_BYTES) */
+    int64_t spare_room = -1;
 };
 
 struct Context;

@@ -1,0 +1,61 @@
+"""GPU: memory that a plan sets aside for matches that may not come, bounded
+by CJ_SPARE_ROOM_BYTES, against the oracle: joins whose result columns the
+probe may not write, or may write in its first run and not in the second."""
+import numpy as np
+import pytest
+
+from calamarijoins_b200 import Context, DataType, Plan, ResidentTable, _lib
+from tests.helpers import assert_same, run_oracle, run_product
+from tests.test_gpu_unique import _plan
+
+pytestmark = pytest.mark.gpu
+I, L, F, V = DataType.INT32, DataType.INT64, DataType.FP64, DataType.VARCHAR
+
+
+@pytest.fixture
+def bounded(monkeypatch):
+    """Contexts with a bound of their own on the room."""
+    made = []
+
+    def make(room):
+        monkeypatch.setenv("CJ_SPARE_ROOM_BYTES", str(room))
+        made.append(Context(0))
+        return made[-1]
+
+    yield make
+    for c in made:
+        c.close()
+
+
+def _resident(plan, ctx):
+    rp = Plan()
+    rp.nodes, rp.root = plan.nodes, plan.root
+    rp.inputs = [ResidentTable(ctx, t) for t in plan.inputs]
+    return rp
+
+
+@pytest.mark.parametrize("flags", [0, _lib.CJ_EXEC_RESULT_ON_DEVICE])
+@pytest.mark.parametrize("gap", [1, 5000])
+@pytest.mark.parametrize("room", [0, 600_000, 1_450_000, 1 << 30])
+def test_room_refused(bounded, room, gap, flags):
+    """Three build rows per key and 60,000 matches for 20,000 probe rows (and
+    4,500 that match nothing): the payload columns' pages take 23 bytes a row,
+    460 (564) KB for the probe rows and 1,380 KB for the matches, so that the
+    bound refuses every run, the second one only (600,000), the pages of a
+    first run with room for all (1,450,000) or nothing."""
+    rng = np.random.default_rng(2)
+    bkeys = rng.permutation(np.repeat(np.arange(2000) * gap, 3))
+    n = 20_000 if gap == 1 else 24_500
+    pkeys = np.concatenate([rng.integers(0, 2000, 20_000) * gap, np.full(n - 20_000, -7)])
+    valid = (rng.random(len(bkeys)) >= 0.1).astype(np.uint8)
+    plan = _plan(bkeys, rng.permutation(pkeys), bpay=[(L, np.arange(6000), None), (I, np.arange(6000), valid)],
+                 ppay=[(F, rng.random(n), None)])
+    ctx = bounded(room)
+    rp = _resident(plan, ctx)
+    got, st = run_product(rp, ctx, flags)
+    assert_same(got, run_oracle(plan), f"room {room}")
+    assert got.num_rows == 60_000
+    if room == 0:
+        assert st.exec["probe_reruns"] == 1
+    for t in rp.inputs:
+        t.free()
