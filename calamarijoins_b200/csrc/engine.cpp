@@ -637,6 +637,14 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 o.direct_only = false;
             }
         };
+        /* At most: the result pages that a probe with room for `cap` matches
+         * writes, the keys' apart. */
+        auto beside_bytes = [&](uint64_t cap) {
+            uint64_t bytes = 0;
+            for (const auto &o : outs)
+                if (is_root && !o.from_keys && o.col.type != CJ_VARCHAR) bytes += cap * (o.col.type == CJ_INT32 ? 5 : 9);
+            return bytes;
+        };
         /* Allocates the match outputs for `cap` pairs and launches the probe
          * of the table built above. */
         auto launch_probe = [&](uint64_t cap) {
@@ -659,11 +667,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                  * ids are collected for the others only. */
                 UniqueOut uo{};
                 uo.match = mo;
-                uint64_t beside_bytes = 0; /* at most: a column's pages for `cap` rows */
-                for (const auto &o : outs)
-                    if (is_root && !o.from_keys && o.col.type != CJ_VARCHAR)
-                        beside_bytes += cap * (o.col.type == CJ_INT32 ? 5 : 9);
-                const bool room = room_for(beside_bytes);
+                const bool room = room_for(beside_bytes(cap));
                 for (auto &o : outs) {
                     if (!is_root || o.from_keys) continue;
                     const auto it = decoded.find({o.col.input, o.col.col});
@@ -815,13 +819,15 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         };
         bool all_fixed = true;
         for (const auto &o : outs) all_fixed &= o.col.type != CJ_VARCHAR;
-        if (is_root && unique && collect && all_fixed && (flags & CJ_EXEC_RESULT_ON_DEVICE) && ctx.opt.defer_count) {
+        if (is_root && unique && collect && all_fixed && (flags & CJ_EXEC_RESULT_ON_DEVICE) && ctx.opt.defer_count &&
+            room_for(beside_bytes(cap))) {
             /* Unique build keys at the root, result left in HBM, no VARCHAR
              * output: at most one match per probe row, so the result is sized
              * for P.rows and its pages are written with the match count read
              * on the device. The execution's one host synchronisation comes
              * last; only if the device refused the table does the join go on
-             * as below. */
+             * as below. Without room for the probe rows the count is read
+             * first, and the pages sized by it. */
             launch_probe(cap);
             std::vector<OutCol> cols;
             std::vector<int32_t> types;

@@ -59,3 +59,21 @@ def test_room_refused(bounded, room, gap, flags):
         assert st.exec["probe_reruns"] == 1
     for t in rp.inputs:
         t.free()
+
+
+@pytest.mark.parametrize("gap", [1, 5000])
+@pytest.mark.parametrize("room", [0, 1 << 30])
+def test_device_counted_result(bounded, room, gap):
+    """Unique keys, result in HBM: written with the count on the device (one
+    synchronisation) only where the probe rows' pages may be set aside."""
+    rng = np.random.default_rng(4)
+    bkeys, n = rng.permutation(3000) * gap, 40_000
+    pkeys = bkeys[rng.integers(0, 3000, n)] + gap * 3000 * (rng.random(n) < 0.9)
+    plan = _plan(bkeys, pkeys, bpay=[(L, np.arange(3000), None)], ppay=[(F, rng.random(n), None)])
+    ctx = bounded(room)
+    rp = _resident(plan, ctx)
+    got, st = run_product(rp, ctx, _lib.CJ_EXEC_RESULT_ON_DEVICE)
+    assert_same(got, run_oracle(plan), f"room {room}")
+    assert st.exec["host_syncs"] == (2 if room == 0 else 1)
+    for t in rp.inputs:
+        t.free()
