@@ -50,6 +50,11 @@ constexpr uint64_t kEmitBesideOpen = 48ull << 20;
  * size (a query of the free memory takes tens of us). */
 constexpr uint64_t kAmpleRoom = 4ull << 30;
 
+/* A result keeps the buffer that its probe wrote, sized for the matches there
+ * might have been, unless less than a quarter of it is used and kKeepSpare or
+ * more is not: the pages then move to a buffer of their size (64 MB in 20 us). */
+constexpr uint64_t kKeepSpare = 32ull << 20;
+
 enum Phase { PH_UPLOAD, PH_DECODE, PH_BUILD, PH_PROBE, PH_NL, PH_INTER, PH_MAT, PH_DOWNLOAD, PH_COUNT };
 /* NVTX range names of the phases (host-side ranges around the enqueueing of
  * each phase; visible in Nsight Systems timelines). */
@@ -157,17 +162,35 @@ class Executor {
         ctx.sync_status(used_cols);
         stats.host_syncs++;
     }
+    /* `pages` itself, or a buffer of `bytes` that its first bytes move to
+     * (kKeepSpare). */
+    DevPtr fitted(const DevPtr &pages, uint64_t bytes) {
+        if (!pages || bytes > pages->bytes / 4 || pages->bytes - bytes < kKeepSpare) return pages;
+        DevPtr fit = ctx.alloc(bytes);
+        if (bytes) ck(cudaMemcpyAsync(fit->ptr, pages->ptr, bytes, cudaMemcpyDeviceToDevice, ctx.stream), "fit pages");
+        return fit;
+    }
     /* A result written with a device-side row count (materialize with
      * rows_dev): its rows and pages once the count is known. */
     void finish_counted(cj_result &r, uint64_t rows) {
         r.num_rows = rows;
         uint64_t pages = 0;
+        bool moved = false;
+        std::map<DevPtr, DevPtr> fit; /* columns may share a buffer */
         for (size_t c = 0; c < r.types.size(); ++c) {
             const uint32_t R = rows_per_page_fixed(r.types[c]);
             r.num_pages[c] = (rows + R - 1) / R;
-            if (!rows) r.dev_pages[c].reset();
+            if (rows) {
+                DevPtr &f = fit[r.dev_pages[c]];
+                if (!f) f = fitted(r.dev_pages[c], r.num_pages[c] * kPageSize);
+                moved |= f != r.dev_pages[c];
+                r.dev_pages[c] = f;
+            } else {
+                r.dev_pages[c].reset();
+            }
             pages += r.num_pages[c];
         }
+        if (moved) ck(cudaStreamSynchronize(ctx.stream), "fit pages");
         stats.output_rows = rows;
         stats.output_pages = pages;
     }
@@ -1041,7 +1064,8 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
                  * shared page array */
                 if (cols[c].pages->bytes < res->num_pages[c] * kPageSize)
                     fail(CJ_ERR_INTERNAL, "result pages smaller than the result");
-                res->dev_pages[c] = cols[c].pages;
+                if (alias[c] >= 0) res->dev_pages[c] = res->dev_pages[alias[c]];
+                else res->dev_pages[c] = rows_dev ? cols[c].pages : fitted(cols[c].pages, res->num_pages[c] * kPageSize);
                 if (cols[c].rel) t.col = out_view(cols[c]);
                 else t.col.type = types[c];
                 t.finish = cols[c].rel ? 2 : 1;

@@ -4,7 +4,8 @@ probe may not write, or may write in its first run and not in the second."""
 import numpy as np
 import pytest
 
-from calamarijoins_b200 import Context, DataType, Plan, ResidentTable, _lib
+from calamarijoins_b200 import Context, DataType, Plan, ResidentTable, _lib, execute_raw
+from oracle import oracle_api as oa
 from tests.helpers import assert_same, run_oracle, run_product
 from tests.test_gpu_unique import _plan
 
@@ -77,3 +78,30 @@ def test_device_counted_result(bounded, room, gap):
     assert st.exec["host_syncs"] == (2 if room == 0 else 1)
     for t in rp.inputs:
         t.free()
+
+
+@pytest.mark.parametrize("flags", [0, _lib.CJ_EXEC_RESULT_ON_DEVICE])
+@pytest.mark.parametrize("keys", ["unique", "repeated"])
+def test_selective_result_gives_room_back(gpu_ctx, keys, flags):
+    """A handful of matches for 10M probe rows: the result holds the pages of
+    its matches, not those of the matches there might have been (41 MB for the
+    keys, 81 MB for each payload)."""
+    nb, n = 3000, 10_000_000
+    bkeys = np.arange(nb) if keys == "unique" else np.arange(nb) // 2
+    pkeys = np.full(n, 10 ** 6)
+    pkeys[::1_000_000] = 7
+    plan = _plan(bkeys, pkeys, bpay=[(L, np.arange(nb), None)], ppay=[(F, np.arange(n) / 2, None)])
+    rp = _resident(plan, gpu_ctx)
+    gpu_ctx.set_option(_lib.CJ_OPT_BUFFER_CACHE_BYTES, 0)  # freed buffers go back to the pool at once
+    try:
+        before, _ = gpu_ctx.memory()
+        res, _ = execute_raw(rp, gpu_ctx, flags)
+        held = gpu_ctx.memory()[0] - before
+        got = oa.PagedResult.from_result(res)
+        res.free()
+        assert held < 1 << 20
+        assert_same(got, run_oracle(plan), keys)
+    finally:
+        gpu_ctx.set_option(_lib.CJ_OPT_BUFFER_CACHE_BYTES, 16 << 30)
+        for t in rp.inputs:
+            t.free()
