@@ -13,26 +13,29 @@ pytestmark = pytest.mark.gpu
 I, L, F, V = DataType.INT32, DataType.INT64, DataType.FP64, DataType.VARCHAR
 
 
-@pytest.fixture
-def bounded(monkeypatch):
-    """Contexts with a bound of their own on the room."""
-    made = []
-
-    def make(room):
-        monkeypatch.setenv("CJ_SPARE_ROOM_BYTES", str(room))
-        made.append(Context(0))
-        return made[-1]
-
-    yield make
-    for c in made:
-        c.close()
-
-
 def _resident(plan, ctx):
     rp = Plan()
     rp.nodes, rp.root = plan.nodes, plan.root
     rp.inputs = [ResidentTable(ctx, t) for t in plan.inputs]
     return rp
+
+
+@pytest.fixture
+def bounded(monkeypatch):
+    """Runs a plan over resident tables in a context with a bound of its own
+    on the room."""
+    def run(plan, room, flags):
+        monkeypatch.setenv("CJ_SPARE_ROOM_BYTES", str(room))
+        ctx = Context(0)
+        rp = _resident(plan, ctx)
+        try:
+            return run_product(rp, ctx, flags)
+        finally:
+            for t in rp.inputs:
+                t.free()
+            ctx.close()
+
+    return run
 
 
 @pytest.mark.parametrize("flags", [0, _lib.CJ_EXEC_RESULT_ON_DEVICE])
@@ -51,15 +54,11 @@ def test_room_refused(bounded, room, gap, flags):
     valid = (rng.random(len(bkeys)) >= 0.1).astype(np.uint8)
     plan = _plan(bkeys, rng.permutation(pkeys), bpay=[(L, np.arange(6000), None), (I, np.arange(6000), valid)],
                  ppay=[(F, rng.random(n), None)])
-    ctx = bounded(room)
-    rp = _resident(plan, ctx)
-    got, st = run_product(rp, ctx, flags)
+    got, st = bounded(plan, room, flags)
     assert_same(got, run_oracle(plan), f"room {room}")
     assert got.num_rows == 60_000
     if room == 0:
         assert st.exec["probe_reruns"] == 1
-    for t in rp.inputs:
-        t.free()
 
 
 @pytest.mark.parametrize("gap", [1, 5000])
@@ -71,13 +70,9 @@ def test_device_counted_result(bounded, room, gap):
     bkeys, n = rng.permutation(3000) * gap, 40_000
     pkeys = bkeys[rng.integers(0, 3000, n)] + gap * 3000 * (rng.random(n) < 0.9)
     plan = _plan(bkeys, pkeys, bpay=[(L, np.arange(3000), None)], ppay=[(F, rng.random(n), None)])
-    ctx = bounded(room)
-    rp = _resident(plan, ctx)
-    got, st = run_product(rp, ctx, _lib.CJ_EXEC_RESULT_ON_DEVICE)
+    got, st = bounded(plan, room, _lib.CJ_EXEC_RESULT_ON_DEVICE)
     assert_same(got, run_oracle(plan), f"room {room}")
     assert st.exec["host_syncs"] == (2 if room == 0 else 1)
-    for t in rp.inputs:
-        t.free()
 
 
 @pytest.mark.parametrize("flags", [0, _lib.CJ_EXEC_RESULT_ON_DEVICE])
