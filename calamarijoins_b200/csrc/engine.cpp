@@ -162,12 +162,23 @@ class Executor {
         ctx.sync_status(used_cols);
         stats.host_syncs++;
     }
+    /* A buffer that the plan can do without: null when the memory is out. */
+    DevPtr spare(uint64_t bytes) {
+        try {
+            return ctx.alloc(bytes);
+        } catch (const Error &e) {
+            if (e.code != CJ_ERR_OUT_OF_MEMORY) throw;
+            return nullptr;
+        }
+    }
+
     /* `pages` itself, or a buffer of `bytes` that its first bytes move to
      * (kKeepSpare). */
     DevPtr fitted(const DevPtr &pages, uint64_t bytes) {
         if (!pages || bytes > pages->bytes / 4 || pages->bytes - bytes < kKeepSpare) return pages;
-        DevPtr fit = ctx.alloc(bytes);
-        if (bytes) ck(cudaMemcpyAsync(fit->ptr, pages->ptr, bytes, cudaMemcpyDeviceToDevice, ctx.stream), "fit pages");
+        DevPtr fit = spare(bytes);
+        if (!fit) return pages;
+        ck(cudaMemcpyAsync(fit->ptr, pages->ptr, bytes, cudaMemcpyDeviceToDevice, ctx.stream), "fit pages");
         return fit;
     }
     /* A result written with a device-side row count (materialize with
@@ -194,13 +205,9 @@ class Executor {
         stats.output_rows = rows;
         stats.output_pages = pages;
     }
-
-    /* Whether `bytes` may be set aside for matches that may not come: above
-     * kAmpleRoom, half of what is left (or the context's own bound). A
-     * selective join whose matches would fit does not fail for room it would
-     * not have used. */
-    bool room_for(uint64_t bytes) {
-        if (ctx.opt.spare_room >= 0) return bytes <= (uint64_t)ctx.opt.spare_room;
+    /* Whether `bytes` may be taken that the plan can do without: up to
+     * kAmpleRoom, above that half of what is left. */
+    bool ample(uint64_t bytes) {
         if (bytes <= kAmpleRoom) return true;
         size_t left = 0, total = 0;
         uint64_t used = 0, reserved = 0;
@@ -209,6 +216,12 @@ class Executor {
         ck(cudaMemPoolGetAttribute(ctx.pool, cudaMemPoolAttrReservedMemCurrent, &reserved), "pool attr");
         std::lock_guard<std::mutex> g(ctx.dev_mu); /* frees of other threads touch the cache too */
         return bytes <= (left + (reserved - std::min(reserved, used)) + ctx.dev_cached) / 2;
+    }
+    /* The same for matches that may not come, under the context's own bound
+     * where it has one. A selective join whose matches would fit does not
+     * fail for room it would not have used. */
+    bool room_for(uint64_t bytes) {
+        return ctx.opt.spare_room >= 0 ? bytes <= (uint64_t)ctx.opt.spare_room : ample(bytes);
     }
 
     const cj_table *resident(uint64_t t) const { return resident_input(plan, t); }
@@ -637,13 +650,16 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                  * if neither, builds another. Direct-mapped: 4 bytes per
                  * slot, at 8 x rows 32 B per build row, at most 2^28 slots (1
                  * GiB); open-addressing: 16 B per build row, 32 for INT64
-                 * keys. One buffer serves both. */
+                 * keys, left out where the memory is short. One buffer serves
+                 * both. */
                 table.max_span = std::min<uint64_t>((uint64_t)ctx.opt.dense_keys * B.rows, 1ull << 28);
                 table.wide = bk.type == CJ_INT64;
-                if (B.rows <= kOpenMaxRows)
-                    table.open_slots = (uint32_t)std::max<uint64_t>(2 * B.rows, 1024);
+                const uint64_t open_slots = std::max<uint64_t>(2 * B.rows, 1024);
+                if (B.rows <= kOpenMaxRows && ample(open_slots * (table.wide ? 16 : 8)))
+                    table.open_slots = (uint32_t)open_slots;
                 table.params = ctx.d_status->table;
-                slots = ctx.alloc(unique_table_bytes(table));
+                if (table.open_slots && !(slots = spare(unique_table_bytes(table)))) table.open_slots = 0;
+                if (!slots) slots = ctx.alloc(unique_table_bytes(table));
                 table.slots = slots->ptr;
                 if (!words_clear) clear_join_words();
                 KScope k(*this, "unique_build");
@@ -670,13 +686,31 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         };
         /* Allocates the match outputs for `cap` pairs and launches the probe
          * of the table built above. */
-        auto launch_probe = [&](uint64_t cap) {
-            drop_pages();
+        uint64_t cap = P.rows;
+        bool widened = false; /* cap is above the probe rows on an estimate */
+        auto match_arrays = [&](uint64_t cap) {
             /* the key columns' result pages, sized for the capacity */
             const uint32_t key_rpp = rows_per_page_fixed(pk.type);
             mk = emit_keys ? ctx.alloc((cap + key_rpp - 1) / key_rpp * kPageSize) : nullptr;
             mb = need_b ? ctx.alloc(cap * 4) : nullptr;
             mp = need_p ? ctx.alloc(cap * 4) : nullptr;
+        };
+        auto launch_probe = [&]() {
+            drop_pages();
+            if (widened) {
+                widened = false;
+                try {
+                    match_arrays(cap);
+                } catch (const Error &e) {
+                    if (e.code != CJ_ERR_OUT_OF_MEMORY) throw;
+                    mk.reset();
+                    mb.reset();
+                    cap = P.rows;
+                    match_arrays(cap);
+                }
+            } else {
+                match_arrays(cap);
+            }
             MatchOut mo;
             mo.build_rids = mb ? mb->as<uint32_t>() : nullptr;
             mo.probe_rids = mp ? mp->as<uint32_t>() : nullptr;
@@ -701,7 +735,9 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                     if (o.col.type != CJ_VARCHAR && it != decoded.end() && it->second.ready && uo.n < kEmitColumns &&
                         beside && room) {
                         const uint32_t R = rows_per_page_fixed(o.col.type);
-                        o.pages = ctx.alloc((cap + R - 1) / R * kPageSize);
+                        o.pages = spare((cap + R - 1) / R * kPageSize);
+                    }
+                    if (o.pages) {
                         o.direct_only = unique && o.from_build && table.open_slots &&
                                         table.open_slots * (table.wide ? 16ull : 8ull) +
                                                         it->second.src.num_pages * kPageSize > kEmitBesideOpen;
@@ -760,7 +796,6 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 }
             }
         };
-        uint64_t cap = P.rows;
         /* The device refused the table of unique keys (its probe did
          * nothing). Keys that repeat get a table of repeated keys: one random
          * access per probe row and one per further match.
@@ -790,14 +825,16 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 const uint64_t more = std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(cap, mean), 4 * P.rows),
                                                          0xFFFFFFFFull);
                 /* a match: two row ids and a key at most, here */
-                if (more > cap && room_for(more * 17)) cap = more;
+                if (more > cap && room_for(more * 17)) {
+                    cap = more;
+                    widened = true;
+                }
             };
-            if ((!tp[kTableRefused] || tp[kTableRefused] == kTableRepeats) && tp[kTableSpan] <= kMultiSpan * B.rows) {
+            if ((!tp[kTableRefused] || tp[kTableRefused] == kTableRepeats) && tp[kTableSpan] <= kMultiSpan * B.rows &&
+                (slots = spare((tp[kTableSpan] + 1) * 8)) && (multi_rows = spare(B.rows * 4))) {
                 multi = true;
                 multi_table.lo = (int64_t)tp[kTableLo];
                 multi_table.span = (uint32_t)tp[kTableSpan];
-                slots = ctx.alloc((tp[kTableSpan] + 1) * 8);
-                multi_rows = ctx.alloc(B.rows * 4);
                 multi_table.entries = slots->as<unsigned long long>();
                 multi_table.rows = multi_rows->as<uint32_t>();
                 widen(tp[kTableSpan]);
@@ -805,16 +842,18 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 ck(launch_multi_build(L, bv, (uint32_t)B.rows, multi_table), "multi_build");
                 return;
             }
+            slots.reset();
+            multi_rows.reset();
+            DevPtr slot_of;
+            const uint32_t open_n = (uint32_t)std::max<uint64_t>(2 * std::min(B.rows, kOpenMaxRows), 1024);
             if (tp[kTableRefused] != kTableWhole && B.rows <= kOpenMaxRows && P.rows / kOpenMultiProbe >= B.rows &&
-                room_for(B.rows * (2 * sizeof(MultiSlot) + 8))) {
-                open_table.nslots = (uint32_t)std::max<uint64_t>(2 * B.rows, 1024);
+                ample(B.rows * (2 * sizeof(MultiSlot) + 8)) && (slots = spare(open_n * sizeof(MultiSlot))) &&
+                (multi_rows = spare(B.rows * 4)) && (slot_of = spare(B.rows * 4))) {
+                open_table.nslots = open_n;
                 open_table.lo = tp[kTableLo];
                 open_table.width = tp[kTableSpan] - 1;
                 open_table.empty = tp[kTableEmpty];
                 open_table.found = ctx.d_status->table;
-                slots = ctx.alloc(open_table.nslots * sizeof(MultiSlot));
-                multi_rows = ctx.alloc(B.rows * 4);
-                DevPtr slot_of = ctx.alloc(B.rows * 4);
                 open_table.slots = slots->as<MultiSlot>();
                 open_table.rows = multi_rows->as<uint32_t>();
                 open_table.slot_of = slot_of->as<uint32_t>();
@@ -829,9 +868,10 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                     widen(ctx.h_status->table[kMultiKeys]);
                     return;
                 }
-                slots.reset();
-                multi_rows.reset();
             }
+            slots.reset();
+            multi_rows.reset();
+            slot_of.reset();
             clear_join_words(); /* the match counter, and words no longer read */
             build_hash();
         };
@@ -840,6 +880,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             stats.num_direct_joins += kind == 1;
             stats.num_open_joins += kind == 2 && !table.wide; /* INT32 keys, as documented */
         };
+        bool probed = false; /* the probe has been launched already */
         bool all_fixed = true;
         for (const auto &o : outs) all_fixed &= o.col.type != CJ_VARCHAR;
         if (is_root && unique && collect && all_fixed && (flags & CJ_EXEC_RESULT_ON_DEVICE) && ctx.opt.defer_count &&
@@ -851,27 +892,37 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
              * last; only if the device refused the table does the join go on
              * as below. Without room for the probe rows the count is read
              * first, and the pages sized by it. */
-            launch_probe(cap);
+            launch_probe();
             std::vector<OutCol> cols;
             std::vector<int32_t> types;
             root_columns(cols, types);
-            std::unique_ptr<cj_result> r(materialize(cols, types, cap, &ctx.d_status->counter));
-            sync();
-            if (table_kind(ctx.h_status->table, table.open_slots)) {
-                M = ctx.h_status->counter;
-                finish_counted(*r, M);
-                count_join();
-                stats.matches += M;
-                synced_last = true;
-                *out = r.release();
-                return Relation{};
+            std::unique_ptr<cj_result> r;
+            try {
+                r.reset(materialize(cols, types, cap, &ctx.d_status->counter));
+            } catch (const Error &e) {
+                if (e.code != CJ_ERR_OUT_OF_MEMORY) throw;
+                probed = true; /* the pages of the matches alone may fit */
             }
-            r.reset();
-            replace_unique();
+            if (r) {
+                sync();
+                if (table_kind(ctx.h_status->table, table.open_slots)) {
+                    M = ctx.h_status->counter;
+                    finish_counted(*r, M);
+                    count_join();
+                    stats.matches += M;
+                    synced_last = true;
+                    *out = r.release();
+                    return Relation{};
+                }
+                r.reset();
+                replace_unique();
+            }
         }
-        for (;;) {
-            if (multi) clear_join_words(); /* the match counter */
-            launch_probe(cap);
+        for (;; probed = false) {
+            if (!probed) {
+                if (multi) clear_join_words(); /* the match counter */
+                launch_probe();
+            }
             sync();
             if (unique && !table_kind(ctx.h_status->table, table.open_slots)) {
                 replace_unique();

@@ -4,7 +4,7 @@ probe may not write, or may write in its first run and not in the second."""
 import numpy as np
 import pytest
 
-from calamarijoins_b200 import Context, DataType, Plan, ResidentTable, _lib, execute_raw
+from calamarijoins_b200 import CJError, Context, DataType, Plan, ResidentTable, _lib, execute_raw
 from oracle import oracle_api as oa
 from tests.helpers import assert_same, run_oracle, run_product
 from tests.test_gpu_unique import _plan
@@ -97,6 +97,44 @@ def test_selective_result_gives_room_back(gpu_ctx, keys, flags):
         assert held < 1 << 20
         assert_same(got, run_oracle(plan), keys)
     finally:
+        gpu_ctx.set_option(_lib.CJ_OPT_BUFFER_CACHE_BYTES, 16 << 30)
+        for t in rp.inputs:
+            t.free()
+
+
+@pytest.mark.parametrize("keys", ["dense", "spread", "wide", "repeated", "repeated_spread"])
+def test_plan_does_without_spare_room(gpu_ctx, keys):
+    """Every allocation of a join fails in turn. What the plan can do without
+    (open-addressing slots, pages that the probe writes, room above the probe
+    rows, tables of repeated keys) must not fail it; the rest must."""
+    rng = np.random.default_rng(5)
+    k, n = rng.permutation(3000) // (2 if "repeated" in keys else 1), 30_000
+    k = k * (1 if keys in ("dense", "repeated") else 10 ** 5)
+    t = L if keys == "wide" else I
+    plan = _plan(k, k[rng.integers(0, 3000, n)], t, t, bpay=[(L, np.arange(3000), None)], ppay=[(F, rng.random(n), None)])
+    want, rp = run_oracle(plan), _resident(plan, gpu_ctx)
+    done_without, failed = [], []
+    gpu_ctx.set_option(_lib.CJ_OPT_BUFFER_CACHE_BYTES, 0)
+    try:
+        used0, _ = gpu_ctx.memory()
+        for at in range(1, 60):
+            gpu_ctx.set_option(_lib.CJ_OPT_FAIL_ALLOC_AT, at)
+            try:
+                got, _ = run_product(rp, gpu_ctx, _lib.CJ_EXEC_RESULT_ON_DEVICE)
+                reached = gpu_ctx.get_option(_lib.CJ_OPT_FAIL_ALLOC_AT) == 0
+                assert_same(got, want, f"{keys}, allocation {at}")
+                if not reached:
+                    break
+                done_without.append(at)
+            except CJError as e:
+                assert e.status == 4 and "injected" in str(e)
+                failed.append(at)
+            gpu_ctx.set_option(_lib.CJ_OPT_FAIL_ALLOC_AT, 0)
+            assert gpu_ctx.memory()[0] == used0
+        assert not reached and len(failed) >= 2
+        assert len(done_without) >= {"dense": 3, "spread": 3, "wide": 3, "repeated": 7, "repeated_spread": 8}[keys]
+    finally:
+        gpu_ctx.set_option(_lib.CJ_OPT_FAIL_ALLOC_AT, 0)
         gpu_ctx.set_option(_lib.CJ_OPT_BUFFER_CACHE_BYTES, 16 << 30)
         for t in rp.inputs:
             t.free()
