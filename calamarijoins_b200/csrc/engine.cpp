@@ -819,8 +819,11 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             unsigned long long tp[kTableWords];
             std::copy(ctx.h_status->table, ctx.h_status->table + kTableWords, tp);
             /* room for the keys' mean number of rows per match, up to 4; a
-             * result above it runs the probe again */
+             * result above it runs the probe again. A server's worker keeps
+             * to the probe rows: admission counts on no more, and what one
+             * plan takes on a guess another might need. */
             auto widen = [&](uint64_t keys) {
+                if (!ctx.owns_pool) return;
                 const uint64_t mean = P.rows * (uint64_t)tp[kTableCount] / std::max<uint64_t>(keys, 1);
                 const uint64_t more = std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(cap, mean), 4 * P.rows),
                                                          0xFFFFFFFFull);

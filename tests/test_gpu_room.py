@@ -4,7 +4,7 @@ probe may not write, or may write in its first run and not in the second."""
 import numpy as np
 import pytest
 
-from calamarijoins_b200 import CJError, Context, DataType, Plan, ResidentTable, _lib, execute_raw
+from calamarijoins_b200 import CJError, Context, DataType, Plan, ResidentTable, Server, _lib, execute_raw
 from oracle import oracle_api as oa
 from tests.helpers import assert_same, run_oracle, run_product
 from tests.test_gpu_unique import _plan
@@ -138,3 +138,21 @@ def test_plan_does_without_spare_room(gpu_ctx, keys):
         gpu_ctx.set_option(_lib.CJ_OPT_BUFFER_CACHE_BYTES, 16 << 30)
         for t in rp.inputs:
             t.free()
+
+
+def test_server_worker_keeps_to_the_estimate():
+    """Two matches per probe row: a context by itself makes room for them at
+    once, a server's worker, whose memory others share, when it has counted."""
+    rng = np.random.default_rng(6)
+    bkeys = rng.permutation(np.repeat(np.arange(4000), 2))
+    pkeys = rng.integers(0, 4000, 50_000)
+    plan = _plan(bkeys, pkeys, bpay=[(L, np.arange(8000), None)])
+    srv = Server(slots=1)
+    try:
+        res, st = srv.wait(srv.submit(plan))
+        got = oa.PagedResult.from_result(res)
+        res.free()
+    finally:
+        srv.close()
+    assert_same(got, run_oracle(plan))
+    assert st["probe_reruns"] == 1
