@@ -85,6 +85,10 @@ struct PlanState {
 
 } // namespace
 
+/* A match array of this size has an allocation of its own (0.4 us of host
+ * time, about as much as writing it takes on the device). */
+constexpr uint64_t kOwnMatches = 1u << 20;
+
 /* What a learning run records for the capture: match counts of every join
  * of every level, in the executor's work order, and page counts of every
  * VARCHAR output column, in materialisation order. */
@@ -442,17 +446,30 @@ void BatchExecutor::run_level(int lvl) {
         unsigned long long *wp = words->as<unsigned long long>();
         unsigned int *ticket = reinterpret_cast<unsigned int *>(wp);
         size_t off = 1;
-        Slab matches;
-        for (size_t k : pidx) {
-            if (work[k].need_b) matches.reserve(work[k].cap * 4);
-            if (work[k].need_p) matches.reserve(work[k].cap * 4);
-        }
-        matches.open(ctx);
-        keep_checks.push_back(matches.mem);
+        /* Match arrays: small ones from a slab for those that a relation or
+         * a root keeps and one for those that only this level's gather
+         * reads; large ones by themselves. Each is given back as soon as a
+         * buffer of its own would be. */
+        Slab kept, passing;
+        auto matches = [&](JoinWork &w, bool build, bool take) -> DevPtr {
+            const uint64_t bytes = w.cap * 4;
+            if (!(build ? w.need_b : w.need_p)) return nullptr;
+            if (bytes >= kOwnMatches) return take ? ctx.alloc(bytes) : nullptr;
+            bool keep = w.is_root;
+            for (const auto &o : w.outs) keep |= o.from_build == build && o.col.vec < 0;
+            Slab &slab = keep ? kept : passing;
+            if (take) return slab.part(bytes);
+            slab.reserve(bytes);
+            return nullptr;
+        };
+        for (size_t k : pidx)
+            for (bool build : {true, false}) matches(work[k], build, false);
+        kept.open(ctx);
+        passing.open(ctx);
         for (size_t k : pidx) {
             auto &w = work[k];
-            w.mb = w.need_b ? matches.part(w.cap * 4) : nullptr;
-            w.mp = w.need_p ? matches.part(w.cap * 4) : nullptr;
+            w.mb = matches(w, true, true);
+            w.mp = matches(w, false, true);
             ProbeTask t{};
             t.pkey = view(w.plan, *w.P, w.pk, nullptr);
             t.n_probe = (uint32_t)w.P->rows;
@@ -591,10 +608,7 @@ void BatchExecutor::materialize_roots() {
             const uint32_t R = rows_per_page_fixed(p.root_types[c]);
             pages.reserve((p.root_rows + R - 1) / R * kPageSize);
         }
-        if (pages.size) {
-            pages.open(ctx);
-            res->keep = pages.mem;
-        }
+        if (pages.size) pages.open(ctx);
         for (size_t c = 0; c < nc; ++c) {
             if (p.root_types[c] == CJ_VARCHAR) {
                 var.push_back({i, c, ctx.alloc(varchar_temp_bytes(p.root_rows, TR))});

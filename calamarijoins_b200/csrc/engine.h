@@ -71,7 +71,8 @@ struct DevBuf {
     void *ptr = nullptr;
     size_t bytes = 0;
     size_t cls = 0;     /* bytes actually held (size class) */
-    bool arena = false; /* carved from the context's arena: not freed alone */
+    bool arena = false; /* carved from the context's arena or from `owner`: not freed alone */
+    std::shared_ptr<DevBuf> owner; /* the buffer it is a part of (Slab) */
     ~DevBuf();
     template <typename T> T *as() const { return reinterpret_cast<T *>(ptr); }
 };

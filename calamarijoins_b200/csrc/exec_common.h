@@ -57,11 +57,12 @@ struct Slab {
         return p;
     }
     template <typename T> T *take_as(size_t bytes) { return reinterpret_cast<T *>(take(bytes)); }
-    /* a buffer object over a part: the slab's owner keeps the memory */
+    /* a buffer object over a part, which keeps the memory */
     DevPtr part(size_t bytes) {
         auto b = std::make_shared<DevBuf>();
         b->bytes = bytes;
         b->arena = true;
+        b->owner = mem;
         b->ptr = take(bytes);
         return b;
     }

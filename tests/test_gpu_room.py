@@ -4,7 +4,8 @@ probe may not write, or may write in its first run and not in the second."""
 import numpy as np
 import pytest
 
-from calamarijoins_b200 import CJError, Context, DataType, Plan, ResidentTable, Server, _lib, execute_raw
+from calamarijoins_b200 import (CJError, ColumnarTable, Context, DataType, Plan, ResidentTable, Server, _lib,
+                                encode_column, execute_batch, execute_raw)
 from oracle import oracle_api as oa
 from tests.helpers import assert_same, run_oracle, run_product
 from tests.test_gpu_unique import _plan
@@ -156,3 +157,36 @@ def test_server_worker_keeps_to_the_estimate():
         srv.close()
     assert_same(got, run_oracle(plan))
     assert st["probe_reruns"] == 1
+
+
+def test_batch_gives_match_arrays_back():
+    """Eight joins of a chain over 8M rows: a level's match arrays (32 MB)
+    are gathered through and given back. Decoded columns (9 x 33 MB), a row-id
+    vector per level and the result stay: 620 MB, and 190 more if the levels'
+    match arrays stayed too."""
+    n, joins = 8_000_000, 8
+    rng = np.random.default_rng(7)
+    fk = encode_column(I, rng.integers(0, 1000, n).astype(np.int32))
+    plan = Plan()
+    plan.inputs = [ColumnarTable(n, [fk] * (joins + 1))]
+    left = plan.new_scan_node(0, [(i, I) for i in range(joins + 1)])
+    for k in range(joins):
+        plan.inputs.append(ColumnarTable(1000, [encode_column(I, rng.permutation(1000).astype(np.int32))]))
+        scan = plan.new_scan_node(k + 1, [(0, I)])
+        last = k == joins - 1
+        left = plan.new_join_node(True, left, scan, k, 0, [(joins, I)] if last else [(i, I) for i in range(joins + 1)])
+    plan.root = left
+    ctx = Context(0)
+    ctx.set_option(_lib.CJ_OPT_BUFFER_CACHE_BYTES, 0)
+    rp = _resident(plan, ctx)
+    try:
+        before = ctx.memory()[1]
+        res, sts, _ = execute_batch([rp], ctx, _lib.CJ_EXEC_RESULT_ON_DEVICE)
+        grown = ctx.memory()[1] - before  # the pool keeps what it has reserved
+        assert sts == [0] and res[0].num_rows == n
+        res[0].free()
+        assert grown < 720 << 20
+    finally:
+        for t in rp.inputs:
+            t.free()
+        ctx.close()
