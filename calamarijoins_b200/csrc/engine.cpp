@@ -235,6 +235,7 @@ class Executor {
     void launch_tasks(std::vector<ColumnTask> &tasks, bool index);
     Decoded &indexed(uint64_t t, uint64_t c);
     Decoded &decode(uint64_t t, uint64_t c);
+    void decode_all(const std::vector<TC> &cols);
     int streamed_key(std::pair<uint64_t, uint64_t> *col) const;
     Relation resolve(uint64_t node, int depth);
     Relation exec_join(uint64_t node, int depth, bool is_root, cj_result **out);
@@ -306,14 +307,21 @@ std::map<Executor::TC, ColumnPages> Executor::upload_small(const std::vector<TC>
  * column's copy only when it decodes that column, so later columns (the
  * payloads) cross PCIe while the joins below the root run.
  *
- * The resident columns among them are indexed and decoded here, all in one
- * launch each (per column those were two to three launches and two memsets:
- * 212 us of a six-table plan's 1.9 ms). Each keeps its errors to itself
- * until the plan reads it: a plan that never gets to a malformed column
- * (an empty join below) still runs. */
+ * The resident columns among them are indexed here in one launch, and those
+ * that the plan is sure to read decoded in another (per column those were two
+ * to three launches and two memsets: 212 us of a six-table plan's 1.9 ms):
+ * all of a plan of one join, the join keys of a larger one, whose other
+ * columns wait for the root (decode_all), since a join below may come out
+ * empty; none when a table is empty. (40M probe rows with two payloads that
+ * hold NULLs: an empty build side 28 us, 504 with everything decoded; an empty
+ * first join of two 358 and 644.) Each column keeps its errors to itself
+ * until the plan reads it: a plan that never gets to a malformed column still
+ * runs. */
 void Executor::prefetch() {
     std::vector<TC> order;
-    std::set<TC> seen;
+    std::set<TC> seen, keys;
+    bool empty = false; /* a table without rows: every join above it is empty too */
+    uint64_t joins = 0;
     auto add = [&](const TC &tc) {
         if (seen.insert(tc).second) order.push_back(tc);
     };
@@ -322,13 +330,19 @@ void Executor::prefetch() {
         const cj_plan_node &n = plan.nodes[node];
         std::vector<TC> out;
         if (n.node_type == CJ_NODE_SCAN) {
+            empty |= table_rows(n.base_table_id) == 0;
             for (uint64_t a = 0; a < n.num_output_attrs; ++a) out.push_back({n.base_table_id, n.output_attrs[a].index});
             return out;
         }
+        ++joins;
         std::vector<TC> both = cols(n.left, depth + 1);
         const std::vector<TC> r = cols(n.right, depth + 1);
-        if (n.left_attr < both.size()) add(both[n.left_attr]);
-        if (n.right_attr < r.size()) add(r[n.right_attr]);
+        auto add_key = [&](const TC &tc) {
+            add(tc);
+            keys.insert(tc);
+        };
+        if (n.left_attr < both.size()) add_key(both[n.left_attr]);
+        if (n.right_attr < r.size()) add_key(r[n.right_attr]);
         both.insert(both.end(), r.begin(), r.end());
         for (uint64_t a = 0; a < n.num_output_attrs; ++a)
             if (n.output_attrs[a].index < both.size()) out.push_back(both[n.output_attrs[a].index]);
@@ -342,7 +356,8 @@ void Executor::prefetch() {
     for (const TC &tc : order) {
         const cj_table *r = resident(tc.first);
         const auto up = small.find(tc);
-        if ((!r && up == small.end()) || table_rows(tc.first) > 0xFFFFFFFFull || now.size() == kStatusColumns) continue;
+        if (empty || (!r && up == small.end()) || table_rows(tc.first) > 0xFFFFFFFFull || now.size() == kStatusColumns)
+            continue;
         Decoded d;
         d.type = column_type(tc.first, tc.second);
         d.rows = table_rows(tc.first);
@@ -361,7 +376,7 @@ void Executor::prefetch() {
             d.mem = slab.mem;
             ColumnState *state = &ctx.d_status->cols[d.status_col];
             tasks.push_back(column_task(d, slab, state, &state->err));
-            d.ready = !(stream && kv.first == streamed);
+            d.ready = joins <= 1 ? !(stream && kv.first == streamed) : keys.count(kv.first) > 0;
             if (d.ready) decodes.push_back(tasks.back());
             decoded.emplace(kv.first, std::move(d));
         }
@@ -375,7 +390,7 @@ void Executor::prefetch() {
         const auto up = small.find(tc);
         if (up != small.end()) {
             if (decoded.count(tc)) continue;
-            Prefetched pf; /* more columns than the status block tracks */
+            Prefetched pf; /* an empty table, or more columns than the status block tracks */
             pf.pages = up->second;
             pf.done = ctx.get_event();
             ck(cudaEventRecord(pf.done, ctx.stream), "event record");
@@ -479,6 +494,20 @@ Decoded &Executor::decode(uint64_t t, uint64_t c) {
         d.ready = true;
     }
     return d;
+}
+
+/* Several columns, in one launch. */
+void Executor::decode_all(const std::vector<TC> &cols) {
+    std::vector<ColumnTask> tasks;
+    for (const TC &tc : cols) {
+        Decoded &d = indexed(tc.first, tc.second);
+        if (d.ready) continue;
+        tasks.push_back(d.task);
+        d.ready = true;
+    }
+    if (tasks.empty()) return;
+    PhaseScope ph(*this, PH_DECODE);
+    launch_tasks(tasks, false);
 }
 
 ColView Executor::view(const Relation &R, const RelCol &c, const uint32_t *rid_a) {
@@ -588,8 +617,11 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
              * synchronisation, where the GPU would wait for the host to
              * enqueue them. Columns still uploading stay lazy, so that the
              * result downloads overlap their uploads. */
+            std::vector<TC> here;
             for (const auto &o : outs)
-                if (!o.from_keys && resident(o.col.input)) decode(o.col.input, o.col.col);
+                if (!o.from_keys && (resident(o.col.input) || decoded.count({o.col.input, o.col.col})))
+                    here.push_back({o.col.input, o.col.col});
+            decode_all(here);
         }
         const uint64_t nl_max = std::min<int64_t>(std::max<int64_t>(ctx.opt.nested_loop_max_build, 0), kNestedLoopMax);
         const bool nl = B.rows <= nl_max;
