@@ -55,6 +55,12 @@ constexpr uint64_t kAmpleRoom = 4ull << 30;
  * more is not: the pages then move to a buffer of their size (64 MB in 20 us). */
 constexpr uint64_t kKeepSpare = 32ull << 20;
 
+/* Pages of payload columns that a plan of several joins decodes before the
+ * first: a launch less, under which the host prepares that join (a star's
+ * 243 MB of them, five joins: 733 us, 747 with the payloads decoded at the root), but
+ * for nothing when a join below the root is empty (256 MB: about 100 us). */
+constexpr uint64_t kDecodeAhead = 256ull << 20;
+
 enum Phase { PH_UPLOAD, PH_DECODE, PH_BUILD, PH_PROBE, PH_NL, PH_INTER, PH_MAT, PH_DOWNLOAD, PH_COUNT };
 /* NVTX range names of the phases (host-side ranges around the enqueueing of
  * each phase; visible in Nsight Systems timelines). */
@@ -321,7 +327,7 @@ void Executor::prefetch() {
     std::vector<TC> order;
     std::set<TC> seen, keys;
     bool empty = false; /* a table without rows: every join above it is empty too */
-    uint64_t joins = 0;
+    uint64_t joins = 0, ahead = 0; /* pages that are decoded for nothing when a join comes out empty */
     auto add = [&](const TC &tc) {
         if (seen.insert(tc).second) order.push_back(tc);
     };
@@ -364,6 +370,7 @@ void Executor::prefetch() {
         d.src = r ? r->cols[tc.second] : up->second;
         d.status_col = (int)now.size();
         d.reserve(slab);
+        if (joins > 1 && !keys.count(tc)) ahead += d.src.num_pages * kPageSize;
         now.emplace_back(tc, std::move(d));
     }
     if (!now.empty()) {
@@ -376,7 +383,7 @@ void Executor::prefetch() {
             d.mem = slab.mem;
             ColumnState *state = &ctx.d_status->cols[d.status_col];
             tasks.push_back(column_task(d, slab, state, &state->err));
-            d.ready = joins <= 1 ? !(stream && kv.first == streamed) : keys.count(kv.first) > 0;
+            d.ready = !(stream && kv.first == streamed) && (ahead <= kDecodeAhead || keys.count(kv.first));
             if (d.ready) decodes.push_back(tasks.back());
             decoded.emplace(kv.first, std::move(d));
         }

@@ -59,20 +59,21 @@ def test_empty_table(gpu_ctx, empty, resident, flags):
 
 
 @pytest.mark.parametrize("flags", [0, _lib.CJ_EXEC_RESULT_ON_DEVICE])
-@pytest.mark.parametrize("resident", [True, False])
 @pytest.mark.parametrize("first", [0, 1000])
-def test_empty_join(gpu_ctx, first, resident, flags):
-    """The first join matches something or nothing: the payloads are decoded
-    (the second launch) only when the root is reached."""
+@pytest.mark.parametrize("n", [20_000, 19_000_000])
+def test_empty_join(gpu_ctx, first, n, flags):
+    """The first join matches something or nothing: payloads of more than 256
+    MB of pages are decoded (the second launch) only when the root is
+    reached."""
     rng = np.random.default_rng(2)
     plan = Plan()
-    plan.inputs = [_fact(20_000, rng), _dim(first), _dim(0)]
+    plan.inputs = [_fact(n, rng), _dim(first), _dim(0, 5)]
     fact = plan.new_scan_node(0, [(0, I), (1, I), (2, F), (3, L)])
     dims = [plan.new_scan_node(k, [(0, I), (1, L)]) for k in (1, 2)]
     j = plan.new_join_node(True, fact, dims[0], 0, 0, [(1, I), (2, F), (3, L), (5, L)])
     plan.root = plan.new_join_node(True, j, dims[1], 0, 0, [(1, F), (2, L), (3, L), (5, L)])
-    got, launches = _run(plan, gpu_ctx, resident, flags)
+    got, launches = _run(plan, gpu_ctx, True, flags)
     assert_same(got, run_oracle(plan))
     assert (got.num_rows == 0) == (first > 0)
-    assert launches["decode"] == (1 if first else 2)
+    assert launches["decode"] == (2 if n > 20_000 and not first else 1)
     assert launches["page_index"] == 1
