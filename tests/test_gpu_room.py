@@ -63,6 +63,26 @@ def test_room_refused(bounded, room, gap, flags):
 
 
 @pytest.mark.parametrize("gap", [1, 5000])
+@pytest.mark.parametrize("rows", [5, 4])
+def test_room_for_the_mean_is_enough(gpu_ctx, rows, gap):
+    """Probe rows that all match, of keys with a row more than the mean a
+    little more often than of the others: one run."""
+    k = np.arange(4000) * gap
+    bkeys = np.concatenate([np.repeat(k, rows - 3), k[:1000]])
+    pkeys = np.concatenate([np.repeat(k, 12), k[:500]])
+    plan = _plan(bkeys, pkeys, bpay=[(L, np.arange(len(bkeys)), None)])
+    rp = _resident(plan, gpu_ctx)
+    try:
+        got, st = run_product(rp, gpu_ctx, _lib.CJ_EXEC_RESULT_ON_DEVICE)
+    finally:
+        for t in rp.inputs:
+            t.free()
+    assert_same(got, run_oracle(plan))
+    assert got.num_rows > len(pkeys) * len(bkeys) // 4000
+    assert st.exec["probe_reruns"] == 0
+
+
+@pytest.mark.parametrize("gap", [1, 5000])
 @pytest.mark.parametrize("room", [0, 1 << 30])
 def test_device_counted_result(bounded, room, gap):
     """Unique keys, result in HBM: written with the count on the device (one
