@@ -863,18 +863,18 @@ CJ_DEV void probe_step(const LK &lk, const typename LK::Code *code, uint32_t ok,
     __syncwarp(); /* done with w before the next step packs */
 }
 
-/* The same over a table of repeated keys, of either kind. The matches of rows with up to
- * three are packed and written together; those of rows with more in rounds,
- * the j-th matches of all of them; the rows of a key with more than kHeavyRun
- * build rows one after the other. 64M x 4M rows over 3M keys, 58.6M matches:
- * 956 us with one result column of two written beside it (bound by the
- * registers of its many paths: 64, some spilled; a separate function for the
- * rare ones cost more in the common one, 1141 us; every match of a row in
- * rounds 1458; warps without rows of more than three on a path of their own
- * 1150). Open addressing, 30M x 3M rows, 31M matches: 955 us with INT32 keys,
- * 1282 with INT64 ones (a 96 MB table); the hash probe takes 455 and 685, but
- * runs twice, having no number of keys to size the result by. */
-constexpr uint32_t kHeavyRun = 32;
+/* The same over a table of repeated keys, of either kind. The matches of rows
+ * with up to three are packed and written together, in three parts where they
+ * outnumber the room; those of rows with more are listed 32 a step, whichever
+ * rows they are of, and written whenever the room is full: all lanes then have
+ * loads in flight however many rows the matches come from. (In rounds of the
+ * j-th matches and, from 33 on, row by row, the 24M matches of 300K x 3M rows,
+ * eight a key, took 808 us, 685 so; the whole join, the hash table 1133.)
+ * 64M x 4M rows over 3M keys, 58.6M matches: 877 us with one result column of
+ * two written beside it (bound by the registers of its many paths: 64, some
+ * spilled; 956 with the rounds, which spilled three times as much; a separate
+ * function for the rare ones cost more in the common one, 1141; warps without
+ * rows of more than three on a path of their own 1150). */
 constexpr uint32_t kMultiRoom = 320; /* matches packed at once: 256 rows and a quarter more */
 struct MultiMatches {
     uint32_t rid[kMultiRoom]; /* the keys first, then the build rows */
@@ -988,15 +988,16 @@ CJ_DEV void probe_step(const LK &lk, const typename LK::Code *code, uint32_t ok,
         if (cnt[it] > 3) many += cnt[it];
     many = warp_sum(many);
     const auto few_of = [&](int it) { return cnt[it] <= 3 ? cnt[it] : 0u; };
-    const uint32_t few = pack_few(few_of, [&](int it, uint32_t i, uint32_t c) {
+    const auto stage = [&](int it, uint32_t i, uint32_t c) {
 #pragma unroll
         for (uint32_t j = 0; j < 3; ++j)
             if (j < c) {
                 if constexpr (LK::kStage) w.rid[i + j] = code[it];
                 w.row[i + j] = (uint8_t)(it * 32 + lane);
             }
-    });
-    const bool packed = few <= kMultiRoom; /* else all of them in rounds */
+    };
+    const uint32_t few = pack_few(few_of, stage);
+    const bool packed = few <= kMultiRoom;
     const unsigned long long total = few + many;
     if (lane == 0) sh.count[buf][part] = total;
     __syncthreads();
@@ -1014,12 +1015,16 @@ CJ_DEV void probe_step(const LK &lk, const typename LK::Code *code, uint32_t ok,
      * with room for the whole count */
     if (base + total > out.match.capacity) return;
     uint32_t at = (uint32_t)base;
-    if (packed && few) {
+    const uint32_t passes = packed ? 1u : 3u;
+    for (uint32_t h = 0; few && h < passes; ++h) {
+        /* all of them, or those of three items (288 matches at most) */
+        const auto part_of = [&](int it) { return packed || (uint32_t)it / 3 == h ? few_of(it) : 0u; };
+        const uint32_t n = packed ? few : pack_few(part_of, stage);
         if constexpr (LK::kStage) {
-            if (out.match.key_pages) emit_keys<T>(lk, out, w, few, at);
+            if (out.match.key_pages) emit_keys<T>(lk, out, w, n, at);
         }
         const PageRun<T> keys(out.match.key_pages, at);
-        pack_few(few_of, [&](int it, uint32_t i, uint32_t c) {
+        pack_few(part_of, [&](int it, uint32_t i, uint32_t c) {
             if constexpr (!LK::kStage) {
                 if (out.match.key_pages)
                     for (uint32_t j = 0; j < c; ++j) __stcs(keys.at(i + j), lk.key_of(code[it]));
@@ -1035,35 +1040,12 @@ CJ_DEV void probe_step(const LK &lk, const typename LK::Code *code, uint32_t ok,
             }
         });
         __syncwarp();
-        emit_packed(out, plan, w, few, at, row0);
-        at += few;
-    }
-    __syncwarp(); /* done with w before it is packed again */
-    if (packed && !many) return;
-    for (uint32_t j = 0;; ++j) {
-        const auto hit_of = [&](int it) {
-            return cnt[it] > j && cnt[it] <= kHeavyRun && (!packed || cnt[it] > 3) ? 1u : 0u;
-        };
-        const uint32_t n = pack_few(hit_of, [&](int it, uint32_t i, uint32_t) {
-            if constexpr (LK::kStage) w.rid[i] = code[it];
-            w.row[i] = (uint8_t)(it * 32 + lane);
-        });
-        if (!n) break;
-        if constexpr (LK::kStage) {
-            if (out.match.key_pages) emit_keys<T>(lk, out, w, n, at);
-        }
-        const PageRun<T> keys(out.match.key_pages, at);
-        pack_few(hit_of, [&](int it, uint32_t i, uint32_t) {
-            if constexpr (!LK::kStage) {
-                if (out.match.key_pages) __stcs(keys.at(i), lk.key_of(code[it]));
-            }
-            w.rid[i] = cnt[it] == 1 ? low[it] : __ldg(lk.rows + (low[it] - cnt[it] + j));
-        });
-        __syncwarp();
         emit_packed(out, plan, w, n, at, row0);
-        __syncwarp();
+        __syncwarp(); /* done with w before it is packed again */
         at += n;
     }
+    if (!many) return;
+    uint32_t left = (uint32_t)many, fill = 0; /* below the capacity */
     for (int it = 0; it < kItems; ++it) {
         uint32_t c = 0, lo = 0; /* item `it`, without indexing registers */
         typename LK::Code cd = 0;
@@ -1074,28 +1056,44 @@ CJ_DEV void probe_step(const LK &lk, const typename LK::Code *code, uint32_t ok,
                 lo = low[q];
                 cd = code[q];
             }
-        uint32_t heavy = __ballot_sync(0xffffffffu, c > kHeavyRun);
-        while (heavy) {
-            const int src = __ffs(heavy) - 1;
-            heavy &= heavy - 1;
-            const uint32_t rows_n = __shfl_sync(0xffffffffu, c, src);
-            const uint32_t first = __shfl_sync(0xffffffffu, lo, src) - rows_n;
-            const typename LK::Code kc = __shfl_sync(0xffffffffu, cd, src);
-            for (uint32_t k0 = 0; k0 < rows_n; k0 += kWarpRows) {
-                const uint32_t n = min(kWarpRows, rows_n - k0);
-                for (uint32_t i = lane; i < n; i += 32) {
-                    w.rid[i] = __ldg(lk.rows + (first + k0 + i));
-                    w.row[i] = (uint8_t)(it * 32 + src);
-                }
-                __syncwarp();
-                if (out.match.key_pages) {
-                    const PageRun<T> keys(out.match.key_pages, at);
-                    for (uint32_t i = lane; i < n; i += 32) __stcs(keys.at(i), lk.key_of(kc));
-                }
-                emit_packed(out, plan, w, n, at, row0);
-                __syncwarp();
-                at += n;
+        if (c <= 3) c = 0;
+        const uint32_t incl = warp_inclusive_scan(c), all = __shfl_sync(0xffffffffu, incl, 31);
+        const uint32_t place = lo - incl; /* of match p of the item's: place + p */
+        for (uint32_t p0 = 0; p0 < all;) {
+            const uint32_t n = min(kMultiRoom - fill, all - p0);
+            const PageRun<T> keys(out.match.key_pages, at);
+            for (uint32_t i = lane; i < ((n + 31) & ~31u); i += 32) {
+                const uint32_t p = p0 + i;
+                uint32_t src = 0; /* the first lane whose matches end above p */
+#pragma unroll
+                for (uint32_t step = 16; step; step >>= 1)
+                    if (__shfl_sync(0xffffffffu, incl, src + step - 1) <= p) src += step;
+                const uint32_t from = __shfl_sync(0xffffffffu, place, src);
+                const typename LK::Code kc = __shfl_sync(0xffffffffu, cd, src);
+                if (i >= n) continue;
+                w.rid[fill + i] = from + p; /* the place of the build row, until the room is full */
+                w.row[fill + i] = (uint8_t)(it * 32 + src);
+                if (out.match.key_pages) __stcs(keys.at(fill + i), lk.key_of(kc));
             }
+            fill += n;
+            left -= n;
+            p0 += n;
+            if (left && fill < kMultiRoom) continue;
+            __syncwarp();
+            for (uint32_t i0 = lane; i0 < fill; i0 += 32 * kEmit) {
+                uint32_t r[kEmit];
+#pragma unroll
+                for (int k = 0; k < kEmit; ++k)
+                    if (i0 + k * 32 < fill) r[k] = __ldg(lk.rows + w.rid[i0 + k * 32]);
+#pragma unroll
+                for (int k = 0; k < kEmit; ++k)
+                    if (i0 + k * 32 < fill) w.rid[i0 + k * 32] = r[k];
+            }
+            __syncwarp();
+            emit_packed(out, plan, w, fill, at, row0);
+            __syncwarp();
+            at += fill;
+            fill = 0;
         }
     }
 }
@@ -1115,10 +1113,28 @@ template <typename T> CJ_DEV bool row_key(const ColView &c, uint32_t i, T *key) 
     return true;
 }
 
+/* The items of a step that a block takes: all, or every `of`-th where the
+ * probe rows are too few to fill the chip and each may have many matches. */
+struct Share {
+    uint32_t which = 0, of = 1; /* a power of two up to kItems */
+    CJ_DEV uint64_t block() const { return blockIdx.x / of; }
+    CJ_DEV uint64_t blocks() const { return gridDim.x / of; }
+    template <typename T, class LK> CJ_DEV void keep(const LK &lk, typename LK::Code *code, uint32_t *ok) const {
+        if (of == 1) return;
+#pragma unroll
+        for (int it = 0; it < kItems; ++it) {
+            bool in;
+            if ((it & (of - 1)) == which) continue;
+            code[it] = lk.code(T(0), false, &in);
+            *ok &= ~(1u << it);
+        }
+    }
+};
+
 /* A step over relation rows t0 ... t0 + 2047. Block-wide. */
 template <typename T, class LK, class SH>
 CJ_DEV void probe_rows(const ColView &col, uint32_t n, uint64_t t0, const LK &lk, const UniqueOut &out,
-                       const EmitPlan &plan, SH &sh, uint32_t part, uint32_t buf) {
+                       const EmitPlan &plan, SH &sh, uint32_t part, uint32_t buf, const Share &share) {
     typename LK::Code code[kItems] = {};
     uint32_t ok = 0;
     const uint64_t r0 = t0 + part * kWarpRows;
@@ -1131,21 +1147,23 @@ CJ_DEV void probe_rows(const ColView &col, uint32_t n, uint64_t t0, const LK &lk
         code[it] = lk.code(key, present, &in);
         if (LK::kMask && in) ok |= 1u << it;
     }
+    share.keep<T>(lk, code, &ok);
     probe_step<T>(lk, code, ok, (uint32_t)r0, out, plan, sh, part, buf);
 }
 
 /* The key column's pages, one a step (INT32) or two (INT64). Block-wide. */
 template <typename T, class LK, class SH>
 CJ_DEV void probe_pages(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueOut &out, const EmitPlan &plan, SH &sh,
-                        uint32_t part) {
+                        uint32_t part, const Share &share) {
     uint32_t buf = 0;
     if constexpr (kStepPages<T> == 1) {
-        for (uint64_t p = blockIdx.x; p < k.num_pages; p += gridDim.x) {
+        const uint32_t stride = share.blocks();
+        for (uint64_t p = share.block(); p < k.num_pages; p += stride) {
             const uint8_t *pg = k.col.pages + p * kPageSize;
             const uint32_t head = __ldg(reinterpret_cast<const uint32_t *>(pg));
             const uint32_t nr = head & 0xFFFFu, nv = head >> 16;
             const uint64_t rs = page_first_row(k.base, k.loc, p);
-            if (p + gridDim.x < k.num_pages) prefetch_part<T>(pg + (uint64_t)gridDim.x * kPageSize, part);
+            if (p + stride < k.num_pages) prefetch_part<T>(pg + (uint64_t)stride * kPageSize, part);
             if (nv > nr || sizeof(T) + sizeof(T) * nv + (nr + 7) / 8 > kPageSize)
                 continue; /* the index has raised the error */
             if (rs + nr > n) {
@@ -1155,15 +1173,16 @@ CJ_DEV void probe_pages(const ProbeKey &k, uint32_t n, const LK &lk, const Uniqu
             uint32_t before = 0;
             for (uint32_t s0 = 0; s0 < nr; s0 += kPageRows<T>) {
                 typename LK::Code code[kItems] = {};
-                const uint32_t ok = page_keys<T>(pg, nr, nv, s0, part, &before, lk, code, k.err);
+                uint32_t ok = page_keys<T>(pg, nr, nv, s0, part, &before, lk, code, k.err);
+                share.keep<T>(lk, code, &ok);
                 probe_step<T>(lk, code, ok, (uint32_t)rs + s0 + part * kWarpRows, out, plan, sh, part, buf);
                 buf ^= 1u;
             }
         }
     } else {
-        const uint64_t stride = (uint64_t)gridDim.x * 2;
+        const uint64_t stride = share.blocks() * 2;
         const uint32_t ppart = part % kPageParts<T>;
-        for (uint64_t p0 = (uint64_t)blockIdx.x * 2; p0 < k.num_pages; p0 += stride) {
+        for (uint64_t p0 = share.block() * 2; p0 < k.num_pages; p0 += stride) {
             const uint64_t p = p0 + part / kPageParts<T>, q = p ^ 1; /* p0 is even */
             const uint8_t *pg = k.col.pages + p * kPageSize;
             uint32_t nr = 0, nv = 0, other = 0;
@@ -1196,6 +1215,7 @@ CJ_DEV void probe_pages(const ProbeKey &k, uint32_t n, const LK &lk, const Uniqu
                         code[it] = lk.code(T(0), false, &in);
                     }
                 }
+                share.keep<T>(lk, code, &ok);
                 probe_step<T>(lk, code, ok, (uint32_t)rs + s0 + ppart * kWarpRows, out, plan, sh, part, buf);
                 buf ^= 1u;
             }
@@ -1204,16 +1224,17 @@ CJ_DEV void probe_pages(const ProbeKey &k, uint32_t n, const LK &lk, const Uniqu
 }
 
 template <bool kPages, typename T, class LK, class SH>
-CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueOut &out, SH &sh) {
+CJ_DEV void probe_all(const ProbeKey &k, uint32_t n, const LK &lk, const UniqueOut &out, SH &sh,
+                      const Share &share = Share()) {
     const EmitPlan plan(out, LK::kMask);
     const uint32_t part = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); /* warp-uniform */
     if constexpr (kPages) {
-        probe_pages<T>(k, n, lk, out, plan, sh, part);
+        probe_pages<T>(k, n, lk, out, plan, sh, part, share);
     } else {
         const ColView col = resolve_view(k.col);
         uint32_t buf = 0;
-        for (uint64_t t0 = (uint64_t)blockIdx.x * kTileRows; t0 < n; t0 += (uint64_t)gridDim.x * kTileRows) {
-            probe_rows<T>(col, n, t0, lk, out, plan, sh, part, buf);
+        for (uint64_t t0 = share.block() * kTileRows; t0 < n; t0 += share.blocks() * kTileRows) {
+            probe_rows<T>(col, n, t0, lk, out, plan, sh, part, buf, share);
             buf ^= 1u;
         }
     }
@@ -1254,23 +1275,35 @@ __global__ void __launch_bounds__(kProbeThreads, kWideBlocks)
 template <bool kPages, typename T>
 __global__ void __launch_bounds__(kProbeThreads, kMultiBlocks)
     k_probe_multi(const __grid_constant__ ProbeKey k, uint32_t n, const __grid_constant__ MultiTable t,
-                  const __grid_constant__ UniqueOut out) {
+                  const __grid_constant__ UniqueOut out, uint32_t shares) {
     __shared__ MultiShared sh;
-    probe_all<kPages, T>(k, n, MultiLookup<T>(t), out, sh);
+    probe_all<kPages, T>(k, n, MultiLookup<T>(t), out, sh, Share{blockIdx.x & (shares - 1), shares});
 }
 
 template <bool kPages, typename T>
 __global__ void __launch_bounds__(kProbeThreads, kOpenMultiBlocks)
     k_probe_open_multi(const __grid_constant__ ProbeKey k, uint32_t n, const __grid_constant__ OpenMultiTable t,
-                       const __grid_constant__ UniqueOut out) {
+                       const __grid_constant__ UniqueOut out, uint32_t shares) {
     __shared__ MultiShared sh;
-    probe_all<kPages, T>(k, n, OpenMultiLookup<T>(t), out, sh);
+    probe_all<kPages, T>(k, n, OpenMultiLookup<T>(t), out, sh, Share{blockIdx.x & (shares - 1), shares});
 }
 
 /* Steps of a probe's CTAs. */
 uint64_t probe_tiles(const ProbeKey &k, uint32_t n) {
     if (!k.base) return ((uint64_t)n + kTileRows - 1) / kTileRows;
     return k.col.type == CJ_INT32 ? k.num_pages : (k.num_pages + 1) / 2;
+}
+
+/* Blocks that share a step's rows of a probe with several matches a row: as
+ * many as the chip holds beside each other and a second wave, up to a block
+ * per item. A warp writes the matches of its 256 rows one room after the
+ * other, which few probe rows with many matches each leave to a few warps:
+ * 50K rows of 40 matches 734 us with a block per step, 290 with eight (the
+ * whole join), 300K rows of 200 matches 2938 and, with four, 1360. */
+uint32_t shares_of(uint64_t tiles, uint64_t wave) {
+    uint32_t s = 1;
+    while (s < (uint32_t)kItems && tiles * s <= wave) s *= 2;
+    return s;
 }
 
 /* Random loads in flight are held in L1: as little of it as possible goes to
@@ -1379,11 +1412,13 @@ cudaError_t launch_probe_multi(const Launch &L, const ProbeKey &k, uint32_t n, c
     if (n == 0) return cudaSuccess;
     const bool pages = k.base != nullptr;
     const uint64_t tiles = probe_tiles(k, n);
-    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * kMultiBlocks));
+    const uint64_t wave = (uint64_t)L.num_sms * kMultiBlocks;
+    const uint32_t shares = shares_of(std::max<uint64_t>(tiles, 1), wave);
+    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, wave)) * shares;
     const auto kernel = k.col.type == CJ_INT32 ? (pages ? k_probe_multi<true, int32_t> : k_probe_multi<false, int32_t>)
                                                : (pages ? k_probe_multi<true, long long> : k_probe_multi<false, long long>);
     prefer_l1(kernel);
-    kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out);
+    kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out, shares);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -1407,12 +1442,14 @@ cudaError_t launch_probe_open_multi(const Launch &L, const ProbeKey &k, uint32_t
     if (n == 0) return cudaSuccess;
     const bool pages = k.base != nullptr;
     const uint64_t tiles = probe_tiles(k, n);
-    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)L.num_sms * kOpenMultiBlocks));
+    const uint64_t wave = (uint64_t)L.num_sms * kOpenMultiBlocks;
+    const uint32_t shares = shares_of(std::max<uint64_t>(tiles, 1), wave);
+    const unsigned g = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, wave)) * shares;
     const auto kernel = k.col.type == CJ_INT32
                             ? (pages ? k_probe_open_multi<true, int32_t> : k_probe_open_multi<false, int32_t>)
                             : (pages ? k_probe_open_multi<true, long long> : k_probe_open_multi<false, long long>);
     prefer_l1(kernel);
-    kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out);
+    kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out, shares);
     count_launches(1);
     return cudaGetLastError();
 }
