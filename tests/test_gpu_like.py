@@ -52,3 +52,19 @@ def test_text_beside_other_conditions(gpu_ctx, rows, keep):
         got = gpu_filter(gpu_ctx, t, pred, [0, 1])
         assert got.num_rows == int(sel.sum())
         assert_same(got, want)
+
+
+@pytest.mark.parametrize("rows", [302_000, 610_001, 1_215_003])
+def test_rows_per_block(gpu_ctx, rows):
+    """Tables whose blocks take 256, 512 and 1,024 rows at a time."""
+    rng = np.random.default_rng(rows)
+    words = [b"", b"a", b"qz", b"aqzb", b"xxqyzz", b"a\nqz"]
+    texts = [words[k] for k in rng.integers(0, len(words), rows)]
+    t = ColumnarTable(rows, [encode_column(DataType.INT32, np.arange(rows, dtype=np.int32)),
+                             encode_column(DataType.VARCHAR, texts, (rng.random(rows) >= 0.1).astype(np.uint8))])
+    like = Comparison(1, Comparison.LIKE, "%_qz%")
+    for pred in (like, LogicalOperation.makeAnd(like, Comparison(0, Comparison.LT, rows // 3))):
+        want, sel = oa.oracle_filter(t, pred, [0])
+        got = gpu_filter(gpu_ctx, t, pred, [0])
+        assert got.num_rows == int(sel.sum())
+        assert_same(got, want)
