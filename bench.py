@@ -294,11 +294,6 @@ def algorithmic_bytes(kernel: str, st: dict, plan_info: dict):
         # build rows) once; per match 2 x 4 B row ids and the 4 B key the
         # probe emits for the root's key columns
         return npr * (4 + 1 / 8) + nb * 4 + m * 12
-    if kernel == "probe_open":
-        # probe keys (4 B + validity bit), the open-addressing table (8 B
-        # slots, 2 per build row) once; per match 2 x 4 B row ids and the
-        # 4 B key the probe emits for the root's key columns
-        return npr * (4 + 1 / 8) + nb * 2 * 8 + m * 12
     if kernel == "probe_unique" and WL["name"] in ("c2", "c2s"):
         # probe keys (4 B + validity bit) and the table once; per match the
         # probe FP64 value read and written and the 4 B key. Direct-mapped (4 B

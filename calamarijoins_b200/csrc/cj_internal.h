@@ -508,9 +508,7 @@ struct PageTask {
     int32_t finish;
     const unsigned long long *table; /* finish 2, with the table words set: also
                                         written through the row ids unless the
-                                        table is direct-mapped or, with
-                                        open_slots, open-addressing            */
-    uint32_t open_slots;
+                                        table is direct-mapped                 */
     uint32_t block_base, blocks; /* place_pages */
 };
 constexpr int kPageArgs = 24; /* tasks passed by value */

@@ -1165,7 +1165,7 @@ cj_result *Executor::materialize(const std::vector<OutCol> &cols, const std::vec
                 if (cols[c].rel) t.col = out_view(cols[c]);
                 else t.col.type = types[c];
                 t.finish = cols[c].rel ? 2 : 1;
-                if (cols[c].direct_only) t.table = ctx.d_status->table; /* open_slots 0: not beside that table */
+                if (cols[c].direct_only) t.table = ctx.d_status->table;
             } else {
                 /* decoded here, not before the loop: the kernel stream waits
                  * for a column's upload only when its pages are written */

@@ -247,8 +247,7 @@ CJ_DEV void decode_fixed_page(const uint8_t *__restrict__ pages, uint64_t p, uin
         return;
     }
     const T *vals = reinterpret_cast<const T *>(pg + DB);
-    const bool dense = nr == nv;
-    if (!dense) {
+    if (nr != nv) {
         load_page_bitmap(pg, nr, sm.bm, sm.pre, sm.wbuf);
         /* Sparse page: a thread takes 4 consecutive rows, whose non-NULL
          * values are consecutive in the page (one bitmap word and its
@@ -297,11 +296,7 @@ CJ_DEV void decode_fixed_page(const uint8_t *__restrict__ pages, uint64_t p, uin
         for (int k = 0; k < kSlabs; ++k) {
             const uint32_t i = base + k * kDecodeThreads + threadIdx.x;
             v[k] = T(0);
-            if (i < nr) {
-                const int idx = dense ? (int)i : value_index(sm.bm, sm.pre, i);
-                if (idx >= (int)nv) atomicOr(err, DEV_ERR_PAGE_HEADER); /* bitmap holds > n_values bits */
-                else if (idx >= 0) v[k] = __ldcs(vals + idx);
-            }
+            if (i < nr) v[k] = __ldcs(vals + i);
         }
 #pragma unroll
         for (int k = 0; k < kSlabs; ++k) {
@@ -309,7 +304,7 @@ CJ_DEV void decode_fixed_page(const uint8_t *__restrict__ pages, uint64_t p, uin
             if (i < nr) values[rs + i] = v[k];
         }
     }
-    write_validity(dense, sm.bm, nr, rs, valid);
+    write_validity(true, sm.bm, nr, rs, valid);
     __syncthreads();
 }
 

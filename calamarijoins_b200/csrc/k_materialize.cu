@@ -245,7 +245,7 @@ CJ_DEV void write_page_blocks(const PageTask &T, uint32_t b, PageSmem &sm) {
     const uint32_t R = rows_per_page_dev(T.col.type);
     const uint64_t num_pages = (rows + R - 1) / R;
     if (b >= num_pages) return;
-    if (T.finish == 1 || (T.finish == 2 && col_null_free(T.col) && !(T.table && !table_kind(T.table, T.open_slots)))) {
+    if (T.finish == 1 || (T.finish == 2 && col_null_free(T.col) && !(T.table && !table_kind(T.table, 0)))) {
         constexpr uint32_t kWarps = kMatThreads / 32;
         for (uint64_t pg = b * kWarps + (threadIdx.x >> 5); pg < num_pages; pg += (uint64_t)T.blocks * kWarps) {
             if (T.col.type == CJ_INT32) finish_dense_page<int32_t>(T.out, rows, pg);
