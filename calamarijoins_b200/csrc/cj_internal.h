@@ -355,11 +355,27 @@ struct EmitColumn {
                             not stay in L2 together                       */
 };
 constexpr int kEmitColumns = 8;
+/* A probe of repeated keys leaves the matches of a row with kRunFrom build
+ * rows or more to a kernel that follows it: runs of at most kRunRows of them.
+ * Room for capacity / kRunFrom runs is enough: one has that many matches at
+ * least, on the mean of its row's. */
+constexpr uint32_t kRunFrom = 64, kRunRows = 960;
+struct alignas(16) MatchRun {
+    int64_t key;
+    uint32_t rows, count; /* place in the table's `rows`, matches */
+    uint32_t at, probe;   /* first output position, probe row     */
+};
+struct RunList {
+    MatchRun *runs = nullptr; /* null: written by the probe itself */
+    unsigned long long *count = nullptr; /* zero before the probe */
+    uint64_t capacity = 0;
+};
 struct UniqueOut {
     MatchOut match;      /* capacity: at least the probe rows         */
     bool need_b, need_p; /* match row ids wanted whatever the columns */
     int n;
     EmitColumn cols[kEmitColumns];
+    RunList runs; /* of a probe of repeated keys */
 };
 /* Probe of a unique table; does nothing when the table is unusable. The
  * match counter must be zero before. */

@@ -25,7 +25,8 @@
  * Keys that repeat get a table of their own (a count, and the row or where
  * the key's rows lie: per value of a dense range, launch_multi_build, else in
  * an open-addressing slot per key, launch_open_multi_build) and the same probe
- * with room for several matches a row.
+ * with room for several matches a row; rows with many are listed and written
+ * by a kernel of their own (k_match_runs).
  *
  * Bound: requests from L1 to L2, about one per clock and SM whatever their
  * size (every random slot or value is one), then the 128-byte lines of L1
@@ -867,7 +868,8 @@ CJ_DEV void probe_step(const LK &lk, const typename LK::Code *code, uint32_t ok,
  * with up to three are packed and written together, in three parts where they
  * outnumber the room; those of rows with more are listed 32 a step, whichever
  * rows they are of, and written whenever the room is full: all lanes then have
- * loads in flight however many rows the matches come from. (In rounds of the
+ * loads in flight however many rows the matches come from. Rows with kRunFrom
+ * or more are only listed where there is a list (RunList). (In rounds of the
  * j-th matches and, from 33 on, row by row, the 24M matches of 300K x 3M rows,
  * eight a key, took 808 us, 685 so; the whole join, the hash table 1133.)
  * 64M x 4M rows over 3M keys, 58.6M matches: 877 us with one result column of
@@ -951,6 +953,18 @@ template <typename T> struct OpenMultiLookup {
         }
     }
 };
+
+/* Lists a row's n matches as runs, for k_match_runs. */
+CJ_DEV void list_runs(const RunList &l, int64_t key, uint32_t rows, uint32_t n, uint32_t at, uint32_t probe) {
+    const uint32_t runs = (n + kRunRows - 1) / kRunRows;
+    unsigned long long first = 0;
+    if (lane_id() == 0) first = atomicAdd(l.count, (unsigned long long)runs);
+    first = __shfl_sync(0xffffffffu, first, 0);
+    for (uint32_t k = lane_id(); k < runs && first + k < l.capacity; k += 32) {
+        const uint32_t q = k * kRunRows;
+        l.runs[first + k] = {key, rows + q, min(kRunRows, n - q), at + q, probe};
+    }
+}
 
 /* The lanes' items of one packing: item `it`'s matches go to places first(it)
  * on, `count(it)` of them (at most three); the packed total is returned. */
@@ -1057,9 +1071,19 @@ CJ_DEV void probe_step(const LK &lk, const typename LK::Code *code, uint32_t ok,
                 cd = code[q];
             }
         if (c <= 3) c = 0;
+        if (out.runs.runs) {
+            for (uint32_t heavy = __ballot_sync(0xffffffffu, c >= kRunFrom); heavy; heavy &= heavy - 1) {
+                const int src = __ffs(heavy) - 1;
+                const uint32_t n = __shfl_sync(0xffffffffu, c, src);
+                left -= n;
+                list_runs(out.runs, (int64_t)lk.key_of(__shfl_sync(0xffffffffu, cd, src)),
+                          __shfl_sync(0xffffffffu, lo, src) - n, n, at + fill + left, row0 + it * 32 + src);
+            }
+            if (c >= kRunFrom) c = 0;
+        }
         const uint32_t incl = warp_inclusive_scan(c), all = __shfl_sync(0xffffffffu, incl, 31);
         const uint32_t place = lo - incl; /* of match p of the item's: place + p */
-        for (uint32_t p0 = 0; p0 < all;) {
+        for (uint32_t p0 = 0; p0 < all || (fill && !left);) { /* the last matches may have been listed before */
             const uint32_t n = min(kMultiRoom - fill, all - p0);
             const PageRun<T> keys(out.match.key_pages, at);
             for (uint32_t i = lane; i < ((n + 31) & ~31u); i += 32) {
@@ -1272,6 +1296,62 @@ __global__ void __launch_bounds__(kProbeThreads, kWideBlocks)
     if (refused == kTableSpread && t.open_slots) probe_all<kPages, T>(k, n, WideLookup<T>(t), out, sh);
 }
 
+/* The matches that a probe of repeated keys listed as runs (list_runs), a
+ * warp a run: the build rows come from the table's `rows` side by side, the
+ * probe row is one for all of them. 60M matches of 400 a row, 5M x 300K INT64
+ * rows of which 3 % match: 1482 us with the probe writing them from its room,
+ * whose listing takes seven warp instructions a match, 870 so. A kernel of its
+ * own, because these loops beside the probe's spill its registers (64M x 4M
+ * rows, at most two matches a row: 1166 us with them, 1007 without). */
+template <typename T>
+CJ_DEV void emit_run_column(const EmitColumn &c, bool direct, const uint32_t *rows, const MatchRun &run) {
+    const PageRun<T> out(c.pages, run.at); /* of one page or two: kRunRows fit one */
+    const auto value = [&](uint32_t r) {
+        if (c.col.rid_b) r = __ldg(c.col.rid_b + r);
+        return direct ? page_value<T>(c.col.pages, r) : __ldg(reinterpret_cast<const T *>(c.col.values) + r);
+    };
+    if (!c.from_build) {
+        const T v = value(run.probe);
+        for (uint32_t i = lane_id(); i < run.count; i += 32) __stcs(out.at(i), v);
+        return;
+    }
+    constexpr int kFlight = 4;
+    for (uint32_t i0 = lane_id(); i0 < run.count; i0 += 32 * kFlight) {
+        T v[kFlight];
+#pragma unroll
+        for (int j = 0; j < kFlight; ++j)
+            if (i0 + j * 32 < run.count) v[j] = value(__ldg(rows + run.rows + i0 + j * 32));
+#pragma unroll
+        for (int j = 0; j < kFlight; ++j)
+            if (i0 + j * 32 < run.count) __stcs(out.at(i0 + j * 32), v[j]);
+    }
+}
+template <typename T>
+__global__ void __launch_bounds__(kProbeThreads) k_match_runs(const uint32_t *rows, const __grid_constant__ UniqueOut out) {
+    static_assert(kRunRows <= PageRun<T>::R && kRunRows <= PageRun<long long>::R, "a run ends on the next page at most");
+    const uint64_t n = min((uint64_t)*out.runs.count, out.runs.capacity);
+    if (blockIdx.x * (uint64_t)kParts >= n) return;
+    const EmitPlan plan(out, false);
+    for (uint64_t k = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32; k < n; k += (uint64_t)gridDim.x * blockDim.x / 32) {
+        const MatchRun run = out.runs.runs[k];
+        const uint32_t lane = lane_id();
+        if (out.match.key_pages) {
+            const PageRun<T> keys(out.match.key_pages, run.at);
+            for (uint32_t i = lane; i < run.count; i += 32) __stcs(keys.at(i), (T)run.key);
+        }
+        for (uint32_t i = lane; plan.want_b && i < run.count; i += 32)
+            __stcs(out.match.build_rids + run.at + i, __ldg(rows + run.rows + i));
+        for (uint32_t i = lane; plan.want_p && i < run.count; i += 32)
+            __stcs(out.match.probe_rids + run.at + i, run.probe);
+        for (int c = 0; c < out.n; ++c) {
+            if (!((plan.active >> c) & 1u)) continue;
+            const EmitColumn &e = out.cols[c];
+            if (e.col.type == CJ_INT32) emit_run_column<int32_t>(e, (plan.direct >> c) & 1u, rows, run);
+            else emit_run_column<long long>(e, (plan.direct >> c) & 1u, rows, run);
+        }
+    }
+}
+
 template <bool kPages, typename T>
 __global__ void __launch_bounds__(kProbeThreads, kMultiBlocks)
     k_probe_multi(const __grid_constant__ ProbeKey k, uint32_t n, const __grid_constant__ MultiTable t,
@@ -1325,6 +1405,17 @@ template <class K> void prefer_l1(K kernel) {
         slot.store(reinterpret_cast<const void *>(kernel), std::memory_order_release);
         return;
     }
+}
+
+/* After a probe that lists runs: their matches. */
+cudaError_t launch_runs(const Launch &L, int32_t key_type, const uint32_t *rows, const UniqueOut &out) {
+    if (!out.runs.runs || !out.runs.capacity) return cudaSuccess;
+    const unsigned g = (unsigned)std::min<uint64_t>((out.runs.capacity + kParts - 1) / kParts, (uint64_t)L.num_sms * 4);
+    const auto kernel = key_type == CJ_INT32 ? k_match_runs<int32_t> : k_match_runs<long long>;
+    prefer_l1(kernel);
+    kernel<<<g, kProbeThreads, 0, L.stream>>>(rows, out);
+    count_launches(1);
+    return cudaGetLastError();
 }
 
 } // namespace
@@ -1420,7 +1511,8 @@ cudaError_t launch_probe_multi(const Launch &L, const ProbeKey &k, uint32_t n, c
     prefer_l1(kernel);
     kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out, shares);
     count_launches(1);
-    return cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? launch_runs(L, k.col.type, t.rows, out) : e;
 }
 
 cudaError_t launch_open_multi_build(const Launch &L, const ColView &key, uint32_t n, const OpenMultiTable &t) {
@@ -1451,7 +1543,8 @@ cudaError_t launch_probe_open_multi(const Launch &L, const ProbeKey &k, uint32_t
     prefer_l1(kernel);
     kernel<<<g, kProbeThreads, 0, L.stream>>>(k, n, t, out, shares);
     count_launches(1);
-    return cudaGetLastError();
+    const cudaError_t e = cudaGetLastError();
+    return e == cudaSuccess ? launch_runs(L, k.col.type, t.rows, out) : e;
 }
 
 } // namespace cj

@@ -5,7 +5,7 @@ probe side and by two, four and eight (few probe rows)."""
 import numpy as np
 import pytest
 
-from calamarijoins_b200 import DataType
+from calamarijoins_b200 import ColumnarTable, DataType, Plan, ResidentTable, _lib, encode_column
 from tests.helpers import assert_same, run_oracle, run_product
 from tests.test_gpu_unique import _check, _plan
 
@@ -46,3 +46,65 @@ def test_blocks_per_step(gpu_ctx, n, gap):
     want = run_oracle(plan)
     got, st = run_product(plan, gpu_ctx)
     assert_same(got, want, f"{n} probe rows")
+
+
+def _resident_run(plan, ctx, flags=0):
+    rp = Plan()
+    rp.nodes, rp.root = plan.nodes, plan.root
+    rp.inputs = [ResidentTable(ctx, t) for t in plan.inputs]
+    try:
+        return run_product(rp, ctx, flags)[0]
+    finally:
+        for t in rp.inputs:
+            t.free()
+
+
+@pytest.mark.parametrize("pay", ["dense", "nulls"])
+@pytest.mark.parametrize("kt,pt,gap", [(I, I, 1), (I, L, 10 ** 5), (L, L, 1), (L, I, 1000)])
+@pytest.mark.parametrize("counts", [[63, 64, 65], [959, 960, 961, 1], [1919, 1920, 1921, 4, 5], [5000, 63, 2], [64]])
+def test_runs(gpu_ctx, counts, kt, pt, gap, pay):
+    """Matches that a kernel of their own writes (64 a row or more, 960 a
+    run), beside rows of fewer: into pages and, with NULLs, as row ids."""
+    rng = np.random.default_rng(len(counts))
+    keys, bkeys = _build(rng, counts * 3, gap)
+    bkeys -= gap  # a negative key too
+    n = max(4 * len(bkeys), 65_536)  # room for fewer: the probe writes them itself
+    pkeys = np.full(n, 10 ** 8)
+    hit = rng.permutation(n)[:40]
+    pkeys[hit] = keys[rng.integers(0, len(keys), 40)] - gap
+    ok = (lambda rows: (rng.random(rows) >= 0.2).astype(np.uint8)) if pay == "nulls" else (lambda rows: None)
+    plan = _plan(bkeys, pkeys, kt, pt, pvalid=(rng.random(n) >= 0.02).astype(np.uint8),
+                 bpay=[(L, np.arange(len(bkeys)), ok(len(bkeys))), (I, np.arange(len(bkeys)), None)],
+                 ppay=[(F, np.arange(n) / 4, ok(n)), (I, np.arange(n), None)])
+    want = run_oracle(plan)
+    for flags in (0, _lib.CJ_EXEC_RESULT_ON_DEVICE):
+        assert_same(_resident_run(plan, gpu_ctx, flags), want, f"{counts}")
+
+
+@pytest.mark.parametrize("gap", [1, 10 ** 5])
+def test_runs_below_the_root(gpu_ctx, gap):
+    """Runs of an intermediate's row ids, and of a probe side and a build side
+    that are intermediates."""
+    rng = np.random.default_rng(3)
+    keys, bkeys = _build(rng, [1, 70, 1000, 3], gap)
+    many = ColumnarTable(len(bkeys), [encode_column(I, bkeys.astype(np.int32)), encode_column(L, np.arange(len(bkeys)))])
+    n = 100_000
+    fk = np.where(rng.random(n) < 0.005, keys[rng.integers(0, len(keys), n)], -9)
+    fact = ColumnarTable(n, [encode_column(I, np.arange(n, dtype=np.int32)), encode_column(I, fk.astype(np.int32)),
+                             encode_column(F, rng.random(n))])
+    ids = rng.permutation(n)[:95_000]
+    some = ColumnarTable(95_000, [encode_column(I, ids.astype(np.int32)), encode_column(I, (ids * 3).astype(np.int32))])
+    plan = Plan()
+    plan.inputs = [many, fact, some]
+    s = [plan.new_scan_node(0, [(0, I), (1, L)]), plan.new_scan_node(1, [(0, I), (1, I), (2, F)]),
+         plan.new_scan_node(2, [(0, I), (1, I)])]
+    j = plan.new_join_node(True, s[0], s[1], 0, 1, [(2, I), (1, L), (3, I), (4, F)])  # below the root
+    plan.root = plan.new_join_node(True, j, s[2], 0, 0, [(0, I), (1, L), (2, I), (3, F), (5, I)])
+    assert_same(_resident_run(plan, gpu_ctx), run_oracle(plan), "below")
+    plan = Plan()
+    plan.inputs = [many, fact, some]
+    s = [plan.new_scan_node(0, [(0, I), (1, L)]), plan.new_scan_node(1, [(0, I), (1, I), (2, F)]),
+         plan.new_scan_node(2, [(0, I), (1, I)])]
+    j = plan.new_join_node(True, s[1], s[2], 0, 0, [(1, I), (2, F), (4, I)])
+    plan.root = plan.new_join_node(True, s[0], j, 0, 0, [(0, I), (1, L), (2, I), (3, F), (4, I)])
+    assert_same(_resident_run(plan, gpu_ctx), run_oracle(plan), "probe side")
