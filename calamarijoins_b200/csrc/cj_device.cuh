@@ -47,10 +47,24 @@ CJ_DEV uint32_t open_slot(int64_t key, uint32_t nslots) {
     return __umulhi((uint32_t)key * 0x9E3779B9u, nslots);
 }
 
-/* The same for INT64 keys, the high word folded in as in hash_key. */
-CJ_DEV uint32_t open_slot_wide(int64_t key, uint32_t nslots) {
-    const uint32_t m = (uint32_t)key ^ ((uint32_t)((uint64_t)key >> 32) * 0x2545F491u);
-    return __umulhi((m ^ (m >> 15)) * 0x9E3779B9u, nslots);
+/* Open-addressing tables of 16-byte slots: groups of eight slots and a tag byte
+ * per slot, 0 where it is empty, else 0x80 | seven bits of its key's hash. One
+ * 8-byte load of a group's tags says whether a key may be there, and in which
+ * slot; a key lies in a later group only if the earlier ones are full. The
+ * high word is folded in as in hash_key. */
+struct TagHash {
+    uint32_t group, tag, first; /* the slot of its group that it tries first */
+};
+CJ_DEV TagHash tag_hash(int64_t key, uint32_t groups) {
+    const uint32_t m = (uint32_t)key ^ ((uint32_t)((uint64_t)key >> 32) * 0x2545F491u), x = m ^ (m >> 15);
+    const uint32_t b = x * 0x85EBCA77u;
+    return {__umulhi(x * 0x9E3779B9u, groups), 0x80u | (b >> 25), (b >> 22) & 7u};
+}
+/* The slot that an insert tries at its step `step` (below the slots). */
+CJ_DEV uint32_t tagged_slot(const TagHash &h, uint32_t step, uint32_t groups) {
+    uint32_t g = h.group + step / 8;
+    if (g >= groups) g -= groups;
+    return g * 8 + ((h.first + step) & 7u);
 }
 
 /* Loads the 2048-entry Bloom tag table into shared memory. */

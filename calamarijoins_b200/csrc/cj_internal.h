@@ -232,9 +232,9 @@ cudaError_t launch_columns_grouped(const Launch &L, const ColumnTask *tasks_dev,
 
 /* Table of unique build keys (k_unique.cu): direct-mapped when their range is
  * at most max_span, else (open_slots > 0) open-addressing, with 8-byte slots
- * for INT32 keys and 16-byte ones for INT64 keys (wide). `slots` holds
+ * for INT32 keys and, for INT64 keys (wide), 16-byte ones and a tag byte each. `slots` holds
  * unique_table_bytes, 16-byte aligned; open_slots is at least twice the build
- * rows. `params` (kTableWords words, zero before the build) receives what the
+ * rows and a multiple of 16. `params` (kTableWords words, zero before the build) receives what the
  * device found. */
 constexpr uint32_t kArrayEmpty = 0xFFFFFFFFu;
 constexpr uint64_t kOpenMaxRows = 1ull << 28;
@@ -271,7 +271,7 @@ struct UniqueTable {
     uint32_t wide;       /* 16-byte slots: INT64 build keys */
 };
 inline uint64_t unique_table_bytes(const UniqueTable &t) {
-    const uint64_t direct = t.max_span * 4, open = (uint64_t)t.open_slots * (t.wide ? 16 : 8);
+    const uint64_t direct = t.max_span * 4, open = (uint64_t)t.open_slots * (t.wide ? 17 : 8); /* wide: tags last */
     return ((direct > open ? direct : open) + 15) & ~15ull;
 }
 /* What the params say (host copy or device): 0 unusable, 1 direct-mapped,
@@ -411,7 +411,8 @@ struct OpenMultiTable {
     unsigned long long *found;   /* kMultiWords words                       */
     unsigned long long lo, width, empty; /* smallest key, largest - smallest,
                                     the key of an empty slot                */
-    uint32_t nslots;             /* at least twice the build rows           */
+    uint32_t nslots;             /* at least twice the build rows, a multiple of 8 */
+    uint8_t *tags;               /* nslots, zero before the build           */
 };
 enum MultiWord {
     kMultiKeys = 0,   /* different keys                                      */

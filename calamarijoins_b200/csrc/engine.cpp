@@ -694,13 +694,13 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                  * host learns it at the probe's own synchronisation and then,
                  * if neither, builds another. Direct-mapped: 4 bytes per
                  * slot, at 8 x rows 32 B per build row, at most 2^28 slots (1
-                 * GiB); open-addressing: 16 B per build row, 32 for INT64
+                 * GiB); open-addressing: 16 B per build row, 34 for INT64
                  * keys, left out where the memory is short. One buffer serves
                  * both. */
                 table.max_span = std::min<uint64_t>((uint64_t)ctx.opt.dense_keys * B.rows, 1ull << 28);
                 table.wide = bk.type == CJ_INT64;
-                const uint64_t open_slots = std::max<uint64_t>(2 * B.rows, 1024);
-                if (B.rows <= kOpenMaxRows && ample(open_slots * (table.wide ? 16 : 8)))
+                const uint64_t open_slots = std::max<uint64_t>((2 * B.rows + 15) & ~15ull, 1024);
+                if (B.rows <= kOpenMaxRows && ample(open_slots * (table.wide ? 17 : 8)))
                     table.open_slots = (uint32_t)open_slots;
                 table.params = ctx.d_status->table;
                 if (table.open_slots && !(slots = spare(unique_table_bytes(table)))) table.open_slots = 0;
@@ -902,9 +902,9 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             slots.reset();
             multi_rows.reset();
             DevPtr slot_of;
-            const uint32_t open_n = (uint32_t)std::max<uint64_t>(2 * std::min(B.rows, kOpenMaxRows), 1024);
+            const uint32_t open_n = (uint32_t)std::max<uint64_t>((2 * std::min(B.rows, kOpenMaxRows) + 7) & ~7ull, 1024);
             if (tp[kTableRefused] != kTableWhole && B.rows <= kOpenMaxRows && P.rows / kOpenMultiProbe >= B.rows &&
-                ample(B.rows * (2 * sizeof(MultiSlot) + 8)) && (slots = spare(open_n * sizeof(MultiSlot))) &&
+                ample(B.rows * (2 * (sizeof(MultiSlot) + 1) + 8)) && (slots = spare(open_n * (sizeof(MultiSlot) + 1))) &&
                 (multi_rows = spare(B.rows * 4)) && (slot_of = spare(B.rows * 4))) {
                 open_table.nslots = open_n;
                 open_table.lo = tp[kTableLo];
@@ -912,6 +912,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 open_table.empty = tp[kTableEmpty];
                 open_table.found = ctx.d_status->table;
                 open_table.slots = slots->as<MultiSlot>();
+                open_table.tags = slots->as<uint8_t>() + open_n * sizeof(MultiSlot);
                 open_table.rows = multi_rows->as<uint32_t>();
                 open_table.slot_of = slot_of->as<uint32_t>();
                 clear_join_words();

@@ -1,12 +1,13 @@
 /*
- * k_unique.cu — joins over unique build keys, and over repeated ones of a
- * dense range: the tables' builds and a probe that reads the key column's
- * pages and writes the result's pages.
+ * k_unique.cu — joins over unique build keys, and over repeated ones: the
+ * tables' builds and a probe that reads the key column's pages and writes the
+ * result's pages.
  *
  * The table (launch_unique_build) is direct-mapped when the keys lie densely
- * (slots[key - lo] = build row), else open-addressing (slots of 8 bytes, key
- * << 32 | build row, or for INT64 keys of 16, key and build row; linear
- * probing from the key's hash, at most half full). Which one, and whether the keys are unique at all, is
+ * (slots[key - lo] = build row), else open-addressing, at most half full
+ * (slots of 8 bytes, key << 32 | build row, and linear probing from the key's
+ * hash; for INT64 keys of 16 bytes, key and build row, in groups of eight with
+ * a tag byte per slot). Which one, and whether the keys are unique at all, is
  * decided on the device: `params` says so to the kernels that follow and,
  * at the next synchronisation, to the host. Both kinds share one buffer.
  *
@@ -31,7 +32,7 @@
  * Bound: requests from L1 to L2, about one per clock and SM whatever their
  * size (every random slot or value is one), then the 128-byte lines of L1
  * that the requests in flight hold. 64M x 4M rows, 43.9M matches, two
- * 8-byte result columns, direct-mapped: 605 us, where decode, probe and
+ * 8-byte result columns, direct-mapped: 580 us, where decode, probe and
  * page writers took 945 us (152 + 390 + 403).
  */
 #include <algorithm>
@@ -122,10 +123,15 @@ struct alignas(16) WideSlot {
     uint32_t rid, pad;
 };
 
-/* Empty slots are all ones, but for wide ones, whose key is kTableEmpty. */
+CJ_DEV uint8_t *wide_tags(const UniqueTable &t) {
+    return reinterpret_cast<uint8_t *>(t.slots) + (uint64_t)t.open_slots * sizeof(WideSlot);
+}
+
+/* Empty slots are all ones, but for wide ones, whose key is kTableEmpty; their
+ * tags are 0. */
 CJ_DEV uint64_t table_bytes(const UniqueTable &t) {
     const unsigned long long refused = t.params[kTableRefused];
-    if (refused == kTableSpread) return (uint64_t)t.open_slots * (t.wide ? 16 : 8);
+    if (refused == kTableSpread) return (uint64_t)t.open_slots * (t.wide ? 17 : 8);
     return refused ? 0ull : t.params[kTableSpan] * 4ull;
 }
 CJ_DEV void fill_table(const UniqueTable &t, uint64_t first, uint64_t stride) {
@@ -135,7 +141,10 @@ CJ_DEV void fill_table(const UniqueTable &t, uint64_t first, uint64_t stride) {
         empty.x = (uint32_t)t.params[kTableEmpty];
         empty.y = (uint32_t)(t.params[kTableEmpty] >> 32);
     }
-    for (uint64_t i = first; i < n16; i += stride) reinterpret_cast<uint4 *>(t.slots)[i] = empty;
+    const bool open = t.params[kTableRefused] == kTableSpread;
+    const uint64_t tags = open && t.wide ? (uint64_t)t.open_slots : n16; /* where they begin */
+    for (uint64_t i = first; i < n16; i += stride)
+        reinterpret_cast<uint4 *>(t.slots)[i] = i < tags ? empty : make_uint4(0u, 0u, 0u, 0u);
 }
 
 /* The keys repeat, or pile up. Written once, or nearly: thousands of stores
@@ -181,13 +190,15 @@ CJ_DEV void insert_rows(const ColView &key, const UniqueTable &t, uint64_t first
             if (*reinterpret_cast<volatile unsigned long long *>(t.params + kTableDup)) return;
             int64_t k;
             if (!load_key(key, (uint32_t)i, &k)) continue;
-            uint32_t h = open_slot_wide(k, t.open_slots);
+            const TagHash h = tag_hash(k, t.open_slots / 8);
             for (uint32_t step = 0;; ++step) {
-                unsigned long long cur = __ldcg(&slots[h].key);
+                const uint32_t at = tagged_slot(h, step, t.open_slots / 8);
+                unsigned long long cur = __ldcg(&slots[at].key);
                 if (cur == empty) {
-                    cur = atomicCAS(&slots[h].key, empty, (unsigned long long)k);
+                    cur = atomicCAS(&slots[at].key, empty, (unsigned long long)k);
                     if (cur == empty) {
-                        slots[h].rid = (uint32_t)i;
+                        slots[at].rid = (uint32_t)i;
+                        wide_tags(t)[at] = (uint8_t)h.tag;
                         break;
                     }
                 }
@@ -195,7 +206,6 @@ CJ_DEV void insert_rows(const ColView &key, const UniqueTable &t, uint64_t first
                     flag_once(t.params + kTableDup);
                     break;
                 }
-                if (++h == t.open_slots) h = 0;
             }
         }
         return;
@@ -386,11 +396,14 @@ __global__ void __launch_bounds__(kUniqueThreads) k_multi_scatter(ColView key_ar
 __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_fill(OpenMultiTable t) {
     const uint4 empty = make_uint4((uint32_t)t.empty, (uint32_t)(t.empty >> 32), 0u, 0u);
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < t.nslots; i += stride)
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < t.nslots; i += stride) {
         reinterpret_cast<uint4 *>(t.slots)[i] = empty;
+        t.tags[i] = 0;
+    }
 }
 __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_claim(ColView key_arg, uint32_t n, OpenMultiTable t) {
     const ColView key = resolve_view(key_arg);
+    const uint32_t groups = t.nslots / 8;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += stride * kUniqueRows) {
         unsigned long long k[kUniqueRows], cur[kUniqueRows];
@@ -402,24 +415,27 @@ __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_claim(ColView key
         }
 #pragma unroll
         for (int q = 0; q < kUniqueRows; ++q)
-            cur[q] = k[q] != t.empty ? __ldcg(&t.slots[open_slot_wide((int64_t)k[q], t.nslots)].key) : t.empty;
+            cur[q] = k[q] != t.empty ? __ldcg(&t.slots[tagged_slot(tag_hash((int64_t)k[q], groups), 0, groups)].key) : t.empty;
 #pragma unroll
         for (int q = 0; q < kUniqueRows; ++q) {
             uint32_t at = ~0u;
             if (k[q] != t.empty) {
-                uint32_t h = open_slot_wide((int64_t)k[q], t.nslots);
+                const TagHash h = tag_hash((int64_t)k[q], groups);
                 unsigned long long c = cur[q];
                 for (uint32_t step = 0; step <= kMaxWalk; ++step) {
+                    const uint32_t s = tagged_slot(h, step, groups);
+                    if (step) c = __ldcg(&t.slots[s].key); /* slots only fill: a full one is final */
                     if (c == t.empty) {
-                        c = atomicCAS(&t.slots[h].key, t.empty, k[q]);
-                        if (c == t.empty) c = k[q];
+                        c = atomicCAS(&t.slots[s].key, t.empty, k[q]);
+                        if (c == t.empty) {
+                            c = k[q];
+                            t.tags[s] = (uint8_t)h.tag;
+                        }
                     }
                     if (c == k[q]) {
-                        at = h;
+                        at = s;
                         break;
                     }
-                    if (++h == t.nslots) h = 0;
-                    c = __ldcg(&t.slots[h].key); /* slots only fill: a full one is final */
                 }
                 if (at != ~0u) atomicAdd(&t.slots[at].count, 1u);
                 else flag_once(t.found + kMultiGaveUp);
@@ -482,7 +498,9 @@ __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_scatter(uint32_t 
  * registers 619, six with 40 (spills) 620. */
 constexpr int kProbeBlocks = 5;
 constexpr int kWideBlocks = 4; /* 64 registers: the codes are 64-bit keys */
-constexpr int kOpenMultiBlocks = 3; /* 80 registers; four with 64: 1291 us where three take 1277 (INT64 keys, below) */
+/* 80 registers; four with 64, more of them spilled: 1347 us where three take
+ * 1314 (30M x 3M INT32 rows, all matching). */
+constexpr int kOpenMultiBlocks = 3;
 constexpr int kMultiBlocks = 4; /* 64 registers; three with 80 1467 us, five with 48 2343 */
 constexpr int kItems = 8;                              /* rows per lane and step       */
 constexpr int kProbeThreads = 2048 / kItems;
@@ -576,45 +594,94 @@ template <typename T> struct OpenLookup {
     }
 };
 
-/* The same over INT64 build keys: a slot is one 16-byte load. */
+/* Lookups in a table of tagged 16-byte slots: the tags of all of a lane's rows
+ * in flight together, then the slots that they point to, four rows' at a time
+ * (16 registers). What is left, a tag that another key shares (one in 128 per
+ * key of the group) or a full group, goes group by group. Bound by the random
+ * accesses, one for a row without a match and two for one with. Walking the
+ * slots to an empty one instead, unique INT64 keys: 30M probe rows over 3M
+ * keys, 97 % of them in the range but no key, 803 us, 416 with tags; 10 % of
+ * them outside it 619 and 605; 5M rows over 300K keys 125 and 118. */
+struct TaggedTable {
+    const ulonglong2 *slots; /* key, payload */
+    const unsigned long long *tags;
+    uint32_t groups;
+    CJ_DEV unsigned long long load_tags(uint32_t g) const { return __ldg(tags + g); }
+    CJ_DEV ulonglong2 load(uint32_t s) const { return __ldg(slots + s); }
+    /* bytes of `w` that may be the tag: their high bits (a byte above a true
+     * one may be set too) */
+    CJ_DEV static unsigned long long may_be(unsigned long long w, uint32_t tag) {
+        const unsigned long long x = w ^ (tag * 0x0101010101010101ull);
+        return (x - 0x0101010101010101ull) & ~x & 0x8080808080808080ull;
+    }
+    CJ_DEV static bool has_empty(unsigned long long w) { return (~w & 0x8080808080808080ull) != 0; }
+    CJ_DEV static uint32_t first(unsigned long long m) { return (uint32_t)(__ffsll((long long)m) - 1) >> 3; }
+    template <class P> CJ_DEV void walk(int64_t key, P put) const {
+        const TagHash h = tag_hash(key, groups);
+        uint32_t g = h.group;
+        for (uint32_t k = 0; k < groups; ++k) {
+            const unsigned long long w = load_tags(g);
+            for (unsigned long long m = may_be(w, h.tag); m; m &= m - 1) {
+                const ulonglong2 v = load(g * 8 + first(m));
+                if (v.x == (unsigned long long)key) {
+                    put(v.y);
+                    return;
+                }
+            }
+            if (has_empty(w)) return;
+            if (++g == groups) g = 0;
+        }
+    }
+    /* put(it, payload) for each row whose key is there */
+    template <typename T, class P> CJ_DEV void find(const T *c, uint32_t ok, P put) const {
+#pragma unroll
+        for (int it = 0; it < kItems; it += 4) {
+            unsigned long long w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                w[j] = 0;
+                if ((ok >> (it + j)) & 1u) w[j] = load_tags(tag_hash((int64_t)c[it + j], groups).group);
+            }
+            ulonglong2 v[4];
+            uint32_t some = 0, more = 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const TagHash h = tag_hash((int64_t)c[it + j], groups);
+                const unsigned long long m = may_be(w[j], h.tag);
+                if (m) {
+                    v[j] = load(h.group * 8 + first(m));
+                    some |= 1u << j;
+                }
+                if ((m & (m - 1)) || (((ok >> (it + j)) & 1u) && !has_empty(w[j]))) more |= 1u << j;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (((some >> j) & 1u) && v[j].x == (unsigned long long)(int64_t)c[it + j]) put(it + j, v[j].y);
+                else if ((more >> j) & 1u) walk((int64_t)c[it + j], [&](unsigned long long y) { put(it + j, y); });
+            }
+        }
+    }
+};
+
+/* Open addressing over INT64 build keys. */
 template <typename T> struct WideLookup {
-    const WideSlot *slots;
-    uint32_t nslots;
-    unsigned long long lo, width, empty;
+    TaggedTable t;
+    unsigned long long lo, width;
     using Code = T;
     static constexpr bool kMask = true;
-    CJ_DEV WideLookup(const UniqueTable &t)
-        : slots(reinterpret_cast<const WideSlot *>(t.slots)), nslots(t.open_slots), lo(t.params[kTableLo]),
-          width(t.params[kTableSpan] - 1), empty(t.params[kTableEmpty]) {}
+    CJ_DEV WideLookup(const UniqueTable &u)
+        : t{reinterpret_cast<const ulonglong2 *>(u.slots), reinterpret_cast<const unsigned long long *>(wide_tags(u)),
+            u.open_slots / 8},
+          lo(u.params[kTableLo]), width(u.params[kTableSpan] - 1) {}
     CJ_DEV T code(T key, bool present, bool *in) const {
         *in = present && (unsigned long long)(int64_t)key - lo <= width;
         return key;
     }
     CJ_DEV T key_of(T c) const { return c; }
-    CJ_DEV ulonglong2 slot(uint32_t h) const { return __ldg(reinterpret_cast<const ulonglong2 *>(slots + h)); }
     CJ_DEV void find(const T *c, uint32_t ok, uint32_t *rid) const {
 #pragma unroll
-        for (int it = 0; it < kItems; it += 4) { /* four rows' slots in flight: 16 registers */
-            ulonglong2 v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                v[j].x = empty;
-                if ((ok >> (it + j)) & 1u) v[j] = slot(open_slot_wide(c[it + j], nslots));
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                rid[it + j] = kArrayEmpty;
-                uint32_t h = open_slot_wide(c[it + j], nslots);
-                for (uint32_t step = 0; v[j].x != empty && step < nslots; ++step) {
-                    if (v[j].x == (unsigned long long)(int64_t)c[it + j]) {
-                        rid[it + j] = (uint32_t)v[j].y;
-                        break;
-                    }
-                    if (++h == nslots) h = 0;
-                    v[j] = slot(h);
-                }
-            }
-        }
+        for (int it = 0; it < kItems; ++it) rid[it] = kArrayEmpty;
+        t.find(c, ok, [&](int it, unsigned long long y) { rid[it] = (uint32_t)y; });
     }
 };
 
@@ -909,48 +976,31 @@ template <typename T> struct MultiLookup {
     }
 };
 
-/* Open addressing: a slot is one 16-byte load; its keys, which need not fit
- * 32 bits, go to their places straight from the lanes. */
+/* Open addressing; its keys, which need not fit 32 bits, go to their places
+ * straight from the lanes. */
 template <typename T> struct OpenMultiLookup {
-    const MultiSlot *slots;
+    TaggedTable t;
     const uint32_t *rows;
-    uint32_t nslots;
-    unsigned long long lo, width, empty;
+    unsigned long long lo, width;
     using Code = T;
     static constexpr bool kMask = true;
     static constexpr bool kStage = false;
-    CJ_DEV OpenMultiLookup(const OpenMultiTable &t)
-        : slots(t.slots), rows(t.rows), nslots(t.nslots), lo(t.lo), width(t.width), empty(t.empty) {}
+    CJ_DEV OpenMultiLookup(const OpenMultiTable &m)
+        : t{reinterpret_cast<const ulonglong2 *>(m.slots), reinterpret_cast<const unsigned long long *>(m.tags),
+            m.nslots / 8},
+          rows(m.rows), lo(m.lo), width(m.width) {}
     CJ_DEV T code(T key, bool present, bool *in) const {
         *in = present && (unsigned long long)(int64_t)key - lo <= width;
         return key;
     }
     CJ_DEV T key_of(T c) const { return c; }
-    CJ_DEV ulonglong2 slot(uint32_t h) const { return __ldg(reinterpret_cast<const ulonglong2 *>(slots + h)); }
     CJ_DEV void find(const T *c, uint32_t ok, uint32_t *low, uint32_t *cnt) const {
 #pragma unroll
-        for (int it = 0; it < kItems; it += 4) { /* four rows' slots in flight: 16 registers */
-            ulonglong2 v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                v[j].x = empty;
-                if ((ok >> (it + j)) & 1u) v[j] = slot(open_slot_wide((int64_t)c[it + j], nslots));
-            }
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                low[it + j] = cnt[it + j] = 0;
-                uint32_t h = open_slot_wide((int64_t)c[it + j], nslots);
-                for (uint32_t step = 0; v[j].x != empty && step < nslots; ++step) {
-                    if (v[j].x == (unsigned long long)(int64_t)c[it + j]) {
-                        low[it + j] = (uint32_t)v[j].y;
-                        cnt[it + j] = (uint32_t)(v[j].y >> 32);
-                        break;
-                    }
-                    if (++h == nslots) h = 0;
-                    v[j] = slot(h);
-                }
-            }
-        }
+        for (int it = 0; it < kItems; ++it) low[it] = cnt[it] = 0;
+        t.find(c, ok, [&](int it, unsigned long long y) {
+            low[it] = (uint32_t)y;
+            cnt[it] = (uint32_t)(y >> 32);
+        });
     }
 };
 
@@ -1422,7 +1472,7 @@ cudaError_t launch_runs(const Launch &L, int32_t key_type, const uint32_t *rows,
 
 cudaError_t launch_unique_build(const Launch &L, const ColView &key, uint32_t n, const UniqueTable &t) {
     if (n == 0) return cudaSuccess;
-    if (t.open_slots && t.open_slots < 2ull * n) return cudaErrorInvalidValue; /* half empty */
+    if (t.open_slots && (t.open_slots < 2ull * n || t.open_slots % 16)) return cudaErrorInvalidValue; /* half empty */
     if (reinterpret_cast<uintptr_t>(t.slots) % 16) return cudaErrorInvalidValue;
     if (n <= kSmallRows) {
         k_unique_small<<<1, kSmallThreads, 0, L.stream>>>(key, n, t);
@@ -1516,7 +1566,9 @@ cudaError_t launch_probe_multi(const Launch &L, const ProbeKey &k, uint32_t n, c
 }
 
 cudaError_t launch_open_multi_build(const Launch &L, const ColView &key, uint32_t n, const OpenMultiTable &t) {
-    if (!n || t.nslots < 2ull * n || reinterpret_cast<uintptr_t>(t.slots) % 16) return cudaErrorInvalidValue;
+    if (!n || t.nslots < 2ull * n || t.nslots % 8 || reinterpret_cast<uintptr_t>(t.slots) % 16 ||
+        reinterpret_cast<uintptr_t>(t.tags) % 8)
+        return cudaErrorInvalidValue;
     const uint64_t wave = (uint64_t)L.num_sms * 8;
     const uint64_t rows_per_block = kUniqueThreads * kUniqueRows, slots_per_block = kUniqueThreads * kPlaceItems;
     const unsigned g = (unsigned)std::min<uint64_t>((n + rows_per_block - 1) / rows_per_block, wave);
