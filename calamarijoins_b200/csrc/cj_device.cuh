@@ -26,7 +26,8 @@ namespace cj {
  * in their tags for every directory size. */
 __host__ __device__ __forceinline__ uint64_t hash_key(int64_t key) {
     const uint64_t x = (uint64_t)key;
-    const uint32_t m = (uint32_t)x ^ ((uint32_t)(x >> 32) * 0x2545F491u);
+    const uint32_t t = (uint32_t)(x >> 32) * 0x2545F491u;
+    const uint32_t m = (uint32_t)x ^ t ^ (t >> 15);
     const uint32_t hi = m * 0x9E3779B1u;
     const uint32_t lo = (m ^ (m >> 15)) * 0x85EBCA77u;
     return ((uint64_t)hi << 32) | lo;

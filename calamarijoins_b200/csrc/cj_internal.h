@@ -420,6 +420,14 @@ enum MultiWord {
     kMultiCursor = 2,
     kMultiWords = 3
 };
+/* Estimate of the different keys among n build rows, from those whose hash ends
+ * in `shift` zero bits (about kSampleRows rows): each sets a bit of `bits`
+ * (kSampleBits, zero before, as *found, the number of bits set). */
+constexpr uint32_t kSampleBits = 1u << 20, kSampleRows = 1u << 17;
+cudaError_t launch_key_sample(const Launch &L, const ColView &key, uint32_t n, uint32_t *bits, unsigned long long *found,
+                              uint32_t *shift);
+uint64_t sampled_keys(unsigned long long found, uint32_t shift);
+
 cudaError_t launch_open_multi_build(const Launch &L, const ColView &key, uint32_t n, const OpenMultiTable &t);
 cudaError_t launch_probe_open_multi(const Launch &L, const ProbeKey &k, uint32_t n, const OpenMultiTable &t,
                                     const UniqueOut &out);

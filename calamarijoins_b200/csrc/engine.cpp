@@ -30,14 +30,26 @@ namespace {
 
 constexpr uint64_t kMultiSpan = 4; /* values of the range per build row */
 
-/* Probe rows per build row from which repeated keys that are not dense get
- * their open-addressing table. Its probe is the cheaper one per row, its build
- * dearer than the hash table's and followed by a synchronisation: 3M x 6M
- * INT64 rows 506 us and 470 on the hash table (sums of the kernels), 3M x 30M
- * 1953 and 2280 (the whole join);
- * a five-join star whose last build side is an intermediate of 86K rows
- * against 105K probe rows 828 us and 766. */
+/* Probe rows per build row from which repeated keys that are not dense may get
+ * their open-addressing table, whose build is dearer than the hash table's and
+ * followed by a synchronisation: 3M x 6M INT64 rows 506 us and 470 on the hash
+ * table (sums of the kernels); a five-join star whose last build side is an
+ * intermediate of 86K rows against 105K probe rows 828 us and 766. */
 constexpr uint64_t kOpenMultiProbe = 4;
+
+/* Build rows per key from which they do get it. A probe row without a match
+ * costs the hash table's small kernel less, one with several the other's; with
+ * their number known both make room for them and probe once. Random INT32
+ * keys, 40 % of the probe rows' in the range but no build key, kernels' sums:
+ * 48M x 3M rows, 1.1 a key, 1980 us on the open-addressing table and 1400 on
+ * the hash table, two a key 2692 and 1737; all matching, 30M x 1M rows, two a
+ * key 1513 and 1287, three 1760 and 2441. */
+constexpr uint64_t kOpenMultiMean2 = 5; /* twice that mean: 2.5 */
+/* Probe rows from which the number of keys is estimated before that choice:
+ * 15 to 30 us and a synchronisation. Below, the open-addressing table is taken
+ * and its build counts them (100K x 1M rows, three a key: 192 us, 204 with the
+ * estimate; 300K x 20M rows of 1.1 a key 667 and 546). */
+constexpr uint64_t kSampleFrom = 1ull << 22;
 
 /* A probe of an open-addressing table reads a build column's values beside
  * it while both stay in L2 (126 MB on two dies, each keeping its own copy of
@@ -647,6 +659,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         bool open_multi = false; /* multi: the keys are not dense */
         OpenMultiTable open_table{};
         DevPtr multi_rows, runs;
+        bool words_ready = false; /* multi: the status words are as its probe needs them */
         const bool words_clear = join_words_clear;
         join_words_clear = false; /* every join counts its matches there */
         UniqueTable table{};
@@ -855,13 +868,14 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
          * probe with one of the columns written beside it; 8 bytes per value
          * of the range, at most kMultiSpan values per build row so that it
          * stays near the hash table's 24 bytes per row.
-         * Over any other range, open addressing, 36 bytes per build row
-         * (30M x 3M rows over 2.25M keys, the whole join, hash table and
-         * this: INT32 keys 2094 and 1599 us, INT64 2312 and 1940; 100K x 5K
-         * INT64 345 and 248).
+         * Over any other range, open addressing, 42 bytes per build row
+         * (30M x 3M INT32 rows, eight a key, half of the probe rows with a
+         * match: the whole join 4916 us on the hash table without room for
+         * them, 2674 here; 100K x 5K INT64 345 and 248).
          * The hash table is left for fewer probe rows than kOpenMultiProbe
-         * per build row, for keys that span all of INT64 or pile up in the
-         * table, and for more build rows than fit kOpenMaxRows or the memory. */
+         * per build row, for keys that hardly repeat (kOpenMultiMean2), that
+         * span all of INT64 or pile up in the table, and for more build rows
+         * than fit kOpenMaxRows or the memory. */
         auto replace_unique = [&]() {
             unique = false;
             slots.reset();
@@ -895,6 +909,8 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 multi_table.entries = slots->as<unsigned long long>();
                 multi_table.rows = multi_rows->as<uint32_t>();
                 widen(tp[kTableSpan]);
+                clear_join_words();
+                words_ready = true;
                 KScope k(*this, "multi_build");
                 ck(launch_multi_build(L, bv, (uint32_t)B.rows, multi_table), "multi_build");
                 return;
@@ -903,9 +919,24 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             multi_rows.reset();
             DevPtr slot_of;
             const uint32_t open_n = (uint32_t)std::max<uint64_t>((2 * std::min(B.rows, kOpenMaxRows) + 7) & ~7ull, 1024);
-            if (tp[kTableRefused] != kTableWhole && B.rows <= kOpenMaxRows && P.rows / kOpenMultiProbe >= B.rows &&
-                ample(B.rows * (2 * (sizeof(MultiSlot) + 1) + 8)) && (slots = spare(open_n * (sizeof(MultiSlot) + 1))) &&
-                (multi_rows = spare(B.rows * 4)) && (slot_of = spare(B.rows * 4))) {
+            const bool many_probes = P.rows / kOpenMultiProbe >= B.rows;
+            uint64_t keys = 0; /* different ones, about; 0: not known */
+            if (DevPtr bits; many_probes && P.rows >= kSampleFrom && (bits = spare(kSampleBits / 8))) {
+                uint32_t shift;
+                clear_join_words();
+                ck(cudaMemsetAsync(bits->ptr, 0, kSampleBits / 8, ctx.stream), "memset");
+                {
+                    KScope k(*this, "key_sample");
+                    ck(launch_key_sample(L, bv, (uint32_t)B.rows, bits->as<uint32_t>(), ctx.d_status->table, &shift),
+                       "key_sample");
+                }
+                sync();
+                keys = std::min<uint64_t>(sampled_keys(ctx.h_status->table[0], shift), tp[kTableCount]);
+            }
+            if (many_probes && (!keys || 2 * tp[kTableCount] >= kOpenMultiMean2 * keys) && tp[kTableRefused] != kTableWhole &&
+                B.rows <= kOpenMaxRows && ample(B.rows * (2 * (sizeof(MultiSlot) + 1) + 8)) &&
+                (slots = spare(open_n * (sizeof(MultiSlot) + 1))) && (multi_rows = spare(B.rows * 4)) &&
+                (slot_of = spare(B.rows * 4))) {
                 open_table.nslots = open_n;
                 open_table.lo = tp[kTableLo];
                 open_table.width = tp[kTableSpan] - 1;
@@ -920,10 +951,15 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                     KScope k(*this, "open_multi_build");
                     ck(launch_open_multi_build(L, bv, (uint32_t)B.rows, open_table), "open_multi_build");
                 }
-                sync(); /* the number of keys, before a probe that might run twice without it */
-                if (!ctx.h_status->table[kMultiGaveUp]) {
-                    multi = open_multi = true;
-                    widen(ctx.h_status->table[kMultiKeys]);
+                multi = open_multi = true;
+                words_ready = true;
+                if (!keys) { /* the number of keys, before a probe that might run twice without it */
+                    sync();
+                    keys = ctx.h_status->table[kMultiKeys];
+                    if (ctx.h_status->table[kMultiGaveUp]) multi = open_multi = false;
+                }
+                if (multi) {
+                    widen(keys);
                     return;
                 }
             }
@@ -931,6 +967,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             multi_rows.reset();
             slot_of.reset();
             clear_join_words(); /* the match counter, and words no longer read */
+            if (keys) widen(keys);
             build_hash();
         };
         auto count_join = [&]() {
@@ -978,10 +1015,22 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         }
         for (;; probed = false) {
             if (!probed) {
-                if (multi) clear_join_words(); /* the match counter */
+                if (multi && !words_ready) clear_join_words(); /* the match counter, the number of runs */
+                words_ready = false;
                 launch_probe();
             }
             sync();
+            if (open_multi && ctx.h_status->table[kMultiGaveUp]) { /* walks given up: the table is unusable */
+                multi = open_multi = false;
+                cap = P.rows;
+                widened = false;
+                slots.reset();
+                multi_rows.reset();
+                drop_pages();
+                clear_join_words();
+                build_hash();
+                continue;
+            }
             if (unique && !table_kind(ctx.h_status->table, table.open_slots)) {
                 replace_unique();
                 continue;

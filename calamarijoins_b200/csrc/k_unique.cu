@@ -37,6 +37,7 @@
  */
 #include <algorithm>
 #include <atomic>
+#include <cmath>
 
 #include "cj_device.cuh"
 
@@ -490,6 +491,48 @@ __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_scatter(uint32_t 
         for (int q = 0; q < kUniqueRows; ++q)
             if (c[q] > 1) t.rows[at[q]] = (uint32_t)(i0 + q * stride);
     }
+}
+
+/* Linear counting (Whang, Vander-Zanden and Taylor) of a part of the keys: b of
+ * m bits set by hashing say -m ln(1 - b / m) keys, within a percent here. The
+ * keys are sampled by their hash, so that all rows of a key are in or out.
+ * Bound by reading the keys and their round trips: 3M rows 29 us. The mixing is
+ * MurmurHash3's 32-bit finaliser. */
+__global__ void __launch_bounds__(kUniqueThreads)
+    k_key_sample(ColView key_arg, uint32_t n, uint32_t shift, uint32_t *bits, unsigned long long *found) {
+    const ColView key = resolve_view(key_arg);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    uint32_t mine = 0;
+    for (uint64_t i0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i0 < n; i0 += stride * kUniqueRows) {
+        int64_t k[kUniqueRows];
+        bool v[kUniqueRows];
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) {
+            const uint64_t i = i0 + q * stride;
+            v[q] = i < n && load_key(key, (uint32_t)i, &k[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < kUniqueRows; ++q) {
+            if (!v[q]) continue;
+            uint32_t h = (uint32_t)(hash_key(k[q]) >> 32);
+            h ^= h >> 16;
+            h *= 0x85EBCA6Bu;
+            h ^= h >> 13;
+            h *= 0xC2B2AE35u;
+            h ^= h >> 16;
+            if (h & ((1u << shift) - 1u)) continue;
+            const uint32_t at = h >> 12, bit = 1u << (at & 31u);
+            static_assert(kSampleBits == 1u << 20, "the hash's 20 top bits");
+            if (!(__ldcg(bits + at / 32) & bit)) mine += (atomicOr(bits + at / 32, bit) & bit) == 0;
+        }
+    }
+    __shared__ uint32_t s_mine;
+    if (threadIdx.x == 0) s_mine = 0;
+    __syncthreads();
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane_id() == 0 && mine) atomicAdd(&s_mine, mine);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_mine) atomicAdd(found, (unsigned long long)s_mine);
 }
 
 /* ---------------- probe ---------------- */
@@ -1563,6 +1606,22 @@ cudaError_t launch_probe_multi(const Launch &L, const ProbeKey &k, uint32_t n, c
     count_launches(1);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? launch_runs(L, k.col.type, t.rows, out) : e;
+}
+
+cudaError_t launch_key_sample(const Launch &L, const ColView &key, uint32_t n, uint32_t *bits, unsigned long long *found,
+                              uint32_t *shift) {
+    *shift = 0;
+    while ((n >> *shift) > kSampleRows) ++*shift; /* at most 15: clear of the bit's place */
+    const uint64_t rows_per_block = kUniqueThreads * kUniqueRows;
+    const unsigned g = (unsigned)std::min<uint64_t>((n + rows_per_block - 1) / rows_per_block, (uint64_t)L.num_sms * 8);
+    k_key_sample<<<g, kUniqueThreads, 0, L.stream>>>(key, n, *shift, bits, found);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+uint64_t sampled_keys(unsigned long long found, uint32_t shift) {
+    const double m = kSampleBits, b = std::min<double>((double)found, m - 1);
+    return (uint64_t)std::max(1.0, -m * std::log1p(-b / m) * (double)(1ull << shift));
 }
 
 cudaError_t launch_open_multi_build(const Launch &L, const ColView &key, uint32_t n, const OpenMultiTable &t) {
