@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(kFilterThreads) k_compare(CmpArgs a) {
 }
 
 /* A VARCHAR column compared with the literal, for the rows whose bit of `mask`
- * is set (null: all); the bits of other rows are 0. A block takes 32 x `take`
+ * is set (null: all); the bits of other rows are 0. A block takes 32 kTake
  * rows at a time (2,048, or fewer in a table too small to fill the chip with
  * such blocks: text_words), packs those that are non-NULL and in the mask, and
  * its threads compare them side by side: a comparison costs tens of
@@ -323,22 +323,22 @@ __global__ void __launch_bounds__(kFilterThreads) k_compare(CmpArgs a) {
  * still in question. 10M strings of 20 characters against '%qz%' beside two conditions
  * that leave a quarter of the rows: the filter 1006 us, 715 so. */
 constexpr uint32_t kTextWords = 64;
-__global__ void __launch_bounds__(kFilterThreads)
-    k_compare_text(CmpArgs a, const uint32_t *__restrict__ mask, uint32_t take) {
+template <uint32_t kTake>
+__global__ void __launch_bounds__(kFilterThreads) k_compare_text(CmpArgs a, const uint32_t *__restrict__ mask) {
     static_assert(kFilterThreads == kTextWords * 4, "a thread lists a byte of the words");
     __shared__ uint32_t s_live[kTextWords], s_pre[kTextWords], s_out[kTextWords];
     __shared__ uint16_t s_row[kTextWords * 32];
     __shared__ uint32_t s_total;
     const ColView c = resolve_view(a.col);
     const uint64_t words = (a.rows + 31) / 32;
-    for (uint64_t w0 = (uint64_t)blockIdx.x * take; w0 < words; w0 += (uint64_t)gridDim.x * take) {
+    for (uint64_t w0 = (uint64_t)blockIdx.x * kTake; w0 < words; w0 += (uint64_t)gridDim.x * kTake) {
         if (threadIdx.x < 32) {
             uint32_t v[2];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const uint64_t w = w0 + 2 * threadIdx.x + j;
                 v[j] = 0;
-                if (w >= words || w - w0 >= take) continue;
+                if (w >= words || (kTake < kTextWords && 2 * threadIdx.x + j >= kTake)) continue;
                 v[j] = __ldg(c.valid + w); /* no bits past the last row */
                 if (mask) v[j] &= __ldg(mask + w);
             }
@@ -376,7 +376,7 @@ __global__ void __launch_bounds__(kFilterThreads)
             if (bit) atomicOr(&s_out[q >> 5], 1u << (q & 31u));
         }
         __syncthreads();
-        if (threadIdx.x < take && w0 + threadIdx.x < words) a.out[w0 + threadIdx.x] = s_out[threadIdx.x];
+        if (threadIdx.x < kTake && w0 + threadIdx.x < words) a.out[w0 + threadIdx.x] = s_out[threadIdx.x];
         __syncthreads();
     }
 }
@@ -424,6 +424,7 @@ unsigned grid_for(const Context &ctx, uint64_t n, unsigned threads) {
  * '%_a_%' (where LIKE cannot skip): the filter 344 us with 64 words, 187
  * with 8; 1,000 strings 209 and 131. */
 uint32_t text_words(const Context &ctx, uint64_t words) {
+    static_assert(kTextWords == 64 && kFilterThreads == 256, "the kernels of 8 to 64 words");
     uint32_t take = kTextWords;
     while (take > kFilterThreads / 32 && words / take < (uint64_t)ctx.num_sms * 8) take /= 2;
     return take;
@@ -648,7 +649,11 @@ class Filter {
             }
             const uint32_t take = text_words(ctx, words);
             const unsigned grid = grid_for(ctx, in.num_rows, text ? take * 32 : kFilterThreads);
-            if (text) k_compare_text<<<grid, kFilterThreads, 0, ctx.stream>>>(a, mask, take);
+            const auto compare_text = take == 64   ? k_compare_text<64>
+                                      : take == 32 ? k_compare_text<32>
+                                      : take == 16 ? k_compare_text<16>
+                                                   : k_compare_text<8>;
+            if (text) compare_text<<<grid, kFilterThreads, 0, ctx.stream>>>(a, mask);
             else k_compare<<<grid, kFilterThreads, 0, ctx.stream>>>(a);
             count_launches(1);
             check_cuda(cudaGetLastError(), "compare");
