@@ -73,6 +73,10 @@ constexpr uint64_t kKeepSpare = 32ull << 20;
  * for nothing when a join below the root is empty (256 MB: about 100 us). */
 constexpr uint64_t kDecodeAhead = 256ull << 20;
 
+/* Probe rows from which a probe of repeated keys gets room for an eighth more
+ * than the mean number of matches. */
+constexpr uint64_t kSpareEighth = 1ull << 15;
+
 /* Room for matches from which the long runs among them are left to a kernel of
  * their own. Its launch takes 5 us also where there are none; 240K matches in
  * runs of 400 take 80 us less with it (5K x 20K rows, the whole join 318 and
@@ -887,14 +891,15 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
              * an eighth more: where every probe row matches, a random half of
              * all results lie just above the mean, and a result above the
              * room runs the probe again (3M x 30M rows, four rows for three
-             * keys: 2104 us, 1296 with the eighth). A server's worker keeps
+             * keys: 2104 us, 1296 with the eighth; below kSpareEighth the
+             * second run is little more than its launch). A server's worker keeps
              * to the probe rows: admission counts on no more, and what one
              * plan takes on a guess another might need. */
             auto widen = [&](uint64_t keys) {
                 if (!ctx.owns_pool) return;
                 const uint64_t mean =
                     std::min<uint64_t>(P.rows * (uint64_t)tp[kTableCount] / std::max<uint64_t>(keys, 1), 4 * P.rows);
-                const uint64_t more = std::min<uint64_t>(mean + mean / 8, 0xFFFFFFFFull);
+                const uint64_t more = std::min<uint64_t>(mean + (P.rows >= kSpareEighth ? mean / 8 : 0), 0xFFFFFFFFull);
                 /* a match: two row ids and a key at most, here */
                 if (mean > cap && more > cap && room_for(more * 17)) {
                     cap = more;
