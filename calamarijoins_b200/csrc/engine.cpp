@@ -30,26 +30,27 @@ namespace {
 
 constexpr uint64_t kMultiSpan = 4; /* values of the range per build row */
 
-/* Probe rows per build row from which repeated keys that are not dense may get
- * their open-addressing table, whose build is dearer than the hash table's and
- * followed by a synchronisation: 3M x 6M INT64 rows 506 us and 470 on the hash
- * table (sums of the kernels); a five-join star whose last build side is an
- * intermediate of 86K rows against 105K probe rows 828 us and 766. */
-constexpr uint64_t kOpenMultiProbe = 4;
-
-/* Build rows per key from which they do get it. A probe row without a match
+/* Repeated keys that are not dense get their open-addressing table from 2.5
+ * build rows per key on, else the hash table. A probe row without a match
  * costs the hash table's small kernel less, one with several the other's; with
  * their number known both make room for them and probe once. Random INT32
  * keys, 40 % of the probe rows' in the range but no build key, kernels' sums:
  * 48M x 3M rows, 1.1 a key, 1980 us on the open-addressing table and 1400 on
  * the hash table, two a key 2692 and 1737; all matching, 30M x 1M rows, two a
- * key 1513 and 1287, three 1760 and 2441. */
-constexpr uint64_t kOpenMultiMean2 = 5; /* twice that mean: 2.5 */
-/* Probe rows from which the number of keys is estimated before that choice:
- * 15 to 30 us and a synchronisation. Below, the open-addressing table is taken
- * and its build counts them (100K x 1M rows, three a key: 192 us, 204 with the
- * estimate; 300K x 20M rows of 1.1 a key 667 and 546). */
-constexpr uint64_t kSampleFrom = 1ull << 22;
+ * key 1513 and 1287, three 1760 and 2441; 2M x 2M rows, four a key 442 and
+ * 471, 40 a key 1621 and 5103. */
+constexpr uint64_t kOpenMultiMean2 = 5; /* twice that mean */
+/* Probe rows from which the number of keys is estimated before that choice: 15
+ * to 30 us and a synchronisation. With fewer, joins of kOpenMultiProbe probe
+ * rows or more per build row take the open-addressing table, whose build
+ * counts the keys (100K x 1M rows, three a key: 192 us, 204 with the estimate;
+ * 300K x 20M rows of 1.1 a key 667 and 546), the others, for whom its dearer
+ * build does not pay, the hash table (2M x 2M INT64 rows of 1.1 a key, all
+ * matching: 392 us, 367 with the estimate and without a second run, half of
+ * them 318 and 349; a five-join star whose last build side is an intermediate
+ * of 86K rows against 105K probe rows 828 on the open-addressing table, 766). */
+constexpr uint64_t kSampleFrom = 1ull << 22, kSampleFromFew = 1ull << 20;
+constexpr uint64_t kOpenMultiProbe = 4;
 
 /* A probe of an open-addressing table reads a build column's values beside
  * it while both stay in L2 (126 MB on two dies, each keeping its own copy of
@@ -876,10 +877,10 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
          * (30M x 3M INT32 rows, eight a key, half of the probe rows with a
          * match: the whole join 4916 us on the hash table without room for
          * them, 2674 here; 100K x 5K INT64 345 and 248).
-         * The hash table is left for fewer probe rows than kOpenMultiProbe
-         * per build row, for keys that hardly repeat (kOpenMultiMean2), that
-         * span all of INT64 or pile up in the table, and for more build rows
-         * than fit kOpenMaxRows or the memory. */
+         * The hash table is left for keys that hardly repeat
+         * (kOpenMultiMean2), few probe rows (kSampleFrom), keys that span all
+         * of INT64 or pile up in the table, and for more build rows than fit
+         * kOpenMaxRows or the memory. */
         auto replace_unique = [&]() {
             unique = false;
             slots.reset();
@@ -926,7 +927,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
             const uint32_t open_n = (uint32_t)std::max<uint64_t>((2 * std::min(B.rows, kOpenMaxRows) + 7) & ~7ull, 1024);
             const bool many_probes = P.rows / kOpenMultiProbe >= B.rows;
             uint64_t keys = 0; /* different ones, about; 0: not known */
-            if (DevPtr bits; many_probes && P.rows >= kSampleFrom && (bits = spare(kSampleBits / 8))) {
+            if (DevPtr bits; P.rows >= (many_probes ? kSampleFrom : kSampleFromFew) && (bits = spare(kSampleBits / 8))) {
                 uint32_t shift;
                 clear_join_words();
                 ck(cudaMemsetAsync(bits->ptr, 0, kSampleBits / 8, ctx.stream), "memset");
@@ -938,7 +939,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 sync();
                 keys = std::min<uint64_t>(sampled_keys(ctx.h_status->table[0], shift), tp[kTableCount]);
             }
-            if (many_probes && (!keys || 2 * tp[kTableCount] >= kOpenMultiMean2 * keys) && tp[kTableRefused] != kTableWhole &&
+            if ((keys ? 2 * tp[kTableCount] >= kOpenMultiMean2 * keys : many_probes) && tp[kTableRefused] != kTableWhole &&
                 B.rows <= kOpenMaxRows && ample(B.rows * (2 * (sizeof(MultiSlot) + 1) + 8)) &&
                 (slots = spare(open_n * (sizeof(MultiSlot) + 1))) && (multi_rows = spare(B.rows * 4)) &&
                 (slot_of = spare(B.rows * 4))) {

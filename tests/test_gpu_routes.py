@@ -50,8 +50,8 @@ CASES = {
 }
 
 
-# from 4M probe rows on the number of keys decides: build keys, their type, the
-# kernels that probe, reruns
+# from 4M probe rows on the number of keys decides, from 1M where there are
+# fewer than four per build row: build keys, their type, the kernels that probe
 MANY = 1 << 22
 WIDE = np.arange(60_000)
 PILED_WIDE = np.arange(1, 20_001, dtype=np.int64)
@@ -65,6 +65,8 @@ SAMPLED = {
     "sampled64": (np.arange(700_000) // 3 * SLOT64, L, {"probe_unique", "probe_open_multi"}),
     "sampled_two": (np.arange(700_000) // 2 * 3000, I, {"probe_unique", "probe_hash"}),
     "piled_up_four": (np.repeat(PILED_WIDE, 4), L, {"probe_unique", "probe_open_multi", "probe_hash"}),
+    "few_two": (np.arange(700_000) // 2 * 3000, I, {"probe_unique", "probe_hash"}),
+    "few_three64": (np.arange(700_000) // 3 * SLOT64, L, {"probe_unique", "probe_open_multi"}),
     "whole_three": (np.repeat(WHOLE, 3), L, {"probe_unique", "probe_hash"}),
 }
 
@@ -75,9 +77,10 @@ def test_route_by_number_of_keys(gpu_ctx, case):
     bkeys, kt, probes = SAMPLED[case]
     rng = np.random.default_rng(1)
     bkeys = rng.permutation(bkeys)
-    pkeys = bkeys[rng.integers(0, len(bkeys), MANY)]
+    n = MANY // 4 if "few" in case else MANY
+    pkeys = bkeys[rng.integers(0, len(bkeys), n)]
     if "piled" in case or "sampled" in case:
-        pkeys[rng.random(MANY) < 0.9] = bkeys.min() - 1
+        pkeys[rng.random(n) < 0.9] = bkeys.min() - 1
     plan = _plan(bkeys, pkeys, kt, kt, bpay=[(I, np.arange(len(bkeys)), None)])
     want = run_oracle(plan)
     rp = Plan()
