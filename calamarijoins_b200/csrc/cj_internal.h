@@ -418,7 +418,8 @@ enum MultiWord {
     kMultiKeys = 0,   /* different keys                                      */
     kMultiGaveUp = 1, /* a key's walk reached kMaxWalk: the table is unusable */
     kMultiCursor = 2,
-    kMultiWords = 3
+    kMultiMost = 3,   /* most build rows of a key                            */
+    kMultiWords = 4
 };
 /* Estimate of the different keys among n build rows, from those whose hash ends
  * in `shift` zero bits (about kSampleRows rows): each sets a bit of `bits`

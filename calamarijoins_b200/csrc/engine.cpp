@@ -79,10 +79,12 @@ constexpr uint64_t kDecodeAhead = 256ull << 20;
 constexpr uint64_t kSpareEighth = 1ull << 15;
 
 /* Room for matches from which the long runs among them are left to a kernel of
- * their own. Its launch takes 5 us also where there are none; 240K matches in
- * runs of 400 take 80 us less with it (5K x 20K rows, the whole join 318 and
- * 237 us). */
-constexpr uint64_t kRunsFrom = 1ull << 16;
+ * their own, where the build found a key with kRunFrom rows or more, and where
+ * the host does not know. 240K matches in runs of 400 take 80 us less with it
+ * (5K x 20K rows, the whole join 318 and 237 us); without any run its launch
+ * and its list cost 5 to 10 us (1,000 x 300K rows over 750 dense keys 199 us,
+ * 188 without). */
+constexpr uint64_t kRunsFrom = 1ull << 16, kRunsFromBlind = 1ull << 20;
 
 enum Phase { PH_UPLOAD, PH_DECODE, PH_BUILD, PH_PROBE, PH_NL, PH_INTER, PH_MAT, PH_DOWNLOAD, PH_COUNT };
 /* NVTX range names of the phases (host-side ranges around the enqueueing of
@@ -664,6 +666,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
         bool open_multi = false; /* multi: the keys are not dense */
         OpenMultiTable open_table{};
         DevPtr multi_rows, runs;
+        uint64_t most_rows = ~0ull; /* multi: of a key, where it is known */
         bool words_ready = false; /* multi: the status words are as its probe needs them */
         const bool words_clear = join_words_clear;
         join_words_clear = false; /* every join counts its matches there */
@@ -788,7 +791,8 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                  * ids are collected for the others only. */
                 UniqueOut uo{};
                 uo.match = mo;
-                if (multi && mo.capacity >= kRunsFrom && (runs = spare(mo.capacity / kRunFrom * sizeof(MatchRun)))) {
+                if (multi && most_rows >= kRunFrom && mo.capacity >= (most_rows == ~0ull ? kRunsFromBlind : kRunsFrom) &&
+                    (runs = spare(mo.capacity / kRunFrom * sizeof(MatchRun)))) {
                     uo.runs.runs = runs->as<MatchRun>();
                     uo.runs.count = ctx.d_status->table + kTableDone; /* zero: clear_join_words */
                     uo.runs.capacity = mo.capacity / kRunFrom;
@@ -962,6 +966,7 @@ Relation Executor::exec_join(uint64_t node_idx, int depth, bool is_root, cj_resu
                 if (!keys) { /* the number of keys, before a probe that might run twice without it */
                     sync();
                     keys = ctx.h_status->table[kMultiKeys];
+                    most_rows = ctx.h_status->table[kMultiMost];
                     if (ctx.h_status->table[kMultiGaveUp]) multi = open_multi = false;
                 }
                 if (multi) {

@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_claim(ColView key
 __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_place(OpenMultiTable t) {
     __shared__ uint32_t wbuf[kUniqueThreads / 32 + 1];
     __shared__ unsigned long long s_base;
-    uint32_t keys = 0;
+    uint32_t keys = 0, most = 0;
     for (uint64_t v0 = (uint64_t)blockIdx.x * kUniqueThreads * kPlaceItems; v0 < t.nslots;
          v0 += (uint64_t)gridDim.x * kUniqueThreads * kPlaceItems) {
         uint32_t c[kPlaceItems], sum = 0, total;
@@ -457,6 +457,7 @@ __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_place(OpenMultiTa
             const uint64_t v = v0 + q * kUniqueThreads + threadIdx.x;
             c[q] = v < t.nslots ? t.slots[v].count : 0u;
             keys += c[q] > 0;
+            most = max(most, c[q]);
             if (c[q] > 1) sum += c[q];
         }
         const uint32_t pre = block_exclusive_scan<uint32_t>(sum, wbuf, &total);
@@ -472,7 +473,11 @@ __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_place(OpenMultiTa
         __syncthreads();
     }
     keys = __reduce_add_sync(0xffffffffu, keys);
-    if (lane_id() == 0 && keys) atomicAdd(t.found + kMultiKeys, (unsigned long long)keys);
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane_id() == 0 && keys) {
+        atomicAdd(t.found + kMultiKeys, (unsigned long long)keys);
+        atomicMax(t.found + kMultiMost, (unsigned long long)most);
+    }
 }
 __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_scatter(uint32_t n, OpenMultiTable t) {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;

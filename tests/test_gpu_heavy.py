@@ -108,3 +108,17 @@ def test_runs_below_the_root(gpu_ctx, gap):
     j = plan.new_join_node(True, s[1], s[2], 0, 0, [(1, I), (2, F), (4, I)])
     plan.root = plan.new_join_node(True, s[0], j, 0, 0, [(0, I), (1, L), (2, I), (3, F), (4, I)])
     assert_same(_resident_run(plan, gpu_ctx), run_oracle(plan), "probe side")
+
+
+@pytest.mark.parametrize("pt", [I, L])
+def test_runs_of_dense_keys(gpu_ctx, pt):
+    """The host does not know the longest run of dense keys: from 1M rows of
+    room on."""
+    rng = np.random.default_rng(8)
+    keys, bkeys = _build(rng, [64, 63, 961, 3, 1, 1920], 1)
+    n = 1 << 20
+    pkeys = np.full(n, 10 ** 8)
+    hit = rng.permutation(n)[:200]
+    pkeys[hit] = keys[rng.integers(0, len(keys), 200)]
+    plan = _plan(bkeys, pkeys, I, pt, bpay=[(L, np.arange(len(bkeys)), None)], ppay=[(I, np.arange(n), None)])
+    assert_same(_resident_run(plan, gpu_ctx, _lib.CJ_EXEC_RESULT_ON_DEVICE), run_oracle(plan))
