@@ -33,8 +33,8 @@ Other workloads (not the default line; --workload):
       measurements as the default line.
   c2s C2 with the build keys spread 500x (unique multiples of 500): the
       open-addressing table instead of the direct-mapped one.
-  c2h C2 with a non-unique build side (4M rows over 3M distinct keys): the
-      unchained hash table; roofline of the hash path's kernels.
+  c2h C2 with a non-unique build side (4M rows over 3M distinct dense keys):
+      the table of repeated dense keys.
   c3  6-way left-deep join: a 36M-row fact table with 5 foreign keys into
       dimensions of 2.5K-4.2M rows (pre-filtered to 10-40 %), VARCHAR
       outputs (lengths log-normal, mean 20 B, 0.01 % long strings);
@@ -87,8 +87,8 @@ WORKLOADS = {
             "unit": UNIT,
             "desc": ("C2 with a non-unique build side: 4,000,000 build rows over 3,000,000 distinct INT32 keys (a "
                      "third twice) + INT64 payload; probe 64,000,000 rows, FK Zipf(0.8) over the distinct keys, "
-                     "30% outside, 2% NULL, + FP64 payload; the unchained hash table (radix-partitioned build, "
-                     "Bloom-tag probe); about 58.5M output rows"),
+                     "30% outside, 2% NULL, + FP64 payload; the table of repeated dense keys (a count and the rows "
+                     "of each key); about 58.5M output rows"),
             "units": "probe rows"},
     "c3": {"metric": "fact rows/s, 6-way join of a 36M-row fact table (plain execute)", "unit": UNIT,
            "desc": ("C3: fact 36,000,000 rows x 5 INT32 FKs (Zipf 0.5-1.2) into dimensions of 2,500 / 130,000 / "

@@ -32,7 +32,7 @@
  * Bound: requests from L1 to L2, about one per clock and SM whatever their
  * size (every random slot or value is one), then the 128-byte lines of L1
  * that the requests in flight hold. 64M x 4M rows, 43.9M matches, two
- * 8-byte result columns, direct-mapped: 580 us, where decode, probe and
+ * 8-byte result columns, direct-mapped: 575 us, where decode, probe and
  * page writers took 945 us (152 + 390 + 403).
  */
 #include <algorithm>
@@ -542,8 +542,8 @@ __global__ void __launch_bounds__(kUniqueThreads)
 
 /* ---------------- probe ---------------- */
 /* 256 threads, 48 registers and 10 KB of shared memory: five CTAs per SM.
- * Measured at 64M x 4M rows (probe alone): five 605 us, four with 64
- * registers 619, six with 40 (spills) 620. */
+ * Measured at 64M x 4M rows (probe alone, 575 us since): five 605 us, four
+ * with 64 registers 619, six with 40 (spills) 620. */
 constexpr int kProbeBlocks = 5;
 constexpr int kWideBlocks = 4; /* 64 registers: the codes are 64-bit keys */
 /* 80 registers; four with 64, more of them spilled: 1347 us where three take
@@ -1485,7 +1485,7 @@ uint32_t shares_of(uint64_t tiles, uint64_t wave) {
 }
 
 /* Random loads in flight are held in L1: as little of it as possible goes to
- * shared memory (default split 628 us, this one 605). Once per kernel and
+ * shared memory (default split 628 us, this one 605, before later gains). Once per kernel and
  * device. */
 template <class K> void prefer_l1(K kernel) {
     constexpr int kDevices = 64;
