@@ -499,7 +499,7 @@ __global__ void __launch_bounds__(kUniqueThreads) k_open_multi_scatter(uint32_t 
 }
 
 /* Linear counting (Whang, Vander-Zanden and Taylor) of a part of the keys: b of
- * m bits set by hashing say -m ln(1 - b / m) keys, within a percent here. The
+ * m bits set by hashing say -m ln(1 - b / m) keys, within about a percent here. The
  * keys are sampled by their hash, so that all rows of a key are in or out.
  * Bound by reading the keys and their round trips: 3M rows 29 us. The mixing is
  * MurmurHash3's 32-bit finaliser. */
@@ -642,14 +642,15 @@ template <typename T> struct OpenLookup {
     }
 };
 
-/* Lookups in a table of tagged 16-byte slots: the tags of all of a lane's rows
- * in flight together, then the slots that they point to, four rows' at a time
- * (16 registers). What is left, a tag that another key shares (one in 128 per
- * key of the group) or a full group, goes group by group. Bound by the random
- * accesses, one for a row without a match and two for one with. Walking the
- * slots to an empty one instead, unique INT64 keys: 30M probe rows over 3M
- * keys, 97 % of them in the range but no key, 803 us, 416 with tags; 10 % of
- * them outside it 619 and 605; 5M rows over 300K keys 125 and 118. */
+/* Lookups in a table of tagged 16-byte slots: the tags of four of a lane's rows
+ * in flight together, then the slots that they point to (all eight rows' tags
+ * at once spill: 661 us where this takes 605, 30M INT64 rows over 3M keys).
+ * What is left, a tag that another key shares (one in 128 per key of the group)
+ * or a full group, goes group by group. Bound by the random accesses, one for a
+ * row without a match and two for one with. Walking the slots to an empty one
+ * instead, unique INT64 keys: 30M probe rows over 3M keys, 97 % of them in the
+ * range but no key, 803 us, 416 with tags; 10 % of them outside it 619 and 605;
+ * 5M rows over 300K keys 125 and 118. */
 struct TaggedTable {
     const ulonglong2 *slots; /* key, payload */
     const unsigned long long *tags;
